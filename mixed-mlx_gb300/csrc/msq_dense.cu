@@ -32,85 +32,168 @@ __device__ __forceinline__ float rootOf(float lambda) {
   return sqrtf(fmaxf(lambda, 0.0f));
 }
 
-// C tile (64 x 64) of C = A^T B (both K-contiguous), FP32 FMA, with an
-// epilogue.  Shared-memory tiles are stored [k][m] so the 4x4 register
-// micro-tile reads broadcast-free rows.
-template <int kEpilogue>
-__global__ void __launch_bounds__(kThreads)
-gemmTNKernel(GemmArgs args) {
-  __shared__ __align__(16) float As[2][kBK][kTile + 4];
-  __shared__ __align__(16) float Bs[2][kBK][kTile + 4];
-  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
+// ---- FP32 GEMM ---------------------------------------------------------------
+// C = op(A) op(B) on the CUDA cores, each element the FMA chain over k in
+// order.  A kT x kT tile of C per CTA: K steps of kBK staged by 4-byte
+// cp.async (any alignment and either operand layout lands as [k][m]; out of
+// range elements are zero-filled) in a ring of kStages, so the loads of the
+// next steps run under the FMAs of this one with one barrier per step.  A
+// thread owns kM x kM outputs (rows kQ apart in groups of 4): per k it reads
+// its rows as packed pairs, broadcasts its columns and issues kM^2 / 2
+// fma.rn.f32x2.  The bound is the FP32 pipe (60% busy at order 2048, a sixth
+// of the rest being the last wave): the four products of a correction of
+// four matrices of order 1000 take 802 us (40 TFLOP/s) against 1437 us with
+// 64 x 64 tiles of 4 x 4 outputs per thread and a load-barrier-compute loop;
+// order 256 alone 46 us against 97.  Tile sizes: gemmClass.
+template <int kT>
+struct GemmShape {
+  static constexpr int kM = kT == 32 ? 4 : 8;              // outputs per thread and dimension
+  static constexpr int kSide = kT / kM;                    // threads per dimension
+  static constexpr int kThr = kSide * kSide;               // 256, 64, 64
+  static constexpr int kK = kT == 32 ? 32 : 16;            // K step
+  static constexpr int kStages = kT == 128 ? 2 : 3;
+  static constexpr int kLd = kT + 4;
+  static constexpr int kQ = kT / (kM / 4);                 // stride between a thread's groups of 4
+  static constexpr int kCtas = kT == 128 ? 2 : 8;          // resident CTAs per SM
+};
+
+__device__ __forceinline__ void copyAsync4(float *smem, const float *gmem, bool valid) {
+  const unsigned dst = static_cast<unsigned>(__cvta_generic_to_shared(smem));
+  const int bytes = valid ? 4 : 0;  // 0: zero-fill, the source is not read
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(dst), "l"(gmem), "r"(bytes)
+               : "memory");
+}
+
+// One operand's K step into its [k][m] stage.  kMajorM: element (m, k) at
+// m + k n (m is the fast thread index), else at k + m n (k fast).
+template <int kT, bool kMajorM>
+__device__ __forceinline__ void gemmStage(float *dst, const float *src, int n, int m0, int k0) {
+  using S = GemmShape<kT>;
+  constexpr int kFast = kMajorM ? kT : S::kK;
+  constexpr int kStep = S::kThr / kFast;                   // slow index per element
+  constexpr int kElems = kT * S::kK / S::kThr;
+  static_assert(S::kThr % kFast == 0, "a thread keeps its fast index");
+  const int fast = threadIdx.x % kFast, slow = threadIdx.x / kFast;
+  const int m = kMajorM ? fast : slow, k = kMajorM ? slow : fast;
+  float *s = dst + k * S::kLd + m;
+  const float *g = src + (kMajorM ? (m0 + m) + static_cast<int64_t>(k0 + k) * n
+                                  : (k0 + k) + static_cast<int64_t>(m0 + m) * n);
+  const int64_t gstep = static_cast<int64_t>(kStep) * n;
+  constexpr int kSmem = kMajorM ? kStep * S::kLd : kStep;
+  const int fast_left = kMajorM ? n - (m0 + m) : n - (k0 + k);   // > 0: in range
+  const int slow_left = kMajorM ? n - (k0 + k) : n - (m0 + m);
+#pragma unroll
+  for (int e = 0; e < kElems; ++e) {
+    const bool valid = fast_left > 0 && slow_left > e * kStep;
+    copyAsync4(s + e * kSmem, valid ? g + e * gstep : src, valid);
+  }
+}
+
+template <int kT>
+__device__ __forceinline__ void gemmStep(const float *as, const float *bs,
+                                         f32x2 (&acc)[GemmShape<kT>::kM / 2][GemmShape<kT>::kM]) {
+  using S = GemmShape<kT>;
+  f32x2 a[S::kM / 2];
+  float b[S::kM];
+#pragma unroll
+  for (int q = 0; q < S::kM / 4; ++q) {
+    const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(as + q * S::kQ);
+    a[2 * q] = v.x;
+    a[2 * q + 1] = v.y;
+    const float4 w = *reinterpret_cast<const float4 *>(bs + q * S::kQ);
+    b[4 * q] = w.x; b[4 * q + 1] = w.y; b[4 * q + 2] = w.z; b[4 * q + 3] = w.w;
+  }
+#pragma unroll
+  for (int c = 0; c < S::kM; ++c) {
+    const f32x2 bb = f2make(b[c], b[c]);
+#pragma unroll
+    for (int p = 0; p < S::kM / 2; ++p) acc[p][c] = f2fma(a[p], bb, acc[p][c]);
+  }
+}
+
+// kMirror: C is symmetric (A and B the same operand): the work list holds
+// the tiles on or above the diagonal and an off-diagonal tile also writes
+// its mirror image (the same products in the same order, so the same bits
+// as a direct tile).
+template <int kT, bool kMajorA, bool kMajorB, int kEpilogue, bool kMirror>
+__global__ void __launch_bounds__(GemmShape<kT>::kThr, GemmShape<kT>::kCtas)
+gemmKernel(GemmArgs args) {
+  using S = GemmShape<kT>;
+  constexpr int kM = S::kM;
+  __shared__ __align__(16) float As[S::kStages][S::kK][S::kLd];
+  __shared__ __align__(16) float Bs[S::kStages][S::kK][S::kLd];
+  const int tx = threadIdx.x % S::kSide, ty = threadIdx.x / S::kSide;
   for (int item = blockIdx.x; item < args.items; item += gridDim.x) {
     const int4 w = args.work[item];  // matrix, tile_i, tile_j, unused
     const int mi = w.x;
     const int n = args.n[mi];
-    const int i0 = w.y * kTile, j0 = w.z * kTile;
+    const int i0 = w.y * kT, j0 = w.z * kT;
     const float *A = args.a + args.a_offset[mi];
     const float *B = args.b + args.b_offset[mi];
-    float acc[4][4] = {};
-    // loader mapping: each thread loads 4 (k, row) elements per operand
-    // Operand layouts: K-major (element (i, k) at k + i*n) loads with k
-    // fastest; M-major (at i + k*n) with i fastest; both coalesced.
-    auto load = [&](int buf, int k0) {
+    f32x2 acc[kM / 2][kM];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int idx = threadIdx.x + e * kThreads;  // 0..1023
-        {
-          const int kk = args.a_mmajor ? idx / kTile : idx % kBK;
-          const int r = args.a_mmajor ? idx % kTile : idx / kBK;
-          const int k = k0 + kk, gi = i0 + r;
-          const int64_t at = args.a_mmajor ? gi + static_cast<int64_t>(k) * n
-                                           : k + static_cast<int64_t>(gi) * n;
-          As[buf][kk][r] = (k < n && gi < n) ? A[at] : 0.0f;
-        }
-        {
-          const int kk = args.b_nmajor ? idx / kTile : idx % kBK;
-          const int r = args.b_nmajor ? idx % kTile : idx / kBK;
-          const int k = k0 + kk, gj = j0 + r;
-          const int64_t at = args.b_nmajor ? gj + static_cast<int64_t>(k) * n
-                                           : k + static_cast<int64_t>(gj) * n;
-          Bs[buf][kk][r] = (k < n && gj < n) ? B[at] : 0.0f;
-        }
+    for (int p = 0; p < kM / 2; ++p)
+#pragma unroll
+      for (int c = 0; c < kM; ++c) acc[p][c] = f2zero();
+    const int steps = (n + S::kK - 1) / S::kK;
+    auto stage = [&](int s) {
+      if (s < steps) {
+        gemmStage<kT, kMajorA>(&As[s % S::kStages][0][0], A, n, i0, s * S::kK);
+        gemmStage<kT, kMajorB>(&Bs[s % S::kStages][0][0], B, n, j0, s * S::kK);
       }
+      asm volatile("cp.async.commit_group;\n" ::: "memory");
     };
-    const int ksteps = (n + kBK - 1) / kBK;
-    load(0, 0);
-    __syncthreads();
-    for (int ks = 0; ks < ksteps; ++ks) {
-      const int buf = ks & 1;
-      if (ks + 1 < ksteps) load(buf ^ 1, (ks + 1) * kBK);
 #pragma unroll
-      for (int kk = 0; kk < kBK; ++kk) {
-        const float4 a4 = *reinterpret_cast<const float4 *>(&As[buf][kk][ty * 4]);
-        const float4 b4 = *reinterpret_cast<const float4 *>(&Bs[buf][kk][tx * 4]);
-        const float av[4] = {a4.x, a4.y, a4.z, a4.w};
-        const float bv[4] = {b4.x, b4.y, b4.z, b4.w};
+    for (int s = 0; s < S::kStages - 1; ++s) stage(s);
+    for (int s = 0; s < steps; ++s) {
+      asm volatile("cp.async.wait_group %0;\n" ::"n"(S::kStages - 2) : "memory");
+      __syncthreads();  // step s landed for every thread; step s - 1's slot is free
+      stage(s + S::kStages - 1);
+      const float *as = &As[s % S::kStages][0][4 * tx], *bs = &Bs[s % S::kStages][0][4 * ty];
+      const int left = n - s * S::kK;
+      if (left >= S::kK) {
 #pragma unroll
-        for (int r = 0; r < 4; ++r)
-#pragma unroll
-          for (int c = 0; c < 4; ++c) acc[r][c] = fmaf(av[r], bv[c], acc[r][c]);
+        for (int k = 0; k < S::kK; ++k) gemmStep<kT>(as + k * S::kLd, bs + k * S::kLd, acc);
+      } else {
+        for (int k = 0; k < left; ++k) gemmStep<kT>(as + k * S::kLd, bs + k * S::kLd, acc);
       }
-      __syncthreads();
     }
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    __syncthreads();  // the ring is free for the next item
     float *C = args.c + args.c_offset[mi];
+    const float *lam = kEpilogue == kEpilogueInverseH ? args.eigenvalues + args.eig_offset[mi] : nullptr;
+    float ri[kM];  // roots of this thread's rows
+    if (kEpilogue == kEpilogueInverseH) {
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const int j = j0 + tx * 4 + c;
+      for (int r = 0; r < kM; ++r) {
+        const int i = i0 + 4 * tx + (r / 4) * S::kQ + r % 4;
+        ri[r] = i < n ? rootOf(lam[i]) : 0.0f;
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < kM; ++c) {
+      const int j = j0 + 4 * ty + (c / 4) * S::kQ + c % 4;
       if (j >= n) continue;
+      const float rj = kEpilogue == kEpilogueInverseH ? rootOf(lam[j]) : 0.0f;
 #pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        const int i = i0 + ty * 4 + r;
-        if (i >= n) continue;
-        float v = acc[r][c];
-        if (kEpilogue == kEpilogueInverseH) {
-          const float *lam = args.eigenvalues + args.eig_offset[mi];
-          // an FP32 eigenvalue <= 0 (below FP32 resolution of a nearly
-          // singular input) has root 0; the pair of two such gets no correction
-          const float d = rootOf(lam[i]) + rootOf(lam[j]);
-          v = d > 0.0f ? v / d : 0.0f;
+      for (int p = 0; p < kM / 2; ++p) {
+        float v[2];
+        f2split(acc[p][c], v[0], v[1]);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int r = 2 * p + h;
+          const int i = i0 + 4 * tx + (r / 4) * S::kQ + r % 4;
+          if (i >= n) continue;
+          float x = v[h];
+          if (kEpilogue == kEpilogueInverseH) {
+            // an FP32 eigenvalue <= 0 (below FP32 resolution of a nearly
+            // singular input) has root 0; the pair of two such gets no correction
+            const float d = ri[r] + rj;
+            x = d > 0.0f ? x / d : 0.0f;
+          }
+          C[i + static_cast<int64_t>(j) * n] = x;
+          if (kMirror && w.z > w.y) C[j + static_cast<int64_t>(i) * n] = x;
         }
-        C[i + static_cast<int64_t>(j) * n] = v;
       }
     }
   }
@@ -378,12 +461,21 @@ __global__ void workingAddKernel(float *__restrict__ x_hi, float *__restrict__ x
 
 }  // namespace
 
-int gemmWork(msq_ctx *ctx, const DeviceBatch *b, int tile, const int4 **work, int *items) {
-  // One list per (layout, tile size); cached on the batch.  A negative tile
-  // size asks for the upper triangle of tiles only (tj >= ti).
+namespace {
+
+// Orders from which the FP32 GEMM may use 128 x 128 tiles, and the first
+// work-list key of the GEMM's lists (the other lists use +-tile).
+constexpr int kGemmLargeOrder = 1000;
+constexpr int kGemmWorkBase = 1 << 16;
+
+// One work list per (batch layout, key), cached on the batch: the tiles of
+// every matrix whose order `in` accepts.
+template <class In>
+int tileWork(msq_ctx *ctx, const DeviceBatch *b, int size, bool upper, int key, const int4 **work,
+             int *items, In in) {
   auto &cache = const_cast<DeviceBatch *>(b)->work_cache;
   for (auto &e : cache) {
-    if (e.tile == tile) {
+    if (e.tile == key) {
       *work = e.work;
       *items = e.items;
       return MSQ_OK;
@@ -391,33 +483,95 @@ int gemmWork(msq_ctx *ctx, const DeviceBatch *b, int tile, const int4 **work, in
   }
   std::vector<int4> list;
   // largest matrices first: their long K loops start early
-  std::vector<int> ids(b->count);
-  for (int i = 0; i < b->count; ++i) ids[i] = i;
+  std::vector<int> ids;
+  for (int i = 0; i < b->count; ++i)
+    if (in(b->host_n[i])) ids.push_back(i);
   std::stable_sort(ids.begin(), ids.end(),
                    [&](int x, int y) { return b->host_n[x] > b->host_n[y]; });
-  const bool upper = tile < 0;
-  const int size = upper ? -tile : tile;
   for (int mi : ids) {
     const int t = (b->host_n[mi] + size - 1) / size;
     for (int ti = 0; ti < t; ++ti)
       for (int tj = upper ? ti : 0; tj < t; ++tj) list.push_back(make_int4(mi, ti, tj, 0));
   }
   int4 *dev = nullptr;
-  MSQ_TRY(cudaCheck(ctx, cudaMalloc(&dev, list.size() * sizeof(int4)), "work list alloc"));
-  MSQ_TRY(cudaCheck(ctx, cudaMemcpy(dev, list.data(), list.size() * sizeof(int4),
-                                    cudaMemcpyHostToDevice), "work list upload"));
-  cache.push_back({tile, dev, static_cast<int>(list.size())});
+  if (!list.empty()) {
+    MSQ_TRY(cudaCheck(ctx, cudaMalloc(&dev, list.size() * sizeof(int4)), "work list alloc"));
+    MSQ_TRY(cudaCheck(ctx, cudaMemcpy(dev, list.data(), list.size() * sizeof(int4),
+                                      cudaMemcpyHostToDevice), "work list upload"));
+  }
+  cache.push_back({key, dev, static_cast<int>(list.size())});
   *work = dev;
   *items = static_cast<int>(list.size());
   return MSQ_OK;
 }
 
+}  // namespace
+
+int gemmWork(msq_ctx *ctx, const DeviceBatch *b, int tile, const int4 **work, int *items) {
+  // A negative tile size asks for the upper triangle of tiles only (tj >= ti).
+  const bool upper = tile < 0;
+  return tileWork(ctx, b, upper ? -tile : tile, upper, tile, work, items, [](int) { return true; });
+}
+
+namespace {
+
+// Tile size of a matrix in the FP32 GEMM.  32 up to order 32 (a 64-tile is
+// mostly padding: a correction of 1000 matrices of order 24 takes 33 us
+// against 53) and for batches with fewer 64-tiles than 1.5 per SM, where
+// one CTA's K loop is the whole launch and a 32-tile's is a quarter as long
+// (order 256 alone: 46 us against 90; order 512 alone: 82 against 150; eight
+// of order 384, 288 tiles: 162 against 133).  128 from order 1000 where
+// the batch's 128-tiles nearly give every SM one (order 2048: 1565 us
+// against 1724; 1500: 648 against 719; 1000 alone, 64 tiles: 443 against
+// 295).  64 otherwise (20 of order 777: 2058 us against 2087 with 128).
+int gemmClass(const DeviceBatch *b, int n) {
+  int64_t tiles64 = 0, tiles128 = 0;
+  for (const int32_t m : b->host_n) {
+    const int64_t t = (m + 63) / 64, u = (m + 127) / 128;
+    tiles64 += t * t;
+    if (m >= kGemmLargeOrder) tiles128 += u * u;
+  }
+  if (n <= 32 || tiles64 < 3 * kSmCount / 2) return 32;
+  return n >= kGemmLargeOrder && tiles128 >= 4 * kSmCount / 5 ? 128 : 64;
+}
+
+// The tiles (matrix, i, j) of every matrix of one tile class, cached on the
+// batch; `upper`: only those on or above the diagonal.
+int gemmTiles(msq_ctx *ctx, const DeviceBatch *b, int tile, bool upper, const int4 **work,
+              int *items) {
+  return tileWork(ctx, b, tile, upper, kGemmWorkBase + (upper ? 1 : 0) + 2 * tile, work, items,
+                  [&](int n) { return gemmClass(b, n) == tile; });
+}
+
+template <int kT, bool kMajorA, bool kMajorB>
+int launchGemm(msq_ctx *ctx, const DeviceBatch *b, GemmArgs args, int epilogue, bool mirror) {
+  using S = GemmShape<kT>;
+  MSQ_TRY(gemmTiles(ctx, b, kT, mirror, &args.work, &args.items));
+  if (args.items == 0) return MSQ_OK;
+  const unsigned grid = std::min<unsigned>(args.items, kSmCount * S::kCtas * 4);
+  if (mirror) {
+    gemmKernel<kT, kMajorA, kMajorA, kEpilogueStore, true><<<grid, S::kThr, 0, ctx->stream>>>(args);
+  } else if (epilogue == kEpilogueInverseH) {
+    gemmKernel<kT, kMajorA, kMajorB, kEpilogueInverseH, false><<<grid, S::kThr, 0, ctx->stream>>>(args);
+  } else {
+    gemmKernel<kT, kMajorA, kMajorB, kEpilogueStore, false><<<grid, S::kThr, 0, ctx->stream>>>(args);
+  }
+  return launched(ctx, "gemm TN fp32");
+}
+
+template <bool kMajorA, bool kMajorB>
+int launchGemmClasses(msq_ctx *ctx, const DeviceBatch *b, const GemmArgs &args, int epilogue,
+                      bool mirror) {
+  MSQ_TRY((launchGemm<128, kMajorA, kMajorB>(ctx, b, args, epilogue, mirror)));
+  MSQ_TRY((launchGemm<64, kMajorA, kMajorB>(ctx, b, args, epilogue, mirror)));
+  return launchGemm<32, kMajorA, kMajorB>(ctx, b, args, epilogue, mirror);
+}
+
+}  // namespace
+
 int gemmTN(msq_ctx *ctx, const DeviceBatch *b, const float *a, const float *bm, float *c,
            int epilogue, const float *eigenvalues, bool a_mmajor, bool b_nmajor) {
   GemmArgs args{};
-  args.a_mmajor = a_mmajor;
-  args.b_nmajor = b_nmajor;
-  MSQ_TRY(gemmWork(ctx, b, kTile, &args.work, &args.items));
   args.a = a;
   args.b = bm;
   args.c = c;
@@ -427,13 +581,13 @@ int gemmTN(msq_ctx *ctx, const DeviceBatch *b, const float *a, const float *bm, 
   args.n = b->n;
   args.eigenvalues = eigenvalues;
   args.eig_offset = b->eig_offset;
-  const unsigned grid = std::min<unsigned>(args.items, kSmCount * 8);
-  if (epilogue == kEpilogueInverseH) {
-    gemmTNKernel<kEpilogueInverseH><<<grid, kThreads, 0, ctx->stream>>>(args);
-  } else {
-    gemmTNKernel<kEpilogueStore><<<grid, kThreads, 0, ctx->stream>>>(args);
-  }
-  return launched(ctx, "gemm TN fp32");
+  // one operand against itself in the same layout (F^T F or F F^T): symmetric
+  const bool mirror = a == bm && a_mmajor == b_nmajor && epilogue == kEpilogueStore;
+  if (a_mmajor)
+    return b_nmajor ? launchGemmClasses<true, true>(ctx, b, args, epilogue, mirror)
+                    : launchGemmClasses<true, false>(ctx, b, args, epilogue, mirror);
+  return b_nmajor ? launchGemmClasses<false, true>(ctx, b, args, epilogue, mirror)
+                  : launchGemmClasses<false, false>(ctx, b, args, epilogue, mirror);
 }
 
 int residualFF(msq_ctx *ctx, const DeviceBatch *b, const float *a, const float *x_hi,
@@ -473,72 +627,10 @@ int transpose(msq_ctx *ctx, const DeviceBatch *b, const float *src, float *dst) 
   return launched(ctx, "transpose");
 }
 
-// C = A B for one n x n column-major matrix, each element the FMA chain
-// sum = fma(A[r, k], B[k, c], sum) over k = 0..n-1 in order, as the
-// reference's matmul kernels accumulate (metal_mixed_sqrt.metal:39-56,
-// matmul_tiled_*: decoded operands, FP32).  16 x 16 outputs per CTA, K
-// staged through shared memory 16 at a time (the chain order is kept).
 namespace {
-constexpr int kMmTile = 16;
 
-__global__ void __launch_bounds__(kMmTile * kMmTile)
-matmulFmaKernel(const float *__restrict__ a, const float *__restrict__ b, float *__restrict__ c,
-                int n) {
-  __shared__ float as[kMmTile][kMmTile + 1];
-  __shared__ float bs[kMmTile][kMmTile + 1];
-  const int tr = threadIdx.x, tc = threadIdx.y;  // row fastest: coalesced column reads
-  const int row = blockIdx.x * kMmTile + tr, col = blockIdx.y * kMmTile + tc;
-  float sum = 0.0f;
-  for (int k0 = 0; k0 < n; k0 += kMmTile) {
-    // A[row, k0 + tc] and B[k0 + tr, col]
-    as[tr][tc] = row < n && k0 + tc < n ? a[row + static_cast<int64_t>(k0 + tc) * n] : 0.0f;
-    bs[tr][tc] = k0 + tr < n && col < n ? b[(k0 + tr) + static_cast<int64_t>(col) * n] : 0.0f;
-    __syncthreads();
-    const int kend = min(kMmTile, n - k0);
-    for (int k = 0; k < kend; ++k) sum = fmaf(as[tr][k], bs[k][tc], sum);
-    __syncthreads();
-  }
-  if (row < n && col < n) c[row + static_cast<int64_t>(col) * n] = sum;
-}
-
-// The same product for every matrix of a batch: one CTA per 16 x 16 output
-// tile of a (matrix, tile_i, tile_j) work list, the same FMA chains.
-__global__ void __launch_bounds__(kMmTile * kMmTile)
-matmulFmaBatchKernel(const float *__restrict__ a, const float *__restrict__ b, float *__restrict__ c,
-                     const int64_t *__restrict__ offset, const int32_t *__restrict__ n,
-                     const int4 *__restrict__ work, int items) {
-  __shared__ float as[kMmTile][kMmTile + 1];
-  __shared__ float bs[kMmTile][kMmTile + 1];
-  const int tr = threadIdx.x, tc = threadIdx.y;
-  for (int item = blockIdx.x; item < items; item += gridDim.x) {
-    const int4 w = work[item];
-    const int nn = n[w.x];
-    const int64_t o = offset[w.x];
-    const int row = w.y * kMmTile + tr, col = w.z * kMmTile + tc;
-    float sum = 0.0f;
-    for (int k0 = 0; k0 < nn; k0 += kMmTile) {
-      as[tr][tc] = row < nn && k0 + tc < nn ? a[o + row + static_cast<int64_t>(k0 + tc) * nn] : 0.0f;
-      bs[tr][tc] = k0 + tr < nn && col < nn ? b[o + (k0 + tr) + static_cast<int64_t>(col) * nn] : 0.0f;
-      __syncthreads();
-      const int kend = min(kMmTile, nn - k0);
-      for (int k = 0; k < kend; ++k) sum = fmaf(as[tr][k], bs[k][tc], sum);
-      __syncthreads();
-    }
-    if (row < nn && col < nn) c[o + row + static_cast<int64_t>(col) * nn] = sum;
-  }
-}
-
-// C_ij = W_ij / (s_i + s_j) (diagonal_sylvester_*, metal_mixed_sqrt.metal:58-74).
-__global__ void diagonalSylvesterKernel(const float *__restrict__ w, const float *__restrict__ s,
-                                        float *__restrict__ c, int n) {
-  const int64_t total = static_cast<int64_t>(n) * n;
-  for (int64_t idx = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; idx < total;
-       idx += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int i = static_cast<int>(idx % n), j = static_cast<int>(idx / n);
-    c[idx] = __fdiv_rn(w[idx], s[i] + s[j]);
-  }
-}
-// The same for every matrix of a batch (grid.y = matrix); s of matrix i at
+// C_ij = W_ij / (s_i + s_j) (diagonal_sylvester_*, metal_mixed_sqrt.metal:58-74)
+// for every matrix of a batch (grid.y = matrix); s of matrix i at
 // eig_offset[i].
 __global__ void diagonalSylvesterBatchKernel(const float *__restrict__ w, const float *__restrict__ s,
                                              float *__restrict__ c, const int64_t *__restrict__ offset,
@@ -557,15 +649,6 @@ __global__ void diagonalSylvesterBatchKernel(const float *__restrict__ w, const 
 }
 }  // namespace
 
-int matmulFmaBatch(msq_ctx *ctx, const DeviceBatch *b, const float *a, const float *bm, float *c) {
-  const int4 *work = nullptr;
-  int items = 0;
-  MSQ_TRY(gemmWork(ctx, b, kMmTile, &work, &items));
-  matmulFmaBatchKernel<<<std::min(items, kSmCount * 16), dim3(kMmTile, kMmTile), 0, ctx->stream>>>(
-      a, bm, c, b->offset, b->n, work, items);
-  return launched(ctx, "native matmul");
-}
-
 int diagonalSylvesterBatch(msq_ctx *ctx, const DeviceBatch *b, const float *w, const float *s,
                            float *c) {
   const int64_t nn = static_cast<int64_t>(b->max_n) * b->max_n;
@@ -573,19 +656,6 @@ int diagonalSylvesterBatch(msq_ctx *ctx, const DeviceBatch *b, const float *w, c
                   static_cast<unsigned>(std::min(b->count, 65535)));
   diagonalSylvesterBatchKernel<<<grid, 256, 0, ctx->stream>>>(w, s, c, b->offset, b->eig_offset,
                                                               b->n, b->count);
-  return launched(ctx, "native diagonal sylvester");
-}
-
-int matmulFma(msq_ctx *ctx, const float *a, const float *b, float *c, int n) {
-  const dim3 grid((n + kMmTile - 1) / kMmTile, (n + kMmTile - 1) / kMmTile);
-  matmulFmaKernel<<<grid, dim3(kMmTile, kMmTile), 0, ctx->stream>>>(a, b, c, n);
-  return launched(ctx, "native matmul");
-}
-
-int diagonalSylvester(msq_ctx *ctx, const float *w, const float *s, float *c, int n) {
-  const int64_t total = static_cast<int64_t>(n) * n;
-  const int grid = static_cast<int>(std::min<int64_t>((total + 255) / 256, kSmCount * 8));
-  diagonalSylvesterKernel<<<grid, 256, 0, ctx->stream>>>(w, s, c, n);
   return launched(ctx, "native diagonal sylvester");
 }
 

@@ -19,8 +19,6 @@ struct GemmArgs {
   const int32_t *n;
   const float *eigenvalues;
   const int64_t *eig_offset;
-  int a_mmajor;  // A(i,k) at i + k*n instead of k + i*n
-  int b_nmajor;  // B(k,j) at j + k*n instead of k + j*n
 };
 
 struct ResidualArgs {
@@ -35,8 +33,9 @@ struct ResidualArgs {
 
 // Flat (matrix, tile_i, tile_j) work list for square tiles of size `tile`.
 int gemmWork(msq_ctx *ctx, const DeviceBatch *b, int tile, const int4 **work, int *items);
-// C = A B per matrix, FP32 FMA; by default A(i,k) = a[k + i*n] and
-// B(k,j) = bm[k + j*n] (C = a^T bm).
+// C = A B per matrix, each element the FP32 FMA chain over k in order; by
+// default A(i,k) = a[k + i*n] and B(k,j) = bm[k + j*n] (C = a^T bm);
+// a_mmajor: A(i,k) = a[i + k*n]; b_nmajor: B(k,j) = bm[j + k*n].
 int gemmTN(msq_ctx *ctx, const DeviceBatch *b, const float *a, const float *bm, float *c,
            int epilogue, const float *eigenvalues, bool a_mmajor = false,
            bool b_nmajor = false);
@@ -51,11 +50,7 @@ int residualFFGeneral(msq_ctx *ctx, const DeviceBatch *b, const float *a, const 
                       const float *x_lo, float *r, double *norms, const float *a_lo = nullptr);
 // X <- X + E in float-float, no symmetrisation.
 int workingAdd(msq_ctx *ctx, const DeviceBatch *b, float *x_hi, float *x_lo, const float *e);
-// One n x n matrix: C = A B with in-order FMA chains; C_ij = W_ij / (s_i + s_j).
-int matmulFma(msq_ctx *ctx, const float *a, const float *b, float *c, int n);
-int diagonalSylvester(msq_ctx *ctx, const float *w, const float *s, float *c, int n);
-// The same for every matrix of a batch in one launch (s at eig_offset).
-int matmulFmaBatch(msq_ctx *ctx, const DeviceBatch *b, const float *a, const float *bm, float *c);
+// C_ij = W_ij / (s_i + s_j) for every matrix of the batch (s at eig_offset).
 int diagonalSylvesterBatch(msq_ctx *ctx, const DeviceBatch *b, const float *w, const float *s,
                            float *c);
 

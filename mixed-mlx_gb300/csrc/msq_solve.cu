@@ -194,6 +194,11 @@ extern "C" int msq_native_sylvester_sweep(msq_ctx *ctx, int format, const float 
   for (int i = 0; i < b->count; ++i)
     extent = std::max(extent, b->host_offset[i] + static_cast<int64_t>(b->host_n[i]) * b->host_n[i]);
   float *rq = workspace, *w1 = workspace + extent, *w2 = workspace + 2 * extent;
+  // C = A B as the reference's matmul kernels accumulate (decoded operands,
+  // FP32, metal_mixed_sqrt.metal:39-56): the GEMM with A column-major.
+  auto product = [&](const float *x, const float *y, float *z) {
+    return gemmTN(ctx, b, x, y, z, kEpilogueStore, nullptr, true, false);
+  };
   // Every matrix of the batch per launch; Q(x) quantizes each matrix to
   // `format` (nearest, per matrix; row length n for the row-scaled format)
   // and decodes it in place.
@@ -201,15 +206,15 @@ extern "C" int msq_native_sylvester_sweep(msq_ctx *ctx, int format, const float 
                                          cudaMemcpyDeviceToDevice, ctx->stream),
                     "native residual copy"));
   MSQ_TRY(quantizeBatch(ctx, format, b, rq));                     // R in the format
-  MSQ_TRY(matmulFmaBatch(ctx, b, vectors_t, rq, w1));              // W1 = V^T R
+  MSQ_TRY(product(vectors_t, rq, w1));              // W1 = V^T R
   MSQ_TRY(quantizeBatch(ctx, format, b, w1));
-  MSQ_TRY(matmulFmaBatch(ctx, b, w1, vectors, w2));                // W2 = W1 V
+  MSQ_TRY(product(w1, vectors, w2));                // W2 = W1 V
   MSQ_TRY(quantizeBatch(ctx, format, b, w2));
   MSQ_TRY(diagonalSylvesterBatch(ctx, b, w2, spectrum, w1));       // C
   MSQ_TRY(quantizeBatch(ctx, format, b, w1));
-  MSQ_TRY(matmulFmaBatch(ctx, b, vectors, w1, w2));                // W1' = V C
+  MSQ_TRY(product(vectors, w1, w2));                // W1' = V C
   MSQ_TRY(quantizeBatch(ctx, format, b, w2));
-  MSQ_TRY(matmulFmaBatch(ctx, b, w2, vectors_t, w1));              // E = W1' V^T
+  MSQ_TRY(product(w2, vectors_t, w1));              // E = W1' V^T
   MSQ_TRY(quantizeBatch(ctx, format, b, w1));
   return symmetricAdd(ctx, b, x_hi, x_lo, w1);                       // X += (E + E^T)/2
 }
