@@ -80,8 +80,9 @@ int msq_set_graphs(msq_ctx *ctx, int enable);
 int msq_synchronize(msq_ctx *ctx);
 /* Failure injection for tests of the bounded device waits (process-wide,
  * default 0).  mode 1: the batched Jacobi sweep kernels' shared-memory flag
- * waits look for a value no warp writes, and their tile loads between
- * sweeps wait on an mbarrier with no copy behind it; mode 2: every tcgen05
+ * waits look for a value no warp writes, their tile loads between
+ * sweeps wait on an mbarrier with no copy behind it, and the grid kernels'
+ * barrier waits for arrivals nobody makes; mode 2: every tcgen05
  * GEMM launch first
  * waits on an mbarrier nothing arrives at (before it issues any copy or
  * MMA).  Each such wait gives up after a short limit, the launch unwinds,

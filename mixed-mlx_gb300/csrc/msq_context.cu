@@ -277,7 +277,6 @@ extern "C" void msq_destroy(msq_ctx *ctx) {
   }
   for (int slot = 0; slot < msq::kScratchSlots; ++slot)
     if (ctx->scratch[slot] != nullptr) cudaFree(ctx->scratch[slot]);
-  if (ctx->grid_exec != nullptr) cudaGraphExecDestroy(ctx->grid_exec);
   for (auto &g : ctx->jacobi_graphs) cudaGraphExecDestroy(g.exec);
   for (auto &g : ctx->solve_graphs) cudaGraphExecDestroy(g.exec);
   if (ctx->pinned != nullptr) cudaFreeHost(ctx->pinned);

@@ -134,13 +134,8 @@ struct msq_ctx {
   // Batched Jacobi launch sequences captured as CUDA graphs (at most 8).
   bool graphs = true;
   std::vector<msq::JacobiGraph> jacobi_graphs;
-  // Grid Jacobi (one large matrix on all SMs): pinned off-norm readback and
-  // the captured graph of one sweep, valid for order grid_n and workspace
-  // grid_work.
+  // Grid Jacobi (one large matrix on all SMs): pinned off-norm readback.
   double *grid_host = nullptr;
-  cudaGraphExec_t grid_exec = nullptr;
-  int grid_n = 0;
-  void *grid_work = nullptr;
   std::vector<cudaEvent_t> sync_pool;
   size_t sync_next = 0;
   // Whole-solve graphs (msq_solve_batched): the plan groups' launch

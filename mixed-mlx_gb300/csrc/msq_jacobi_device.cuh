@@ -374,6 +374,181 @@ __device__ __forceinline__ void pivotSweep(float (&ra)[8], float (&rb)[8], float
   }
 }
 
+// Round-robin slot and pair of a round inside one sweep (round < m - 1: no
+// modulo), and the pair that holds a block.
+__host__ __device__ __forceinline__ int sweepSlot(int slot, int round, int m) {
+  if (slot == 0) return 0;
+  const int k = slot - 1 - round;
+  return 1 + (k < 0 ? k + m - 1 : k);
+}
+__host__ __device__ __forceinline__ void sweepPair(int pair, int round, int m, int &p, int &q) {
+  const int a = sweepSlot(pair, round, m), b = sweepSlot(m - 1 - pair, round, m);
+  p = a < b ? a : b;
+  q = a < b ? b : a;
+}
+__host__ __device__ __forceinline__ int sweepPairOf(int block, int round, int m) {
+  int slot = 0;
+  if (block != 0) {
+    const int k = block - 1 + round;
+    slot = 1 + (k >= m - 1 ? k - (m - 1) : k);
+  }
+  return slot < m - 1 - slot ? slot : m - 1 - slot;
+}
+
+// ---------------------------------------------------------------------------
+// The same pivot sweep on 16 lanes, where its latency is what counts (the
+// grid kernels: a round's critical path is one pivot): the same rotations
+// and the same bits.
+//
+// The pivot is kept in tournament positions: in every group pair t holds
+// positions (t, 7 - t), and between groups position 0 stays and positions
+// 1..7 rotate by one, so every group has the same data movement.  Lane
+// (t, j) holds the 2x2 block of pairs lo = min(t, j), hi = max(t, j): rows
+// (lo, 7 - lo), columns (hi, 7 - hi), row rotation first, then the column
+// rotation, which is the sequential order of the upper triangle (the lower
+// one is its transpose bit for bit: each of its elements sees the same two
+// operations).  Lanes (t, j) and (j, t) do the same work and write the two
+// triangles.  The diagonal lanes compute the four angles of a group at once;
+// the blocks move through shared memory, double-buffered (no bank conflict
+// in either direction for the two pivots of a warp).  Positions order a pair
+// by tournament slot, the angle by index: where they differ the angle is
+// taken of the swapped pair and s negated (x - y and x + (-y) round alike).
+// Q is formed by another warp that follows the pivot warp (PivotQ): the
+// diagonal lanes leave each group's (c, s) in shared memory and a flag says
+// how far they are; 32 more rotations per group would otherwise sit on the
+// critical path.
+constexpr int kPivotOffset = 132;  // floats of a pivot (two 8x8 buffers); the second one
+                                   // of a warp starts on other banks
+// Shared memory of a pivot warp (two pivots) and the warp that forms their Q.
+struct PivotPair {
+  float m[2 * kPivotOffset];
+  float2 cs[2][7][4];  // (cosine or 2 for no rotation, sine), position order
+  int groups;          // 8 x sweeps + groups done by the pivot warp
+  int taken;           // sweeps whose (c, s) the other warp has read
+};
+
+__device__ __forceinline__ void storeFlag(int *p, int v) {
+  asm volatile("st.release.cta.shared.s32 [%0], %1;" ::"r"(static_cast<unsigned>(__cvta_generic_to_shared(p))), "r"(v) : "memory");
+}
+__device__ __forceinline__ int loadFlag(const int *p) {
+  int v;
+  asm volatile("ld.acquire.cta.shared.s32 %0, [%1];" : "=r"(v) : "r"(static_cast<unsigned>(__cvta_generic_to_shared(p))) : "memory");
+  return v;
+}
+// Bounded wait for *p >= target (false on expiry).
+constexpr int kPairWaitLimit = 1 << 22;
+__device__ __forceinline__ bool waitFlag(const int *p, int target) {
+  for (int i = 0; i < kPairWaitLimit; ++i)
+    if (loadFlag(p) - target >= 0) return true;
+  return false;
+}
+
+__host__ __device__ constexpr int tournamentItem(int pos, int g) {
+  return pos == 0 ? 0 : 1 + (pos - 1 - g + 7) % 7;
+}
+// bit g: the item at position t of group g has the larger index of its pair
+__host__ __device__ constexpr uint32_t flipWord(int t) {
+  uint32_t w = 0;
+  for (int g = 0; g < 7; ++g)
+    w |= (tournamentItem(t, g) > tournamentItem(7 - t, g) ? 1u : 0u) << g;
+  return w;
+}
+
+struct Pivot16 {
+  int w[4], r[4];    // shared-memory element of x00, x01, x10, x11: written, read
+  uint32_t flips;
+  int lo, hi;
+  bool diag;
+  __device__ explicit Pivot16(int L) {
+    const int t = L >> 2, j = L & 3;
+    lo = t < j ? t : j;
+    hi = t < j ? j : t;
+    diag = t == j;
+    flips = t == 0 ? flipWord(0) : t == 1 ? flipWord(1) : t == 2 ? flipWord(2) : flipWord(3);
+    const int rr[2] = {lo, 7 - lo}, cc[2] = {hi, 7 - hi};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int a = rr[e >> 1], b = cc[e & 1];
+      // group g + 1 finds at position p what group g left at position p - 1
+      const int pa = a == 0 ? 0 : (a == 1 ? 7 : a - 1), pb = b == 0 ? 0 : (b == 1 ? 7 : b - 1);
+      w[e] = t <= j ? 8 * a + b : 8 * b + a;
+      r[e] = t <= j ? 8 * pa + pb : 8 * pb + pa;
+    }
+  }
+};
+
+// Sweeps the two symmetric 8x8 matrices of the warp (row-major, stride 8, at
+// pair.m and pair.m + kPivotOffset, synchronised by the caller), which hold
+// the rotated matrices on return.  `seq` counts the pair's sweeps.  False if
+// the warp that forms Q does not follow.  The groups are a loop, not
+// unrolled: the sweep runs once per round beside other warps' code, and 28 KB
+// of instructions were fetched anew each time.
+__device__ __forceinline__ bool pivotSweep16(const Pivot16 &p, PivotPair &pair, int half, int lane,
+                                             int seq) {
+  float *M = pair.m + half * kPivotOffset;
+  float x[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) x[e] = M[p.w[e]];
+  const bool ok = waitFlag(&pair.taken, seq);  // the last sweep's (c, s) have been read
+  __syncwarp();
+#pragma unroll 1
+  for (int g = 0; g < 7; ++g) {
+    const bool flip = (p.flips >> g) & 1;
+    float c = 1.0f, s = 0.0f;
+    // off-diagonal lanes have no angle (a zero off-diagonal element)
+    const bool on = jacobiAngle(flip ? x[3] : x[0], flip ? x[0] : x[3], p.diag ? x[1] : 0.0f, c, s);
+    const float mark = on ? c : 2.0f;  // no rotation: 2 in the place of the cosine
+    s = flip ? -s : s;
+    const float c1 = __shfl_sync(0xffffffffu, mark, 5 * p.lo, 16);
+    const float s1 = __shfl_sync(0xffffffffu, s, 5 * p.lo, 16);
+    const float c2 = __shfl_sync(0xffffffffu, mark, 5 * p.hi, 16);
+    const float s2 = __shfl_sync(0xffffffffu, s, 5 * p.hi, 16);
+    if (p.diag) pair.cs[half][g][p.lo] = make_float2(mark, s);
+    const bool on1 = c1 != 2.0f, on2 = c2 != 2.0f;
+    rot2(x[0], x[2], c1, s1, on1);  // rows
+    rot2(x[1], x[3], c1, s1, on1);
+    rot2(x[0], x[1], c2, s2, on2);  // columns
+    rot2(x[2], x[3], c2, s2, on2);
+    if (p.diag && on) x[1] = x[2] = 0.0f;
+    float *m = M + (g & 1) * 64;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) m[p.w[e]] = x[e];
+    __syncwarp();
+#pragma unroll
+    for (int e = 0; e < 4; ++e) x[e] = m[p.r[e]];
+    if (lane == 0) storeFlag(&pair.groups, 8 * seq + g + 1);
+  }
+  // after the seventh exchange position i holds index i again
+#pragma unroll
+  for (int e = 0; e < 4; ++e) M[64 + p.w[e]] = x[e];
+  __syncwarp();
+  return ok;
+}
+
+// Q of the same two pivots, in tournament positions as well (columns t and
+// 7 - t rotate, then 1..7 move on): lane L of a half holds row L & 7.
+__device__ __forceinline__ bool pivotQ(PivotPair &pair, int half, int lane, int seq, float (&q)[8]) {
+  bool ok = true;
+#pragma unroll
+  for (int y = 0; y < 8; ++y) q[y] = y == (lane & 7) ? 1.0f : 0.0f;
+#pragma unroll 1
+  for (int g = 0; g < 7; ++g) {
+    ok = waitFlag(&pair.groups, 8 * seq + g + 1) && ok;
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      const float2 cs = pair.cs[half][g][t];
+      rot2(q[t], q[7 - t], cs.x, cs.y, cs.x != 2.0f);
+    }
+    const float last = q[7];
+#pragma unroll
+    for (int y = 7; y > 1; --y) q[y] = q[y - 1];
+    q[1] = last;
+  }
+  __syncwarp();
+  if (lane == 0) storeFlag(&pair.taken, seq + 1);
+  return ok;
+}
+
 // Tile lookup through the shared table tri[J] = J (J + 1) / 2 ...
 struct SharedTri {
   const int *tri;
@@ -394,6 +569,8 @@ struct ComputedTri {
 struct FlatTiles {
   float *t;
   __device__ __forceinline__ float *base(int ti) const { return t + static_cast<int64_t>(ti) * kTileF; }
+  __device__ __forceinline__ void load(int ti, bool transposed, float (&b)[4][4]) const;
+  __device__ __forceinline__ void store(int ti, bool transposed, const float (&b)[4][4]) const;
 };
 // ... or tiles [0, split) in shared memory and the rest in the global
 // workspace (the global-tile sweep keeps what fits on chip).
@@ -404,6 +581,8 @@ struct SplitTiles {
   __device__ __forceinline__ float *base(int ti) const {
     return ti < split ? s + ti * kTileF : g + static_cast<int64_t>(ti) * kTileF;
   }
+  __device__ __forceinline__ void load(int ti, bool transposed, float (&b)[4][4]) const;
+  __device__ __forceinline__ void store(int ti, bool transposed, const float (&b)[4][4]) const;
 };
 // Element e = tileElement(t, i, j) of a tile store.
 template <class Mem>
@@ -431,6 +610,36 @@ __device__ __forceinline__ void storeTileAt(float *p, int ti, bool transposed, c
     dst[i ^ (ti & 3)] = transposed ? make_float4(t[0][i], t[1][i], t[2][i], t[3][i])
                                    : make_float4(t[i][0], t[i][1], t[i][2], t[i][3]);
   }
+}
+
+__device__ __forceinline__ void FlatTiles::load(int ti, bool transposed, float (&b)[4][4]) const {
+  loadTileAt(base(ti), ti, transposed, b);
+}
+__device__ __forceinline__ void FlatTiles::store(int ti, bool transposed, const float (&b)[4][4]) const {
+  storeTileAt(base(ti), ti, transposed, b);
+}
+__device__ __forceinline__ void SplitTiles::load(int ti, bool transposed, float (&b)[4][4]) const {
+  loadTileAt(base(ti), ti, transposed, b);
+}
+__device__ __forceinline__ void SplitTiles::store(int ti, bool transposed, const float (&b)[4][4]) const {
+  storeTileAt(base(ti), ti, transposed, b);
+}
+
+// 32-byte global accesses (32-byte aligned addresses).  Lanes of a warp that
+// each touch their own 64-byte tile pay per instruction for 32 lines: two of
+// these per tile instead of four 16-byte ones (166 against 218 cycles per 64
+// tiles loaded, 206 against 377 stored, tiles in L2).
+__device__ __forceinline__ void loadGlobal32(const float *p, float (&v)[8]) {
+  asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]),
+                 "=f"(v[7])
+               : "l"(p)
+               : "memory");
+}
+__device__ __forceinline__ void storeGlobal32(float *p, const float (&v)[8]) {
+  asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(v[0]),
+               "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
+               : "memory");
 }
 
 // Super-tile update T' = Q_k^T T Q_l on two lanes (h = 0, 1 of an adjacent
@@ -462,7 +671,7 @@ __device__ __forceinline__ void superTileHalfMem(const Mem &mem, TileOf tileOf, 
     if (valid) {
       bool tr;
       const int ti = tileOf(x ? rb1 : rb0, cbh, tr);
-      loadTileAt(mem.base(ti), ti, tr, b4);
+      mem.load(ti, tr, b4);
     } else {
 #pragma unroll
       for (int i = 0; i < 4; ++i)
@@ -537,7 +746,7 @@ __device__ __forceinline__ void superTileHalfMem(const Mem &mem, TileOf tileOf, 
       }
       bool tr;
       const int ti = tileOf(rbh, y ? cb1 : cb0, tr);
-      storeTileAt(mem.base(ti), ti, tr, b4);
+      mem.store(ti, tr, b4);
     }
   }
 }

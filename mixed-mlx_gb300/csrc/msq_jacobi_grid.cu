@@ -2,19 +2,33 @@
 //
 // The batched eigensolver gives each matrix one CTA, which leaves a single
 // large matrix (or a handful) on a few SMs.  Here every SM works on the same
-// matrix, with the same blocked rotations and the same bits:
-//  * A is kept as the same packed, row-swizzled 4x4 tiles of the upper
-//    triangle, in global memory (L2-resident up to n ~ 4096);
-//  * a round is two launches: gridPivotKernel sweeps the P pivots (a quad of
-//    lanes each, writing the round's rotations), gridUpdateKernel applies
-//    every super-tile update T' = Q_k^T T Q_l (two lanes each) and the V
-//    update V <- V Q on row-major V (lanes = rows, so Q_k is a broadcast);
-//  * the rounds of one sweep are captured once into a CUDA graph and the
-//    graph is launched once per sweep;
+// matrix, with the same blocked rotations and the same bits.  One cooperative
+// launch runs a whole sweep, one grid barrier per round:
+//  * A is kept as packed 4x4 tiles of the upper triangle (rows in
+//    order: a lane moves a whole tile with two 32-byte accesses), in global
+//    memory (L2-resident up to n ~ 4096), twice: a round
+//    reads one copy and writes the other, so nobody waits for a reader;
+//  * step r: one warp per CTA (two pivots at a time) rebuilds the cross tile
+//    that each pivot of round r + 1 needs from round r's input tiles and
+//    rotations (the diagonal tiles come from round r's pivots) and sweeps
+//    those pivots on 16 lanes each, a second warp forms their Q, and the
+//    others apply round r's super-tile updates T' = Q_k^T T Q_l (two lanes
+//    each);
+//  * V <- V Q: up to n ~ 2300 a CTA keeps its rows of V in shared memory for
+//    the whole sweep and applies round r's rotations after it has arrived at
+//    the barrier, while the others arrive (rows are independent); beyond,
+//    launches of kLogRounds rounds log the rotations and gridReplayKernel
+//    applies them to V;
 //  * after each sweep the FP64 off-norm is reduced on the device and read by
 //    the host, which decides whether another sweep is needed (the reference
 //    runs a fixed 8 sweeps, MetalRuntime::symmetricJacobi,
 //    src/metal_runtime.cpp:584-646).
+// A round is bound by its latency up to n ~ 1600 (one pivot's chain of 28
+// angles 2.1 us, the exchange through L2 and the barrier as much again) and
+// beyond by the updates (uncoalesced tile accesses, L2).  Microseconds per
+// round, sweeps of a random matrix, against two launches per round with V in
+// global memory and quad pivots: n = 512 4.6 (13), 1024 4.8 (18), 2048 7.8
+// (36), 4096 28 (62).
 // Every element update is the same ordered FP32 chain as in the batched
 // kernels and the CPU restatement, so results agree bit for bit after the
 // same number of sweeps.
@@ -22,23 +36,83 @@
 #include "msq_jacobi_device.cuh"
 #include "msq_jacobi_grid.cuh"
 
+#include <algorithm>
+#include <atomic>
 #include <cmath>
-#include <cstring>
 
 namespace msq {
 namespace {
 
-constexpr int kGridThreads = 256;
+constexpr int kNormThreads = 256;
+constexpr int kSweepThreads = 512;          // one CTA per SM at 128 registers
+constexpr int kSweepWarps = kSweepThreads / 32;
+constexpr size_t kGridSmemLimit = 223 * 1024;  // beside the static part (3 KB)
+// Up to this order the pivots are the critical path and the update warps of
+// their scheduler are left out (n = 1536: 5.3 us per round against 6.7); at
+// 2048 the updates need every warp (8.0 against 8.9).
+constexpr int kQuietOrder = 1600;
+// Polls of the grid barrier before the kernel reports kStatusFlagTimeout and
+// returns (seconds), and the limit under the failure-injection mode.
+constexpr int kBarrierWaitLimit = 1 << 22;
+constexpr int kBarrierTestLimit = 256;
+constexpr int kLogRounds = 128;             // rounds per launch where V is replayed from a log
+constexpr int kMaxPasses = 8;               // pivot pairs per CTA: P <= 2 * 8 * CTAs
 
 struct GridArgs {
-  float *tiles;  // packed tiles of A
-  float *v;      // V, row-major n x m
+  float *tiles[2];  // packed tiles of A: round r reads copy (copy + r - first) & 1
+  float *v;         // V, row-major n x m
   const float *v_in;  // column-major starting V (null: the identity)
-  float *q;      // this round's rotations, P x 64 (row-major 8x8 each)
-  double *acc;   // off2, diag2 accumulators
+  float *q;         // rotations, P x kQS (row-major 8x8 each) per round slot:
+                    // two slots by round parity, or one per round of the launch
+  float *diag;      // diagonal tiles after the pivots of two rounds: 2 x nb x 16
+  double *acc;      // off2, diag2 accumulators
+  unsigned *barrier;  // arrivals so far
+  int *status;      // device status word
   int n, m, nb, P;
-  int round;
-  int super_items;  // 2 x folded super-tile items, rounded up to 32
+  int first, last;  // rounds [first, last) of the sweep
+  int copy;         // copy of A that holds the current matrix
+  int rows;         // rows of V per CTA
+  int update_warps;
+  unsigned base;    // barrier arrivals before this launch
+  int wait_test;    // 1: the barrier waits for a count nobody reaches
+};
+
+// Element (i, j) of tile t.
+__device__ __forceinline__ int64_t gridElement(int t, int i, int j) {
+  return static_cast<int64_t>(t) * kTileF + 4 * i + j;
+}
+
+// The two copies of A's tiles: read from one, written to the other.
+struct PingPongTiles {
+  const float *in;
+  float *out;
+  __device__ __forceinline__ void load(int ti, bool transposed, float (&b)[4][4]) const {
+    const float *p = in + static_cast<int64_t>(ti) * kTileF;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      float v[8];
+      loadGlobal32(p + 8 * h, v);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const int i = 2 * h + e / 4, j = e % 4;
+        if (transposed) b[j][i] = v[e];
+        else b[i][j] = v[e];
+      }
+    }
+  }
+  __device__ __forceinline__ void store(int ti, bool transposed, const float (&b)[4][4]) const {
+    float *p = out + static_cast<int64_t>(ti) * kTileF;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      float v[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const int i = 2 * h + e / 4, j = e % 4;
+        v[e] = transposed ? b[j][i] : b[i][j];
+      }
+      storeGlobal32(p + 8 * h, v);
+    }
+  }
 };
 
 // A (column-major, n x n) -> symmetrised tiles (the same averaged load as
@@ -54,7 +128,7 @@ __global__ void gridLoadKernel(const float *a, GridArgs g) {
     if (gi < g.n && gj < g.n) {
       val = 0.5f * (a[gi + static_cast<int64_t>(gj) * g.n] + a[gj + static_cast<int64_t>(gi) * g.n]);
     }
-    g.tiles[tileElement(triTile(I, J), e / 4, e % 4)] = val;
+    g.tiles[0][gridElement(triTile(I, J), e / 4, e % 4)] = val;
   }
   // V rows 4J .. 4J + 3
   for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < 4 * g.m; idx += gridDim.x * blockDim.x) {
@@ -68,26 +142,20 @@ __global__ void gridLoadKernel(const float *a, GridArgs g) {
 }
 
 // off2 (strictly off-diagonal) and diag2, FP64, as the batched kernel.
-__global__ void gridNormKernel(GridArgs g) {
-  __shared__ double red[2][kGridThreads / 32];
-  const int64_t tiles = static_cast<int64_t>(g.nb) * (g.nb + 1) / 2;
+// grid.y = column block J.
+__global__ void __launch_bounds__(kNormThreads) gridNormKernel(GridArgs g) {
+  __shared__ double red[2][kNormThreads / 32];
+  const int J = blockIdx.y;
+  const float *column = g.tiles[g.copy] + static_cast<int64_t>(triTile(0, J)) * kTileF;
   double off2 = 0.0, diag2 = 0.0;
-  for (int64_t idx = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; idx < tiles * kTileF;
-       idx += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int64_t t = idx / kTileF;
-    const int e = static_cast<int>(idx % kTileF);
-    // t = J (J + 1) / 2 + I, I <= J
-    int J = static_cast<int>((sqrt(8.0 * static_cast<double>(t) + 1.0) - 1.0) / 2.0);
-    while (static_cast<int64_t>(J) * (J + 1) / 2 > t) --J;
-    while (static_cast<int64_t>(J + 1) * (J + 2) / 2 <= t) ++J;
-    const int I = static_cast<int>(t - static_cast<int64_t>(J) * (J + 1) / 2);
-    const double v = g.tiles[idx];  // any element of tile t (rows are only permuted)
+  for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < (J + 1) * kTileF;
+       idx += gridDim.x * blockDim.x) {
+    const int I = idx / kTileF, e = idx % kTileF;
+    const double v = column[idx];
     if (I < J) {
       off2 += 2.0 * v * v;
     } else {
-      const int phys = e / 4, col = e % 4;
-      const int row = phys ^ static_cast<int>(t & 3);
-      if (row == col) diag2 += v * v;
+      if (e / 4 == e % 4) diag2 += v * v;
       else off2 += v * v;
     }
   }
@@ -103,7 +171,7 @@ __global__ void gridNormKernel(GridArgs g) {
   __syncthreads();
   if (threadIdx.x == 0) {
     double a = 0.0, b = 0.0;
-    for (int w = 0; w < kGridThreads / 32; ++w) {
+    for (int w = 0; w < kNormThreads / 32; ++w) {
       a += red[0][w];
       b += red[1][w];
     }
@@ -112,100 +180,414 @@ __global__ void gridNormKernel(GridArgs g) {
   }
 }
 
-// The P pivots of one round: a quad of lanes per pivot (pivotSweep), the
-// rotations written row-major to g.q.  Warp-uniform: every lane of a warp
-// takes part in the quad shuffles.
-__global__ void __launch_bounds__(kGridThreads) gridPivotKernel(GridArgs g) {
-  __shared__ __align__(16) float qcol[kGridThreads / 4][kQS];
-  const int t4 = threadIdx.x & 3;
-  const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 2;
-  const bool active = k < g.P;
-  float ra[8], rb[8];
-  int tII = 0, tIJ = 0, tJJ = 0;
-  if (active) {
-    int I, J;
-    rrPair(k, g.round, g.nb, I, J);
-    tII = triTile(I, I);
-    tIJ = triTile(I, J);
-    tJJ = triTile(J, J);
-    const float4 *sII = reinterpret_cast<const float4 *>(g.tiles + static_cast<int64_t>(tII) * kTileF);
-    const float4 *sIJ = reinterpret_cast<const float4 *>(g.tiles + static_cast<int64_t>(tIJ) * kTileF);
-    const float4 *sJJ = reinterpret_cast<const float4 *>(g.tiles + static_cast<int64_t>(tJJ) * kTileF);
-    const int jr = 3 - t4;
-    const float4 v0 = sII[t4 ^ (tII & 3)], v1 = sIJ[t4 ^ (tIJ & 3)], v2 = sJJ[jr ^ (tJJ & 3)];
-    ra[0] = v0.x; ra[1] = v0.y; ra[2] = v0.z; ra[3] = v0.w;
-    ra[4] = v1.x; ra[5] = v1.y; ra[6] = v1.z; ra[7] = v1.w;
+// Where a sweep CTA keeps a round's rotations and its rows of V.
+enum GridStore : int {
+  kVShared = 0,   // both in shared memory
+  kQShared = 1,   // rotations in shared memory; V is replayed from the log
+  kNoneShared = 2,
+};
+
+__device__ __forceinline__ unsigned loadAcquire(const unsigned *p) {
+  unsigned v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
+__device__ __forceinline__ void namedSync(int id, int threads) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void namedArrive(int id, int threads) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
+__device__ __forceinline__ void prefetchL1(const float *p) {
+  asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
+}
+
+// Element (i, c) of block (R, C), R != C, of the packed upper triangle.
+__device__ __forceinline__ float blockElement(const float *tiles, int R, int C, int i, int c) {
+  return R < C ? tiles[gridElement(triTile(R, C), i, c)] : tiles[gridElement(triTile(C, R), c, i)];
+}
+
+// o = x q for kRows rows' 8 elements and an 8x8 rotation: the ordered chains
+// o_c = sum_j x_j q_jc, two columns per packed FMA.
+template <int kRows>
+__device__ __forceinline__ void rotateRow(float *v, int m, int I, int J, const f32x2 (&q)[8][4]) {
+  float x[kRows][8];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) rb[i] = g.tiles[tileElement(tIJ, i, jr)];
-    rb[4] = v2.x; rb[5] = v2.y; rb[6] = v2.z; rb[7] = v2.w;
-  } else {
-#pragma unroll
-    for (int y = 0; y < 8; ++y) ra[y] = rb[y] = 0.0f;
+  for (int e = 0; e < kRows; ++e) {
+    const float4 a = *reinterpret_cast<const float4 *>(v + static_cast<int64_t>(e) * m + 4 * I);
+    const float4 b = *reinterpret_cast<const float4 *>(v + static_cast<int64_t>(e) * m + 4 * J);
+    x[e][0] = a.x; x[e][1] = a.y; x[e][2] = a.z; x[e][3] = a.w;
+    x[e][4] = b.x; x[e][5] = b.y; x[e][6] = b.z; x[e][7] = b.w;
   }
-  float *qs = qcol[threadIdx.x >> 2];
-  pivotSweep(ra, rb, qs, t4, active);
-  if (active) {
-    float4 *sII = reinterpret_cast<float4 *>(g.tiles + static_cast<int64_t>(tII) * kTileF);
-    float4 *sIJ = reinterpret_cast<float4 *>(g.tiles + static_cast<int64_t>(tIJ) * kTileF);
-    float4 *sJJ = reinterpret_cast<float4 *>(g.tiles + static_cast<int64_t>(tJJ) * kTileF);
-    sII[t4 ^ (tII & 3)] = make_float4(ra[0], ra[1], ra[2], ra[3]);
-    sIJ[t4 ^ (tIJ & 3)] = make_float4(ra[4], ra[5], ra[6], ra[7]);
-    sJJ[t4 ^ (tJJ & 3)] = make_float4(rb[4], rb[5], rb[6], rb[7]);
-    // the quad's Q (row-major in qs) -> g.q[k]: lane t copies rows 2t, 2t+1
-    const float4 *src = reinterpret_cast<const float4 *>(qs);
-    float4 *dst = reinterpret_cast<float4 *>(g.q + static_cast<int64_t>(k) * kQF);
 #pragma unroll
-    for (int x = 0; x < 4; ++x) dst[4 * t4 + x] = src[4 * t4 + x];
+  for (int e = 0; e < kRows; ++e) {
+    f32x2 o[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) o[c] = f2zero();
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const f32x2 xx = f2make(x[e][j], x[e][j]);
+#pragma unroll
+      for (int c = 0; c < 4; ++c) o[c] = f2fma(xx, q[j][c], o[c]);
+    }
+    *reinterpret_cast<ulonglong2 *>(v + static_cast<int64_t>(e) * m + 4 * I) = make_ulonglong2(o[0], o[1]);
+    *reinterpret_cast<ulonglong2 *>(v + static_cast<int64_t>(e) * m + 4 * J) = make_ulonglong2(o[2], o[3]);
   }
 }
 
-// Super-tile updates (items [0, super_items)) and the V update (items
-// beyond: row fastest, then pair) of one round.
-__global__ void __launch_bounds__(kGridThreads) gridUpdateKernel(GridArgs g) {
-  const int64_t total = g.super_items + static_cast<int64_t>(g.n) * g.P;
-  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-  for (int64_t base = blockIdx.x * static_cast<int64_t>(blockDim.x) + (threadIdx.x & ~31); base < total;
-       base += stride) {
-    const int64_t w = base + (threadIdx.x & 31);
-    if (base < g.super_items) {
-      // warp-uniform branch: super_items is a multiple of 32
-      const int w2 = static_cast<int>(w);
-      const int h = w2 & 1;
-      int k = 0, l = 0;
-      const bool valid = foldedBlock(w2 >> 1, g.P, k, l) && k != l && (w2 >> 1) < ((g.P + 1) / 2) * (g.P + 1);
-      if (!valid) k = l = 0;
-      int rb0, rb1, cb0, cb1;
-      rrPair(k, g.round, g.nb, rb0, rb1);
-      rrPair(l, g.round, g.nb, cb0, cb1);
-      const float4 *qk = reinterpret_cast<const float4 *>(g.q + static_cast<int64_t>(k) * kQF);
-      const float4 *ql = reinterpret_cast<const float4 *>(g.q + static_cast<int64_t>(l) * kQF);
-      superTileHalf(g.tiles, ComputedTri{}, qk, ql, rb0, rb1, cb0, cb1, h, valid);
-    } else {
-      const int64_t idx = w - g.super_items;
-      if (idx >= static_cast<int64_t>(g.n) * g.P) continue;
-      const int row = static_cast<int>(idx % g.n), k = static_cast<int>(idx / g.n);
-      int I, J;
-      rrPair(k, g.round, g.nb, I, J);
-      const float4 *qk = reinterpret_cast<const float4 *>(g.q + static_cast<int64_t>(k) * kQF);
-      float *vrow = g.v + static_cast<int64_t>(row) * g.m;
-      const float4 a = *reinterpret_cast<const float4 *>(vrow + 4 * I);
-      const float4 b = *reinterpret_cast<const float4 *>(vrow + 4 * J);
-      const float x[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-      float o[8];
-#pragma unroll
-      for (int c = 0; c < 8; ++c) o[c] = 0.0f;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float4 lo = qk[2 * j], hi = qk[2 * j + 1];
-        o[0] = fmaf(x[j], lo.x, o[0]); o[1] = fmaf(x[j], lo.y, o[1]);
-        o[2] = fmaf(x[j], lo.z, o[2]); o[3] = fmaf(x[j], lo.w, o[3]);
-        o[4] = fmaf(x[j], hi.x, o[4]); o[5] = fmaf(x[j], hi.y, o[5]);
-        o[6] = fmaf(x[j], hi.z, o[6]); o[7] = fmaf(x[j], hi.w, o[7]);
-      }
-      *reinterpret_cast<float4 *>(vrow + 4 * I) = make_float4(o[0], o[1], o[2], o[3]);
-      *reinterpret_cast<float4 *>(vrow + 4 * J) = make_float4(o[4], o[5], o[6], o[7]);
+// Shares of `rows` rows for `groups` groups of 32 pairs on `warps` warps:
+// the fewest row steps of the busiest warp, a rotation's load counting as
+// three rows.
+__host__ __device__ __forceinline__ int rowShares(int rows, int groups, int warps) {
+  int best = 1, cost = 1 << 30;
+  for (int s = 1; s <= rows && s <= 8; ++s) {
+    const int c = ((groups * s + warps - 1) / warps) * (3 + (rows + s - 1) / s);
+    if (c < cost) {
+      cost = c;
+      best = s;
     }
   }
+  return best;
+}
+
+// V <- V Q on `row_count` rows (stride m) by warp `w` of `warps`: a lane
+// holds one pair's rotation and walks rows (consecutive pairs are
+// consecutive blocks, so the lanes' accesses are contiguous); a warp takes
+// 32 pairs and one of `shares` shares of the rows.
+template <class PairOf>
+__device__ __forceinline__ void rotateRows(float *rows, int row_count, int shares, int m, int P,
+                                           const float *q, int w, int warps, int lane, PairOf pairOf) {
+  const int groups = (P + 31) / 32;
+  for (int unit = w; unit < groups * shares; unit += warps) {
+    const int k = 32 * (unit % groups) + lane, share = unit / groups;
+    int row = row_count * share / shares;
+    const int hi = row_count * (share + 1) / shares;
+    if (k >= P) continue;
+    int I, J;
+    pairOf(k, I, J);
+    f32x2 qq[8][4];
+    const ulonglong2 *src = reinterpret_cast<const ulonglong2 *>(q + static_cast<int64_t>(k) * kQS);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const ulonglong2 x = src[2 * j], y = src[2 * j + 1];
+      qq[j][0] = x.x; qq[j][1] = x.y; qq[j][2] = y.x; qq[j][3] = y.y;
+    }
+    for (; row + 2 <= hi; row += 2) rotateRow<2>(rows + static_cast<int64_t>(row) * m, m, I, J, qq);
+    if (row < hi) rotateRow<1>(rows + static_cast<int64_t>(row) * m, m, I, J, qq);
+  }
+}
+
+// Rounds [first, last) of one sweep on gridDim.x CTAs that are all resident
+// (cooperative launch).  Warp 0 sweeps the CTA's pivots, warp 1 forms their
+// Q, update_warps others apply the updates; with fewer than 14 of those the
+// warps that share warp 0's scheduler are left out.
+template <int kStore>
+__global__ void __launch_bounds__(kSweepThreads, 1) gridSweepKernel(GridArgs g) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ PivotPair pair;
+  __shared__ float crosses[kMaxPasses][32];  // the pivots' cross tiles of the current round
+  __shared__ int counters[2];                // update items taken, by round parity
+  __shared__ int arrived, give_up;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int G = gridDim.x, cta = blockIdx.x;
+  const int P = g.P, nb = g.nb, m = g.m;
+  const int update_warps = g.update_warps, update_threads = 32 * update_warps;
+  const int active = update_warps + 2;
+  const bool quiet = update_warps < kSweepWarps - 2;
+  const int uw = quiet ? warp - 2 - warp / 4 : warp - 2;  // index among the update warps
+  float *qs = reinterpret_cast<float *>(smem_raw);                    // [P][kQS]
+  float *vs = qs + (kStore == kNoneShared ? 0 : P * kQS);             // [rows][m]
+  short2 *pairs = reinterpret_cast<short2 *>(vs + (kStore == kVShared ? g.rows * m : 0));  // [2][P]
+  const int row0 = min(g.n, cta * g.rows), row_count = min(g.rows, g.n - row0);
+  const int64_t qround = static_cast<int64_t>(P) * kQS;
+  auto qslot = [&](int r) { return g.q + (kStore == kVShared ? r & 1 : r - g.first) * qround; };
+  auto tilesOf = [&](int r) { return g.tiles[(g.copy + r - g.first) & 1]; };
+  // pivots: half h of pass p takes pair cta + G (2 p + h) of each round
+  // (a CTA without one still takes part in every barrier)
+  const int passes = max(1, (P - cta + 2 * G - 1) / (2 * G));
+
+  if (threadIdx.x == 0) {
+    counters[0] = counters[1] = arrived = pair.groups = pair.taken = 0;
+    // an earlier launch gave up: its arrivals are missing from the count
+    give_up = *static_cast<volatile int *>(g.status) != kStatusOk;
+  }
+  __syncthreads();
+  if (give_up || (quiet && warp != 0 && warp % 4 == 0)) return;
+
+  // A warp is done with what others wait for; the CTA's last one arrives at
+  // the grid barrier.
+  auto arrive = [&]() {
+    __syncwarp();
+    if (lane == 0) {
+      __threadfence_block();
+      if (atomicAdd(&arrived, 1) == active - 1) {
+        arrived = 0;
+        __threadfence();
+        atomicAdd(g.barrier, 1u);
+      }
+    }
+  };
+  // Warp 0 polls (bounded: on expiry the launch reports and returns), the
+  // others wait for it and for each other.
+  auto waitAll = [&](unsigned count) {
+    if (warp == 0) {
+      if (lane == 0) {
+        const unsigned target = g.base + count * G + (g.wait_test ? (1u << 30) : 0u);
+        const int limit = g.wait_test ? kBarrierTestLimit : kBarrierWaitLimit;
+        int polls = 0;
+        while (static_cast<int>(loadAcquire(g.barrier) - target) < 0) {
+          if (++polls > limit) {
+            atomicExch(g.status, kStatusFlagTimeout);
+            give_up = 1;
+            break;
+          }
+        }
+      }
+      __syncwarp();
+      namedArrive(2, 32 * active);
+    } else {
+      namedSync(2, 32 * active);
+    }
+    return *static_cast<volatile int *>(&give_up) == 0;
+  };
+
+  if (warp == 0) {
+    const int L = lane & 15, half = lane >> 4, a = L >> 2, b = L & 3;
+    const Pivot16 p16(L);
+    float *M = pair.m + half * kPivotOffset;
+    int seq = 0;
+    // Sweeps the pivot of blocks (I, J) in round r from this lane's elements
+    // (a, b) of its tiles (`xrow`: the cross element belongs to row block I
+    // and column block J, else the other way round) and publishes the
+    // diagonal tiles.
+    auto sweepPivot = [&](int r, int pass, bool present, int I, int J, float dI, float dJ,
+                          float cross, bool xrow) {
+      M[8 * a + b] = dI;
+      M[8 * (4 + a) + 4 + b] = dJ;
+      M[xrow ? 8 * a + 4 + b : 8 * b + 4 + a] = cross;  // (row, column) of the upper block
+      M[xrow ? 8 * (4 + b) + a : 8 * (4 + a) + b] = cross;
+      __syncwarp();
+      if (!pivotSweep16(p16, pair, half, lane, seq) && lane == 0) atomicExch(g.status, kStatusFlagTimeout);
+      ++seq;
+      if (present) {
+        float *d = g.diag + static_cast<int64_t>(r & 1) * nb * kTileF;
+        d[I * kTileF + L] = M[64 + 8 * a + b];
+        d[J * kTileF + L] = M[64 + 8 * (4 + a) + 4 + b];
+      }
+      crosses[pass][lane] = M[64 + 8 * a + 4 + b];
+      __syncwarp();
+    };
+    for (int pass = 0; pass < passes; ++pass) {
+      // the pivots of the first round, from the matrix itself
+      const int kk = cta + G * (2 * pass + half);
+      int I = 0, J = 0;
+      float dI = 0.0f, dJ = 0.0f, cross = 0.0f;
+      if (kk < P) {
+        sweepPair(kk, g.first, nb, I, J);
+        const float *t = tilesOf(g.first);
+        dI = t[gridElement(triTile(I, I), a, b)];
+        dJ = t[gridElement(triTile(J, J), a, b)];
+        cross = t[gridElement(triTile(I, J), a, b)];
+      }
+      sweepPivot(g.first, pass, kk < P, I, J, dI, dJ, cross, true);
+    }
+    arrive();
+    for (int r = g.first; r < g.last; ++r) {
+      const float *tin = tilesOf(r);
+      float *tout = tilesOf(r + 1);
+      for (int pass = 0; pass < passes; ++pass) {
+        // Everything that can be known before the barrier: the pivot's
+        // blocks in round r + 1; the super-tile (k, l), k < l, of round r
+        // that holds the tile of those blocks; this lane's element (a, b)
+        // of that tile and columns 2b, 2b + 1 of the super-tile's rows.
+        const int kk = cta + G * (2 * pass + half);
+        const bool present = kk < P, more = present && r + 1 < g.last;
+        int I = 0, J = 0, rb0 = 0, rb1 = 0, cb0 = 1, cb1 = 1, k = 0, l = 0;
+        bool xrow = true;
+        if (more) {
+          sweepPair(kk, r + 1, nb, I, J);
+          k = sweepPairOf(I, r, nb);
+          l = sweepPairOf(J, r, nb);
+          xrow = k < l;
+          if (!xrow) {
+            const int x = k;
+            k = l;
+            l = x;
+          }
+          sweepPair(k, r, nb, rb0, rb1);
+          sweepPair(l, r, nb, cb0, cb1);
+        }
+        const int row_half = (xrow ? I : J) == rb1 ? 4 : 0;
+        const int col_half = (xrow ? J : I) == cb1 ? 4 : 0;
+        const float *qk = qslot(r) + static_cast<int64_t>(k) * kQS + row_half + a;
+        const float *ql = qslot(r) + static_cast<int64_t>(l) * kQS + col_half + b;
+        const float *d = g.diag + static_cast<int64_t>(r & 1) * nb * kTileF;
+        const int cb = b < 2 ? cb0 : cb1, c0 = 2 * (b & 1);
+        if (pass == 0 && !waitAll(r - g.first + 1)) return;
+        float t0[8], t1[8], qa[8], qb[8], dI = 0.0f, dJ = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) t0[i] = t1[i] = qa[i] = qb[i] = 0.0f;
+        if (more) {
+          dI = d[I * kTileF + L];
+          dJ = d[J * kTileF + L];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const int rb = i < 4 ? rb0 : rb1;
+            t0[i] = blockElement(tin, rb, cb, i & 3, c0);
+            t1[i] = blockElement(tin, rb, cb, i & 3, c0 + 1);
+            qa[i] = qk[8 * i];
+            qb[i] = ql[8 * i];
+          }
+        }
+        if (present) {
+          // round r's cross tile, rotated by its pivot, into the new copy;
+          // the diagonal tiles too after the last round (until then they
+          // travel from pivot to pivot through g.diag)
+          int pI, pJ;
+          sweepPair(kk, r, nb, pI, pJ);
+          tout[gridElement(triTile(pI, pJ), a, b)] = crosses[pass][lane];
+          if (r + 1 == g.last) {
+            tout[gridElement(triTile(pI, pI), a, b)] = d[pI * kTileF + L];
+            tout[gridElement(triTile(pJ, pJ), a, b)] = d[pJ * kTileF + L];
+          }
+        }
+        if (r + 1 == g.last) continue;
+        // U[a][2b], U[a][2b + 1], then T'[a][b]: the chains of superTileHalf
+        float u0 = 0.0f, u1 = 0.0f, cross = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          u0 = fmaf(qa[i], t0[i], u0);
+          u1 = fmaf(qa[i], t1[i], u1);
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const float u = __shfl_sync(0xffffffffu, j & 1 ? u1 : u0, 4 * a + (j >> 1), 16);
+          cross = fmaf(u, qb[j], cross);
+        }
+        sweepPivot(r + 1, pass, more, I, J, dI, dJ, cross, xrow);
+      }
+      arrive();
+    }
+  } else if (warp == 1) {
+    const int half = lane >> 4, L = lane & 15;
+    int seq = 0;
+    for (int r = g.first; r <= g.last; ++r) {  // Q of round r
+      if (r < g.last) {
+        for (int pass = 0; pass < passes; ++pass) {
+          const int kk = cta + G * (2 * pass + half);
+          float q[8];
+          if (!pivotQ(pair, half, lane, seq, q) && lane == 0) atomicExch(g.status, kStatusFlagTimeout);
+          ++seq;
+          if (kk < P && L < 8) {
+            float4 *out = reinterpret_cast<float4 *>(qslot(r) + static_cast<int64_t>(kk) * kQS);
+            out[2 * L] = make_float4(q[0], q[1], q[2], q[3]);
+            out[2 * L + 1] = make_float4(q[4], q[5], q[6], q[7]);
+          }
+        }
+      }
+      arrive();
+      if (r < g.last && !waitAll(r - g.first + 1)) return;
+    }
+  } else {
+    const int ut = 32 * uw + lane;
+    // this CTA's part of the update items (two lanes per super-tile)
+    const int items = 2 * ((P + 1) / 2) * (P + 1);
+    const int chunks = (items + 31) / 32;
+    const int chunk_lo = static_cast<int>(static_cast<int64_t>(chunks) * cta / G);
+    const int chunk_hi = static_cast<int>(static_cast<int64_t>(chunks) * (cta + 1) / G);
+    const int shares = rowShares(row_count, (P + 31) / 32, update_warps);
+    arrive();
+    if (kStore == kVShared) {
+      const float4 *src = reinterpret_cast<const float4 *>(g.v + static_cast<int64_t>(row0) * m);
+      float4 *dst = reinterpret_cast<float4 *>(vs);
+      for (int x = ut; x < row_count * (m / 4); x += update_threads) dst[x] = src[x];
+    }
+    for (int r = g.first; r < g.last; ++r) {
+      short2 *pr = pairs + (r & 1) * P;
+      for (int k = ut; k < P; k += update_threads) {
+        int I, J;
+        sweepPair(k, r, nb, I, J);
+        pr[k] = make_short2(static_cast<short>(I), static_cast<short>(J));
+      }
+      if (ut == 0) counters[r & 1] = 0;
+      if (!waitAll(r - g.first + 1)) return;
+      const float *qr = qslot(r);
+      const float *tin = tilesOf(r);
+      float *tout = tilesOf(r + 1);
+      // the first chunk's tiles on their way while the rotations arrive
+      if (uw < chunk_hi - chunk_lo) {
+        const int w2 = 32 * (chunk_lo + uw) + lane;
+        int k = 0, l = 0;
+        if (w2 < items && foldedBlock(w2 >> 1, P, k, l) && k != l) {
+          const short2 rb = pr[k], cb = pr[l];
+          const int C = w2 & 1 ? cb.y : cb.x;
+          const ComputedTri tri;
+          bool tr;
+          prefetchL1(tin + static_cast<int64_t>(tri(rb.x, C, tr)) * kTileF);
+          prefetchL1(tin + static_cast<int64_t>(tri(rb.y, C, tr)) * kTileF);
+        }
+      }
+      if (kStore != kNoneShared) {
+        for (int x = ut; x < P * (kQS / 4); x += update_threads) copyAsync16(qs + 4 * x, qr + 4 * x);
+        copyAsyncCommit();
+        copyAsyncWaitAll();
+        namedSync(1, update_threads);
+        qr = qs;
+      }
+      // chunks: the first by warp, the others as warps come free
+      for (int chunk = chunk_lo + uw; chunk < chunk_hi;) {
+        const int w2 = 32 * chunk + lane;
+        int k = 0, l = 0;
+        const bool valid = w2 < items && foldedBlock(w2 >> 1, P, k, l) && k != l;
+        if (!valid) k = l = 0;
+        const short2 rb = pr[k], cb = pr[l];
+        superTileHalfMem(PingPongTiles{tin, tout}, ComputedTri{},
+                         reinterpret_cast<const float4 *>(qr + static_cast<int64_t>(k) * kQS),
+                         reinterpret_cast<const float4 *>(qr + static_cast<int64_t>(l) * kQS), rb.x,
+                         rb.y, cb.x, cb.y, w2 & 1, valid);
+        if (lane == 0) chunk = chunk_lo + update_warps + atomicAdd(&counters[r & 1], 1);
+        chunk = __shfl_sync(0xffffffffu, chunk, 0);
+      }
+      arrive();
+      if (kStore == kVShared) {
+        rotateRows(vs, row_count, shares, m, P, qr, uw, update_warps, lane, [&](int k, int &I, int &J) {
+          const short2 ij = pr[k];
+          I = ij.x;
+          J = ij.y;
+        });
+      }
+    }
+    if (kStore == kVShared) {
+      namedSync(1, update_threads);
+      float4 *dst = reinterpret_cast<float4 *>(g.v + static_cast<int64_t>(row0) * m);
+      const float4 *src = reinterpret_cast<const float4 *>(vs);
+      for (int x = ut; x < row_count * (m / 4); x += update_threads) dst[x] = src[x];
+    }
+  }
+}
+
+// Applies the logged rotations of rounds [first, last) to g.rows rows of V
+// per CTA, kept in shared memory meanwhile; the rotations come straight from
+// the log (L2): a warp's 32 lanes each load one pair's and use it for every
+// row.
+__global__ void __launch_bounds__(kSweepThreads, 1) gridReplayKernel(GridArgs g) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  float4 *vs = reinterpret_cast<float4 *>(smem_raw);
+  const int row0 = blockIdx.x * g.rows, row_count = min(g.rows, g.n - row0);
+  float4 *v = reinterpret_cast<float4 *>(g.v + static_cast<int64_t>(row0) * g.m);
+  const int chunks = row_count * (g.m / 4);
+  const int shares = rowShares(row_count, (g.P + 31) / 32, kSweepWarps);
+  for (int x = threadIdx.x; x < chunks; x += kSweepThreads) vs[x] = v[x];
+  __syncthreads();
+  for (int r = g.first; r < g.last; ++r) {
+    rotateRows(reinterpret_cast<float *>(vs), row_count, shares, g.m, g.P,
+               g.q + static_cast<int64_t>(r - g.first) * g.P * kQS, threadIdx.x >> 5, kSweepWarps,
+               threadIdx.x & 31, [&](int k, int &I, int &J) { sweepPair(k, r, g.nb, I, J); });
+    __syncthreads();
+  }
+  for (int x = threadIdx.x; x < chunks; x += kSweepThreads) v[x] = vs[x];
 }
 
 // Eigenvalues (the diagonal), the rotated matrix written back in full
@@ -219,8 +601,9 @@ __global__ void gridFinishKernel(GridArgs g, float *a, float *vectors, float *ei
     const int r = r0 + idx % 32, c = c0 + idx / 32;
     if (r < g.n && c < g.n) {
       const int I = r / 4, J = c / 4;
-      const float val = I <= J ? g.tiles[tileElement(triTile(I, J), r % 4, c % 4)]
-                               : g.tiles[tileElement(triTile(J, I), c % 4, r % 4)];
+      const float *t = g.tiles[g.copy];
+      const float val = I <= J ? t[gridElement(triTile(I, J), r % 4, c % 4)]
+                               : t[gridElement(triTile(J, I), c % 4, r % 4)];
       a[r + static_cast<int64_t>(c) * g.n] = val;
       if (r == c) eigenvalues[r] = val;
     }
@@ -239,15 +622,50 @@ __global__ void gridFinishKernel(GridArgs g, float *a, float *vectors, float *ei
   }
 }
 
+size_t gridSweepSmem(int store, int P, int m, int rows) {
+  size_t bytes = static_cast<size_t>(2) * P * sizeof(short2);
+  if (store != kNoneShared) bytes += static_cast<size_t>(P) * kQS * sizeof(float);
+  if (store == kVShared) bytes += static_cast<size_t>(rows) * m * sizeof(float);
+  return bytes;
+}
+
+// Opt-in shared memory sizes, set once per device.
+int gridAttributes(msq_ctx *ctx) {
+  static std::atomic<uint64_t> done_mask{0};
+  const uint64_t bit = ctx->device >= 0 && ctx->device < 64 ? uint64_t{1} << ctx->device : 0;
+  if (bit != 0 && (done_mask.load() & bit)) return MSQ_OK;
+  const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  const int bytes = static_cast<int>(kGridSmemLimit);
+  MSQ_TRY(cudaCheck(ctx, cudaFuncSetAttribute(gridSweepKernel<kVShared>, a, bytes), "grid attr"));
+  MSQ_TRY(cudaCheck(ctx, cudaFuncSetAttribute(gridSweepKernel<kQShared>, a, bytes), "grid attr"));
+  MSQ_TRY(cudaCheck(ctx, cudaFuncSetAttribute(gridSweepKernel<kNoneShared>, a, bytes), "grid attr"));
+  MSQ_TRY(cudaCheck(ctx, cudaFuncSetAttribute(gridReplayKernel, a, bytes), "grid attr"));
+  done_mask.fetch_or(bit);
+  return MSQ_OK;
+}
+
 }  // namespace
 
 int gridJacobiSolve(msq_ctx *ctx, float *matrix, float *vectors, float *eigenvalues, int n,
                     double tolerance, int max_sweeps, int *sweeps_out, double *off_ratio_out,
                     double *norm2_out, bool keep_vectors) {
-  const int m = padded8(n), nb = m / 4, P = nb / 2;
+  const int m = padded8(n), nb = m / 4, P = nb / 2, rounds = nb - 1;
+  int sms = 0;
+  MSQ_TRY(cudaCheck(ctx, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device),
+                    "grid SM count"));
+  const int ctas = std::min(sms, kSmCount);  // all resident, one per SM
+  if (P > 2 * kMaxPasses * ctas) return setError(ctx, MSQ_ERR_UNSUPPORTED, "grid jacobi: order too large");
+  GridArgs g{};
+  g.rows = (n + ctas - 1) / ctas;
+  int store = kVShared;
+  while (store < kNoneShared && gridSweepSmem(store, P, m, g.rows) > kGridSmemLimit) ++store;
+  const size_t smem = gridSweepSmem(store, P, m, g.rows);
+  const int launch_rounds = store == kVShared ? rounds : std::min(rounds, kLogRounds);
   const int64_t tile_floats = static_cast<int64_t>(nb) * (nb + 1) / 2 * kTileF;
   const int64_t v_floats = static_cast<int64_t>(n) * m;
-  const size_t bytes = 256 + ((tile_floats + v_floats + static_cast<int64_t>(P) * kQF) * sizeof(float) + 255) / 256 * 256;
+  const int64_t q_floats = static_cast<int64_t>(store == kVShared ? 2 : launch_rounds) * P * kQS;
+  const int64_t diag_floats = static_cast<int64_t>(2) * nb * kTileF;
+  const size_t bytes = 256 + ((2 * tile_floats + v_floats + q_floats + diag_floats) * sizeof(float) + 255) / 256 * 256;
   char *work = static_cast<char *>(scratch(ctx, bytes, kScratchGrid));
   if (work == nullptr) return MSQ_ERR_CUDA;
   if (ctx->grid_host == nullptr &&
@@ -255,69 +673,44 @@ int gridJacobiSolve(msq_ctx *ctx, float *matrix, float *vectors, float *eigenval
                 "grid pinned") != MSQ_OK) {
     return MSQ_ERR_CUDA;
   }
-  GridArgs g{};
+  MSQ_TRY(gridAttributes(ctx));
   g.acc = reinterpret_cast<double *>(work);
-  g.tiles = reinterpret_cast<float *>(work + 256);
-  g.v = g.tiles + tile_floats;
+  g.barrier = reinterpret_cast<unsigned *>(work + 128);
+  g.tiles[0] = reinterpret_cast<float *>(work + 256);
+  g.tiles[1] = g.tiles[0] + tile_floats;
+  g.v = g.tiles[1] + tile_floats;
   g.q = g.v + v_floats;
+  g.diag = g.q + q_floats;
   g.v_in = keep_vectors ? vectors : nullptr;
+  g.status = ctx->d_status;
+  g.wait_test = waitTestMode() == kWaitTestFlag;
   g.n = n;
   g.m = m;
   g.nb = nb;
   g.P = P;
-  g.super_items = (2 * ((P + 1) / 2) * (P + 1) + 31) / 32 * 32;
+  g.update_warps = n <= kQuietOrder ? kSweepWarps - 2 - (kSweepWarps / 4 - 1) : kSweepWarps - 2;
   cudaStream_t s = ctx->stream;
+  MSQ_TRY(cudaCheck(ctx, cudaMemsetAsync(work, 0, 256, s), "grid reset"));
   {
     dim3 grid(std::max(1, std::min(64, (nb * kTileF + 255) / 256)), nb);
     gridLoadKernel<<<grid, 256, 0, s>>>(matrix, g);
     MSQ_TRY(launched(ctx, "jacobi grid load"));
   }
-  const int pivot_ctas = (4 * P + kGridThreads - 1) / kGridThreads;
-  const int64_t update_items = g.super_items + static_cast<int64_t>(n) * P;
-  const int update_ctas = static_cast<int>(std::min<int64_t>((update_items + kGridThreads - 1) / kGridThreads,
-                                                             static_cast<int64_t>(kSmCount) * 16));
-  // One sweep = nb - 1 rounds of (pivots, updates).  Captured into a graph
-  // once per (order, buffers); launched directly while the launch timer runs.
-  auto enqueueSweep = [&](cudaStream_t st) -> int {
-    for (int r = 0; r < nb - 1; ++r) {
-      g.round = r;
-      gridPivotKernel<<<pivot_ctas, kGridThreads, 0, st>>>(g);
-      MSQ_TRY(st == s ? launched(ctx, "jacobi grid pivots") : cudaCheck(ctx, cudaGetLastError(), "grid pivots"));
-      gridUpdateKernel<<<update_ctas, kGridThreads, 0, st>>>(g);
-      MSQ_TRY(st == s ? launched(ctx, "jacobi grid updates") : cudaCheck(ctx, cudaGetLastError(), "grid updates"));
-    }
-    return MSQ_OK;
-  };
-  const bool use_graph = !ctx->timing;
-  if (use_graph && (ctx->grid_exec == nullptr || ctx->grid_n != n || ctx->grid_work != work)) {
-    if (ctx->grid_exec != nullptr) {
-      cudaGraphExecDestroy(ctx->grid_exec);
-      ctx->grid_exec = nullptr;
-    }
-    cudaStream_t cs = auxStream(ctx, 4);
-    if (cs == s) return setError(ctx, MSQ_ERR_CUDA, "grid jacobi: no capture stream");
-    MSQ_TRY(cudaCheck(ctx, cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal), "graph capture"));
-    const int status = enqueueSweep(cs);
-    cudaGraph_t graph = nullptr;
-    const cudaError_t end = cudaStreamEndCapture(cs, &graph);
-    if (status != MSQ_OK) {
-      if (graph != nullptr) cudaGraphDestroy(graph);
-      return status;
-    }
-    MSQ_TRY(cudaCheck(ctx, end, "graph capture end"));
-    const cudaError_t inst = cudaGraphInstantiate(&ctx->grid_exec, graph, 0);
-    cudaGraphDestroy(graph);
-    MSQ_TRY(cudaCheck(ctx, inst, "graph instantiate"));
-    ctx->grid_n = n;
-    ctx->grid_work = work;
-  }
+  const void *kernel = store == kVShared   ? reinterpret_cast<const void *>(gridSweepKernel<kVShared>)
+                       : store == kQShared ? reinterpret_cast<const void *>(gridSweepKernel<kQShared>)
+                                           : reinterpret_cast<const void *>(gridSweepKernel<kNoneShared>);
+  // replay: the most rows per CTA that fit, spread evenly over whole waves
+  const int fit = std::max<int>(1, static_cast<int>(kGridSmemLimit / (m * sizeof(float))));
+  const int waves = (n + fit * ctas - 1) / (fit * ctas);
+  const int replay_rows = std::min(fit, (n + waves * ctas - 1) / (waves * ctas));
   double norm2 = 0.0, ratio = 0.0;
   int sweeps = 0;
-  const int norm_ctas = static_cast<int>(std::min<int64_t>((tile_floats + kGridThreads - 1) / kGridThreads,
-                                                           static_cast<int64_t>(kSmCount) * 8));
   for (;;) {
     MSQ_TRY(cudaCheck(ctx, cudaMemsetAsync(g.acc, 0, 2 * sizeof(double), s), "grid norm reset"));
-    gridNormKernel<<<norm_ctas, kGridThreads, 0, s>>>(g);
+    {
+      dim3 grid(std::max(1, std::min(8, nb * kTileF / (4 * kNormThreads))), nb);
+      gridNormKernel<<<grid, kNormThreads, 0, s>>>(g);
+    }
     MSQ_TRY(launched(ctx, "jacobi grid norm"));
     MSQ_TRY(cudaCheck(ctx, cudaMemcpyAsync(ctx->grid_host, g.acc, 2 * sizeof(double), cudaMemcpyDeviceToHost, s),
                       "grid norm read"));
@@ -326,12 +719,23 @@ int gridJacobiSolve(msq_ctx *ctx, float *matrix, float *vectors, float *eigenval
     if (sweeps == 0) norm2 = off2 + diag2;
     ratio = norm2 > 0.0 ? std::sqrt(off2 / norm2) : 0.0;
     if (ratio <= tolerance || sweeps >= max_sweeps) break;
-    if (use_graph) {
-      MSQ_TRY(cudaCheck(ctx, cudaGraphLaunch(ctx->grid_exec, s), "graph launch"));
-      ++ctx->graph_launches;
-      ctx->launches += 2 * static_cast<uint64_t>(nb - 1);
-    } else {
-      MSQ_TRY(enqueueSweep(s));
+    for (int r = 0; r < rounds; r += launch_rounds) {
+      g.first = r;
+      g.last = std::min(rounds, r + launch_rounds);
+      void *params[] = {&g};
+      MSQ_TRY(cudaCheck(ctx, cudaLaunchCooperativeKernel(kernel, dim3(ctas), dim3(kSweepThreads),
+                                                         params, smem, s), "grid sweep launch"));
+      MSQ_TRY(launched(ctx, "jacobi grid sweep"));
+      // one arrival per round and one after the first pivots
+      g.base += static_cast<unsigned>(ctas) * static_cast<unsigned>(g.last - g.first + 1);
+      g.copy = (g.copy + g.last - g.first) & 1;
+      if (store != kVShared) {
+        GridArgs v = g;
+        v.rows = replay_rows;
+        gridReplayKernel<<<(n + replay_rows - 1) / replay_rows, kSweepThreads,
+                           static_cast<size_t>(replay_rows) * m * sizeof(float), s>>>(v);
+        MSQ_TRY(launched(ctx, "jacobi grid replay"));
+      }
     }
     ++sweeps;
   }
