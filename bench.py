@@ -54,9 +54,9 @@ def _tiles_fit_shared(n: int) -> bool:
     """The sweep keeps the packed tiles in shared memory when they fit 227 KB."""
     m = (n + 7) // 8 * 8
     nb, p = m // 4, m // 8
-    # reduction scratch, tile table, counters, done flags, three 16-bit round
-    # tables; two rotation buffers (68-float stride); the packed tiles
-    head = (32 * 8 + (nb + 1 + 2 + p) * 4 + 3 * (3 * p + 2 * nb) * 2 + 15) // 16 * 16
+    # reduction scratch, counters, done flags, four round tables; two rotation
+    # buffers (68-float stride); the packed tiles
+    head = (32 * 8 + (2 + p) * 4 + 4 * 8 * p + 15) // 16 * 16
     return head + 2 * p * 68 * 4 + nb * (nb + 1) // 2 * 16 * 4 <= 227 * 1024 - 256
 
 

@@ -28,6 +28,15 @@
 //    that ends the sweeps is accumulated in FP64 — sweeps stop once
 //    off(A) <= tol * ||A||_F instead of after a fixed 8;
 //  * launches are size-bucketed (threads per CTA grow with n), largest first.
+//
+// What bounds the sweep: the L1 data pipe beyond n = 320 (71% of its peak at
+// n = 512: tiles a lane at a time, rotations from shared memory), the pivots'
+// latency below.  Rolled pivots in tournament positions, 32-byte accesses to
+// global tiles, computed tile indexes and byte tables (two reads per
+// super-tile) took a sweep of 152 matrices from 4.45 to 3.75 ms at n = 512,
+// 2.49 to 2.17 at 400, 1.10 to 0.98 at 300, 304 of n = 256 from 1.47 to 1.27,
+// and one of n = 32 alone from 73 to 51 us.  Eight lanes per pivot are
+// faster below n = 64 only (n = 256: 1.50 ms).
 #include "msq_internal.cuh"
 #include "msq_jacobi_device.cuh"
 #include "msq_jacobi_grid.cuh"
@@ -167,36 +176,42 @@ __device__ __forceinline__ SplitTiles tileMem(std::false_type, float *s, float *
   return SplitTiles{s, g, split};
 }
 
-// Entries (16-bit) of one round table of the sweep kernel: pairs (I, J),
-// rotate flags, per block its pair and its partner (-1: not rotated).
-__host__ __device__ constexpr int roundTableShorts(int nb) { return 3 * (nb / 2) + 2 * nb; }
-
 // One round's table in shared memory and its P 8x8 rotations (kQS floats
-// apart).
+// apart).  Blocks and pairs fit bytes (one CTA solves n <= 1024: 256 blocks).
+// item(k): the pair's blocks I (bits 0-7) and J (8-15) and the pairs whose
+// super-tile with k holds a cross tile of the next round's pivots (16-23,
+// 24-31; 255: none), so a super-tile costs two table reads; slot(b): the
+// pair of block b; partner(b): its partner, itself when not rotated.
 struct RoundTable {
-  short *t;
+  uint32_t *items;
   float *q;
   int P;
-  __device__ short &pi(int k) const { return t[k]; }
-  __device__ short &pj(int k) const { return t[P + k]; }
-  __device__ short &on(int k) const { return t[2 * P + k]; }
-  __device__ short &slot(int b) const { return t[3 * P + b]; }
-  __device__ short &partner(int b) const { return t[5 * P + b]; }
+  __device__ uint32_t &item(int k) const { return items[k]; }
+  __device__ int pi(int k) const { return items[k] & 255; }
+  __device__ int pj(int k) const { return (items[k] >> 8) & 255; }
+  __device__ uint8_t &slot(int b) const { return reinterpret_cast<uint8_t *>(items + P)[b]; }
+  __device__ uint8_t &partner(int b) const { return reinterpret_cast<uint8_t *>(items + P)[2 * P + b]; }
+  __device__ bool on(int k) const {
+    const int i = pi(k);
+    return partner(i) != i;
+  }
 };
+constexpr int kNoPair = 255;
+__host__ __device__ constexpr int roundTableBytes(int P) { return 8 * P; }
+constexpr int kRoundTables = 4;  // rounds r .. r + 3
 
 // Polls of a done flag before the sweep kernel reports kStatusFlagTimeout
 // (kFlagWaitTestLimit under the failure-injection mode).
 constexpr int kFlagWaitLimit = 1 << 22;
 constexpr int kFlagWaitTestLimit = 64;
 
-// Shared memory of the sweep kernel: reduction scratch; the tile table, two
-// work counters, P done flags and three round tables; the rotations of two
-// rounds; then the packed tiles (with_tiles).
+// Shared memory of the sweep kernel: reduction scratch; two work counters, P
+// done flags and the round tables; the rotations of two rounds; then the
+// packed tiles (with_tiles).
 __host__ __device__ constexpr size_t sweepSmemLayout(int n, bool with_tiles, size_t *q_off,
                                                     size_t *tile_off) {
   const int m = padded8(n), nb = m / 4, P = nb / 2;
-  size_t bytes = 32 * sizeof(double) + (nb + 1 + 2 + P) * sizeof(int) +
-                 3 * roundTableShorts(nb) * sizeof(short);
+  size_t bytes = 32 * sizeof(double) + (2 + P) * sizeof(int) + kRoundTables * roundTableBytes(P);
   bytes = (bytes + 15) & ~static_cast<size_t>(15);
   *q_off = bytes;
   bytes += 2 * static_cast<size_t>(P) * kQS * sizeof(float);
@@ -225,10 +240,9 @@ jacobiSweepKernel(JacobiArgs args) {
   size_t q_off, tile_off;
   sweepSmemLayout(n, kSmem, &q_off, &tile_off);
   double *red = reinterpret_cast<double *>(smem_raw);
-  int *tri = reinterpret_cast<int *>(red + 32);
-  int *counters = tri + nb + 1;
+  int *counters = reinterpret_cast<int *>(red + 32);
   int *flags = counters + 2;
-  short *tables = reinterpret_cast<short *>(flags + P);
+  uint32_t *tables = reinterpret_cast<uint32_t *>(flags + P);
   float *qs = reinterpret_cast<float *>(smem_raw + q_off);
   float *gtiles = args.tiles + args.t_offset[mi];
   float *stiles = reinterpret_cast<float *>(smem_raw + tile_off);
@@ -242,9 +256,6 @@ jacobiSweepKernel(JacobiArgs args) {
   const int2 *sched = sched_at >= 0 ? args.sched + sched_at : nullptr;
   const int rounds = sched != nullptr ? twoLevelRounds(nb) : nb - 1;
 
-  for (int k = threadIdx.x; k <= nb; k += blockDim.x) tri[k] = k * (k + 1) / 2;
-  __syncthreads();
-
   if (args.first) {
     // Symmetrised load, as working_from_symmetric_f32 and the averaged a_pq
     // of jacobi_rotations_f32 do (metal_mixed_sqrt.metal:1349-1350, 1922).
@@ -256,7 +267,7 @@ jacobiSweepKernel(JacobiArgs args) {
         if (gi < n && gj < n) {
           v = 0.5f * (full[gi + static_cast<int64_t>(gj) * n] + full[gj + static_cast<int64_t>(gi) * n]);
         }
-        tileAt(tiles, tileElement(tri[J] + I, e / 4, e % 4)) = v;
+        tileAt(tiles, tileElement(triTile(I, J), e / 4, e % 4)) = v;
       }
     }
   } else if (split > 0) {
@@ -280,7 +291,7 @@ jacobiSweepKernel(JacobiArgs args) {
   for (int J = 0; J < nb; ++J) {
     for (int idx = threadIdx.x; idx < (J + 1) * kTileF; idx += blockDim.x) {
       const int I = idx / kTileF, e = idx % kTileF;
-      const double v = tileAt(tiles, tileElement(tri[J] + I, e / 4, e % 4));
+      const double v = tileAt(tiles, tileElement(triTile(I, J), e / 4, e % 4));
       if (I < J) off2 += 2.0 * v * v;
       else if (e / 4 == e % 4) diag2 += v * v;
       else off2 += v * v;
@@ -297,14 +308,14 @@ jacobiSweepKernel(JacobiArgs args) {
     // later, :1436-1444); full symmetric write-back of the matrix.
     float *eig = args.eigenvalues + args.eig_offset[mi];
     for (int k = threadIdx.x; k < n; k += blockDim.x) {
-      eig[k] = tileAt(tiles, tileElement(tri[k / 4] + k / 4, k % 4, k % 4));
+      eig[k] = tileAt(tiles, tileElement(triTile(k / 4, k / 4), k % 4, k % 4));
     }
     float *out = args.a + args.a_offset[mi];
     for (int c = 0; c < n; ++c) {
       for (int r = threadIdx.x; r < n; r += blockDim.x) {
         const int I = r / 4, J = c / 4;
-        const float v = I <= J ? tileAt(tiles, tileElement(tri[J] + I, r % 4, c % 4))
-                               : tileAt(tiles, tileElement(tri[I] + J, c % 4, r % 4));
+        const float v = I <= J ? tileAt(tiles, tileElement(triTile(I, J), r % 4, c % 4))
+                               : tileAt(tiles, tileElement(triTile(J, I), c % 4, r % 4));
         out[r + static_cast<int64_t>(c) * n] = v;
       }
     }
@@ -331,9 +342,9 @@ jacobiSweepKernel(JacobiArgs args) {
   float *log = args.log + args.log_offset[mi];
   const int items = ((P + 1) / 2) * (P + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
-  // round r's table is buffer r % 3, its rotations buffer r & 1
+  // round r's table is buffer r mod 4, its rotations buffer r & 1
   auto table = [&](int r) {
-    return RoundTable{tables + (r % 3) * roundTableShorts(nb), qs + (r & 1) * P * kQS, P};
+    return RoundTable{tables + (r % kRoundTables) * (roundTableBytes(P) / 4), qs + (r & 1) * P * kQS, P};
   };
 
   // Pairs of round r into its table (threads [first, blockDim) take part).
@@ -343,13 +354,23 @@ jacobiSweepKernel(JacobiArgs args) {
       int I, J;
       bool on;
       roundPair(sched, k, r, nb, I, J, on);
-      t.pi(k) = static_cast<short>(I);
-      t.pj(k) = static_cast<short>(J);
-      t.on(k) = static_cast<short>(on);
-      t.slot(I) = static_cast<short>(k);
-      t.slot(J) = static_cast<short>(k);
-      t.partner(I) = static_cast<short>(on ? J : -1);
-      t.partner(J) = static_cast<short>(on ? I : -1);
+      t.item(k) = static_cast<uint32_t>(I | (J << 8)) | 0xffff0000u;
+      t.slot(I) = static_cast<uint8_t>(k);
+      t.slot(J) = static_cast<uint8_t>(k);
+      t.partner(I) = static_cast<uint8_t>(on ? J : I);
+      t.partner(J) = static_cast<uint8_t>(on ? I : J);
+    }
+  };
+  // The pairs that share a critical super-tile with each pair of round r, from
+  // the tables of r and r + 1 (none in the last round).
+  auto stageCritical = [&](int r, int first) {
+    if (r + 1 >= rounds) return;
+    const RoundTable t = table(r), nxt = table(r + 1);
+    for (int k = threadIdx.x - first; k < P; k += blockDim.x - first) {
+      const int x = t.pi(k), y = t.pj(k);
+      const int px = nxt.partner(x), py = nxt.partner(y);
+      const uint32_t cx = px != x ? t.slot(px) : kNoPair, cy = py != y ? t.slot(py) : kNoPair;
+      t.item(k) = static_cast<uint32_t>(x | (y << 8)) | (cx << 16) | (cy << 24);
     }
   };
 
@@ -365,16 +386,16 @@ jacobiSweepKernel(JacobiArgs args) {
     int tII = 0, tIJ = 0, tJJ = 0;
     if (active) {
       const int I = t.pi(k), J = t.pj(k);
-      tII = tileIndex(tri, I, I);
-      tIJ = tileIndex(tri, I, J);
-      tJJ = tileIndex(tri, J, J);
+      tII = triTile(I, I);
+      tIJ = triTile(I, J);
+      tJJ = triTile(J, J);
       // lane t starts with rows t (block I) and 7 - t (block J row 3 - t;
       // its left half is the mirror of tile (I, J))
       const float4 *sII = reinterpret_cast<const float4 *>(tiles.base(tII));
       const float4 *sIJ = reinterpret_cast<const float4 *>(tiles.base(tIJ));
       const float4 *sJJ = reinterpret_cast<const float4 *>(tiles.base(tJJ));
       const int jr = 3 - t4;
-      const float4 v0 = sII[t4 ^ (tII & 3)], v1 = sIJ[t4 ^ (tIJ & 3)], v2 = sJJ[jr ^ (tJJ & 3)];
+      const float4 v0 = sII[t4 ^ tileSwizzle(tII)], v1 = sIJ[t4 ^ tileSwizzle(tIJ)], v2 = sJJ[jr ^ tileSwizzle(tJJ)];
       ra[0] = v0.x; ra[1] = v0.y; ra[2] = v0.z; ra[3] = v0.w;
       ra[4] = v1.x; ra[5] = v1.y; ra[6] = v1.z; ra[7] = v1.w;
 #pragma unroll
@@ -386,14 +407,14 @@ jacobiSweepKernel(JacobiArgs args) {
     }
     pivotSweep(ra, rb, t.q + (active ? k : 0) * kQS, t4, active);
     if (active) {
-      // rows t (tiles (I, I), (I, J)) and 4 + t (tile (J, J)); the lower
+      // rows t (tiles (I, I), (I, J)) and 7 - t (tile (J, J)); the lower
       // left block is the mirror of tile (I, J) and is not stored
       float4 *sII = reinterpret_cast<float4 *>(tiles.base(tII));
       float4 *sIJ = reinterpret_cast<float4 *>(tiles.base(tIJ));
       float4 *sJJ = reinterpret_cast<float4 *>(tiles.base(tJJ));
-      sII[t4 ^ (tII & 3)] = make_float4(ra[0], ra[1], ra[2], ra[3]);
-      sIJ[t4 ^ (tIJ & 3)] = make_float4(ra[4], ra[5], ra[6], ra[7]);
-      sJJ[t4 ^ (tJJ & 3)] = make_float4(rb[4], rb[5], rb[6], rb[7]);
+      sII[t4 ^ tileSwizzle(tII)] = make_float4(ra[0], ra[1], ra[2], ra[3]);
+      sIJ[t4 ^ tileSwizzle(tIJ)] = make_float4(ra[4], ra[5], ra[6], ra[7]);
+      sJJ[(3 - t4) ^ tileSwizzle(tJJ)] = make_float4(rb[4], rb[5], rb[6], rb[7]);
     } else if (present) {
       // identity pair: Q = I (lane t writes rows 2t and 2t + 1)
       float4 *q4 = reinterpret_cast<float4 *>(t.q + k * kQS);
@@ -406,12 +427,13 @@ jacobiSweepKernel(JacobiArgs args) {
     }
   };
 
-  // Off-pivot super-tiles: T' = Q_k^T T Q_l for pairs k < l of a round, two
-  // lanes per super-tile (warp-uniform: the pair shuffle has all lanes).
-  auto superTile = [&](const RoundTable &t, int k, int l, int h, bool valid) {
-    superTileHalfMem(tiles, SharedTri{tri}, reinterpret_cast<const float4 *>(t.q + k * kQS),
-                     reinterpret_cast<const float4 *>(t.q + l * kQS), t.pi(k), t.pj(k), t.pi(l),
-                     t.pj(l), h, valid);
+  // Off-pivot super-tiles: T' = Q_k^T T Q_l for pairs k < l of a round (table
+  // words ik, il), two lanes per super-tile (warp-uniform: the pair shuffle
+  // has all lanes).
+  auto superTile = [&](const RoundTable &t, int k, int l, uint32_t ik, uint32_t il, int h, bool valid) {
+    superTileHalfMem(tiles, ComputedTri{}, reinterpret_cast<const float4 *>(t.q + k * kQS),
+                     reinterpret_cast<const float4 *>(t.q + l * kQS), ik & 255, (ik >> 8) & 255,
+                     il & 255, (il >> 8) & 255, h, valid);
   };
   // The super-tile (k, l) of round `cur` holding the tile (x, y) that pivot
   // kk of round `nxt` reads (none when cur paired x and y: its pivot wrote
@@ -435,14 +457,9 @@ jacobiSweepKernel(JacobiArgs args) {
     }
     return true;
   };
-  // Whether super-tile (k, l) of cur is one of those.
-  auto isCritical = [&](const RoundTable &cur, const RoundTable &nxt, int k, int l) {
-    const int p1 = nxt.partner(cur.pi(k)), p2 = nxt.partner(cur.pj(k));
-    return (p1 >= 0 && cur.slot(p1) == l) || (p2 >= 0 && cur.slot(p2) == l);
-  };
   // The other super-tiles of cur (all of them without a next round), taken
   // by warps 32 lanes (16 super-tiles) at a time from a shared counter.
-  auto otherItems = [&](const RoundTable &cur, const RoundTable &nxt, bool more, int *counter) {
+  auto otherItems = [&](const RoundTable &cur, int *counter) {
     for (;;) {
       int base = 0;
       if (lane == 0) base = atomicAdd(counter, 32);
@@ -451,9 +468,10 @@ jacobiSweepKernel(JacobiArgs args) {
       const int w2 = base + lane;
       int k = 0, l = 0;
       bool valid = w2 < 2 * items && foldedBlock(w2 >> 1, P, k, l) && k != l;
-      if (valid && more && isCritical(cur, nxt, k, l)) valid = false;
       if (!valid) k = l = 0;
-      superTile(cur, k, l, w2 & 1, valid);
+      const uint32_t ik = cur.item(k), il = cur.item(l);
+      valid = valid && static_cast<int>((ik >> 16) & 255) != l && static_cast<int>(ik >> 24) != l;
+      superTile(cur, k, l, ik, il, w2 & 1, valid);
     }
   };
 
@@ -465,11 +483,11 @@ jacobiSweepKernel(JacobiArgs args) {
   // the plain round order (pivots, then all super-tiles, round by round).
   const int pw = min(warps, (P + 7) / 8);
   const int stage_first = pw < warps ? 32 * pw : 0;  // threads that stage tables and log
-  stagePairs(0, 0);
-  if (rounds > 1) stagePairs(1, 0);
+  for (int r = 0; r < kRoundTables - 1 && r < rounds; ++r) stagePairs(r, 0);
   if (threadIdx.x == 0) counters[0] = counters[1] = 0;
   for (int k = threadIdx.x; k < P; k += blockDim.x) flags[k] = 0;
   __syncthreads();
+  stageCritical(0, 0);
   for (int base = 8 * warp; base < P; base += 8 * warps) pivot(table(0), base + (lane >> 2));
   __syncthreads();
   for (int round = 0; round < rounds; ++round) {
@@ -484,7 +502,7 @@ jacobiSweepKernel(JacobiArgs args) {
         int k = 0, l = 0, owner = kk;
         const bool own = (lane & 2) == 0 && criticalItem(cur, nxt, kk, k, l, owner) && owner == kk;
         if (!own) k = l = 0;
-        superTile(cur, k, l, lane & 1, own);
+        superTile(cur, k, l, cur.item(k), cur.item(l), lane & 1, own);
         __syncwarp();
         if (own && (lane & 3) == 0) {
           __threadfence_block();
@@ -514,7 +532,8 @@ jacobiSweepKernel(JacobiArgs args) {
       }
     }
     if (static_cast<int>(threadIdx.x) >= stage_first) {
-      if (round + 2 < rounds) stagePairs(round + 2, stage_first);
+      if (round + 3 < rounds) stagePairs(round + 3, stage_first);
+      stageCritical(round + 1, stage_first);
       if (threadIdx.x == stage_first) counters[(round + 1) & 1] = 0;
       // this round's rotations, logged for the V replay (coalesced copy)
       const float4 *src = reinterpret_cast<const float4 *>(cur.q);
@@ -523,7 +542,7 @@ jacobiSweepKernel(JacobiArgs args) {
         dst[x] = src[(x >> 4) * (kQS / 4) + (x & 15)];
       }
     }
-    otherItems(cur, nxt, more, counters + (round & 1));
+    otherItems(cur, counters + (round & 1));
     __syncthreads();
   }
   if (split > 0) {

@@ -138,12 +138,15 @@ __device__ double blockReduceSum(double v, double *red) {
 // Packed tile (I, J), I <= J, of a matrix's tile array: tile index
 // tri[J] + I, 16 floats.  A 4x4 tile spans half the 32 shared-memory banks,
 // so without care the rows of all tiles would fall on two bank groups; row
-// i of tile t is stored at physical row i ^ (t & 3), which spreads the
-// float4 rows a warp touches over all eight 4-bank groups.
+// i of tile t is stored at physical row i ^ tileSwizzle(t), which with the
+// tile's half spreads the float4 rows a warp touches.  Rows move in pairs
+// (0, 1), (2, 3), so a 32-byte access still finds two adjacent rows in
+// order.
+__device__ __forceinline__ int tileSwizzle(int t) { return t & 2; }
 __device__ __forceinline__ int tileIndex(const int *tri, int I, int J) { return tri[J] + I; }
 
 __device__ __forceinline__ int64_t tileElement(int t, int i, int j) {
-  return static_cast<int64_t>(t) * kTileF + (((i ^ (t & 3)) << 2) | j);
+  return static_cast<int64_t>(t) * kTileF + (((i ^ tileSwizzle(t)) << 2) | j);
 }
 
 // Loads block (R, C) of A (4x4, row-major in t) from packed tile ti, which
@@ -160,7 +163,7 @@ __device__ __forceinline__ void loadTile(const float *tiles, int ti, bool transp
   const float4 *src = reinterpret_cast<const float4 *>(tiles + static_cast<int64_t>(ti) * kTileF);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const float4 v = src[i ^ (ti & 3)];
+    const float4 v = src[i ^ tileSwizzle(ti)];
     if (!transposed) {
       t[i][0] = v.x; t[i][1] = v.y; t[i][2] = v.z; t[i][3] = v.w;
     } else {
@@ -173,7 +176,7 @@ __device__ __forceinline__ void storeTile(float *tiles, int ti, bool transposed,
   float4 *dst = reinterpret_cast<float4 *>(tiles + static_cast<int64_t>(ti) * kTileF);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    dst[i ^ (ti & 3)] = transposed ? make_float4(t[0][i], t[1][i], t[2][i], t[3][i])
+    dst[i ^ tileSwizzle(ti)] = transposed ? make_float4(t[0][i], t[1][i], t[2][i], t[3][i])
                                    : make_float4(t[i][0], t[i][1], t[i][2], t[i][3]);
   }
 }
@@ -201,49 +204,45 @@ __device__ __forceinline__ int triTile(int I, int J) { return J * (J + 1) / 2 + 
 // a' = c a - s b, column b' = s a + c b; p <- J^T p J, p_ab = p_ba = 0;
 // Q <- Q J.
 //
-// A quad of lanes sweeps one pivot.  In group g lane t owns the two rows
-// (a_t, b_t) of its pair.  The four angles of a group depend only on the
-// pair's own 2x2 block, which no other rotation of the group touches, so
-// they are computed at once and shared with shuffles; each lane then
-// updates its two rows.  Element (x, y) of a row pair t and column pair j is
-// touched by the row rotation of t and the column rotation of j, applied in
-// the order of the pairs in the group (the sequential order); the diagonal
-// block (j = t) takes the column rotation first.  Every operation is an
-// explicitly rounded one (no FMA contraction, no approximate reciprocal
-// square root), so the sweep equals, bit for bit, the sequential sweep of
-// the C restatement compiled with -ffp-contract=off.
+// The pivot is kept in tournament positions: in every group pair t holds
+// positions (t, 7 - t), and between groups position 0 stays and positions
+// 1..7 rotate by one, so the seven groups are one loop (unrolled in index
+// order they are 40 KB of instructions, fetched anew every round beside the
+// super-tile code).  Positions order a pair by tournament slot, the angle by
+// index: where they differ the angle is taken of the swapped pair and s
+// negated (x - y and x + (-y) round alike).
+//
+// A quad of lanes sweeps one pivot.  Lane t owns the two rows of pair t.  The
+// four angles of a group depend only on the pair's own 2x2 block, which no
+// other rotation of the group touches, so they are computed at once and
+// shared with shuffles; each lane then updates its two rows.  Element (x, y)
+// of a row pair t and column pair j is touched by the row rotation of t and
+// the column rotation of j, applied in the order of the pairs in the group
+// (the sequential order); the diagonal block (j = t) takes the column
+// rotation first.  Every operation is an explicitly rounded one (no FMA
+// contraction, no approximate reciprocal square root), so the sweep equals,
+// bit for bit, the sequential sweep of the C restatement compiled with
+// -ffp-contract=off.
 
-// Pairs of group g packed as 4 x (a: 3 bits, b: 3 bits), a < b.
-__host__ __device__ constexpr uint32_t groupWord(int g) {
-  constexpr int pairs[8][8] = {{0, 7, 1, 6, 2, 5, 3, 4}, {0, 6, 5, 7, 1, 4, 2, 3},
-                               {0, 5, 4, 6, 3, 7, 1, 2}, {0, 4, 3, 5, 2, 6, 1, 7},
-                               {0, 3, 2, 4, 1, 5, 6, 7}, {0, 2, 1, 3, 4, 7, 5, 6},
-                               {0, 1, 2, 7, 3, 6, 4, 5},
-                               // layout used to store the pivot: rows (t, 4 + t)
-                               {0, 4, 1, 5, 2, 6, 3, 7}};
+// The item at position pos of group g, and (bit g) whether the item at
+// position t of group g has the larger index of its pair.
+__host__ __device__ constexpr int tournamentItem(int pos, int g) {
+  return pos == 0 ? 0 : 1 + (pos - 1 - g + 7) % 7;
+}
+__host__ __device__ constexpr uint32_t flipWord(int t) {
   uint32_t w = 0;
-  for (int t = 0; t < 4; ++t)
-    w |= static_cast<uint32_t>(pairs[g][2 * t] | (pairs[g][2 * t + 1] << 3)) << (6 * t);
+  for (int g = 0; g < 7; ++g)
+    w |= (tournamentItem(t, g) > tournamentItem(7 - t, g) ? 1u : 0u) << g;
   return w;
 }
-
-// For each row r: owner lane (2 bits) and slot (1 bit, 1 = second row of
-// the pair) in group g, packed 3 bits per row.
-__host__ __device__ constexpr uint32_t ownerWord(int g) {
-  uint32_t w = 0;
-  for (int t = 0; t < 4; ++t) {
-    const uint32_t a = (groupWord(g) >> (6 * t)) & 7, b = (groupWord(g) >> (6 * t + 3)) & 7;
-    w |= static_cast<uint32_t>(t) << (3 * a);
-    w |= static_cast<uint32_t>(t | 4) << (3 * b);
-  }
-  return w;
+__device__ __forceinline__ uint32_t laneFlips(int t) {
+  return t == 0 ? flipWord(0) : t == 1 ? flipWord(1) : t == 2 ? flipWord(2) : flipWord(3);
 }
 
-__device__ __forceinline__ float pick8(const float (&r)[8], int i) {
-  float v = r[0];
-#pragma unroll
-  for (int k = 1; k < 8; ++k) v = i == k ? r[k] : v;
-  return v;
+// r[t] of four values
+__device__ __forceinline__ float pick4(float a, float b, float c, float d, int t) {
+  const float lo = t & 1 ? b : a, hi = t & 1 ? d : c;
+  return t & 2 ? hi : lo;
 }
 
 // Rotation angle of one pair (explicitly rounded; renormalised so that
@@ -278,93 +277,81 @@ __device__ __forceinline__ void rot2(float &x, float &y, float c, float s, bool 
   y = on ? ny : y;
 }
 
-// One group of 4 rotations on the quad.  ra / rb: this lane's rows a_t / b_t
-// (all 8 columns); q: rows 2t and 2t + 1 of the pivot's Q, which every lane
-// updates for all four rotations of the group (Q <- Q J touches columns a, b
-// of each row; the group's pairs are disjoint, so their order is free).
-template <int G>
-__device__ __forceinline__ void pivotGroup(float (&ra)[8], float (&rb)[8], float (&q)[2][8], int t) {
-  constexpr uint32_t W = groupWord(G);
-  const int a = (W >> (6 * t)) & 7, b = (W >> (6 * t + 3)) & 7;
-  float c, s;
-  const bool on = jacobiAngle(pick8(ra, a), pick8(rb, b), pick8(ra, b), c, s);
-  float cj[4], sj[4];
-  bool onj[4];
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    cj[j] = __shfl_sync(0xffffffffu, c, j, 4);
-    sj[j] = __shfl_sync(0xffffffffu, s, j, 4);
-    onj[j] = __shfl_sync(0xffffffffu, static_cast<int>(on), j, 4) != 0;
-  }
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const int A = (W >> (6 * j)) & 7, B = (W >> (6 * j + 3)) & 7;
-    // 2x2 block X: rows (a_t, b_t), columns (A, B) of pair j.  If j comes
-    // first in the group (or j = t) the column rotation precedes the row
-    // rotation: Y = (C_t(R_j(X^T)))^T, else Y = C_j(R_t(X)), where R mixes
-    // rows and C mixes columns with the same two-term arithmetic.
-    const bool swap = j <= t;
-    float x00 = ra[A], x01 = swap ? rb[A] : ra[B];
-    float x10 = swap ? ra[B] : rb[A], x11 = rb[B];
-    const float c1 = swap ? cj[j] : c, s1 = swap ? sj[j] : s;
-    const bool on1 = swap ? onj[j] : on;
-    const float c2 = swap ? c : cj[j], s2 = swap ? s : sj[j];
-    const bool on2 = swap ? on : onj[j];
-    rot2(x00, x10, c1, s1, on1);  // rows of X'
-    rot2(x01, x11, c1, s1, on1);
-    rot2(x00, x01, c2, s2, on2);  // columns of X'
-    rot2(x10, x11, c2, s2, on2);
-    const bool diag = j == t && on;
-    ra[A] = x00;
-    rb[B] = x11;
-    const float y01 = swap ? x10 : x01, y10 = swap ? x01 : x10;
-    ra[B] = diag ? 0.0f : y01;
-    rb[A] = diag ? 0.0f : y10;
-    rot2(q[0][A], q[0][B], cj[j], sj[j], onj[j]);
-    rot2(q[1][A], q[1][B], cj[j], sj[j], onj[j]);
-  }
-}
-
-// Moves the rows from the ownership of group G to that of group G + 1.
-template <int G>
-__device__ __forceinline__ void pivotExchange(float (&ra)[8], float (&rb)[8], int t) {
-  constexpr uint32_t O = ownerWord(G), W1 = groupWord(G + 1);
-  const int a1 = (W1 >> (6 * t)) & 7, b1 = (W1 >> (6 * t + 3)) & 7;
-  const int src_a = (O >> (3 * a1)) & 3, slot_a = (O >> (3 * a1 + 2)) & 1;
-  const int src_b = (O >> (3 * b1)) & 3, slot_b = (O >> (3 * b1 + 2)) & 1;
-  float na[8], nb[8];
-#pragma unroll
-  for (int y = 0; y < 8; ++y) {
-    const float u0 = __shfl_sync(0xffffffffu, ra[y], src_a, 4);
-    const float u1 = __shfl_sync(0xffffffffu, rb[y], src_a, 4);
-    const float v0 = __shfl_sync(0xffffffffu, ra[y], src_b, 4);
-    const float v1 = __shfl_sync(0xffffffffu, rb[y], src_b, 4);
-    na[y] = slot_a ? u1 : u0;
-    nb[y] = slot_b ? v1 : v0;
-  }
-#pragma unroll
-  for (int y = 0; y < 8; ++y) {
-    ra[y] = na[y];
-    rb[y] = nb[y];
-  }
-}
-
-// Full pivot sweep on the quad; on return ra / rb hold rows (t, 4 + t) and,
-// if active, qrow holds Q row-major (lane t writes rows 2t and 2t + 1).
+// Full pivot sweep on the quad: lane t holds rows t (ra) and 7 - t (rb), all
+// 8 columns, before and after; if active, qrow receives Q row-major (lane t
+// keeps and writes its rows 2t and 2t + 1).
 __device__ __forceinline__ void pivotSweep(float (&ra)[8], float (&rb)[8], float *qrow, int t,
                                            bool active) {
+  const uint32_t flips = laneFlips(t);
   float q[2][8];
 #pragma unroll
   for (int x = 0; x < 2; ++x)
 #pragma unroll
     for (int y = 0; y < 8; ++y) q[x][y] = y == 2 * t + x ? 1.0f : 0.0f;
-  pivotGroup<0>(ra, rb, q, t); pivotExchange<0>(ra, rb, t);
-  pivotGroup<1>(ra, rb, q, t); pivotExchange<1>(ra, rb, t);
-  pivotGroup<2>(ra, rb, q, t); pivotExchange<2>(ra, rb, t);
-  pivotGroup<3>(ra, rb, q, t); pivotExchange<3>(ra, rb, t);
-  pivotGroup<4>(ra, rb, q, t); pivotExchange<4>(ra, rb, t);
-  pivotGroup<5>(ra, rb, q, t); pivotExchange<5>(ra, rb, t);
-  pivotGroup<6>(ra, rb, q, t); pivotExchange<6>(ra, rb, t);
+#pragma unroll 1
+  for (int g = 0; g < 7; ++g) {
+    const bool flip = (flips >> g) & 1;
+    const float p0 = pick4(ra[0], ra[1], ra[2], ra[3], t);  // (t, t)
+    const float p1 = pick4(rb[7], rb[6], rb[5], rb[4], t);  // (7 - t, 7 - t)
+    float c, s;
+    const bool on = jacobiAngle(flip ? p1 : p0, flip ? p0 : p1,
+                                pick4(ra[7], ra[6], ra[5], ra[4], t), c, s);
+    s = flip ? -s : s;
+    const float mark = on ? c : 2.0f;  // no rotation: 2 in the place of the cosine
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float cj = __shfl_sync(0xffffffffu, mark, j, 4);
+      const float sj = __shfl_sync(0xffffffffu, s, j, 4);
+      const bool onj = cj != 2.0f;
+      // 2x2 block X: rows (t, 7 - t), columns (j, 7 - j).  If j comes first
+      // in the group (or j = t) the column rotation precedes the row
+      // rotation: Y = (C_t(R_j(X^T)))^T, else Y = C_j(R_t(X)), where R mixes
+      // rows and C mixes columns with the same two-term arithmetic.
+      const bool swap = j <= t;
+      float x00 = ra[j], x01 = swap ? rb[j] : ra[7 - j];
+      float x10 = swap ? ra[7 - j] : rb[j], x11 = rb[7 - j];
+      const float c1 = swap ? cj : c, s1 = swap ? sj : s;
+      const bool on1 = swap ? onj : on;
+      const float c2 = swap ? c : cj, s2 = swap ? s : sj;
+      const bool on2 = swap ? on : onj;
+      rot2(x00, x10, c1, s1, on1);  // rows of X'
+      rot2(x01, x11, c1, s1, on1);
+      rot2(x00, x01, c2, s2, on2);  // columns of X'
+      rot2(x10, x11, c2, s2, on2);
+      const bool diag = j == t && on;
+      ra[j] = x00;
+      rb[7 - j] = x11;
+      const float y01 = swap ? x10 : x01, y10 = swap ? x01 : x10;
+      ra[7 - j] = diag ? 0.0f : y01;
+      rb[j] = diag ? 0.0f : y10;
+      rot2(q[0][j], q[0][7 - j], cj, sj, onj);
+      rot2(q[1][j], q[1][7 - j], cj, sj, onj);
+    }
+    // Positions 1..7 move on: the rows between the lanes (position t takes
+    // position t - 1, position 1 takes 7, position 7 - t takes 6 - t), the
+    // columns in registers.
+    float na[8], nb[8];
+#pragma unroll
+    for (int y = 0; y < 8; ++y) {
+      const float up = __shfl_up_sync(0xffffffffu, t == 0 ? rb[y] : ra[y], 1, 4);
+      const float down = __shfl_down_sync(0xffffffffu, rb[y], 1, 4);
+      na[y] = t == 0 ? ra[y] : up;
+      nb[y] = t == 3 ? ra[y] : down;
+    }
+#pragma unroll
+    for (int y = 0; y < 8; ++y) {
+      const int from = y == 0 ? 0 : (y == 1 ? 7 : y - 1);
+      ra[y] = na[from];
+      rb[y] = nb[from];
+    }
+#pragma unroll
+    for (int x = 0; x < 2; ++x) {
+      const float last = q[x][7];
+#pragma unroll
+      for (int y = 7; y > 1; --y) q[x][y] = q[x][y - 1];
+      q[x][1] = last;
+    }
+  }
   if (active) {
     float4 *q4 = reinterpret_cast<float4 *>(qrow);
     q4[4 * t + 0] = make_float4(q[0][0], q[0][1], q[0][2], q[0][3]);
@@ -400,10 +387,7 @@ __host__ __device__ __forceinline__ int sweepPairOf(int block, int round, int m)
 // grid kernels: a round's critical path is one pivot): the same rotations
 // and the same bits.
 //
-// The pivot is kept in tournament positions: in every group pair t holds
-// positions (t, 7 - t), and between groups position 0 stays and positions
-// 1..7 rotate by one, so every group has the same data movement.  Lane
-// (t, j) holds the 2x2 block of pairs lo = min(t, j), hi = max(t, j): rows
+// In tournament positions as well.  Lane (t, j) holds the 2x2 block of pairs lo = min(t, j), hi = max(t, j): rows
 // (lo, 7 - lo), columns (hi, 7 - hi), row rotation first, then the column
 // rotation, which is the sequential order of the upper triangle (the lower
 // one is its transpose bit for bit: each of its elements sees the same two
@@ -443,17 +427,6 @@ __device__ __forceinline__ bool waitFlag(const int *p, int target) {
   return false;
 }
 
-__host__ __device__ constexpr int tournamentItem(int pos, int g) {
-  return pos == 0 ? 0 : 1 + (pos - 1 - g + 7) % 7;
-}
-// bit g: the item at position t of group g has the larger index of its pair
-__host__ __device__ constexpr uint32_t flipWord(int t) {
-  uint32_t w = 0;
-  for (int g = 0; g < 7; ++g)
-    w |= (tournamentItem(t, g) > tournamentItem(7 - t, g) ? 1u : 0u) << g;
-  return w;
-}
-
 struct Pivot16 {
   int w[4], r[4];    // shared-memory element of x00, x01, x10, x11: written, read
   uint32_t flips;
@@ -464,7 +437,7 @@ struct Pivot16 {
     lo = t < j ? t : j;
     hi = t < j ? j : t;
     diag = t == j;
-    flips = t == 0 ? flipWord(0) : t == 1 ? flipWord(1) : t == 2 ? flipWord(2) : flipWord(3);
+    flips = laneFlips(t);
     const int rr[2] = {lo, 7 - lo}, cc[2] = {hi, 7 - hi};
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
@@ -549,7 +522,7 @@ __device__ __forceinline__ bool pivotQ(PivotPair &pair, int half, int lane, int 
   return ok;
 }
 
-// Tile lookup through the shared table tri[J] = J (J + 1) / 2 ...
+// Tile lookup through a shared table tri[J] = J (J + 1) / 2 ...
 struct SharedTri {
   const int *tri;
   __device__ __forceinline__ int operator()(int R, int C, bool &transposed) const {
@@ -557,7 +530,8 @@ struct SharedTri {
     return transposed ? tri[R] + C : tri[C] + R;
   }
 };
-// ... or computed (grid kernels).
+// ... or computed (two integer instructions against a shared read with
+// conflicts).
 struct ComputedTri {
   __device__ __forceinline__ int operator()(int R, int C, bool &transposed) const {
     transposed = R > C;
@@ -594,7 +568,7 @@ __device__ __forceinline__ void loadTileAt(const float *p, int ti, bool transpos
   const float4 *src = reinterpret_cast<const float4 *>(p);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const float4 v = src[i ^ (ti & 3)];
+    const float4 v = src[i ^ tileSwizzle(ti)];
     if (!transposed) {
       t[i][0] = v.x; t[i][1] = v.y; t[i][2] = v.z; t[i][3] = v.w;
     } else {
@@ -607,22 +581,9 @@ __device__ __forceinline__ void storeTileAt(float *p, int ti, bool transposed, c
   float4 *dst = reinterpret_cast<float4 *>(p);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    dst[i ^ (ti & 3)] = transposed ? make_float4(t[0][i], t[1][i], t[2][i], t[3][i])
+    dst[i ^ tileSwizzle(ti)] = transposed ? make_float4(t[0][i], t[1][i], t[2][i], t[3][i])
                                    : make_float4(t[i][0], t[i][1], t[i][2], t[i][3]);
   }
-}
-
-__device__ __forceinline__ void FlatTiles::load(int ti, bool transposed, float (&b)[4][4]) const {
-  loadTileAt(base(ti), ti, transposed, b);
-}
-__device__ __forceinline__ void FlatTiles::store(int ti, bool transposed, const float (&b)[4][4]) const {
-  storeTileAt(base(ti), ti, transposed, b);
-}
-__device__ __forceinline__ void SplitTiles::load(int ti, bool transposed, float (&b)[4][4]) const {
-  loadTileAt(base(ti), ti, transposed, b);
-}
-__device__ __forceinline__ void SplitTiles::store(int ti, bool transposed, const float (&b)[4][4]) const {
-  storeTileAt(base(ti), ti, transposed, b);
 }
 
 // 32-byte global accesses (32-byte aligned addresses).  Lanes of a warp that
@@ -640,6 +601,55 @@ __device__ __forceinline__ void storeGlobal32(float *p, const float (&v)[8]) {
   asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(v[0]),
                "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
                : "memory");
+}
+
+__device__ __forceinline__ void FlatTiles::load(int ti, bool transposed, float (&b)[4][4]) const {
+  loadTileAt(base(ti), ti, transposed, b);
+}
+__device__ __forceinline__ void FlatTiles::store(int ti, bool transposed, const float (&b)[4][4]) const {
+  storeTileAt(base(ti), ti, transposed, b);
+}
+// The global part in 32-byte accesses.
+__device__ __forceinline__ void SplitTiles::load(int ti, bool transposed, float (&b)[4][4]) const {
+  if (ti < split) {
+    loadTileAt(s + ti * kTileF, ti, transposed, b);
+    return;
+  }
+  const float *p = g + static_cast<int64_t>(ti) * kTileF;
+  const int sw = tileSwizzle(ti);
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    float v[8];
+    loadGlobal32(p + 4 * ((2 * h) ^ sw), v);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      if (transposed) {
+        b[e][2 * h] = v[e];
+        b[e][2 * h + 1] = v[4 + e];
+      } else {
+        b[2 * h][e] = v[e];
+        b[2 * h + 1][e] = v[4 + e];
+      }
+    }
+  }
+}
+__device__ __forceinline__ void SplitTiles::store(int ti, bool transposed, const float (&b)[4][4]) const {
+  if (ti < split) {
+    storeTileAt(s + ti * kTileF, ti, transposed, b);
+    return;
+  }
+  float *p = g + static_cast<int64_t>(ti) * kTileF;
+  const int sw = tileSwizzle(ti);
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    float v[8];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      v[e] = transposed ? b[e][2 * h] : b[2 * h][e];
+      v[4 + e] = transposed ? b[e][2 * h + 1] : b[2 * h + 1][e];
+    }
+    storeGlobal32(p + 4 * ((2 * h) ^ sw), v);
+  }
 }
 
 // Super-tile update T' = Q_k^T T Q_l on two lanes (h = 0, 1 of an adjacent

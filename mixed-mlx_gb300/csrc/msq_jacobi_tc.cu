@@ -652,7 +652,7 @@ __global__ void __launch_bounds__(kInnerThreads, 4) tlInnerKernel(InnerArgs args
         const float4 *sIJ = reinterpret_cast<const float4 *>(tiles + tIJ * kTileF);
         const float4 *sJJ = reinterpret_cast<const float4 *>(tiles + tJJ * kTileF);
         const int jr = 3 - t4;
-        const float4 v0 = sII[t4 ^ (tII & 3)], v1 = sIJ[t4 ^ (tIJ & 3)], v2 = sJJ[jr ^ (tJJ & 3)];
+        const float4 v0 = sII[t4 ^ tileSwizzle(tII)], v1 = sIJ[t4 ^ tileSwizzle(tIJ)], v2 = sJJ[jr ^ tileSwizzle(tJJ)];
         ra[0] = v0.x; ra[1] = v0.y; ra[2] = v0.z; ra[3] = v0.w;
         ra[4] = v1.x; ra[5] = v1.y; ra[6] = v1.z; ra[7] = v1.w;
 #pragma unroll
@@ -667,9 +667,9 @@ __global__ void __launch_bounds__(kInnerThreads, 4) tlInnerKernel(InnerArgs args
         float4 *sII = reinterpret_cast<float4 *>(tiles + tII * kTileF);
         float4 *sIJ = reinterpret_cast<float4 *>(tiles + tIJ * kTileF);
         float4 *sJJ = reinterpret_cast<float4 *>(tiles + tJJ * kTileF);
-        sII[t4 ^ (tII & 3)] = make_float4(ra[0], ra[1], ra[2], ra[3]);
-        sIJ[t4 ^ (tIJ & 3)] = make_float4(ra[4], ra[5], ra[6], ra[7]);
-        sJJ[t4 ^ (tJJ & 3)] = make_float4(rb[4], rb[5], rb[6], rb[7]);
+        sII[t4 ^ tileSwizzle(tII)] = make_float4(ra[0], ra[1], ra[2], ra[3]);
+        sIJ[t4 ^ tileSwizzle(tIJ)] = make_float4(ra[4], ra[5], ra[6], ra[7]);
+        sJJ[(3 - t4) ^ tileSwizzle(tJJ)] = make_float4(rb[4], rb[5], rb[6], rb[7]);
       } else {
         float4 *q4 = reinterpret_cast<float4 *>(qs + k * kQS);
 #pragma unroll
