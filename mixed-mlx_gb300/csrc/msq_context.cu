@@ -208,6 +208,30 @@ const DeviceBatch *prepareBatch(msq_ctx *ctx, const int32_t *n,
   return b;
 }
 
+bool findWork(const DeviceBatch *b, int key, const int4 **work, int *items) {
+  for (const WorkList &e : b->work_cache) {
+    if (e.tile != key) continue;
+    *work = e.work;
+    *items = e.items;
+    return true;
+  }
+  return false;
+}
+
+int keepWork(msq_ctx *ctx, const DeviceBatch *b, int key, const std::vector<int4> &list,
+             const int4 **work, int *items) {
+  int4 *dev = nullptr;
+  if (!list.empty()) {
+    MSQ_TRY(cudaCheck(ctx, cudaMalloc(&dev, list.size() * sizeof(int4)), "work list alloc"));
+    MSQ_TRY(cudaCheck(ctx, cudaMemcpy(dev, list.data(), list.size() * sizeof(int4),
+                                      cudaMemcpyHostToDevice), "work list upload"));
+  }
+  const_cast<DeviceBatch *>(b)->work_cache.push_back({key, dev, static_cast<int>(list.size())});
+  *work = dev;
+  *items = static_cast<int>(list.size());
+  return MSQ_OK;
+}
+
 void *scratch(msq_ctx *ctx, size_t bytes, int slot) {
   if (bytes <= ctx->scratch_bytes[slot]) return ctx->scratch[slot];
   if (ctx->scratch[slot] != nullptr) {

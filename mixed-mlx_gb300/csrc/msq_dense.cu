@@ -17,6 +17,7 @@
 #include "msq_dense.cuh"
 #include "msq_internal.cuh"
 #include "msq_f32x2.cuh"
+#include "msq_residual.cuh"
 
 #include <algorithm>
 #include <vector>
@@ -467,20 +468,14 @@ namespace {
 // work-list key of the GEMM's lists (the other lists use +-tile).
 constexpr int kGemmLargeOrder = 1000;
 constexpr int kGemmWorkBase = 1 << 16;
+constexpr int kResidualWork = 1 << 18;
 
 // One work list per (batch layout, key), cached on the batch: the tiles of
 // every matrix whose order `in` accepts.
 template <class In>
 int tileWork(msq_ctx *ctx, const DeviceBatch *b, int size, bool upper, int key, const int4 **work,
              int *items, In in) {
-  auto &cache = const_cast<DeviceBatch *>(b)->work_cache;
-  for (auto &e : cache) {
-    if (e.tile == key) {
-      *work = e.work;
-      *items = e.items;
-      return MSQ_OK;
-    }
-  }
+  if (findWork(b, key, work, items)) return MSQ_OK;
   std::vector<int4> list;
   // largest matrices first: their long K loops start early
   std::vector<int> ids;
@@ -493,16 +488,7 @@ int tileWork(msq_ctx *ctx, const DeviceBatch *b, int size, bool upper, int key, 
     for (int ti = 0; ti < t; ++ti)
       for (int tj = upper ? ti : 0; tj < t; ++tj) list.push_back(make_int4(mi, ti, tj, 0));
   }
-  int4 *dev = nullptr;
-  if (!list.empty()) {
-    MSQ_TRY(cudaCheck(ctx, cudaMalloc(&dev, list.size() * sizeof(int4)), "work list alloc"));
-    MSQ_TRY(cudaCheck(ctx, cudaMemcpy(dev, list.data(), list.size() * sizeof(int4),
-                                      cudaMemcpyHostToDevice), "work list upload"));
-  }
-  cache.push_back({key, dev, static_cast<int>(list.size())});
-  *work = dev;
-  *items = static_cast<int>(list.size());
-  return MSQ_OK;
+  return keepWork(ctx, b, key, list, work, items);
 }
 
 }  // namespace
@@ -593,7 +579,9 @@ int gemmTN(msq_ctx *ctx, const DeviceBatch *b, const float *a, const float *bm, 
 int residualFF(msq_ctx *ctx, const DeviceBatch *b, const float *a, const float *x_hi,
                const float *x_lo, float *r, double *norms, const float *a_lo) {
   ResidualArgs args{};
-  MSQ_TRY(gemmWork(ctx, b, -kTile, &args.work, &args.items));  // upper tiles
+  // upper tiles of the small matrices; the others on the tensor cores
+  MSQ_TRY(tileWork(ctx, b, kTile, true, kResidualWork, &args.work, &args.items,
+                   [](int n) { return !residualOnTensorCores(n); }));
   args.a = a;
   args.a_lo = a_lo;
   args.x_hi = x_hi;
@@ -604,6 +592,8 @@ int residualFF(msq_ctx *ctx, const DeviceBatch *b, const float *a, const float *
   args.n = b->n;
   MSQ_TRY(cudaCheck(ctx, cudaMemsetAsync(norms, 0, 2 * b->count * sizeof(double), ctx->stream),
                     "norm reset"));
+  MSQ_TRY(residualMma(ctx, b, a, x_hi, x_lo, r, norms, a_lo));
+  if (args.items == 0) return MSQ_OK;
   const unsigned grid = std::min<unsigned>(args.items, kSmCount * 8);
   residualFFKernel<false><<<grid, kThreads, 0, ctx->stream>>>(args);
   return launched(ctx, "residual float-float");

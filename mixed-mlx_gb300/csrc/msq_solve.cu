@@ -396,21 +396,14 @@ int enqueuePass(msq_ctx *ctx, const float *a_user, const int32_t *n_user,
     MSQ_TRY(reconstructFromFactor(ctx, sb, g.plan.format, pb->F, pb->Xh));
     // Corrections use the FP32 stable basis V, as the reference's fp32_frozen
     // stage does (src/metal_solver.cpp:304-325).  The plain FP32 plan runs its
-    // GEMMs and residuals on the CUDA cores in FP32 / float-float; low-bit
-    // plans run the correction GEMMs on the tensor cores (split BF16, FP32
-    // accumulation) and the residual of the low-bit X0 too.  A tensor-core
-    // residual carries the FP32 accumulation error of an n-long sum (about
-    // sqrt(n) 2^-24 of ||A||): negligible against the quantization residual of
-    // X0, not against the residual after a correction, which a further
-    // correction could not push below it.  So every residual after the first
-    // correction, and the one that decides acceptance, are float-float.
-    const bool low_bit = g.plan.format != MSQ_PLAN_FP32;
-    const int gemm_format = low_bit ? MSQ_FMT_BF16 : MSQ_FMT_FP32;
-    auto residual = [&](bool accurate) {
-      return low_bit && !accurate ? residualTc(ctx, sb, pb->A, pb->Xh, pb->Xl, pb->R, norms)
-                                  : residualFF(ctx, sb, pb->A, pb->Xh, pb->Xl, pb->R, norms);
+    // GEMMs on the CUDA cores in FP32; low-bit plans run the correction GEMMs
+    // on the tensor cores (split BF16, FP32 accumulation).  Every residual is
+    // float-float.
+    const int gemm_format = g.plan.format != MSQ_PLAN_FP32 ? MSQ_FMT_BF16 : MSQ_FMT_FP32;
+    auto residual = [&]() {
+      return residualFF(ctx, sb, pb->A, pb->Xh, pb->Xl, pb->R, norms);
     };
-    MSQ_TRY(residual(g.plan.sweeps == 0));
+    MSQ_TRY(residual());
     MSQ_TRY(cudaCheck(ctx, cudaMemcpyAsync(rep.initial, norms, 2 * c * sizeof(double),
                                            cudaMemcpyDeviceToHost, ctx->stream), "norms read"));
     for (int s = 0; s < g.plan.sweeps; ++s) {
@@ -418,7 +411,7 @@ int enqueuePass(msq_ctx *ctx, const float *a_user, const int32_t *n_user,
       // sweeps only the float-float residual runs
       MSQ_TRY(sylvesterSweep(ctx, sb, gemm_format, pb->V, lam, pb->R, pb->Xh, pb->Xl, pb->F,
                              pb->W1, s > 0));
-      MSQ_TRY(residual(true));
+      MSQ_TRY(residual());
     }
     MSQ_TRY(cudaCheck(ctx, cudaMemcpyAsync(rep.final, norms, 2 * c * sizeof(double),
                                            cudaMemcpyDeviceToHost, ctx->stream), "norms read"));

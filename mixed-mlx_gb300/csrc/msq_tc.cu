@@ -64,12 +64,11 @@ constexpr int kScaleTileBytes = 2 * kScaleAtomBytes;
 // columns (A atoms at +0, +4, B atoms at +8, +12).
 constexpr uint32_t kTmemColsMx = 512;
 constexpr uint32_t kScaleCol0 = 256;
-constexpr int kMaxSegments = 6;
+constexpr int kMaxSegments = 3;
 enum Epilogue : int {
   kEpiStore = 0,     // X = acc
   kEpiRowScale = 1,  // X_ij = acc * r_i * r_j (FP8 row-scaled factor)
   kEpiInverseH = 2,  // X_ij = acc / (s_i + s_j), s = sqrt(lambda)
-  kEpiResidual = 3,  // X = A - acc, FP64 ||X||^2 and ||A||^2 per matrix
 };
 
 // Bounded wait: false (and the status word set) if the phase never completes.
@@ -122,8 +121,6 @@ struct TcArgs {
   const int64_t *eig_offset;
   const float *row_scale;  // kEpiRowScale: per matrix row scales at eig_offset
   const float *eigenvalues;// kEpiInverseH: lambda, s = sqrt(max(lambda, 0))
-  const float *a_in;       // kEpiResidual: R = A - acc
-  double *norms;           // kEpiResidual: ||R||^2, ||A||^2 per matrix
   float *x;
   int *status;
   int wait_test;           // 1: the producer first waits on a barrier nothing arrives at
@@ -300,8 +297,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcGemmKernel(TcArgs args) {
       const float *lam = kEpi == kEpiInverseH ? args.eigenvalues + args.eig_offset[mi] : nullptr;
       const float si = kEpi == kEpiInverseH && i < n ? sqrtf(fmaxf(lam[i], 0.0f)) : 0.0f;
 
-      const float *A = kEpi == kEpiResidual ? args.a_in + args.x_offset[mi] : nullptr;
-      double rn = 0.0, an = 0.0;
 #pragma unroll 1
       for (int c = 0; c < 4; ++c) {
         float v[32];
@@ -329,27 +324,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcGemmKernel(TcArgs args) {
                 const float d = si + sj[q];
                 val = d > 0.0f ? val / d : 0.0f;  // both roots 0: no correction
               }
-              if (kEpi == kEpiResidual) {
-                const float a = A[at];
-                val = a - val;
-                rn += static_cast<double>(val) * val;
-                an += static_cast<double>(a) * a;
-              }
               X[at] = val;
             }
           }
-        }
-      }
-      if (kEpi == kEpiResidual) {
-        // epilogue warps 0-3 reduce, then one atomic per warp
-#pragma unroll
-        for (int s = 16; s > 0; s >>= 1) {
-          rn += __shfl_xor_sync(0xffffffffu, rn, s);
-          an += __shfl_xor_sync(0xffffffffu, an, s);
-        }
-        if (lane == 0) {
-          atomicAdd(&args.norms[2 * mi], rn);
-          atomicAdd(&args.norms[2 * mi + 1], an);
         }
       }
       asm volatile("tcgen05.fence::before_thread_sync;");
@@ -560,34 +537,29 @@ __global__ void __launch_bounds__(128) packMxKernel(MxPackArgs args) {
   }
 }
 
-// Split-BF16 packing of an FP32 (or float-float hi + lo) matrix M, n x n
-// column-major, as the K-major MMA operand: operand row i is column i of M
-// (kTranspose false) or row i of M (kTranspose true).  Piece p is the BF16
-// rounding of what pieces 0..p-1 left over, so three pieces carry the FP32
-// mantissa and the products p_a p_b (exact in FP32) sum to M_a M_b.
+// Split-BF16 packing of an FP32 matrix M, n x n column-major, as the K-major
+// MMA operand: operand row i is column i of M (kTranspose false) or row i of
+// M (kTranspose true).  The second piece is the BF16 rounding of what the
+// first left over.
 struct SplitArgs {
   const int4 *work;
   int items;
-  const float *hi;
-  const float *lo;  // may be null
+  const float *m;
   const int64_t *offset;
   const int64_t *tile_base;
   const int32_t *n;
-  int pieces;
-  uint8_t *out[3];
+  uint8_t *out[2];
 };
 
-template <bool kTranspose, bool kLo>
+template <bool kTranspose>
 __global__ void __launch_bounds__(128) packSplitKernel(SplitArgs args) {
   // kTranspose false reads operand row i from column i of M: the tile's 128
   // columns x 64 rows are staged in shared memory with coalesced loads (a
   // warp reads 32 consecutive elements of one column, eight columns in
   // flight), then each thread reads its row there (stride 65: no bank
-  // conflicts).  kLo: M is float-float (hi + lo).
+  // conflicts).
   constexpr int kLd = 65;
-  constexpr int kStage = kTranspose ? 1 : kTileRows * kLd;
-  __shared__ float stage_hi[kStage];
-  __shared__ float stage_lo[kLo ? kStage : 1];
+  __shared__ float stage[kTranspose ? 1 : kTileRows * kLd];
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   for (int item = blockIdx.x; item < args.items; item += gridDim.x) {
     const int4 w = args.work[item];
@@ -595,62 +567,48 @@ __global__ void __launch_bounds__(128) packSplitKernel(SplitArgs args) {
     const int r = threadIdx.x;
     const int i = w.y * kTileRows + r;
     const int k0 = w.z * 64;
-    const float *H = args.hi + args.offset[mi];
-    const float *L = kLo ? args.lo + args.offset[mi] : nullptr;
+    const float *M = args.m + args.offset[mi];
     const int64_t tile = (args.tile_base[mi] + static_cast<int64_t>(w.y) * w.w + w.z) * kTileBytes;
     if (!kTranspose) {
       __syncthreads();  // the previous item's rows have been read
 #pragma unroll 1
       for (int c0 = 8 * warp; c0 < kTileRows; c0 += 32) {
-        float xh[8][2], xl[8][2];
+        float x[8][2];
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
           const int col = w.y * kTileRows + c0 + q;
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             const int k = k0 + lane + 32 * h;
-            const bool in = col < n && k < n;
-            const int64_t at = k + static_cast<int64_t>(col) * n;
-            xh[q][h] = in ? H[at] : 0.0f;
-            xl[q][h] = kLo && in ? L[at] : 0.0f;
+            x[q][h] = col < n && k < n ? M[k + static_cast<int64_t>(col) * n] : 0.0f;
           }
         }
 #pragma unroll
         for (int q = 0; q < 8; ++q)
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            stage_hi[(c0 + q) * kLd + lane + 32 * h] = xh[q][h];
-            if (kLo) stage_lo[(c0 + q) * kLd + lane + 32 * h] = xl[q][h];
-          }
+          for (int h = 0; h < 2; ++h) stage[(c0 + q) * kLd + lane + 32 * h] = x[q][h];
       }
       __syncthreads();
     }
 #pragma unroll 1
     for (int c = 0; c < 8; ++c) {
-      uint32_t word[3][4] = {};
+      uint32_t word[2][4] = {};
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
         const int k = k0 + c * 8 + e;
-        float x = 0.0f, xl = 0.0f;
+        float x = 0.0f;
         if (kTranspose) {
-          if (i < n && k < n) {
-            const int64_t at = i + static_cast<int64_t>(k) * n;
-            x = H[at];
-            xl = kLo ? L[at] : 0.0f;
-          }
+          if (i < n && k < n) x = M[i + static_cast<int64_t>(k) * n];
         } else {
-          x = stage_hi[r * kLd + c * 8 + e];
-          xl = kLo ? stage_lo[r * kLd + c * 8 + e] : 0.0f;
+          x = stage[r * kLd + c * 8 + e];
         }
         const uint32_t h0 = encodeBf16(x);
-        const float rem = (x - decodeBf16(static_cast<uint16_t>(h0))) + xl;
-        const uint32_t h1 = encodeBf16(rem);
-        const uint32_t h2 = encodeBf16(rem - decodeBf16(static_cast<uint16_t>(h1)));
+        const uint32_t h1 = encodeBf16(x - decodeBf16(static_cast<uint16_t>(h0)));
         word[0][e / 2] |= h0 << (16 * (e % 2));
         word[1][e / 2] |= h1 << (16 * (e % 2));
-        word[2][e / 2] |= h2 << (16 * (e % 2));
       }
-      for (int p = 0; p < args.pieces; ++p) {
+#pragma unroll
+      for (int p = 0; p < 2; ++p) {
         *reinterpret_cast<uint4 *>(args.out[p] + tile + swizzle128(r, c)) =
             make_uint4(word[p][0], word[p][1], word[p][2], word[p][3]);
       }
@@ -796,7 +754,6 @@ int tcAttributes(msq_ctx *ctx) {
   MSQ_TRY(cudaCheck(ctx, cudaFuncSetAttribute(tcGemmKernel<kOpBf16, kEpiStore>, a, bytes), "tc attr"));
   MSQ_TRY(cudaCheck(ctx, cudaFuncSetAttribute(tcGemmKernel<kOpFp8, kEpiRowScale>, a, bytes), "tc attr"));
   MSQ_TRY(cudaCheck(ctx, cudaFuncSetAttribute(tcGemmKernel<kOpBf16, kEpiInverseH>, a, bytes), "tc attr"));
-  MSQ_TRY(cudaCheck(ctx, cudaFuncSetAttribute(tcGemmKernel<kOpBf16, kEpiResidual>, a, bytes), "tc attr"));
   const int mx_bytes = static_cast<int>(tcSmemBytes(kOpMxf4));
   MSQ_TRY(cudaCheck(ctx, cudaFuncSetAttribute(tcGemmKernel<kOpMxf4, kEpiStore>, a, mx_bytes), "tc attr"));
   MSQ_TRY(cudaCheck(ctx, cudaFuncSetAttribute(tcGemmKernel<kOpMxf8, kEpiStore>, a, mx_bytes), "tc attr"));
@@ -808,8 +765,7 @@ int tcAttributes(msq_ctx *ctx) {
 // X = sum_s A_s B_s^T per matrix with the given epilogue.
 int launchTcGemm(msq_ctx *ctx, const DeviceBatch *b, TcPlan *p, int epilogue, int segments,
                  const uint8_t *const *a_tiles, const uint8_t *const *b_tiles,
-                 const float *row_scale, const float *eigenvalues, const float *a_in,
-                 double *norms, float *x, const char *what,
+                 const float *row_scale, const float *eigenvalues, float *x, const char *what,
                  const uint8_t *scale_tiles = nullptr) {
   MSQ_TRY(tcAttributes(ctx));
   TcArgs args{};
@@ -828,8 +784,6 @@ int launchTcGemm(msq_ctx *ctx, const DeviceBatch *b, TcPlan *p, int epilogue, in
   args.eig_offset = b->eig_offset;
   args.row_scale = row_scale;
   args.eigenvalues = eigenvalues;
-  args.a_in = a_in;
-  args.norms = norms;
   args.x = x;
   args.status = ctx->d_status;
   args.wait_test = waitTestMode() == kWaitTestMbarrier;
@@ -853,9 +807,6 @@ int launchTcGemm(msq_ctx *ctx, const DeviceBatch *b, TcPlan *p, int epilogue, in
     case kEpiInverseH:
       tcGemmKernel<kOpBf16, kEpiInverseH><<<grid, kTcThreads, smem, ctx->stream>>>(args);
       break;
-    case kEpiResidual:
-      tcGemmKernel<kOpBf16, kEpiResidual><<<grid, kTcThreads, smem, ctx->stream>>>(args);
-      break;
     default:
       tcGemmKernel<kOpBf16, kEpiStore><<<grid, kTcThreads, smem, ctx->stream>>>(args);
       break;
@@ -867,7 +818,7 @@ int runTcGemm(msq_ctx *ctx, const DeviceBatch *b, TcPlan *p, const uint8_t *tile
               const float *row_scale, float *x) {
   const uint8_t *t[1] = {tiles};
   return launchTcGemm(ctx, b, p, p->kind == kOpFp8 ? kEpiRowScale : kEpiStore, 1, t, t,
-                      row_scale, nullptr, nullptr, nullptr, x, "tcgen05 reconstruction");
+                      row_scale, nullptr, x, "tcgen05 reconstruction");
 }
 
 template <int kSource>
@@ -893,7 +844,7 @@ int launchPackMx(msq_ctx *ctx, const DeviceBatch *b, TcPlan *p, const float *f,
 int runMxGemm(msq_ctx *ctx, const DeviceBatch *b, TcPlan *p, const uint8_t *tiles,
               const uint8_t *scale_tiles, float *x) {
   const uint8_t *t[1] = {tiles};
-  return launchTcGemm(ctx, b, p, kEpiStore, 1, t, t, nullptr, nullptr, nullptr, nullptr, x,
+  return launchTcGemm(ctx, b, p, kEpiStore, 1, t, t, nullptr, nullptr, x,
                       "tcgen05 reconstruction", scale_tiles);
 }
 
@@ -929,26 +880,20 @@ int launchPack(msq_ctx *ctx, const DeviceBatch *b, TcPlan *p, const float *f,
 
 namespace {
 
-int packSplit(msq_ctx *ctx, const DeviceBatch *b, TcPlan *p, const float *hi, const float *lo,
-              bool transpose, int pieces, uint8_t *const *out) {
+int packSplit(msq_ctx *ctx, const DeviceBatch *b, TcPlan *p, const float *m, bool transpose,
+              uint8_t *const *out) {
   SplitArgs args{};
   args.work = p->pack_work;
   args.items = p->pack_items;
-  args.hi = hi;
-  args.lo = lo;
+  args.m = m;
   args.offset = b->offset;
   args.tile_base = p->tile_base;
   args.n = b->n;
-  args.pieces = pieces;
-  for (int q = 0; q < pieces; ++q) args.out[q] = out[q];
+  args.out[0] = out[0];
+  args.out[1] = out[1];
   const unsigned grid = std::min(p->pack_items, kSmCount * 16);
-  if (transpose) {
-    if (lo) packSplitKernel<true, true><<<grid, 128, 0, ctx->stream>>>(args);
-    else packSplitKernel<true, false><<<grid, 128, 0, ctx->stream>>>(args);
-  } else {
-    if (lo) packSplitKernel<false, true><<<grid, 128, 0, ctx->stream>>>(args);
-    else packSplitKernel<false, false><<<grid, 128, 0, ctx->stream>>>(args);
-  }
+  if (transpose) packSplitKernel<true><<<grid, 128, 0, ctx->stream>>>(args);
+  else packSplitKernel<false><<<grid, 128, 0, ctx->stream>>>(args);
   return launched(ctx, "pack split-BF16");
 }
 
@@ -968,8 +913,7 @@ int gemmSplit2(msq_ctx *ctx, const DeviceBatch *b, TcPlan *p, uint8_t *const *a,
                int epilogue, const float *eigenvalues, float *out, const char *what) {
   const uint8_t *sa[3] = {a[0], a[0], a[1]};
   const uint8_t *sb[3] = {bb[0], bb[1], bb[0]};
-  return launchTcGemm(ctx, b, p, epilogue, 3, sa, sb, nullptr, eigenvalues, nullptr, nullptr, out,
-                      what);
+  return launchTcGemm(ctx, b, p, epilogue, 3, sa, sb, nullptr, eigenvalues, out, what);
 }
 
 }  // namespace
@@ -987,39 +931,19 @@ int sylvesterTc(msq_ctx *ctx, const DeviceBatch *b, const float *v, const float 
   if (splitBuffers(ctx, p, buf) == nullptr) return MSQ_ERR_CUDA;
   uint8_t *vn[2] = {buf[0], buf[1]}, *vt[2] = {buf[2], buf[3]}, *op[2] = {buf[4], buf[5]};
   if (!basis_packed) {
-    MSQ_TRY(packSplit(ctx, b, p, v, nullptr, false, 2, vn));  // rows = columns of V
-    MSQ_TRY(packSplit(ctx, b, p, v, nullptr, true, 2, vt));   // rows = rows of V
+    MSQ_TRY(packSplit(ctx, b, p, v, false, vn));  // rows = columns of V
+    MSQ_TRY(packSplit(ctx, b, p, v, true, vt));   // rows = rows of V
   }
-  MSQ_TRY(packSplit(ctx, b, p, r, nullptr, false, 2, op));  // R (symmetric)
+  MSQ_TRY(packSplit(ctx, b, p, r, false, op));  // R (symmetric)
   MSQ_TRY(gemmSplit2(ctx, b, p, op, vn, kEpiStore, nullptr, ws0, "tc sylvester G=RV"));
-  MSQ_TRY(packSplit(ctx, b, p, ws0, nullptr, false, 2, op));
+  MSQ_TRY(packSplit(ctx, b, p, ws0, false, op));
   MSQ_TRY(gemmSplit2(ctx, b, p, vn, op, kEpiInverseH, lam, ws1, "tc sylvester C=V'G/H"));
-  MSQ_TRY(packSplit(ctx, b, p, ws1, nullptr, false, 2, op));
+  MSQ_TRY(packSplit(ctx, b, p, ws1, false, op));
   MSQ_TRY(gemmSplit2(ctx, b, p, op, vt, kEpiStore, nullptr, ws0, "tc sylvester Zt=CV'"));
-  MSQ_TRY(packSplit(ctx, b, p, ws0, nullptr, false, 2, op));
+  MSQ_TRY(packSplit(ctx, b, p, ws0, false, op));
   MSQ_TRY(gemmSplit2(ctx, b, p, op, vt, kEpiStore, nullptr, ws1, "tc sylvester E=ZV'"));
   *correction = ws1;
   return MSQ_OK;
-}
-
-// R = A - X X on the tensor cores: X = x0 + x1 + x2 (BF16 pieces of the
-// float-float X), X X ~ x0x0 + x0x1 + x1x0 + x0x2 + x2x0 + x1x1 accumulated
-// in FP32 in one TMEM accumulator; the epilogue forms R and the FP64 norms.
-// About FP32 accuracy: used between sweeps; the accepting residual is the
-// float-float one.
-int residualTc(msq_ctx *ctx, const DeviceBatch *b, const float *a, const float *x_hi,
-               const float *x_lo, float *r, double *norms) {
-  TcPlan *p = tcPlan(ctx, b, kOpBf16);
-  if (p == nullptr) return MSQ_ERR_CUDA;
-  uint8_t *buf[kBuffers];
-  if (splitBuffers(ctx, p, buf) == nullptr) return MSQ_ERR_CUDA;
-  MSQ_TRY(packSplit(ctx, b, p, x_hi, x_lo, false, 3, buf));
-  const uint8_t *sa[6] = {buf[0], buf[0], buf[1], buf[0], buf[2], buf[1]};
-  const uint8_t *sb[6] = {buf[0], buf[1], buf[0], buf[2], buf[0], buf[1]};
-  MSQ_TRY(cudaCheck(ctx, cudaMemsetAsync(norms, 0, 2 * b->count * sizeof(double), ctx->stream),
-                    "norm reset"));
-  return launchTcGemm(ctx, b, p, kEpiResidual, 6, sa, sb, nullptr, nullptr, a, norms, r,
-                      "tc residual");
 }
 
 int reconstructLowBit(msq_ctx *ctx, const DeviceBatch *b, int format, const float *f, float *x) {
