@@ -142,7 +142,8 @@ std::vector<char> routeToGrid(const int32_t *n, int count, int mode) {
   return grid;
 }
 constexpr int kSweepThreadsMax = 512;
-constexpr int kReplayThreads = 256;
+constexpr int kReplayThreads = 256;       // two CTAs per SM (up to 112 KB each)
+constexpr int kReplayThreadsLarge = 512;  // one CTA per SM
 
 struct JacobiArgs {
   float *a;                  // user matrices (full, column-major)
@@ -587,7 +588,7 @@ __host__ __device__ __forceinline__ size_t replaySmemBytes(int max_n, int rows) 
 // rotations are copied from the log with cp.async while the current round
 // runs, so a round costs one barrier.  Each element is the ordered chain
 // o_c = sum_j x_j q_jc in FP32 FMA, as the CPU restatement.
-__global__ void __launch_bounds__(kReplayThreads)
+__global__ void __launch_bounds__(kReplayThreadsLarge)
 jacobiReplayKernel(VArgs args) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int mi = args.work_matrix[blockIdx.x];
@@ -645,32 +646,12 @@ jacobiReplayKernel(VArgs args) {
       const int r_in = lanes_shift > 0 ? item & 31 : item % lanes_r;
       const int2 ij = pr[k];
       const int I = ij.x, J = ij.y;
-      const float4 *qk = reinterpret_cast<const float4 *>(qs + k * kQF);
-      float q[8][8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float4 lo = qk[2 * j], hi = qk[2 * j + 1];
-        q[j][0] = lo.x; q[j][1] = lo.y; q[j][2] = lo.z; q[j][3] = lo.w;
-        q[j][4] = hi.x; q[j][5] = hi.y; q[j][6] = hi.z; q[j][7] = hi.w;
-      }
-      for (int e = 0; e < per_lane; ++e) {
-        const int r = r_in + 32 * e;
-        if (r >= rows) break;
-        float *row = vs + r * ld;
-        const float4 a = *reinterpret_cast<const float4 *>(row + 4 * I);
-        const float4 b = *reinterpret_cast<const float4 *>(row + 4 * J);
-        const float x[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-        float o[8];
-#pragma unroll
-        for (int c = 0; c < 8; ++c) {
-          float acc = 0.0f;
-#pragma unroll
-          for (int j = 0; j < 8; ++j) acc = fmaf(x[j], q[j][c], acc);
-          o[c] = acc;
-        }
-        *reinterpret_cast<float4 *>(row + 4 * I) = make_float4(o[0], o[1], o[2], o[3]);
-        *reinterpret_cast<float4 *>(row + 4 * J) = make_float4(o[4], o[5], o[6], o[7]);
-      }
+      f32x2 q[8][4];
+      loadRotation(qs + k * kQF, q);
+      int e = 0;
+      for (; e + 2 <= per_lane && r_in + 32 * (e + 1) < rows; e += 2)
+        rotateRow<2>(vs + (r_in + 32 * e) * ld, 32 * ld, I, J, q);
+      if (e < per_lane && r_in + 32 * e < rows) rotateRow<1>(vs + (r_in + 32 * e) * ld, 0, I, J, q);
     }
   }
   copyAsyncWaitAll();
@@ -728,14 +709,18 @@ bool fitsSmem(int n) {
 }
 
 // Rows of V per replay CTA for matrices up to order max_n: the whole matrix
-// when it is small, else the most rows (a multiple of 32) that keep two CTAs
-// per SM (<= 112 KB of shared memory each), at least 8.
+// when it is small; else the most rows (a multiple of 32) that keep two CTAs
+// per SM (<= 112 KB of shared memory each), or 64 with one CTA of 512 threads
+// per SM where that is more and fits (a rotation read from shared memory then
+// serves two rows per lane: 152 matrices of order 512 take 2.9 ms per sweep
+// against 3.7 with 32 rows), at least 8.
 int replayRows(int max_n) {
   if (max_n <= 32) return padded8(max_n);
   int best = 0;
   const int cap = (max_n + 31) / 32 * 32;
   for (int rows = 32; rows <= cap; rows += 32)
     if (replaySmemBytes(max_n, rows) <= 112 * 1024) best = rows;
+  if (best < 64 && max_n > 64 && replaySmemBytes(max_n, 64) <= kSmemLimit) return 64;
   if (best > 0) return best;
   for (int rows = 32; rows >= 8; rows -= 8)
     if (replaySmemBytes(max_n, rows) <= kSmemLimit) return rows;
@@ -1347,7 +1332,8 @@ int jacobiEnqueue(msq_ctx *ctx, const DeviceBatch *b, float *matrices, float *ve
         vargs.work_row = plan->work_row + g.first;
         vargs.rows_per_cta = g.rows;
         launchBegin(ctx, rs);
-        jacobiReplayKernel<<<g.count, kReplayThreads, g.smem, rs>>>(vargs);
+        jacobiReplayKernel<<<g.count, g.smem > 112 * 1024 ? kReplayThreadsLarge : kReplayThreads, g.smem,
+                             rs>>>(vargs);
         MSQ_TRY(launchedOn(ctx, rs, "jacobi replay"));
       }
       MSQ_TRY(tcVectorsEnqueue(ctx, rs, plan->tcv, vectors, b->offset, b->n, args.state, args.log,

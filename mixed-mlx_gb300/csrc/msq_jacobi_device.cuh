@@ -769,6 +769,45 @@ __device__ __forceinline__ void superTileHalf(float *tiles, TileOf tileOf, const
 }
 
 
+// A row-major 8x8 rotation in registers, columns in pairs.
+__device__ __forceinline__ void loadRotation(const float *p, f32x2 (&q)[8][4]) {
+  const ulonglong2 *src = reinterpret_cast<const ulonglong2 *>(p);
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const ulonglong2 x = src[2 * j], y = src[2 * j + 1];
+    q[j][0] = x.x; q[j][1] = x.y; q[j][2] = y.x; q[j][3] = y.y;
+  }
+}
+
+// o = x q for kRows rows' 8 elements and an 8x8 rotation: the ordered chains
+// o_c = sum_j x_j q_jc, two columns per packed FMA; rows `stride`
+// apart, blocks I and J of each.
+template <int kRows>
+__device__ __forceinline__ void rotateRow(float *v, int stride, int I, int J, const f32x2 (&q)[8][4]) {
+  float x[kRows][8];
+#pragma unroll
+  for (int e = 0; e < kRows; ++e) {
+    const float4 a = *reinterpret_cast<const float4 *>(v + static_cast<int64_t>(e) * stride + 4 * I);
+    const float4 b = *reinterpret_cast<const float4 *>(v + static_cast<int64_t>(e) * stride + 4 * J);
+    x[e][0] = a.x; x[e][1] = a.y; x[e][2] = a.z; x[e][3] = a.w;
+    x[e][4] = b.x; x[e][5] = b.y; x[e][6] = b.z; x[e][7] = b.w;
+  }
+#pragma unroll
+  for (int e = 0; e < kRows; ++e) {
+    f32x2 o[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) o[c] = f2zero();
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const f32x2 xx = f2make(x[e][j], x[e][j]);
+#pragma unroll
+      for (int c = 0; c < 4; ++c) o[c] = f2fma(xx, q[j][c], o[c]);
+    }
+    *reinterpret_cast<ulonglong2 *>(v + static_cast<int64_t>(e) * stride + 4 * I) = make_ulonglong2(o[0], o[1]);
+    *reinterpret_cast<ulonglong2 *>(v + static_cast<int64_t>(e) * stride + 4 * J) = make_ulonglong2(o[2], o[3]);
+  }
+}
+
 // TMA bulk copies (cp.async.bulk) of a contiguous block between global and
 // shared memory; both addresses 16-byte aligned, size a multiple of 16.  The
 // load completes on an mbarrier (expect_tx); the wait is bounded.

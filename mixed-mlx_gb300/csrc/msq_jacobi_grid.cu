@@ -209,34 +209,6 @@ __device__ __forceinline__ float blockElement(const float *tiles, int R, int C, 
   return R < C ? tiles[gridElement(triTile(R, C), i, c)] : tiles[gridElement(triTile(C, R), c, i)];
 }
 
-// o = x q for kRows rows' 8 elements and an 8x8 rotation: the ordered chains
-// o_c = sum_j x_j q_jc, two columns per packed FMA.
-template <int kRows>
-__device__ __forceinline__ void rotateRow(float *v, int m, int I, int J, const f32x2 (&q)[8][4]) {
-  float x[kRows][8];
-#pragma unroll
-  for (int e = 0; e < kRows; ++e) {
-    const float4 a = *reinterpret_cast<const float4 *>(v + static_cast<int64_t>(e) * m + 4 * I);
-    const float4 b = *reinterpret_cast<const float4 *>(v + static_cast<int64_t>(e) * m + 4 * J);
-    x[e][0] = a.x; x[e][1] = a.y; x[e][2] = a.z; x[e][3] = a.w;
-    x[e][4] = b.x; x[e][5] = b.y; x[e][6] = b.z; x[e][7] = b.w;
-  }
-#pragma unroll
-  for (int e = 0; e < kRows; ++e) {
-    f32x2 o[4];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) o[c] = f2zero();
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const f32x2 xx = f2make(x[e][j], x[e][j]);
-#pragma unroll
-      for (int c = 0; c < 4; ++c) o[c] = f2fma(xx, q[j][c], o[c]);
-    }
-    *reinterpret_cast<ulonglong2 *>(v + static_cast<int64_t>(e) * m + 4 * I) = make_ulonglong2(o[0], o[1]);
-    *reinterpret_cast<ulonglong2 *>(v + static_cast<int64_t>(e) * m + 4 * J) = make_ulonglong2(o[2], o[3]);
-  }
-}
-
 // Shares of `rows` rows for `groups` groups of 32 pairs on `warps` warps:
 // the fewest row steps of the busiest warp, a rotation's load counting as
 // three rows.
@@ -268,12 +240,7 @@ __device__ __forceinline__ void rotateRows(float *rows, int row_count, int share
     int I, J;
     pairOf(k, I, J);
     f32x2 qq[8][4];
-    const ulonglong2 *src = reinterpret_cast<const ulonglong2 *>(q + static_cast<int64_t>(k) * kQS);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const ulonglong2 x = src[2 * j], y = src[2 * j + 1];
-      qq[j][0] = x.x; qq[j][1] = x.y; qq[j][2] = y.x; qq[j][3] = y.y;
-    }
+    loadRotation(q + static_cast<int64_t>(k) * kQS, qq);
     for (; row + 2 <= hi; row += 2) rotateRow<2>(rows + static_cast<int64_t>(row) * m, m, I, J, qq);
     if (row < hi) rotateRow<1>(rows + static_cast<int64_t>(row) * m, m, I, J, qq);
   }

@@ -89,7 +89,7 @@ void twoLevelSchedule(int nb, std::vector<int32_t> &out) {
 
 namespace {
 
-constexpr int kFormThreads = 256;    // one warp per super-pair (at most 8)
+constexpr int kFormThreads = 512;    // two warps per super-pair (at most 8)
 constexpr int kFormLd = 68;          // row stride of a 64x64 Z block in shared memory
 constexpr int kApplyThreads = 320;   // warps 0-7 rows (two per TMEM lane quarter), 8 MMA, 9 copies
 constexpr int kRowWarps = 8;
@@ -146,14 +146,17 @@ __global__ void __launch_bounds__(kFormThreads) tcvFormKernel(FormArgs args) {
   const int n = args.n[mi], m = padded8(n), nb = m / 4, P = nb / 2;
   const int supers = twoLevelSupers(nb), pairs = supers / 2;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const bool owner = warp < pairs;  // warp x forms the block of super-pair x
-  float *z = zs + warp * 64 * kFormLd;
+  // warps x and x + 8 form the block of super-pair x: a round's rotations act
+  // on disjoint columns, so each takes every other one
+  const int pair = warp & 7, half = warp >> 3;
+  const bool owner = pair < pairs;
+  float *z = zs + pair * 64 * kFormLd;
   float *qbuf = zs + 8 * 64 * kFormLd;  // [2][P][64]: a round's rotations, double-buffered
   if (owner) {
-    for (int i = lane; i < 64; i += 32)
-      for (int c = 0; c < 64; c += 4)
-        *reinterpret_cast<float4 *>(z + i * kFormLd + c) =
-            make_float4(i == c, i == c + 1, i == c + 2, i == c + 3);
+    const int i = lane + 32 * half;
+    for (int c = 0; c < 64; c += 4)
+      *reinterpret_cast<float4 *>(z + i * kFormLd + c) =
+          make_float4(i == c, i == c + 1, i == c + 2, i == c + 3);
   }
   const float *log = args.log + args.log_offset[mi];
   const int32_t *prog = args.prog + args.prog_off[mi];
@@ -174,49 +177,26 @@ __global__ void __launch_bounds__(kFormThreads) tcvFormKernel(FormArgs args) {
     }
     if (!owner) continue;
     const float *qs = qbuf + (t & 1) * P * kQF;
-    const int mine = lane < 8 ? prog[(r * pairs + warp) * 8 + lane] : -1;
-    for (int e = 0; e < 8; ++e) {
+    const int mine = lane < 8 ? prog[(r * pairs + pair) * 8 + lane] : -1;
+    for (int e = half; e < 8; e += 2) {
       const int code = __shfl_sync(0xffffffffu, mine, e);
       if (code < 0) break;
       const int k = code & 255, la = (code >> 8) & 255, lb = code >> 16;
-      const float4 *q4 = reinterpret_cast<const float4 *>(qs + k * kQF);
-      float q[8][8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float4 lo = q4[2 * j], hi = q4[2 * j + 1];
-        q[j][0] = lo.x; q[j][1] = lo.y; q[j][2] = lo.z; q[j][3] = lo.w;
-        q[j][4] = hi.x; q[j][5] = hi.y; q[j][6] = hi.z; q[j][7] = hi.w;
-      }
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        float *row = z + (lane + 32 * h) * kFormLd;
-        const float4 a = *reinterpret_cast<const float4 *>(row + 4 * la);
-        const float4 b = *reinterpret_cast<const float4 *>(row + 4 * lb);
-        const float x[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-        float o[8];
-#pragma unroll
-        for (int c = 0; c < 8; ++c) {
-          float acc = 0.0f;
-#pragma unroll
-          for (int j = 0; j < 8; ++j) acc = fmaf(x[j], q[j][c], acc);
-          o[c] = acc;
-        }
-        *reinterpret_cast<float4 *>(row + 4 * la) = make_float4(o[0], o[1], o[2], o[3]);
-        *reinterpret_cast<float4 *>(row + 4 * lb) = make_float4(o[4], o[5], o[6], o[7]);
-      }
+      f32x2 q[8][4];
+      loadRotation(qs + k * kQF, q);
+      rotateRow<2>(z + lane * kFormLd, 32 * kFormLd, la, lb, q);
     }
   }
   copyAsyncWaitAll();
-  __syncwarp();
+  __syncthreads();
   if (!owner) return;
   // B operand rows j (output columns), K = the 64 local indices: Z^T, as
   // hi rows 0..63 then lo rows 0..63 (rows 32..63, super-block Q, start
   // 4 KB into each term).
   uint8_t *img = args.images +
-                 (args.image_off[mi] + static_cast<int64_t>(stage) * pairs + warp) * kRotationImageBytes;
-#pragma unroll 1
-  for (int h = 0; h < 2; ++h) {
-    const int j = lane + 32 * h;
+                 (args.image_off[mi] + static_cast<int64_t>(stage) * pairs + pair) * kRotationImageBytes;
+  {
+    const int j = lane + 32 * half;
 #pragma unroll 1
     for (int c = 0; c < 8; ++c) {
       uint32_t hi[4], lo[4];
@@ -341,20 +321,21 @@ __global__ void __launch_bounds__(kApplyThreads, 1) tcvApplyKernel(ApplyArgs arg
           const uint32_t a_hi = smemAddr(ops + buf * 2 * kOperandBytes);
           const uint32_t a_lo = a_hi + kOperandBytes;
           const uint32_t zimg = smemAddr(ring + slot * kRotationImageBytes);
-#pragma unroll 1
-          for (int h = 0; h < 2; ++h) {
-            const int S = h ? Qs : Ps;
-            if (S >= real) continue;
-            const uint32_t d = tmem + 32 * S;
-            const uint64_t ah = smemDesc(a_hi), al = smemDesc(a_lo);
-            const uint64_t zh = smemDesc(zimg + h * 4096);
-            const uint64_t zl = smemDesc(zimg + kImageTermBytes + h * 4096);
+          // the two halves of the pair take turns, so that consecutive MMAs
+          // use different accumulators
+          const uint64_t ah = smemDesc(a_hi), al = smemDesc(a_lo);
+          const uint64_t zh = smemDesc(zimg), zl = smemDesc(zimg + kImageTermBytes);
+          const uint32_t d0 = tmem + 32 * Ps, d1 = tmem + 32 * Qs;
+          const bool on0 = Ps < real, on1 = Qs < real;
 #pragma unroll
-            for (int kk = 0; kk < 4; ++kk) {
-              mmaBf16(d, ah + 2 * kk, zh + 2 * kk, idesc, kk > 0);
-              mmaBf16(d, al + 2 * kk, zh + 2 * kk, idesc, 1);
-              mmaBf16(d, ah + 2 * kk, zl + 2 * kk, idesc, 1);
-            }
+          for (int kk = 0; kk < 4; ++kk) {
+            const uint64_t a = ah + 2 * kk, b = al + 2 * kk, z = zh + 2 * kk, y = zl + 2 * kk;
+            if (on0) mmaBf16(d0, a, z, idesc, kk > 0);
+            if (on1) mmaBf16(d1, a, z + 256, idesc, kk > 0);
+            if (on0) mmaBf16(d0, b, z, idesc, 1);
+            if (on1) mmaBf16(d1, b, z + 256, idesc, 1);
+            if (on0) mmaBf16(d0, a, y, idesc, 1);
+            if (on1) mmaBf16(d1, a, y + 256, idesc, 1);
           }
           mmaCommit(smemAddr(&a_empty[buf]));
           mmaCommit(smemAddr(&z_empty[slot]));
