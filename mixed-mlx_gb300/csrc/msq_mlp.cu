@@ -18,6 +18,9 @@
 #include "msq_codec_device.cuh"
 #include "msq_internal.cuh"
 
+#include <algorithm>
+#include <vector>
+
 namespace msq {
 namespace {
 
@@ -28,7 +31,97 @@ static_assert(kParams == MSQ_MLP_PARAMS, "parameter layout");
 
 __device__ __forceinline__ float bf16Round(float x) { return decodeBf16(encodeBf16(x)); }
 
-// Features of one matrix (one CTA), all from O(n^2) passes:
+// Sum of FP32 values in float-float (about 48 bits): on this GPU an FP64
+// addition costs as much as 64 FP32 ones.
+struct FloatSum {
+  float s = 0.0f, c = 0.0f;
+  __device__ __forceinline__ void add(float v, float err = 0.0f) {
+    const float t = s + v, z = t - s;
+    c += ((s - (t - z)) + (v - z)) + err;
+    s = t;
+  }
+  __device__ __forceinline__ void square(float v) {
+    const float q = __fmul_rn(v, v);
+    add(q, fmaf(v, v, -q));
+  }
+  // the warp's total in every lane
+  __device__ __forceinline__ void warp() {
+#pragma unroll
+    for (int k = 16; k; k >>= 1)
+      add(__shfl_xor_sync(0xffffffffu, s, k), __shfl_xor_sync(0xffffffffu, c, k));
+  }
+  __device__ double value() const { return static_cast<double>(s) + static_cast<double>(c); }
+};
+
+// Per column i of a symmetric matrix (element (j, i) at j + i n): the sums of
+// |a_ji| and a_ji^2 over j != i.  A warp per column, lanes down the column:
+// coalesced, bound by the latency of a few loads per column and, at large
+// orders, by memory.  A thread per column read with a stride of n and summed
+// in FP64; features of 256 matrices of orders 64 .. 512: 417 us, 74 so; of
+// one matrix of order 1024: 1067 and 49; of 4096 of order 64: 275 and 223.
+struct ColumnStat {
+  double abs_sum, squares;
+};
+constexpr int kStatColumns = 32;  // columns per work item
+
+__global__ void __launch_bounds__(256) columnStatsKernel(const float *__restrict__ a,
+                                                         const int32_t *__restrict__ nn,
+                                                         const int64_t *__restrict__ off,
+                                                         const int64_t *__restrict__ eoff,
+                                                         const int4 *__restrict__ work, int items,
+                                                         ColumnStat *__restrict__ stats) {
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  for (int item = blockIdx.x; item < items; item += gridDim.x) {
+    const int mi = work[item].x, n = nn[mi];
+    const int hi = min(n, (work[item].y + 1) * kStatColumns);
+    for (int i = work[item].y * kStatColumns + warp; i < hi; i += 8) {
+      const float *col = a + off[mi] + static_cast<int64_t>(i) * n;
+      FloatSum sum, squares;
+      if (n % 4 == 0 && (reinterpret_cast<uintptr_t>(col) & 15) == 0) {
+        const float4 *c4 = reinterpret_cast<const float4 *>(col);
+#pragma unroll 4
+        for (int j = lane; j < n / 4; j += 32) {
+          const float4 v = c4[j];
+          const float x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float y = 4 * j + e == i ? 0.0f : x[e];
+            sum.add(fabsf(y));
+            squares.square(y);
+          }
+        }
+      } else {
+#pragma unroll 4
+        for (int j = lane; j < n; j += 32) {
+          const float y = j == i ? 0.0f : col[j];
+          sum.add(fabsf(y));
+          squares.square(y);
+        }
+      }
+      sum.warp();
+      squares.warp();
+      double rs = sum.value(), r2 = squares.value();
+      // Squares that FP32 overflows or loses (a square below 2^-126 beside a
+      // sum of 1e-20 is 1e-18 of it), and infinities and NaN: in FP64.
+      if (!(r2 >= 1e-20 && r2 <= 1e37) && rs != 0.0) {
+        rs = r2 = 0.0;
+        for (int j = lane; j < n; j += 32) {
+          const double y = j == i ? 0.0 : static_cast<double>(col[j]);
+          rs += fabs(y);
+          r2 += y * y;
+        }
+#pragma unroll
+        for (int s = 16; s; s >>= 1) {
+          rs += __shfl_xor_sync(0xffffffffu, rs, s);
+          r2 += __shfl_xor_sync(0xffffffffu, r2, s);
+        }
+      }
+      if (lane == 0) stats[eoff[mi] + i] = {rs, r2};
+    }
+  }
+}
+
+// Features of one matrix (one warp) from its diagonal and column sums:
 //  0 log2 n            1 log10 trace/n        2 log10 ||A||_F / n
 //  3 log10 min diag    4 log10 max diag       5 log10(max/min diag)
 //  6 Gershgorin lower / (trace/n) (clamped)   7 log10 Gershgorin upper/(trace/n)
@@ -36,23 +129,25 @@ __device__ __forceinline__ float bf16Round(float x) { return decodeBf16(encodeBf
 // 10 mean |a_ij| off-diagonal / mean diag     11 log10 (||A||_F^2 / trace^2 * n)
 // 12 std diag / mean diag                     13 fraction of rows diagonally dominant
 // 14 log10 tolerance (filled by the caller; 0 here)   15 bias term 1
-__global__ void featuresKernel(const float *__restrict__ a, const int32_t *__restrict__ nn,
-                               const int64_t *__restrict__ off, float *__restrict__ out) {
-  const int mi = blockIdx.x;
+// Lane k forms feature k, so the FP64 logarithms (and square roots) of a
+// matrix are one instruction stream.
+__global__ void __launch_bounds__(128) featuresKernel(const float *__restrict__ a,
+                                                      const int32_t *__restrict__ nn,
+                                                      const int64_t *__restrict__ off,
+                                                      const int64_t *__restrict__ eoff,
+                                                      const ColumnStat *__restrict__ stats, int count,
+                                                      float *__restrict__ out) {
+  const int lane = threadIdx.x % 32, mi = blockIdx.x * 4 + threadIdx.x / 32;
+  if (mi >= count) return;
   const int n = nn[mi];
   const float *A = a + off[mi];
-  __shared__ double red[8][32];
+  const ColumnStat *col = stats + eoff[mi];
   double tr = 0, fro = 0, offm = 0, offabs = 0, dmin = 1e300, dmax = -1e300, d2 = 0;
-  double glo = 1e300, ghi = -1e300, rowmax = 0, dom = 0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+  double glo = 1e300, ghi = -1e300, rowmax = 0;
+  int dominant = 0;
+  for (int i = lane; i < n; i += 32) {
     const double d = A[i + static_cast<int64_t>(i) * n];
-    double rs = 0, ro2 = 0;
-    for (int j = 0; j < n; ++j) {
-      if (j == i) continue;
-      const double v = A[j + static_cast<int64_t>(i) * n];  // row i = column i (symmetric)
-      rs += fabs(v);
-      ro2 += v * v;
-    }
+    const double rs = col[i].abs_sum, ro2 = col[i].squares;
     tr += d;
     d2 += d * d;
     fro += d * d + ro2;
@@ -63,161 +158,198 @@ __global__ void featuresKernel(const float *__restrict__ a, const int32_t *__res
     glo = fmin(glo, d - rs);
     ghi = fmax(ghi, d + rs);
     rowmax = fmax(rowmax, rs);
-    dom += d > rs ? 1.0 : 0.0;
+    dominant += d > rs;
   }
-  double vals[8] = {tr, fro, offm, offabs, d2, dom, 0, 0};
-  double mins[2] = {dmin, glo}, maxs[3] = {dmax, ghi, rowmax};
-  const int lane = threadIdx.x % 32, warp = threadIdx.x / 32, warps = blockDim.x / 32;
-  for (int k = 0; k < 6; ++k) {
-    double v = vals[k];
-    for (int s = 16; s; s >>= 1) v += __shfl_xor_sync(0xffffffffu, v, s);
-    if (lane == 0) red[k][warp] = v;
+#pragma unroll
+  for (int s = 16; s; s >>= 1) {
+    auto other = [&](double v) { return __shfl_xor_sync(0xffffffffu, v, s); };
+    tr += other(tr);
+    d2 += other(d2);
+    fro += other(fro);
+    offm += other(offm);
+    offabs += other(offabs);
+    dmin = fmin(dmin, other(dmin));
+    dmax = fmax(dmax, other(dmax));
+    glo = fmin(glo, other(glo));
+    ghi = fmax(ghi, other(ghi));
+    rowmax = fmax(rowmax, other(rowmax));
+    dominant += __shfl_xor_sync(0xffffffffu, dominant, s);
   }
-  for (int k = 0; k < 2; ++k) {
-    double v = mins[k];
-    for (int s = 16; s; s >>= 1) v = fmin(v, __shfl_xor_sync(0xffffffffu, v, s));
-    mins[k] = v;
-  }
-  for (int k = 0; k < 3; ++k) {
-    double v = maxs[k];
-    for (int s = 16; s; s >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, s));
-    maxs[k] = v;
-  }
-  __shared__ double rmin[2][32], rmax[3][32];
-  if (lane == 0) {
-    rmin[0][warp] = mins[0]; rmin[1][warp] = mins[1];
-    rmax[0][warp] = maxs[0]; rmax[1][warp] = maxs[1]; rmax[2][warp] = maxs[2];
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int k = 0; k < 6; ++k) {
-      double s = 0;
-      for (int w = 0; w < warps; ++w) s += red[k][w];
-      vals[k] = s;
-    }
-    double mn0 = 1e300, mn1 = 1e300, mx0 = -1e300, mx1 = -1e300, mx2 = 0;
-    for (int w = 0; w < warps; ++w) {
-      mn0 = fmin(mn0, rmin[0][w]); mn1 = fmin(mn1, rmin[1][w]);
-      mx0 = fmax(mx0, rmax[0][w]); mx1 = fmax(mx1, rmax[1][w]); mx2 = fmax(mx2, rmax[2][w]);
-    }
-    const double trace = vals[0], fnorm = sqrt(vals[1]), mean_d = trace / n;
-    const double tiny = 1e-30;
-    float *f = out + static_cast<int64_t>(mi) * kIn;
-    f[0] = static_cast<float>(log2(static_cast<double>(n)));
-    f[1] = static_cast<float>(log10(fmax(mean_d, tiny)));
-    f[2] = static_cast<float>(log10(fmax(fnorm / n, tiny)));
-    f[3] = static_cast<float>(log10(fmax(mn0, tiny)));
-    f[4] = static_cast<float>(log10(fmax(mx0, tiny)));
-    f[5] = static_cast<float>(log10(fmax(mx0, tiny) / fmax(mn0, tiny)));
-    f[6] = static_cast<float>(fmax(-10.0, fmin(1.0, mn1 / fmax(mean_d, tiny))));
-    f[7] = static_cast<float>(log10(fmax(mx1, tiny) / fmax(mean_d, tiny)));
-    f[8] = static_cast<float>(sqrt(vals[2]) / fmax(fnorm, tiny));
-    f[9] = static_cast<float>(fmin(100.0, mx2 / fmax(mn0, tiny)));
-    f[10] = static_cast<float>(n > 1 ? (vals[3] / (static_cast<double>(n) * (n - 1))) / fmax(mean_d, tiny) : 0.0);
-    f[11] = static_cast<float>(log10(fmax(vals[1] * n / fmax(trace * trace, tiny), tiny)));
-    f[12] = static_cast<float>(sqrt(fmax(vals[4] / n - mean_d * mean_d, 0.0)) / fmax(mean_d, tiny));
-    f[13] = static_cast<float>(vals[5] / n);
-    f[14] = 0.0f;
-    f[15] = 1.0f;
+  if (lane >= kIn) return;
+  const double tiny = 1e-30, mean = tr / n, mean_t = fmax(mean, tiny), dmin_t = fmax(dmin, tiny);
+  // square roots: ||A||_F, the off-diagonal mass (8), the deviation (12)
+  const double root = sqrt(lane == 8 ? offm : lane == 12 ? fmax(d2 / n - mean * mean, 0.0) : fro);
+  const double fnorm = __shfl_sync(0xffffu, root, 0);
+  const double numerator = lane == 0    ? static_cast<double>(n)
+                           : lane == 1  ? mean_t
+                           : lane == 2  ? fmax(root / n, tiny)
+                           : lane == 3  ? dmin_t
+                           : lane == 4  ? fmax(dmax, tiny)
+                           : lane == 5  ? fmax(dmax, tiny)
+                           : lane == 6  ? glo
+                           : lane == 7  ? fmax(ghi, tiny)
+                           : lane == 8  ? root
+                           : lane == 9  ? rowmax
+                           : lane == 10 ? (n > 1 ? offabs / (static_cast<double>(n) * (n - 1)) : 0.0)
+                           : lane == 11 ? fro * n
+                           : lane == 12 ? root
+                           : lane == 13 ? static_cast<double>(dominant)
+                                        : 0.0;
+  const double denominator = lane == 5 || lane == 9                                 ? dmin_t
+                             : lane == 6 || lane == 7 || lane == 10 || lane == 12   ? mean_t
+                             : lane == 8                                            ? fmax(fnorm, tiny)
+                             : lane == 11                                           ? fmax(tr * tr, tiny)
+                             : lane == 13                                           ? static_cast<double>(n)
+                                                                                    : 1.0;
+  double v = numerator / denominator;
+  const bool logarithm = lane <= 5 || lane == 7 || lane == 11;
+  const double l = log10(logarithm ? (lane == 11 ? fmax(v, tiny) : v) : 1.0);
+  if (logarithm) v = l;
+  if (lane == 0) v = log2(static_cast<double>(n));
+  if (lane == 6) v = fmax(-10.0, fmin(1.0, v));
+  if (lane == 9) v = fmin(100.0, v);
+  if (lane == 15) v = 1.0;
+  out[static_cast<int64_t>(mi) * kIn + lane] = static_cast<float>(v);
+}
+
+// The network's weights, rounded to BF16 and widened, in shared memory: W2 and
+// W3 with a row stride of 65 so that the threads of a hidden layer, one row
+// each, read different banks.  Rows of features go in groups of kRows per CTA
+// of 64 x kRows threads (a thread per hidden unit and row).
+constexpr int kRows = 4;
+constexpr int kMlpThreads = kHid * kRows;
+constexpr int kLd1 = kIn + 1, kLd2 = kHid + 1;
+struct MlpShared {
+  float w1[kHid * kLd1], b1[kHid], w2[kHid * kLd2], b2[kHid], w3[kOut * kLd2], b3[kOut];
+  float x[kRows][kIn], h1[kRows][kHid], h2[kRows][kHid], z[kRows][kOut];
+};
+
+__device__ __forceinline__ void mlpLoad(const float *__restrict__ p, MlpShared &m) {
+  for (int i = threadIdx.x; i < kHid * kIn; i += blockDim.x) m.w1[i / kIn * kLd1 + i % kIn] = bf16Round(p[kW1 + i]);
+  for (int i = threadIdx.x; i < kHid * kHid; i += blockDim.x)
+    m.w2[i / kHid * kLd2 + i % kHid] = bf16Round(p[kW2 + i]);
+  for (int i = threadIdx.x; i < kOut * kHid; i += blockDim.x)
+    m.w3[i / kHid * kLd2 + i % kHid] = bf16Round(p[kW3 + i]);
+  for (int i = threadIdx.x; i < kHid; i += blockDim.x) {
+    m.b1[i] = bf16Round(p[kB1 + i]);
+    m.b2[i] = bf16Round(p[kB2 + i]);
+    if (i < kOut) m.b3[i] = bf16Round(p[kB3 + i]);
   }
 }
 
-// Forward for rows of features: thread block of 64 threads, 8 rows per block
-// iteration; h1 and h2 staged in shared memory.  Logits are FP32.
-template <bool kKeep>
-__device__ void mlpForwardRow(const float *__restrict__ p, const float *__restrict__ x,
-                              float *h1, float *h2, float *z) {
-  const int t = threadIdx.x;  // hidden unit
-  float s = bf16Round(p[kB1 + t]);
-  for (int i = 0; i < kIn; ++i) s = fmaf(bf16Round(p[kW1 + t * kIn + i]), x[i], s);
-  h1[t] = fmaxf(s, 0.0f);
+// Logits of rows first .. first + kRows - 1 (those below `rows`) into m.z.
+__device__ __forceinline__ void mlpForwardRows(MlpShared &m, const float *__restrict__ x, int first,
+                                               int rows) {
+  const int t = threadIdx.x % kHid, r = threadIdx.x / kHid;  // hidden unit, row
+  __syncthreads();  // the weights are loaded, the last group is done
+  if (t < kIn) m.x[r][t] = first + r < rows ? x[static_cast<int64_t>(first + r) * kIn + t] : 0.0f;
   __syncthreads();
-  s = bf16Round(p[kB2 + t]);
-  for (int i = 0; i < kHid; ++i) s = fmaf(bf16Round(p[kW2 + t * kHid + i]), h1[i], s);
-  h2[t] = fmaxf(s, 0.0f);
+  float s = m.b1[t];
+#pragma unroll
+  for (int i = 0; i < kIn; ++i) s = fmaf(m.w1[t * kLd1 + i], m.x[r][i], s);
+  m.h1[r][t] = fmaxf(s, 0.0f);
+  __syncthreads();
+  s = m.b2[t];
+#pragma unroll 16
+  for (int i = 0; i < kHid; ++i) s = fmaf(m.w2[t * kLd2 + i], m.h1[r][i], s);
+  m.h2[r][t] = fmaxf(s, 0.0f);
   __syncthreads();
   if (t < kOut) {
-    s = bf16Round(p[kB3 + t]);
-    for (int i = 0; i < kHid; ++i) s = fmaf(bf16Round(p[kW3 + t * kHid + i]), h2[i], s);
-    z[t] = s;
+    s = m.b3[t];
+#pragma unroll 16
+    for (int i = 0; i < kHid; ++i) s = fmaf(m.w3[t * kLd2 + i], m.h2[r][i], s);
+    m.z[r][t] = s;
   }
   __syncthreads();
 }
 
-__global__ void __launch_bounds__(64) mlpForwardKernel(const float *__restrict__ p,
-                                                       const float *__restrict__ x, int rows,
-                                                       float *__restrict__ logits) {
-  __shared__ float xs[kIn], h1[kHid], h2[kHid], z[kOut];
-  for (int r = blockIdx.x; r < rows; r += gridDim.x) {
-    if (threadIdx.x < kIn) xs[threadIdx.x] = x[static_cast<int64_t>(r) * kIn + threadIdx.x];
-    __syncthreads();
-    mlpForwardRow<false>(p, xs, h1, h2, z);
-    if (threadIdx.x < kOut) logits[static_cast<int64_t>(r) * kOut + threadIdx.x] = z[threadIdx.x];
-    __syncthreads();
+__global__ void __launch_bounds__(kMlpThreads) mlpForwardKernel(const float *__restrict__ p,
+                                                                const float *__restrict__ x, int rows,
+                                                                float *__restrict__ logits) {
+  __shared__ MlpShared m;
+  mlpLoad(p, m);
+  for (int first = blockIdx.x * kRows; first < rows; first += gridDim.x * kRows) {
+    mlpForwardRows(m, x, first, rows);
+    const int r = threadIdx.x / kOut;
+    if (threadIdx.x < kRows * kOut && first + r < rows)
+      logits[static_cast<int64_t>(first) * kOut + threadIdx.x] = m.z[r][threadIdx.x % kOut];
   }
 }
 
 // Backward of L = mean over rows and outputs of softplus(z) - y z (sigmoid
 // cross-entropy), accumulating dL/dparams (w.r.t. the FP32 masters, through
-// the BF16 rounding as a straight-through identity) with block-local
-// partial sums flushed by atomics.  loss gets the mean loss.
-__global__ void __launch_bounds__(64) mlpBackwardKernel(const float *__restrict__ p,
-                                                        const float *__restrict__ x,
-                                                        const float *__restrict__ y, int rows,
-                                                        float *__restrict__ grad,
-                                                        float *__restrict__ loss) {
-  __shared__ float xs[kIn], h1[kHid], h2[kHid], z[kOut], dz[kOut], dh2[kHid], dh1[kHid];
-  const int t = threadIdx.x;
-  // per-thread accumulators for the rows this block handles
-  float gW1[kIn], gB1 = 0.0f, gW2[kHid], gB2 = 0.0f, gW3[kHid], gB3 = 0.0f;
-  for (int i = 0; i < kIn; ++i) gW1[i] = 0.0f;
-  for (int i = 0; i < kHid; ++i) { gW2[i] = 0.0f; gW3[i] = 0.0f; }
-  float lsum = 0.0f;
+// the BF16 rounding as a straight-through identity).  A CTA keeps its rows'
+// sums of the gradient in registers, every thread a fixed set of parameters,
+// and adds them once at the end; at most kGradCtas, so that the additions
+// into the one gradient do not dominate.  loss gets the mean loss.
+constexpr int kGradCtas = 64;
+__global__ void __launch_bounds__(kMlpThreads) mlpBackwardKernel(const float *__restrict__ p,
+                                                                 const float *__restrict__ x,
+                                                                 const float *__restrict__ y, int rows,
+                                                                 float *__restrict__ grad,
+                                                                 float *__restrict__ loss) {
+  __shared__ MlpShared m;
+  __shared__ float dz[kRows][kOut], dh2[kRows][kHid], dh1[kRows][kHid];
+  const int t = threadIdx.x % kHid, r = threadIdx.x / kHid;
+  // this thread's parameters: column t of kHid / kRows rows of W2, and of
+  // kOut / kRows rows of W3, 4 elements of W1
+  constexpr int k2 = kHid / kRows, k3 = kOut / kRows, k1 = kHid * kIn / kMlpThreads;
+  float g1[k1] = {}, g2[k2] = {}, g3[k3] = {}, gb1 = 0.0f, gb2 = 0.0f, gb3 = 0.0f, lsum = 0.0f;
   const float inv = 1.0f / (static_cast<float>(rows) * kOut);
-  for (int r = blockIdx.x; r < rows; r += gridDim.x) {
-    if (t < kIn) xs[t] = x[static_cast<int64_t>(r) * kIn + t];
-    __syncthreads();
-    mlpForwardRow<true>(p, xs, h1, h2, z);
+  mlpLoad(p, m);
+  for (int first = blockIdx.x * kRows; first < rows; first += gridDim.x * kRows) {
+    mlpForwardRows(m, x, first, rows);
     if (t < kOut) {
-      const float zz = z[t], yy = y[static_cast<int64_t>(r) * kOut + t];
-      const float sig = 1.0f / (1.0f + expf(-zz));
-      dz[t] = (sig - yy) * inv;
-      lsum += (fmaxf(zz, 0.0f) + log1pf(expf(-fabsf(zz))) - yy * zz) * inv;
+      float d = 0.0f;
+      if (first + r < rows) {
+        const float zz = m.z[r][t], yy = y[static_cast<int64_t>(first + r) * kOut + t];
+        const float sig = 1.0f / (1.0f + expf(-zz));
+        d = (sig - yy) * inv;
+        lsum += (fmaxf(zz, 0.0f) + log1pf(expf(-fabsf(zz))) - yy * zz) * inv;
+      }
+      dz[r][t] = d;  // rows beyond the last contribute nothing
     }
     __syncthreads();
-    // layer 3: thread t < 8 owns output t
-    if (t < kOut) {
-      for (int i = 0; i < kHid; ++i) gW3[i] += dz[t] * h2[i];
-      gB3 += dz[t];
-    }
-    // dh2
-    {
-      float s = 0.0f;
-      for (int o = 0; o < kOut; ++o) s = fmaf(bf16Round(p[kW3 + o * kHid + t]), dz[o], s);
-      dh2[t] = h2[t] > 0.0f ? s : 0.0f;
-    }
+    float s = 0.0f;
+#pragma unroll
+    for (int o = 0; o < kOut; ++o) s = fmaf(m.w3[o * kLd2 + t], dz[r][o], s);
+    dh2[r][t] = m.h2[r][t] > 0.0f ? s : 0.0f;
     __syncthreads();
-    for (int i = 0; i < kHid; ++i) gW2[i] += dh2[t] * h1[i];
-    gB2 += dh2[t];
-    {
-      float s = 0.0f;
-      for (int o = 0; o < kHid; ++o) s = fmaf(bf16Round(p[kW2 + o * kHid + t]), dh2[o], s);
-      dh1[t] = h1[t] > 0.0f ? s : 0.0f;
+    s = 0.0f;
+#pragma unroll 16
+    for (int o = 0; o < kHid; ++o) s = fmaf(m.w2[o * kLd2 + t], dh2[r][o], s);
+    dh1[r][t] = m.h1[r][t] > 0.0f ? s : 0.0f;
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < kRows; ++q) {
+#pragma unroll
+      for (int e = 0; e < k2; ++e) g2[e] = fmaf(dh2[q][r * k2 + e], m.h1[q][t], g2[e]);
+#pragma unroll
+      for (int e = 0; e < k3; ++e) g3[e] = fmaf(dz[q][r * k3 + e], m.h2[q][t], g3[e]);
+#pragma unroll
+      for (int e = 0; e < k1; ++e) {
+        const int i = threadIdx.x + e * kMlpThreads;
+        g1[e] = fmaf(dh1[q][i / kIn], m.x[q][i % kIn], g1[e]);
+      }
+      if (r == 0) {
+        gb1 += dh1[q][t];
+        gb2 += dh2[q][t];
+        if (t < kOut) gb3 += dz[q][t];
+      }
     }
-    __syncthreads();
-    for (int i = 0; i < kIn; ++i) gW1[i] += dh1[t] * xs[i];
-    gB1 += dh1[t];
-    __syncthreads();
   }
-  for (int i = 0; i < kIn; ++i) atomicAdd(&grad[kW1 + t * kIn + i], gW1[i]);
-  atomicAdd(&grad[kB1 + t], gB1);
-  for (int i = 0; i < kHid; ++i) atomicAdd(&grad[kW2 + t * kHid + i], gW2[i]);
-  atomicAdd(&grad[kB2 + t], gB2);
-  if (t < kOut) {
-    for (int i = 0; i < kHid; ++i) atomicAdd(&grad[kW3 + t * kHid + i], gW3[i]);
-    atomicAdd(&grad[kB3 + t], gB3);
-    atomicAdd(loss, lsum);
+#pragma unroll
+  for (int e = 0; e < k2; ++e) atomicAdd(&grad[kW2 + (r * k2 + e) * kHid + t], g2[e]);
+#pragma unroll
+  for (int e = 0; e < k3; ++e) atomicAdd(&grad[kW3 + (r * k3 + e) * kHid + t], g3[e]);
+#pragma unroll
+  for (int e = 0; e < k1; ++e) atomicAdd(&grad[kW1 + threadIdx.x + e * kMlpThreads], g1[e]);
+  if (r == 0) {
+    atomicAdd(&grad[kB1 + t], gb1);
+    atomicAdd(&grad[kB2 + t], gb2);
+    if (t < kOut) atomicAdd(&grad[kB3 + t], gb3);
   }
+  if (t < kOut) atomicAdd(loss, lsum);
 }
 
 // Adam (beta1 0.9, beta2 0.999, eps 1e-8) on the FP32 masters.
@@ -245,7 +377,23 @@ extern "C" int msq_features(msq_ctx *ctx, const float *a, const int32_t *n, cons
   if (!a || !features) return setError(ctx, MSQ_ERR_INVALID_ARGUMENT, "msq_features: null buffer");
   const DeviceBatch *b = prepareBatch(ctx, n, offset, count);
   if (b == nullptr) return MSQ_ERR_INVALID_ARGUMENT;
-  featuresKernel<<<count, 128, 0, ctx->stream>>>(a, b->n, b->offset, features);
+  constexpr int kStatWork = 1 << 19;
+  const int4 *work = nullptr;
+  int items = 0;
+  if (!findWork(b, kStatWork, &work, &items)) {
+    std::vector<int4> list;
+    for (int mi = 0; mi < b->count; ++mi)
+      for (int t = 0; t < (b->host_n[mi] + kStatColumns - 1) / kStatColumns; ++t)
+        list.push_back(make_int4(mi, t, 0, 0));
+    MSQ_TRY(keepWork(ctx, b, kStatWork, list, &work, &items));
+  }
+  auto *stats = static_cast<ColumnStat *>(scratch(ctx, b->total_order * sizeof(ColumnStat), kScratchOperand));
+  if (stats == nullptr) return MSQ_ERR_CUDA;
+  columnStatsKernel<<<std::min(items, kSmCount * 8), 256, 0, ctx->stream>>>(
+      a, b->n, b->offset, b->eig_offset, work, items, stats);
+  MSQ_TRY(launched(ctx, "mlp column sums"));
+  featuresKernel<<<(count + 3) / 4, 128, 0, ctx->stream>>>(a, b->n, b->offset, b->eig_offset, stats,
+                                                         count, features);
   return launched(ctx, "mlp features");
 }
 
@@ -256,8 +404,8 @@ extern "C" int msq_mlp_forward(msq_ctx *ctx, const float *params, const float *f
   if (!params || !features || !logits || rows < 0)
     return setError(ctx, MSQ_ERR_INVALID_ARGUMENT, "msq_mlp_forward: bad argument");
   if (rows == 0) return MSQ_OK;
-  mlpForwardKernel<<<std::min(rows, kSmCount * 16), 64, 0, ctx->stream>>>(params, features, rows,
-                                                                          logits);
+  mlpForwardKernel<<<std::min((rows + kRows - 1) / kRows, kSmCount * 4), kMlpThreads, 0, ctx->stream>>>(
+      params, features, rows, logits);
   return launched(ctx, "mlp forward");
 }
 
@@ -267,7 +415,7 @@ extern "C" int msq_mlp_backward(msq_ctx *ctx, const float *params, const float *
   msq::DeviceGuard device_guard(ctx);
   if (!params || !features || !targets || !grad_params || !loss || rows <= 0)
     return setError(ctx, MSQ_ERR_INVALID_ARGUMENT, "msq_mlp_backward: bad argument");
-  mlpBackwardKernel<<<std::min(rows, kSmCount * 4), 64, 0, ctx->stream>>>(
+  mlpBackwardKernel<<<std::min((rows + kRows - 1) / kRows, kGradCtas), kMlpThreads, 0, ctx->stream>>>(
       params, features, targets, rows, grad_params, loss);
   return launched(ctx, "mlp backward");
 }

@@ -28,12 +28,9 @@
 // brings the slices of 32 of K (64 KB of A, 32 KB of B) into one of two
 // stages, an MMA warp issues the 36 pairs, sixteen warps read the eight
 // accumulators (all 512 TMEM columns) every 512 of K (eight epilogue warps
-// took 396 us on 1000 matrices of order 128 against 244).  The pairs are issued
-// so that two of one weight are at least four apart: an MMA of N = 64 that
-// waits for the accumulator of the one before it takes 113 cycles against 32
-// on the pipe (152 matrices of order 512: 1322 us with the pairs' four K steps
-// in a row, 865 so).  Large matrices are bound by the operand loads from L2
-// (96 KB per 72 MMAs, 5.4 TB/s).
+// took 396 us on 1000 matrices of order 128 against 244).  What bounds it is
+// the tensor pipe's read of A: an MMA of M = 128 takes 68 cycles for N = 32,
+// 64 and 128 alike (152 matrices of order 512: 80 per MMA with the drain).
 //
 // Residual of four matrices of order 1000: 216 us with the slicing against
 // 908 on the CUDA cores; 152 of order 512: 1085 against 4247; 1000 of order
@@ -82,8 +79,7 @@ __device__ __forceinline__ uint64_t smemDesc64(uint32_t addr) {
          (static_cast<uint64_t>(4) << 61);            // SWIZZLE_64B
 }
 
-// The pairs (p, q), p + q < kSlices, as 16 p + q: equal weights at least four
-// apart (also from the end to the start), (0, g) first of its weight.
+// The pairs (p, q), p + q < kSlices, as 16 p + q, (0, g) first of its weight.
 constexpr int kPairs = kSlices * (kSlices + 1) / 2;
 __device__ constexpr uint8_t kPairOrder[kPairs] = {
     0x07, 0x06, 0x05, 0x04, 0x16, 0x15, 0x14, 0x03, 0x25, 0x24, 0x13, 0x23,
