@@ -358,28 +358,55 @@ residualFFKernel(ResidualArgs args) {
 // F^T (K-major factor): F[k + i*n] = V[i + k*n] * lambda_k^(1/4), so that
 // X = F^T F = V diag(sqrt(lambda)) V^T (scale_columns_f32,
 // metal_mixed_sqrt.metal:21-38, split symmetrically over both factors).
-__global__ void makeFactorKernel(const float *__restrict__ v, const float *__restrict__ lam,
-                                 const int32_t *__restrict__ nn, const int64_t *__restrict__ off,
-                                 const int64_t *__restrict__ eoff, float *__restrict__ f,
-                                 const int4 *__restrict__ work, int items) {
-  __shared__ float tile[32][33];
+//
+// 64 x 64 tiles through shared memory, 16 loads in flight per thread, a
+// quartic root per column of the tile: bound by memory (order 8192: 272 us
+// with 32 x 32 tiles and a root per element, 120 us so).
+constexpr int kFactorTile = 64;
+__global__ void __launch_bounds__(256) makeFactorKernel(
+    const float *__restrict__ v, const float *__restrict__ lam, const int32_t *__restrict__ nn,
+    const int64_t *__restrict__ off, const int64_t *__restrict__ eoff, float *__restrict__ f,
+    const int4 *__restrict__ work, int items) {
+  constexpr int kT = kFactorTile, kRows = kT / 8;
+  __shared__ float tile[kT][kT + 1], root[kT];
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   for (int item = blockIdx.x; item < items; item += gridDim.x) {
-  const int mi = work[item].x;
-  const int n = nn[mi];
-  const int i0 = work[item].y * 32, k0 = work[item].z * 32;
-  __syncthreads();
-  const float *V = v + off[mi];
-  float *F = f + off[mi];
-  const float *L = lam + eoff[mi];
-  for (int r = threadIdx.y; r < 32; r += blockDim.y) {
-    const int k = k0 + r, i = i0 + threadIdx.x;
-    tile[r][threadIdx.x] = (k < n && i < n) ? V[i + static_cast<int64_t>(k) * n] * sqrtf(rootOf(L[k])) : 0.0f;
-  }
-  __syncthreads();
-  for (int r = threadIdx.y; r < 32; r += blockDim.y) {
-    const int i = i0 + r, k = k0 + threadIdx.x;
-    if (i < n && k < n) F[k + static_cast<int64_t>(i) * n] = tile[threadIdx.x][r];
-  }
+    const int mi = work[item].x;
+    const int n = nn[mi];
+    const int i0 = work[item].y * kT, k0 = work[item].z * kT;
+    const float *V = v + off[mi];
+    float *F = f + off[mi];
+    float x[kRows][2];
+#pragma unroll
+    for (int q = 0; q < kRows; ++q) {
+      const int k = k0 + kRows * warp + q;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int i = i0 + 32 * h + lane;
+        x[q][h] = k < n && i < n ? V[i + static_cast<int64_t>(k) * n] : 0.0f;
+      }
+    }
+    if (threadIdx.x < kT) {
+      const int k = k0 + threadIdx.x;
+      root[threadIdx.x] = k < n ? sqrtf(rootOf(lam[eoff[mi] + k])) : 0.0f;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < kRows; ++q)
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        tile[kRows * warp + q][32 * h + lane] = x[q][h] * root[kRows * warp + q];
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < kRows; ++q) {
+      const int r = kRows * warp + q, i = i0 + r;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int k = k0 + 32 * h + lane;
+        if (i < n && k < n) F[k + static_cast<int64_t>(i) * n] = tile[32 * h + lane][r];
+      }
+    }
+    __syncthreads();  // the tile is free for the next item
   }
 }
 
@@ -602,8 +629,8 @@ int residualFF(msq_ctx *ctx, const DeviceBatch *b, const float *a, const float *
 int makeFactor(msq_ctx *ctx, const DeviceBatch *b, const float *v, const float *lam, float *f) {
   const int4 *work;
   int items;
-  MSQ_TRY(gemmWork(ctx, b, 32, &work, &items));
-  makeFactorKernel<<<std::min(items, kSmCount * 16), dim3(32, 8), 0, ctx->stream>>>(
+  MSQ_TRY(gemmWork(ctx, b, kFactorTile, &work, &items));
+  makeFactorKernel<<<std::min(items, kSmCount * 8), 256, 0, ctx->stream>>>(
       v, lam, b->n, b->offset, b->eig_offset, f, work, items);
   return launched(ctx, "make factor");
 }

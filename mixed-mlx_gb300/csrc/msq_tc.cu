@@ -67,9 +67,33 @@ constexpr uint32_t kScaleCol0 = 256;
 constexpr int kMaxSegments = 3;
 enum Epilogue : int {
   kEpiStore = 0,     // X = acc
-  kEpiRowScale = 1,  // X_ij = acc * r_i * r_j (FP8 row-scaled factor)
+  kEpiRowScale = 1,  // X_ij = acc * r_i * r_j (FP8 row-scaled factor), mirrored
   kEpiInverseH = 2,  // X_ij = acc / (s_i + s_j), s = sqrt(lambda)
+  kEpiMirror = 3,    // X = acc, mirrored
 };
+// X = W W^T: its tiles below the diagonal are the transposes, bit for bit, of
+// those above it (the same products in the same order), so the work list
+// holds the upper ones and the epilogue stores both.  Half the MMAs and half
+// the operand traffic, which is what bounds a large order: MXFP4 at order
+// 8192 205 us (369 with every tile computed).
+constexpr bool isMirrored(int epilogue) {
+  return epilogue == kEpiRowScale || epilogue == kEpiMirror;
+}
+
+// v[q] of lane l <-> v[l] of lane q.
+__device__ __forceinline__ void transpose32(float *v, int lane) {
+#pragma unroll
+  for (int s = 16; s; s >>= 1) {
+    const bool high = lane & s;
+#pragma unroll
+    for (int q = 0; q < 32; ++q) {
+      if (q & s) continue;
+      const float got = __shfl_xor_sync(0xffffffffu, high ? v[q] : v[q + s], s);
+      if (high) v[q] = got;
+      else v[q + s] = got;
+    }
+  }
+}
 
 // Bounded wait: false (and the status word set) if the phase never completes.
 __device__ __forceinline__ bool mbarWait(uint32_t bar, uint32_t parity, int *status,
@@ -316,16 +340,24 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcGemmKernel(TcArgs args) {
             const int j = j0 + c * 32 + q;
             if (j < n) {
               const int64_t at = i + static_cast<int64_t>(j) * n;
-              float val = v[q];
               // (r_i r_j) first: the product of the two scales is the same
-              // for (i, j) and (j, i), so X stays exactly symmetric
-              if (kEpi == kEpiRowScale) val = val * (ri * rs[j]);
+              // for (i, j) and (j, i)
+              if (kEpi == kEpiRowScale) v[q] = v[q] * (ri * rs[j]);
               if (kEpi == kEpiInverseH) {
                 const float d = si + sj[q];
-                val = d > 0.0f ? val / d : 0.0f;  // both roots 0: no correction
+                v[q] = d > 0.0f ? v[q] / d : 0.0f;  // both roots 0: no correction
               }
-              X[at] = val;
+              X[at] = v[q];
             }
+          }
+        }
+        if (isMirrored(kEpi) && w.y != w.z) {
+          transpose32(v, lane);
+          const int j = j0 + c * 32 + lane, i0 = i - lane;
+          if (j < n) {
+#pragma unroll
+            for (int q = 0; q < 32; ++q)
+              if (i0 + q < n) X[j + static_cast<int64_t>(i0 + q) * n] = v[q];
           }
         }
       }
@@ -370,62 +402,113 @@ struct PackArgs {
   uint8_t *tiles;
 };
 
-// One CTA of 128 threads per tile; thread r packs row r (128 bytes).
+// kN consecutive elements at k of a row of n, zero beyond it; `vec`: the row
+// starts on a boundary of min(kN, 4) floats (and so does k).
+template <int kN>
+__device__ __forceinline__ void loadRow(const float *__restrict__ row, int k, int n, bool vec,
+                                        float *v) {
+  if (vec && k + kN <= n) {
+    if constexpr (kN == 2) {
+      const float2 t = *reinterpret_cast<const float2 *>(row + k);
+      v[0] = t.x; v[1] = t.y;
+    } else {
+#pragma unroll
+      for (int q = 0; q < kN; q += 4) {
+        const float4 t = *reinterpret_cast<const float4 *>(row + k + q);
+        v[q] = t.x; v[q + 1] = t.y; v[q + 2] = t.z; v[q + 3] = t.w;
+      }
+    }
+  } else {
+#pragma unroll
+    for (int q = 0; q < kN; ++q) v[q] = k + q < n ? row[k + q] : 0.0f;
+  }
+}
+
+// Rows of `f` (n apart) start on a boundary of kN floats, at most 16 bytes.
+template <int kN>
+__device__ __forceinline__ bool rowsAligned(const float *f, int n) {
+  constexpr uintptr_t kMask = 4 * (kN < 4 ? kN : 4) - 1;
+  return ((reinterpret_cast<uintptr_t>(f) | (4 * static_cast<uintptr_t>(n))) & kMask) == 0;
+}
+
+// Byte offset in a tile of 32-bit word `word` of row `row`.
+__device__ __forceinline__ uint32_t tileWord(int row, int word) {
+  return swizzle128(row, word >> 2) + 4 * (word & 3);
+}
+
+// One CTA of 128 threads per tile, a warp per 32 of its rows: lane l forms
+// word l of a row, so a row is read and written as whole lines, kBatch rows
+// in flight.  Bound by memory.  (A thread per row, each lane on its own
+// line: 522 us for the BF16 factors of 4096 matrices of orders 16 .. 512, 247
+// so.)
 template <int kSource>
 __global__ void __launch_bounds__(128) packKernel(PackArgs args) {
+  constexpr bool kFp8 = kSource == kPackF32Fp8Row || kSource == kPackFp8Codes;
+  constexpr bool kF32 = kSource == kPackF32Fp8Row || kSource == kPackF32Bf16;
+  constexpr int kElems = kFp8 ? 128 : 64;  // elements per 128-byte row
+  constexpr int kWord = kElems / 32;       // elements per lane
+  constexpr int kBatch = 8;
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   for (int item = blockIdx.x; item < args.items; item += gridDim.x) {
     const int4 w = args.work[item];
     const int mi = w.x, n = args.n[mi];
-    const int r = threadIdx.x;
-    const int i = w.y * kTileRows + r;
-    constexpr bool kFp8 = kSource == kPackF32Fp8Row || kSource == kPackFp8Codes;
-    constexpr int kElems = kFp8 ? 128 : 64;  // elements per 128-byte row
-    const int k0 = w.z * kElems;
+    const int k = w.z * kElems + kWord * lane;
     const int64_t off = args.f_offset[mi];
     uint8_t *tile = args.tiles + (args.tile_base[mi] + static_cast<int64_t>(w.y) * w.w + w.z) *
                                      kTileBytes;
-    const bool row_ok = i < n;
-    float inv_scale_row = 1.0f;
-    if (kSource == kPackF32Fp8Row && row_ok) inv_scale_row = args.row_scale[args.eig_offset[mi] + i];
+    const float *f = args.f + off;
+    const bool vec = kF32 && rowsAligned<kWord>(f, n);
 #pragma unroll 1
-    for (int c = 0; c < 8; ++c) {
-      uint32_t word[4] = {0, 0, 0, 0};
-      if (row_ok) {
-        if constexpr (kFp8) {
+    for (int r0 = 32 * warp; r0 < 32 * warp + 32; r0 += kBatch) {
+      const int i0 = w.y * kTileRows + r0;
+      if constexpr (kF32) {
+        float v[kBatch][kWord] = {};
+        float scale[kBatch];
 #pragma unroll
-          for (int e = 0; e < 16; ++e) {
-            const int k = k0 + c * 16 + e;
-            uint32_t code = 0;
-            if (k < n) {
-              const int64_t at = off + k + static_cast<int64_t>(i) * n;
-              code = kSource == kPackFp8Codes ? args.codes[at]
-                                              : encodeE4M3(rowDivide(args.f[at], inv_scale_row));
-            }
-            word[e / 4] |= code << (8 * (e % 4));
+        for (int q = 0; q < kBatch; ++q) {
+          if (i0 + q < n) loadRow<kWord>(f + static_cast<int64_t>(i0 + q) * n, k, n, vec, v[q]);
+          scale[q] = kSource == kPackF32Fp8Row && i0 + q < n
+                         ? args.row_scale[args.eig_offset[mi] + i0 + q]
+                         : 1.0f;
+        }
+#pragma unroll
+        for (int q = 0; q < kBatch; ++q) {
+          uint32_t word = 0;
+#pragma unroll
+          for (int e = 0; e < kWord; ++e) {
+            if (kFp8) word |= static_cast<uint32_t>(encodeE4M3(rowDivide(v[q][e], scale[q]))) << (8 * e);
+            else word |= static_cast<uint32_t>(encodeBf16(v[q][e])) << (16 * e);
           }
-        } else {
+          *reinterpret_cast<uint32_t *>(tile + tileWord(r0 + q, lane)) = word;
+        }
+      } else {
+        uint32_t word[kBatch] = {};
 #pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            const int k = k0 + c * 8 + e;
-            uint32_t h = 0;
-            if (k < n) {
-              const int64_t at = off + k + static_cast<int64_t>(i) * n;
-              if (kSource == kPackF32Bf16) {
-                h = encodeBf16(args.f[at]);
+        for (int q = 0; q < kBatch; ++q) {
+          const int64_t at0 = off + k + static_cast<int64_t>(i0 + q) * n;
+          if (i0 + q < n) {
+#pragma unroll
+            for (int e = 0; e < kWord; ++e) {
+              if (k + e >= n) continue;
+              const int64_t at = at0 + e;
+              if (kSource == kPackFp8Codes) {
+                word[q] |= static_cast<uint32_t>(args.codes[at]) << (8 * e);
               } else if (kSource == kPackBf16Codes) {
-                h = reinterpret_cast<const uint16_t *>(args.codes)[at];
+                word[q] |= static_cast<uint32_t>(reinterpret_cast<const uint16_t *>(args.codes)[at])
+                           << (16 * e);
               } else {  // kPackMxfp4Codes: exact, at most 2 significant bits
                 const uint32_t byte = args.codes[at / 2];
                 const float d = decodeE2M1((byte >> ((at & 1) * 4)) & 0xfu);
-                h = encodeBf16(mxScale(d, args.mx_scales[at / 32]));
+                word[q] |= static_cast<uint32_t>(encodeBf16(mxScale(d, args.mx_scales[at / 32])))
+                           << (16 * e);
               }
             }
-            word[e / 2] |= h << (16 * (e % 2));
           }
         }
+#pragma unroll
+        for (int q = 0; q < kBatch; ++q)
+          *reinterpret_cast<uint32_t *>(tile + tileWord(r0 + q, lane)) = word[q];
       }
-      *reinterpret_cast<uint4 *>(tile + swizzle128(r, c)) =
-          make_uint4(word[0], word[1], word[2], word[3]);
     }
   }
 }
@@ -438,8 +521,10 @@ __global__ void __launch_bounds__(128) packKernel(PackArgs args) {
 //   kMxCodesFp4  flat MXFP4 codes and scales (order divisible by 32, so
 //                the flat 32-element blocks are row blocks)
 //   kMxCodesFp8  flat MXFP8 E4M3 codes and scales (same condition)
-// One CTA of 128 threads per tile; thread r packs row r.  Blocks beyond the
-// order get zero codes and the unit scale (byte 127).
+// One CTA of 128 threads per tile, a warp per 32 of its rows, lane l word l
+// of a row (8 or 4 elements: a block is 4 or 8 lanes).  Blocks beyond the
+// order get zero codes and the unit scale (byte 127).  Bound by memory: the
+// FP32 factor of order 8192 in 64 us (244 with a thread per row).
 enum MxSource : int { kMxF32Fp4 = 0, kMxCodesFp4 = 1, kMxCodesFp8 = 2 };
 
 struct MxPackArgs {
@@ -459,80 +544,80 @@ template <int kSource>
 __global__ void __launch_bounds__(128) packMxKernel(MxPackArgs args) {
   constexpr bool kFp4 = kSource != kMxCodesFp8;
   constexpr int kElems = kFp4 ? 256 : 128;  // K per 128-byte tile row
-  constexpr int kBlocks = kElems / 32;
+  constexpr int kWord = kElems / 32;
+  constexpr int kGroup = 32 / kWord;        // lanes per block
+  constexpr int kBatch = 4;
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   for (int item = blockIdx.x; item < args.items; item += gridDim.x) {
     const int4 w = args.work[item];
     const int mi = w.x, n = args.n[mi];
-    const int r = threadIdx.x;
-    const int i = w.y * kTileRows + r;
-    const int k0 = w.z * kElems;
+    const int k = w.z * kElems + kWord * lane;
     const int64_t off = args.f_offset[mi];
     const int64_t t = args.tile_base[mi] + static_cast<int64_t>(w.y) * w.w + w.z;
     uint8_t *tile = args.tiles + t * kTileBytes;
     uint8_t *sft = args.scale_tiles + t * kScaleTileBytes;
-    uint32_t sf_word[2] = {0x7f7f7f7fu, 0x7f7f7f7fu};
+    const bool block_ok = k / 32 * 32 < n;  // the lane's block has an element
+    const float *f = args.f + off;
+    const bool vec = kSource == kMxF32Fp4 && rowsAligned<kWord>(f, n);
 #pragma unroll 1
-    for (int blk = 0; blk < kBlocks; ++blk) {
-      const int kb = k0 + 32 * blk;
-      uint32_t words[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // 32 codes: 16 (E2M1) or 32 bytes
-      uint32_t sf = 127;
-      if (i < n && kb < n) {
-        const int64_t at = off + kb + static_cast<int64_t>(i) * n;
-        if constexpr (kSource == kMxF32Fp4) {
-          float x[32];
+    for (int r0 = 32 * warp; r0 < 32 * warp + 32; r0 += kBatch) {
+      const int i0 = w.y * kTileRows + r0;
+      uint32_t word[kBatch] = {}, sf[kBatch];
+      if constexpr (kSource == kMxF32Fp4) {
+        float v[kBatch][kWord] = {};
+#pragma unroll
+        for (int q = 0; q < kBatch; ++q)
+          if (i0 + q < n) loadRow<kWord>(f + static_cast<int64_t>(i0 + q) * n, k, n, vec, v[q]);
+#pragma unroll
+        for (int q = 0; q < kBatch; ++q) {
           float m = 0.0f;
 #pragma unroll
-          for (int e = 0; e < 32; ++e) {
-            x[e] = kb + e < n ? args.f[at + e] : 0.0f;
-            const float a = fabsf(x[e]);
+          for (int e = 0; e < kWord; ++e) {
+            const float a = fabsf(v[q][e]);
             if (a <= 3.402823466e38f) m = fmaxf(m, a);
           }
-          const int ex = mxExponent(m, 2);
-          sf = static_cast<uint32_t>(ex + 127);
 #pragma unroll
-          for (int e = 0; e < 32; ++e) {
-            const uint32_t code = kb + e < n ? encodeE2M1(mxDivide(x[e], ex)) : 0u;
-            words[e / 8] |= code << (4 * (e % 8));
+          for (int s = 1; s < kGroup; s <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, s));
+          const int ex = mxExponent(m, 2);
+          sf[q] = i0 + q < n && block_ok ? static_cast<uint32_t>(ex + 127) : 127u;
+          if (ex >= -126 && ex <= 126) {
+            const float s = exp2Int(-ex);
+#pragma unroll
+            for (int e = 0; e < kWord; e += 2)
+              word[q] |= encodeE2M1Pair(v[q][e] * s, v[q][e + 1] * s, v[q][e], v[q][e + 1])
+                         << (4 * e);
+          } else {
+#pragma unroll
+            for (int e = 0; e < kWord; e += 2) {
+              const float x = mxDivide(v[q][e], ex), y = mxDivide(v[q][e + 1], ex);
+              word[q] |= encodeE2M1Pair(x, y, x, y) << (4 * e);
+            }
           }
-        } else if constexpr (kSource == kMxCodesFp4) {
-          // 16 bytes of codes at byte at / 2 (a multiple of 16), one scale
-          const uint4 c = *reinterpret_cast<const uint4 *>(args.codes + at / 2);
-          words[0] = c.x;
-          words[1] = c.y;
-          words[2] = c.z;
-          words[3] = c.w;
-          sf = args.mx_scales[at / 32];
-        } else {
-          const uint4 c0 = *reinterpret_cast<const uint4 *>(args.codes + at);
-          const uint4 c1 = *reinterpret_cast<const uint4 *>(args.codes + at + 16);
-          words[0] = c0.x;
-          words[1] = c0.y;
-          words[2] = c0.z;
-          words[3] = c0.w;
-          words[4] = c1.x;
-          words[5] = c1.y;
-          words[6] = c1.z;
-          words[7] = c1.w;
-          sf = args.mx_scales[at / 32];
+        }
+      } else {
+#pragma unroll
+        for (int q = 0; q < kBatch; ++q) {
+          sf[q] = 127;
+          if (i0 + q < n && block_ok) {
+            const int64_t at = off + k + static_cast<int64_t>(i0 + q) * n;
+            word[q] = *reinterpret_cast<const uint32_t *>(args.codes + (kFp4 ? at / 2 : at));
+            sf[q] = args.mx_scales[at / 32];
+          }
         }
       }
-      if constexpr (kFp4) {
-        *reinterpret_cast<uint4 *>(tile + swizzle128(r, blk)) =
-            make_uint4(words[0], words[1], words[2], words[3]);
-      } else {
-        *reinterpret_cast<uint4 *>(tile + swizzle128(r, 2 * blk)) =
-            make_uint4(words[0], words[1], words[2], words[3]);
-        *reinterpret_cast<uint4 *>(tile + swizzle128(r, 2 * blk + 1)) =
-            make_uint4(words[4], words[5], words[6], words[7]);
-      }
-      const int shift = 8 * (blk % 4);
-      sf_word[blk / 4] = (sf_word[blk / 4] & ~(0xffu << shift)) | (sf << shift);
-    }
-    // row r of atom a: 4 bytes at 16 (r mod 32) + 4 (r / 32)
-    const int at_row = 16 * (r % 32) + 4 * (r / 32);
 #pragma unroll
-    for (int a = 0; a < kBlocks / 4; ++a) {
-      *reinterpret_cast<uint32_t *>(sft + a * kScaleAtomBytes + at_row) = sf_word[a];
+      for (int q = 0; q < kBatch; ++q) {
+        *reinterpret_cast<uint32_t *>(tile + tileWord(r0 + q, lane)) = word[q];
+        // the four scale bytes of an atom's row: 4 bytes at 16 (r mod 32) + 4 (r / 32)
+        uint32_t bytes = sf[q] << (8 * (lane / kGroup % 4));
+        bytes |= __shfl_xor_sync(0xffffffffu, bytes, kGroup);
+        bytes |= __shfl_xor_sync(0xffffffffu, bytes, 2 * kGroup);
+        if (lane % (4 * kGroup) == 0) {
+          const int r = r0 + q;
+          *reinterpret_cast<uint32_t *>(sft + lane / (4 * kGroup) * kScaleAtomBytes +
+                                        16 * (r % 32) + 4 * (r / 32)) = bytes;
+        }
+      }
     }
   }
 }
@@ -551,66 +636,80 @@ struct SplitArgs {
   uint8_t *out[2];
 };
 
+// x, y as the low and high halves of a word of each piece.
+__device__ __forceinline__ void splitPair(float x, float y, uint32_t &first, uint32_t &second) {
+  const uint32_t x0 = encodeBf16(x), y0 = encodeBf16(y);
+  first = x0 | (y0 << 16);
+  second = static_cast<uint32_t>(encodeBf16(x - decodeBf16(static_cast<uint16_t>(x0)))) |
+           (static_cast<uint32_t>(encodeBf16(y - decodeBf16(static_cast<uint16_t>(y0)))) << 16);
+}
+
+// Bound by memory: both directions read M and write the tiles in whole
+// lines.  kTranspose false: a warp per 32 rows, lane l word l (two elements)
+// of a row, as packKernel.  kTranspose true: a thread per operand row reads
+// along M's columns with its warp, and the tile goes through shared memory
+// in its own (swizzled) layout, from which it is copied out in order.
 template <bool kTranspose>
 __global__ void __launch_bounds__(128) packSplitKernel(SplitArgs args) {
-  // kTranspose false reads operand row i from column i of M: the tile's 128
-  // columns x 64 rows are staged in shared memory with coalesced loads (a
-  // warp reads 32 consecutive elements of one column, eight columns in
-  // flight), then each thread reads its row there (stride 65: no bank
-  // conflicts).
-  constexpr int kLd = 65;
-  __shared__ float stage[kTranspose ? 1 : kTileRows * kLd];
+  __shared__ __align__(16) unsigned char image[kTranspose ? 2 : 1][kTranspose ? kTileBytes : 16];
+  constexpr int kBatch = 8;
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   for (int item = blockIdx.x; item < args.items; item += gridDim.x) {
     const int4 w = args.work[item];
     const int mi = w.x, n = args.n[mi];
-    const int r = threadIdx.x;
-    const int i = w.y * kTileRows + r;
     const int k0 = w.z * 64;
     const float *M = args.m + args.offset[mi];
     const int64_t tile = (args.tile_base[mi] + static_cast<int64_t>(w.y) * w.w + w.z) * kTileBytes;
-    if (!kTranspose) {
-      __syncthreads();  // the previous item's rows have been read
+    if constexpr (kTranspose) {
+      const int r = threadIdx.x, i = w.y * kTileRows + r;
 #pragma unroll 1
-      for (int c0 = 8 * warp; c0 < kTileRows; c0 += 32) {
-        float x[8][2];
+      for (int c = 0; c < 8; c += 2) {
+        float x[16];
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const int col = w.y * kTileRows + c0 + q;
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int k = k0 + lane + 32 * h;
-            x[q][h] = col < n && k < n ? M[k + static_cast<int64_t>(col) * n] : 0.0f;
-          }
+        for (int e = 0; e < 16; ++e) {
+          const int k = k0 + c * 8 + e;
+          x[e] = i < n && k < n ? M[i + static_cast<int64_t>(k) * n] : 0.0f;
         }
 #pragma unroll
-        for (int q = 0; q < 8; ++q)
+        for (int h = 0; h < 2; ++h) {
+          uint32_t word[2][4];
 #pragma unroll
-          for (int h = 0; h < 2; ++h) stage[(c0 + q) * kLd + lane + 32 * h] = x[q][h];
+          for (int e = 0; e < 4; ++e)
+            splitPair(x[8 * h + 2 * e], x[8 * h + 2 * e + 1], word[0][e], word[1][e]);
+#pragma unroll
+          for (int p = 0; p < 2; ++p)
+            *reinterpret_cast<uint4 *>(image[p] + swizzle128(r, c + h)) =
+                make_uint4(word[p][0], word[p][1], word[p][2], word[p][3]);
+        }
       }
       __syncthreads();
-    }
-#pragma unroll 1
-    for (int c = 0; c < 8; ++c) {
-      uint32_t word[2][4] = {};
-#pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        const int k = k0 + c * 8 + e;
-        float x = 0.0f;
-        if (kTranspose) {
-          if (i < n && k < n) x = M[i + static_cast<int64_t>(k) * n];
-        } else {
-          x = stage[r * kLd + c * 8 + e];
-        }
-        const uint32_t h0 = encodeBf16(x);
-        const uint32_t h1 = encodeBf16(x - decodeBf16(static_cast<uint16_t>(h0)));
-        word[0][e / 2] |= h0 << (16 * (e % 2));
-        word[1][e / 2] |= h1 << (16 * (e % 2));
-      }
 #pragma unroll
       for (int p = 0; p < 2; ++p) {
-        *reinterpret_cast<uint4 *>(args.out[p] + tile + swizzle128(r, c)) =
-            make_uint4(word[p][0], word[p][1], word[p][2], word[p][3]);
+        const uint4 *src = reinterpret_cast<const uint4 *>(image[p]);
+        uint4 *dst = reinterpret_cast<uint4 *>(args.out[p] + tile);
+#pragma unroll
+        for (int q = 0; q < kTileBytes / 16 / 128; ++q)
+          dst[128 * q + threadIdx.x] = src[128 * q + threadIdx.x];
+      }
+      __syncthreads();  // the image is free for the next item
+    } else {
+      const int k = k0 + 2 * lane;
+      const bool vec = rowsAligned<2>(M, n);
+#pragma unroll 1
+      for (int r0 = 32 * warp; r0 < 32 * warp + 32; r0 += kBatch) {
+        const int i0 = w.y * kTileRows + r0;
+        float v[kBatch][2] = {};
+#pragma unroll
+        for (int q = 0; q < kBatch; ++q)
+          if (i0 + q < n) loadRow<2>(M + static_cast<int64_t>(i0 + q) * n, k, n, vec, v[q]);
+#pragma unroll
+        for (int q = 0; q < kBatch; ++q) {
+          uint32_t word[2];
+          splitPair(v[q][0], v[q][1], word[0], word[1]);
+#pragma unroll
+          for (int p = 0; p < 2; ++p)
+            *reinterpret_cast<uint32_t *>(args.out[p] + tile + tileWord(r0 + q, lane)) = word[p];
+        }
       }
     }
   }
@@ -647,9 +746,9 @@ struct TcPlan {
   int count;
   int kind;
   int device_id;
-  int pack_items, gemm_items;
+  int pack_items, gemm_items, upper_items;
   int64_t total_tiles;
-  int4 *pack_work, *gemm_work;
+  int4 *pack_work, *gemm_work, *upper_work;  // upper: tiles on or above the diagonal
   int64_t *tile_base;
   int32_t *row_matrix;
   void *device;
@@ -682,7 +781,7 @@ TcPlan *tcPlan(msq_ctx *ctx, const DeviceBatch *b, int kind) {
   // K per 128-byte tile row
   const int elems = kind == kOpMxf4 ? 256 : (kind == kOpFp8 || kind == kOpMxf8) ? 128 : 64;
   std::vector<int64_t> base(b->count);
-  std::vector<int4> pack, gemm;
+  std::vector<int4> pack, gemm, upper;
   std::vector<int32_t> row_matrix;
   int64_t tiles = 0;
   std::vector<int> ids(b->count);
@@ -702,7 +801,10 @@ TcPlan *tcPlan(msq_ctx *ctx, const DeviceBatch *b, int kind) {
     const int n = b->host_n[mi];
     const int mt = (n + kTileRows - 1) / kTileRows, kt = (n + elems - 1) / elems;
     for (int a = 0; a < mt; ++a)
-      for (int c = 0; c < mt; ++c) gemm.push_back(make_int4(mi, a, c, kt));
+      for (int c = 0; c < mt; ++c) {
+        gemm.push_back(make_int4(mi, a, c, kt));
+        if (c >= a) upper.push_back(gemm.back());
+      }
   }
   auto *p = new TcPlan{};
   p->key = b->key;
@@ -711,8 +813,10 @@ TcPlan *tcPlan(msq_ctx *ctx, const DeviceBatch *b, int kind) {
   p->device_id = ctx->device;
   p->pack_items = static_cast<int>(pack.size());
   p->gemm_items = static_cast<int>(gemm.size());
+  p->upper_items = static_cast<int>(upper.size());
   p->total_tiles = tiles;
-  const size_t bytes = (pack.size() + gemm.size()) * sizeof(int4) + base.size() * sizeof(int64_t) +
+  const size_t bytes = (pack.size() + gemm.size() + upper.size()) * sizeof(int4) +
+                       base.size() * sizeof(int64_t) +
                        row_matrix.size() * sizeof(int32_t) + 64;
   char *dev = nullptr;
   if (cudaCheck(ctx, cudaMalloc(&dev, bytes), "tc plan alloc") != MSQ_OK) {
@@ -722,10 +826,12 @@ TcPlan *tcPlan(msq_ctx *ctx, const DeviceBatch *b, int kind) {
   p->device = dev;
   p->pack_work = reinterpret_cast<int4 *>(dev);
   p->gemm_work = p->pack_work + pack.size();
-  p->tile_base = reinterpret_cast<int64_t *>(p->gemm_work + gemm.size());
+  p->upper_work = p->gemm_work + gemm.size();
+  p->tile_base = reinterpret_cast<int64_t *>(p->upper_work + upper.size());
   p->row_matrix = reinterpret_cast<int32_t *>(p->tile_base + base.size());
   cudaMemcpy(p->pack_work, pack.data(), pack.size() * sizeof(int4), cudaMemcpyHostToDevice);
   cudaMemcpy(p->gemm_work, gemm.data(), gemm.size() * sizeof(int4), cudaMemcpyHostToDevice);
+  cudaMemcpy(p->upper_work, upper.data(), upper.size() * sizeof(int4), cudaMemcpyHostToDevice);
   cudaMemcpy(p->tile_base, base.data(), base.size() * sizeof(int64_t), cudaMemcpyHostToDevice);
   cudaMemcpy(p->row_matrix, row_matrix.data(), row_matrix.size() * sizeof(int32_t),
              cudaMemcpyHostToDevice);
@@ -754,9 +860,10 @@ int tcAttributes(msq_ctx *ctx) {
   MSQ_TRY(cudaCheck(ctx, cudaFuncSetAttribute(tcGemmKernel<kOpBf16, kEpiStore>, a, bytes), "tc attr"));
   MSQ_TRY(cudaCheck(ctx, cudaFuncSetAttribute(tcGemmKernel<kOpFp8, kEpiRowScale>, a, bytes), "tc attr"));
   MSQ_TRY(cudaCheck(ctx, cudaFuncSetAttribute(tcGemmKernel<kOpBf16, kEpiInverseH>, a, bytes), "tc attr"));
+  MSQ_TRY(cudaCheck(ctx, cudaFuncSetAttribute(tcGemmKernel<kOpBf16, kEpiMirror>, a, bytes), "tc attr"));
   const int mx_bytes = static_cast<int>(tcSmemBytes(kOpMxf4));
-  MSQ_TRY(cudaCheck(ctx, cudaFuncSetAttribute(tcGemmKernel<kOpMxf4, kEpiStore>, a, mx_bytes), "tc attr"));
-  MSQ_TRY(cudaCheck(ctx, cudaFuncSetAttribute(tcGemmKernel<kOpMxf8, kEpiStore>, a, mx_bytes), "tc attr"));
+  MSQ_TRY(cudaCheck(ctx, cudaFuncSetAttribute(tcGemmKernel<kOpMxf4, kEpiMirror>, a, mx_bytes), "tc attr"));
+  MSQ_TRY(cudaCheck(ctx, cudaFuncSetAttribute(tcGemmKernel<kOpMxf8, kEpiMirror>, a, mx_bytes), "tc attr"));
   done_mask.fetch_or(bit);
   return MSQ_OK;
 }
@@ -771,8 +878,8 @@ int launchTcGemm(msq_ctx *ctx, const DeviceBatch *b, TcPlan *p, int epilogue, in
   TcArgs args{};
   args.scales_a = scale_tiles;
   args.scales_b = scale_tiles;
-  args.work = p->gemm_work;
-  args.items = p->gemm_items;
+  args.work = isMirrored(epilogue) ? p->upper_work : p->gemm_work;
+  args.items = isMirrored(epilogue) ? p->upper_items : p->gemm_items;
   args.segments = segments;
   for (int s = 0; s < segments; ++s) {
     args.tiles_a[s] = a_tiles[s];
@@ -787,22 +894,25 @@ int launchTcGemm(msq_ctx *ctx, const DeviceBatch *b, TcPlan *p, int epilogue, in
   args.x = x;
   args.status = ctx->d_status;
   args.wait_test = waitTestMode() == kWaitTestMbarrier;
-  const unsigned grid = std::min(p->gemm_items, kSmCount);
+  const unsigned grid = std::min(args.items, kSmCount);
   const size_t smem = tcSmemBytes(p->kind);
   if (isBlockScaled(p->kind)) {
-    if (scale_tiles == nullptr || segments != 1 || epilogue != kEpiStore) {
-      return setError(ctx, MSQ_ERR_INVALID_ARGUMENT, "block-scaled GEMM: one segment, store");
+    if (scale_tiles == nullptr || segments != 1 || epilogue != kEpiMirror) {
+      return setError(ctx, MSQ_ERR_INVALID_ARGUMENT, "block-scaled GEMM: one segment, W W^T");
     }
     if (p->kind == kOpMxf4) {
-      tcGemmKernel<kOpMxf4, kEpiStore><<<grid, kTcThreads, smem, ctx->stream>>>(args);
+      tcGemmKernel<kOpMxf4, kEpiMirror><<<grid, kTcThreads, smem, ctx->stream>>>(args);
     } else {
-      tcGemmKernel<kOpMxf8, kEpiStore><<<grid, kTcThreads, smem, ctx->stream>>>(args);
+      tcGemmKernel<kOpMxf8, kEpiMirror><<<grid, kTcThreads, smem, ctx->stream>>>(args);
     }
     return launched(ctx, what);
   }
   switch (epilogue) {
     case kEpiRowScale:
       tcGemmKernel<kOpFp8, kEpiRowScale><<<grid, kTcThreads, smem, ctx->stream>>>(args);
+      break;
+    case kEpiMirror:
+      tcGemmKernel<kOpBf16, kEpiMirror><<<grid, kTcThreads, smem, ctx->stream>>>(args);
       break;
     case kEpiInverseH:
       tcGemmKernel<kOpBf16, kEpiInverseH><<<grid, kTcThreads, smem, ctx->stream>>>(args);
@@ -817,7 +927,7 @@ int launchTcGemm(msq_ctx *ctx, const DeviceBatch *b, TcPlan *p, int epilogue, in
 int runTcGemm(msq_ctx *ctx, const DeviceBatch *b, TcPlan *p, const uint8_t *tiles,
               const float *row_scale, float *x) {
   const uint8_t *t[1] = {tiles};
-  return launchTcGemm(ctx, b, p, p->kind == kOpFp8 ? kEpiRowScale : kEpiStore, 1, t, t,
+  return launchTcGemm(ctx, b, p, p->kind == kOpFp8 ? kEpiRowScale : kEpiMirror, 1, t, t,
                       row_scale, nullptr, x, "tcgen05 reconstruction");
 }
 
@@ -844,7 +954,7 @@ int launchPackMx(msq_ctx *ctx, const DeviceBatch *b, TcPlan *p, const float *f,
 int runMxGemm(msq_ctx *ctx, const DeviceBatch *b, TcPlan *p, const uint8_t *tiles,
               const uint8_t *scale_tiles, float *x) {
   const uint8_t *t[1] = {tiles};
-  return launchTcGemm(ctx, b, p, kEpiStore, 1, t, t, nullptr, nullptr, x,
+  return launchTcGemm(ctx, b, p, kEpiMirror, 1, t, t, nullptr, nullptr, x,
                       "tcgen05 reconstruction", scale_tiles);
 }
 

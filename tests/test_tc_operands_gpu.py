@@ -1,0 +1,75 @@
+"""The operand packs and the mirrored tiles of the tensor-core products at the
+edges of tiles, of 32-element blocks and of vector alignment (an odd order
+before an even one), against FP64 products of the oracle's quantized factor.
+
+Tolerances (relative Frobenius): FP32 accumulation of exact products, 2e-6;
+the split-BF16 correction drops a term of 2^-18 and rounds two second pieces
+at 2^-18 in each of its four products, 12 2^-18 and four accumulations; the
+factor is two square roots and a product, each rounded once (2^-22)."""
+import numpy as np
+import pytest
+
+import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+ACC = 2e-6
+ORDERS = [[1, 2, 31], [33, 64, 128], [127, 129, 34, 255], [257, 256, 63, 130], [640]]
+
+
+def _dev(x):
+    import torch
+    return torch.from_numpy(np.ascontiguousarray(x, np.float32)).cuda()
+
+
+def _quantized(fmt, f):
+    n = f.shape[0]
+    row = n if fmt == 8 else 0
+    cols = [O.decode(fmt, *O.encode(fmt, np.ascontiguousarray(f[:, i]), row_length=row), n, row_length=row)
+            for i in range(n)]
+    return np.stack(cols, axis=1).astype(np.float64)
+
+
+@pytest.mark.parametrize("orders", ORDERS)
+@pytest.mark.parametrize("plan,fmt", [(1, 1), (2, 8), (3, 7)])
+def test_reconstruction_from_the_factor(ctx, msq, orders, plan, fmt):
+    import torch
+    b = msq.Batch.from_orders(orders)
+    rng = np.random.default_rng(orders[0])
+    fs = []
+    for n in orders:
+        f = rng.standard_normal((n, n)) * 2.0 ** rng.integers(-12, 1, (n, n))
+        f[: n // 2, n // 3] = 0.0  # zero blocks of a row
+        fs.append(f.astype(np.float32))
+    x = ctx.reconstruct_factor(plan, _dev(b.pack(fs)), b)
+    torch.cuda.synchronize()
+    for f, xg in zip(fs, b.unpack(x.cpu().numpy())):
+        q = _quantized(fmt, f)
+        ref = q.T @ q
+        assert np.linalg.norm(xg - ref) <= ACC * np.linalg.norm(ref), f.shape
+        assert np.array_equal(xg, xg.T)
+
+
+@pytest.mark.parametrize("orders", ORDERS)
+def test_factor_and_split_correction(ctx, msq, orders):
+    import torch
+    b = msq.Batch.from_orders(orders)
+    rng = np.random.default_rng(orders[-1])
+    mats = [(rng.standard_normal((n, n)) / np.sqrt(n)).astype(np.float32) for n in orders]
+    res = [rng.standard_normal((n, n)) * 1e-3 for n in orders]
+    res = [(r + r.T).astype(np.float32) for r in res]
+    lam = rng.uniform(0.1, 1.0, int(b.n.sum())).astype(np.float32)
+    v = _dev(b.pack(mats))
+    f = ctx.make_factor(v, _dev(lam), b)
+    hi, lo = torch.zeros_like(v), torch.zeros_like(v)
+    ctx.sylvester_sweep(msq.BF16, v, _dev(lam), _dev(b.pack(res)), b, hi, lo)
+    torch.cuda.synchronize()
+    at = 0
+    for n, m, r, fg, eg in zip(orders, mats, res, b.unpack(f.cpu().numpy()), b.unpack(hi.cpu().numpy())):
+        m, r, s = m.astype(np.float64), r.astype(np.float64), np.sqrt(lam[at:at + n].astype(np.float64))
+        at += n
+        np.testing.assert_allclose(fg, (m * np.sqrt(s)).T, rtol=2.0**-22, atol=0)
+        c = (m.T @ r @ m) / (s[:, None] + s[None, :])
+        e = m @ c @ m.T
+        e = 0.5 * (e + e.T)
+        assert np.linalg.norm(eg - e) <= (12 * 2.0**-18 + 4 * ACC) * np.linalg.norm(e), n
