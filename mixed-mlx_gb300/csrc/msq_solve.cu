@@ -42,9 +42,8 @@ int sylvesterSweep(msq_ctx *ctx, const DeviceBatch *b, int gemm_format, const fl
                    const float *lam, const float *r, float *x_hi, float *x_lo, float *ws0,
                    float *ws1, bool basis_packed) {
   if (gemm_format == MSQ_FMT_BF16) {
-    float *e = nullptr;
-    MSQ_TRY(sylvesterTc(ctx, b, v, lam, r, ws0, ws1, &e, basis_packed));
-    return symmetricAdd(ctx, b, x_hi, x_lo, e);
+    MSQ_TRY(sylvesterTc(ctx, b, v, lam, r, ws1, basis_packed));
+    return symmetricAdd(ctx, b, x_hi, x_lo, ws1);
   }
   return sylvesterFp32(ctx, b, v, lam, r, x_hi, x_lo, ws0, ws1);
 }

@@ -29,14 +29,12 @@ int reconstructLowBit(msq_ctx *ctx, const DeviceBatch *b, int format, const floa
 int reconstructEncoded(msq_ctx *ctx, const DeviceBatch *b, int format, const void *values,
                        const void *scales, float *x);
 
-// msq_tc.cu — tensor-core Sylvester GEMM chain (the correction is returned in
-// *correction, one of ws0/ws1).  basis_packed:
+// msq_tc.cu — tensor-core Sylvester GEMM chain into `correction`.  basis_packed:
 // the split operands of V and V^T are still those of the previous chain on
 // the same V and batch (no tensor-core call in between), so they are not
 // packed again.
 int sylvesterTc(msq_ctx *ctx, const DeviceBatch *b, const float *v, const float *lam,
-                const float *r, float *ws0, float *ws1, float **correction,
-                bool basis_packed = false);
+                const float *r, float *correction, bool basis_packed = false);
 
 // msq_codecs.cu — x <- decode(encode(x)) for every matrix of the batch in
 // one launch (MX blocks and scale rows within each matrix).

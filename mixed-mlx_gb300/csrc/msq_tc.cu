@@ -10,11 +10,11 @@
 //     (16-byte chunk index XOR row mod 8 inside each 1024-byte atom), so a
 //     tile is one contiguous 16 KB block that a single TMA bulk copy
 //     (cp.async.bulk) lands in shared memory ready for the MMA;
-//   * tcGemmKernel is a persistent, warp-specialized kernel: warp 4 issues
-//     the bulk copies into a 4-stage mbarrier ring, warp 5 owns TMEM (256
+//   * tcGemmKernel is a persistent, warp-specialized kernel: one warp issues
+//     the bulk copies into an mbarrier ring, one owns TMEM (256
 //     columns: two 128x128 FP32 accumulators) and issues tcgen05.mma
 //     (kind::f16 for BF16, kind::f8f6f4 for FP8 E4M3) from one thread, and
-//     warps 0-3 drain the other accumulator with tcgen05.ld while the next
+//     sixteen warps drain the other accumulator with tcgen05.ld while the next
 //     tile accumulates, applying the per-row FP8 scales r_i r_j.
 // MX factors (E2M1 or E4M3 with one UE8M0 scale per 32 along K of a row;
 // the reference's K-major MX operand with scale stride ld / 32,
@@ -44,7 +44,6 @@ namespace {
 constexpr int kTileRows = 128;
 constexpr int kTileBytes = 16384;  // 128 rows x 128 bytes
 constexpr int kStages = 4;
-constexpr int kTcThreads = 192;    // warps 0-3 epilogue, 4 producer, 5 MMA
 constexpr uint32_t kTmemCols = 256;
 constexpr long long kWaitLimit = 1ll << 26;
 
@@ -64,13 +63,38 @@ constexpr int kScaleTileBytes = 2 * kScaleAtomBytes;
 // columns (A atoms at +0, +4, B atoms at +8, +12).
 constexpr uint32_t kTmemColsMx = 512;
 constexpr uint32_t kScaleCol0 = 256;
-constexpr int kMaxSegments = 3;
 enum Epilogue : int {
-  kEpiStore = 0,     // X = acc
+  kEpiStore = 0,     // split product, X = acc
   kEpiRowScale = 1,  // X_ij = acc * r_i * r_j (FP8 row-scaled factor), mirrored
-  kEpiInverseH = 2,  // X_ij = acc / (s_i + s_j), s = sqrt(lambda)
+  kEpiInverseH = 2,  // split product, acc / (s_i + s_j), s = sqrt(lambda), packed
   kEpiMirror = 3,    // X = acc, mirrored
+  kEpiPacked = 4,    // split product, acc packed
 };
+// Split products: A and B each in two BF16 pieces, a0 b0 + a0 b1 + a1 b0 (the
+// dropped a1 b1 is below 2^-16 of the product).  A stage holds the four tiles
+// of 64 of K, so each is brought once (with one product after the other the
+// first pieces came twice): operand traffic bounds the loop.  E = Z V^T of
+// 4096 matrices of orders 16 .. 512: 0.60 ms with a segment per product, 0.44
+// so.
+constexpr bool isSplit(int epilogue) {
+  return epilogue == kEpiStore || epilogue == kEpiInverseH || epilogue == kEpiPacked;
+}
+// Packed: the result goes out as the two pieces of the next product's
+// operand (operand row j = column j of X) instead of to FP32 and through
+// packSplitKernel, a third of the bytes: 0.57 ms, of which the pack alone
+// took 0.39 after a product of 0.60.
+constexpr bool isPacked(int epilogue) { return epilogue == kEpiInverseH || epilogue == kEpiPacked; }
+constexpr int stageTiles(int epilogue) { return isSplit(epilogue) ? 4 : 2; }
+constexpr int ringStages(int epilogue) { return isSplit(epilogue) ? 3 : kStages; }
+// Epilogue warps; then the producer warp and the MMA warp.  A split product's
+// epilogue (a division, two roundings, a shuffle per element) is as long as
+// its K loop at orders up to 512, and one warp per TMEM sub-partition does
+// not hide its latency: C = V^T G / H of 4096 matrices of orders 16 .. 512
+// takes 2.58 ms with four warps, 1.05 with sixteen.  A mirrored one only
+// stores, and sixteen warps' bursts of stores come in the way of the operand
+// loads: order 8192 in MXFP4 205 us with four warps, 213 with sixteen.
+constexpr int epilogueWarps(int epilogue) { return isSplit(epilogue) ? 16 : 4; }
+constexpr int tcThreads(int epilogue) { return 32 * (epilogueWarps(epilogue) + 2); }
 // X = W W^T: its tiles below the diagonal are the transposes, bit for bit, of
 // those above it (the same products in the same order), so the work list
 // holds the upper ones and the epilogue stores both.  Half the MMAs and half
@@ -132,12 +156,12 @@ __device__ __forceinline__ void mmaIssue(uint32_t tmem, uint64_t a, uint64_t b, 
 struct TcArgs {
   const int4 *work;        // (matrix, tile_m, tile_n, k_tiles)
   int items;
-  // The accumulator sums A_s B_s^T over `segments` operand pairs (split-BF16
-  // products); every packed operand shares the plan's tile geometry.
-  int segments;
-  const uint8_t *tiles_a[kMaxSegments];
-  const uint8_t *tiles_b[kMaxSegments];
-  const uint8_t *scales_a; // block-scaled kinds: scale-factor tiles (one segment)
+  // the operands' pieces (one, or two of a split product); every packed
+  // operand shares the plan's tile geometry
+  const uint8_t *tiles_a[2];
+  const uint8_t *tiles_b[2];
+  uint8_t *out[2];         // packed epilogues: the pieces of the result
+  const uint8_t *scales_a; // block-scaled kinds: scale-factor tiles
   const uint8_t *scales_b;
   const int64_t *tile_base;// per matrix: first tile index
   const int32_t *n;
@@ -151,36 +175,39 @@ struct TcArgs {
 };
 
 template <int kKind, int kEpi>
-__global__ void __launch_bounds__(kTcThreads, 1) tcGemmKernel(TcArgs args) {
+__global__ void __launch_bounds__(tcThreads(kEpi), 1) tcGemmKernel(TcArgs args) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char *base = reinterpret_cast<unsigned char *>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   constexpr bool kMx = isBlockScaled(kKind);
+  constexpr int kWarps = epilogueWarps(kEpi), kProducerWarp = kWarps, kMmaWarp = kWarps + 1;
   constexpr uint32_t kCols = kMx ? kTmemColsMx : kTmemCols;
-  unsigned char *stage_mem = base;  // kStages x (A 16 KB, B 16 KB)
+  constexpr int kPieces = isSplit(kEpi) ? 2 : 1, kRing = ringStages(kEpi);
+  constexpr int kStageBytes = stageTiles(kEpi) * kTileBytes;
+  unsigned char *stage_mem = base;  // kRing x (pieces of A, pieces of B)
   // block-scaled kinds: kStages x (SFA 1 KB, SFB 1 KB) after the operands
-  unsigned char *scale_mem = base + kStages * 2 * kTileBytes;
-  uint64_t *bars = reinterpret_cast<uint64_t *>(base + kStages * 2 * kTileBytes +
-                                                (kMx ? kStages * 2 * kScaleTileBytes : 0));
-  uint64_t *full = bars, *empty = bars + kStages;
-  uint64_t *acc_full = bars + 2 * kStages, *acc_empty = acc_full + 2;
+  unsigned char *scale_mem = base + kRing * kStageBytes;
+  uint64_t *bars = reinterpret_cast<uint64_t *>(base + kRing * kStageBytes +
+                                                (kMx ? kRing * 2 * kScaleTileBytes : 0));
+  uint64_t *full = bars, *empty = bars + kRing;
+  uint64_t *acc_full = bars + 2 * kRing, *acc_empty = acc_full + 2;
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_empty + 2);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kStages; ++s) {
+    for (int s = 0; s < kRing; ++s) {
       mbarInit(smemAddr(&full[s]), 1);
       mbarInit(smemAddr(&empty[s]), 1);
     }
     for (int a = 0; a < 2; ++a) {
       mbarInit(smemAddr(&acc_full[a]), 1);
-      mbarInit(smemAddr(&acc_empty[a]), 128);
+      mbarInit(smemAddr(&acc_empty[a]), 32 * kWarps);
     }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 5) {
+  if (warp == kMmaWarp) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      smemAddr(tmem_slot)),
                  "r"(kCols));
@@ -191,7 +218,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcGemmKernel(TcArgs args) {
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t tmem = *tmem_slot;
 
-  if (warp == 4) {
+  if (warp == kProducerWarp) {
     if (lane == 0) {
       int stage = 0;
       uint32_t phase = 0;
@@ -204,37 +231,35 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcGemmKernel(TcArgs args) {
       }
       for (int item = blockIdx.x; item < args.items && !*abort_flag; item += gridDim.x) {
         const int4 w = args.work[item];
-        const int64_t base = args.tile_base[w.x] * kTileBytes;
-        for (int seg = 0; seg < args.segments; ++seg) {
-          const uint8_t *ta = args.tiles_a[seg] + base;
-          const uint8_t *tb = args.tiles_b[seg] + base;
-          for (int kt = 0; kt < w.w; ++kt) {
-            if (!mbarWait(smemAddr(&empty[stage]), phase ^ 1, args.status, abort_flag)) break;
-            const uint32_t bar = smemAddr(&full[stage]);
-            mbarArriveExpectTx(bar, 2 * kTileBytes + (kMx ? 2 * kScaleTileBytes : 0));
-            unsigned char *dst = stage_mem + stage * 2 * kTileBytes;
-            const int64_t tile_a = args.tile_base[w.x] + static_cast<int64_t>(w.y) * w.w + kt;
-            const int64_t tile_b = args.tile_base[w.x] + static_cast<int64_t>(w.z) * w.w + kt;
-            bulkLoad(smemAddr(dst), ta + (static_cast<int64_t>(w.y) * w.w + kt) * kTileBytes,
+        const int64_t tile_a = args.tile_base[w.x] + static_cast<int64_t>(w.y) * w.w;
+        const int64_t tile_b = args.tile_base[w.x] + static_cast<int64_t>(w.z) * w.w;
+        for (int kt = 0; kt < w.w; ++kt) {
+          if (!mbarWait(smemAddr(&empty[stage]), phase ^ 1, args.status, abort_flag)) break;
+          const uint32_t bar = smemAddr(&full[stage]);
+          mbarArriveExpectTx(bar, kStageBytes + (kMx ? 2 * kScaleTileBytes : 0));
+          unsigned char *dst = stage_mem + stage * kStageBytes;
+#pragma unroll
+          for (int p = 0; p < kPieces; ++p) {
+            bulkLoad(smemAddr(dst + p * kTileBytes), args.tiles_a[p] + (tile_a + kt) * kTileBytes,
                      kTileBytes, bar);
-            bulkLoad(smemAddr(dst + kTileBytes),
-                     tb + (static_cast<int64_t>(w.z) * w.w + kt) * kTileBytes, kTileBytes, bar);
-            if constexpr (kMx) {
-              unsigned char *sdst = scale_mem + stage * 2 * kScaleTileBytes;
-              bulkLoad(smemAddr(sdst), args.scales_a + tile_a * kScaleTileBytes, kScaleTileBytes,
-                       bar);
-              bulkLoad(smemAddr(sdst + kScaleTileBytes), args.scales_b + tile_b * kScaleTileBytes,
-                       kScaleTileBytes, bar);
-            }
-            if (++stage == kStages) {
-              stage = 0;
-              phase ^= 1;
-            }
+            bulkLoad(smemAddr(dst + (kPieces + p) * kTileBytes),
+                     args.tiles_b[p] + (tile_b + kt) * kTileBytes, kTileBytes, bar);
+          }
+          if constexpr (kMx) {
+            unsigned char *sdst = scale_mem + stage * 2 * kScaleTileBytes;
+            bulkLoad(smemAddr(sdst), args.scales_a + (tile_a + kt) * kScaleTileBytes,
+                     kScaleTileBytes, bar);
+            bulkLoad(smemAddr(sdst + kScaleTileBytes),
+                     args.scales_b + (tile_b + kt) * kScaleTileBytes, kScaleTileBytes, bar);
+          }
+          if (++stage == kRing) {
+            stage = 0;
+            phase ^= 1;
           }
         }
       }
     }
-  } else if (warp == 5) {
+  } else if (warp == kMmaWarp) {
     if (lane == 0) {
       int stage = 0;
       uint32_t phase = 0;
@@ -245,13 +270,12 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcGemmKernel(TcArgs args) {
         if (!mbarWait(smemAddr(&acc_empty[acc]), acc_phase ^ 1, args.status, abort_flag)) break;
         asm volatile("tcgen05.fence::after_thread_sync;");
         const uint32_t d = tmem + acc * 128;
-        const int steps = args.segments * w.w;
-        for (int step = 0; step < steps; ++step) {
+        for (int step = 0; step < w.w; ++step) {
           if (!mbarWait(smemAddr(&full[stage]), phase, args.status, abort_flag)) break;
           asm volatile("tcgen05.fence::after_thread_sync;");
-          const uint32_t a_addr = smemAddr(stage_mem + stage * 2 * kTileBytes);
+          const uint32_t a_addr = smemAddr(stage_mem + stage * kStageBytes);
           const uint64_t adesc = smemDesc(a_addr);
-          const uint64_t bdesc = smemDesc(a_addr + kTileBytes);
+          const uint64_t bdesc = smemDesc(a_addr + kPieces * kTileBytes);
           // 128 bytes of K per stage: four MMAs of 32 bytes (K = 16 BF16, 32
           // FP8 or 64 E2M1); the start address advances inside the swizzle
           // atom.
@@ -284,10 +308,15 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcGemmKernel(TcArgs args) {
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk) {
               mmaIssue<kKind>(d, adesc + 2 * kk, bdesc + 2 * kk, (step | kk) != 0);
+              if constexpr (isSplit(kEpi)) {
+                constexpr uint64_t kSecond = kTileBytes >> 4;  // the second piece's tile
+                mmaIssue<kKind>(d, adesc + 2 * kk, bdesc + kSecond + 2 * kk, 1);
+                mmaIssue<kKind>(d, adesc + kSecond + 2 * kk, bdesc + 2 * kk, 1);
+              }
             }
           }
           mmaCommit(smemAddr(&empty[stage]));
-          if (++stage == kStages) {
+          if (++stage == kRing) {
             stage = 0;
             phase ^= 1;
           }
@@ -300,7 +329,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcGemmKernel(TcArgs args) {
       }
     }
   } else {
-    // Epilogue: thread t owns accumulator row t (TMEM lane t).
+    // Epilogue: warp w has rows 32 (w mod 4) .. of the accumulator, a lane one
+    // row (TMEM lane), and every kWarps / 4 th chunk of 32 columns.
+    const int row = 32 * (warp % 4) + lane;
     int acc = 0;
     uint32_t acc_phase = 0;
     for (int item = blockIdx.x; item < args.items; item += gridDim.x) {
@@ -309,8 +340,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcGemmKernel(TcArgs args) {
       asm volatile("tcgen05.fence::after_thread_sync;");
       const int mi = w.x;
       const int n = args.n[mi];
-      const int i = w.y * kTileRows + threadIdx.x;
-      const int j0 = w.z * kTileRows;
+      const int i = w.y * kTileRows + row;
       float *X = args.x + args.x_offset[mi];
       float ri = 1.0f;
       const float *rs = nullptr;
@@ -322,38 +352,60 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcGemmKernel(TcArgs args) {
       const float si = kEpi == kEpiInverseH && i < n ? sqrtf(fmaxf(lam[i], 0.0f)) : 0.0f;
 
 #pragma unroll 1
-      for (int c = 0; c < 4; ++c) {
+      for (int c = warp / 4; c < 4; c += kWarps / 4) {
+        const int j0 = w.z * kTileRows + 32 * c;
         float v[32];
-        tmemLoad32(tmem + ((32u * warp) << 16) + acc * 128 + c * 32, v);
+        tmemLoad32(tmem + ((32u * (warp % 4)) << 16) + acc * 128 + c * 32, v);
+        asm volatile("tcgen05.fence::before_thread_sync;");
+        if (c + kWarps / 4 >= 4) mbarArrive(smemAddr(&acc_empty[acc]));  // in registers: it is free
         // s_j of this chunk's 32 columns: one square root per lane (not one
         // per element), spread over the warp by shuffles that every lane runs
-        float sj[32];
         if (kEpi == kEpiInverseH) {
-          const int jl = j0 + c * 32 + lane;
+          const int jl = j0 + lane;
           const float mine = jl < n ? sqrtf(fmaxf(lam[jl], 0.0f)) : 0.0f;
 #pragma unroll
-          for (int q = 0; q < 32; ++q) sj[q] = __shfl_sync(0xffffffffu, mine, q);
+          for (int q = 0; q < 32; ++q) {
+            const float d = si + __shfl_sync(0xffffffffu, mine, q);
+            v[q] = d > 0.0f ? v[q] / d : 0.0f;  // both roots 0: no correction
+          }
         }
-        if (i < n) {
+        if constexpr (isPacked(kEpi)) {
+          // Element (i, j) is k = i of operand row j.  Lanes 2l and 2l + 1
+          // exchange pieces: the even one stores both first pieces, the odd
+          // one both second pieces, zeros beyond the order.
+          const int k = (w.y * kTileRows + row) & ~1, kt = k / 64;
+          uint8_t *out = (lane & 1 ? args.out[1] : args.out[0]) +
+                         (args.tile_base[mi] + static_cast<int64_t>(w.z) * w.w + kt) * kTileBytes +
+                         4 * (k / 2 % 4);
 #pragma unroll
           for (int q = 0; q < 32; ++q) {
-            const int j = j0 + c * 32 + q;
+            float x = v[q];
+            if (i >= n || j0 + q >= n) x = 0.0f;
+            const uint32_t first = encodeBf16(x);
+            const uint32_t second =
+                encodeBf16(x - decodeBf16(static_cast<uint16_t>(first)));
+            const uint32_t mine = lane & 1 ? second : first;
+            const uint32_t other = __shfl_xor_sync(0xffffffffu, lane & 1 ? first : second, 1);
+            if (kt < w.w) {
+              *reinterpret_cast<uint32_t *>(out + swizzle128(c * 32 + q, k / 8 % 8)) =
+                  lane & 1 ? other | (mine << 16) : mine | (other << 16);
+            }
+          }
+        } else if (i < n) {
+#pragma unroll
+          for (int q = 0; q < 32; ++q) {
+            const int j = j0 + q;
             if (j < n) {
-              const int64_t at = i + static_cast<int64_t>(j) * n;
               // (r_i r_j) first: the product of the two scales is the same
               // for (i, j) and (j, i)
               if (kEpi == kEpiRowScale) v[q] = v[q] * (ri * rs[j]);
-              if (kEpi == kEpiInverseH) {
-                const float d = si + sj[q];
-                v[q] = d > 0.0f ? v[q] / d : 0.0f;  // both roots 0: no correction
-              }
-              X[at] = v[q];
+              X[i + static_cast<int64_t>(j) * n] = v[q];
             }
           }
         }
         if (isMirrored(kEpi) && w.y != w.z) {
           transpose32(v, lane);
-          const int j = j0 + c * 32 + lane, i0 = i - lane;
+          const int j = j0 + lane, i0 = i - lane;
           if (j < n) {
 #pragma unroll
             for (int q = 0; q < 32; ++q)
@@ -361,8 +413,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcGemmKernel(TcArgs args) {
           }
         }
       }
-      asm volatile("tcgen05.fence::before_thread_sync;");
-      mbarArrive(smemAddr(&acc_empty[acc]));
       if (++acc == 2) {
         acc = 0;
         acc_phase ^= 1;
@@ -372,7 +422,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcGemmKernel(TcArgs args) {
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;");
-  if (warp == 5) {
+  if (warp == kMmaWarp) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
                  "r"(kCols));
   }
@@ -845,90 +895,61 @@ TcPlan *tcPlan(msq_ctx *ctx, const DeviceBatch *b, int kind) {
   return p;
 }
 
-size_t tcSmemBytes(int kind = kOpBf16) {
-  return kStages * 2 * kTileBytes + (isBlockScaled(kind) ? kStages * 2 * kScaleTileBytes : 0) +
+size_t tcSmemBytes(int kind, int epilogue) {
+  return ringStages(epilogue) *
+             (stageTiles(epilogue) * kTileBytes + (isBlockScaled(kind) ? 2 * kScaleTileBytes : 0)) +
          1024 + 256;
 }
 
-// Opt-in shared memory of the GEMM kernels, once per device.
-int tcAttributes(msq_ctx *ctx) {
+// One launch of tcGemmKernel<kKind, kEpi>, its opt-in shared memory set once
+// per device.
+template <int kKind, int kEpi>
+int launchTcKernel(msq_ctx *ctx, const TcArgs &args, const char *what) {
   static std::atomic<uint64_t> done_mask{0};
   const uint64_t bit = ctx->device >= 0 && ctx->device < 64 ? uint64_t{1} << ctx->device : 0;
-  if (bit != 0 && (done_mask.load() & bit)) return MSQ_OK;
-  const int bytes = static_cast<int>(tcSmemBytes());
-  const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
-  MSQ_TRY(cudaCheck(ctx, cudaFuncSetAttribute(tcGemmKernel<kOpBf16, kEpiStore>, a, bytes), "tc attr"));
-  MSQ_TRY(cudaCheck(ctx, cudaFuncSetAttribute(tcGemmKernel<kOpFp8, kEpiRowScale>, a, bytes), "tc attr"));
-  MSQ_TRY(cudaCheck(ctx, cudaFuncSetAttribute(tcGemmKernel<kOpBf16, kEpiInverseH>, a, bytes), "tc attr"));
-  MSQ_TRY(cudaCheck(ctx, cudaFuncSetAttribute(tcGemmKernel<kOpBf16, kEpiMirror>, a, bytes), "tc attr"));
-  const int mx_bytes = static_cast<int>(tcSmemBytes(kOpMxf4));
-  MSQ_TRY(cudaCheck(ctx, cudaFuncSetAttribute(tcGemmKernel<kOpMxf4, kEpiMirror>, a, mx_bytes), "tc attr"));
-  MSQ_TRY(cudaCheck(ctx, cudaFuncSetAttribute(tcGemmKernel<kOpMxf8, kEpiMirror>, a, mx_bytes), "tc attr"));
-  done_mask.fetch_or(bit);
-  return MSQ_OK;
+  const size_t smem = tcSmemBytes(kKind, kEpi);
+  if (bit == 0 || !(done_mask.load() & bit)) {
+    MSQ_TRY(cudaCheck(ctx, cudaFuncSetAttribute(tcGemmKernel<kKind, kEpi>,
+                                                cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                static_cast<int>(smem)), "tc attr"));
+    done_mask.fetch_or(bit);
+  }
+  const unsigned grid = std::min(args.items, kSmCount);
+  tcGemmKernel<kKind, kEpi><<<grid, tcThreads(kEpi), smem, ctx->stream>>>(args);
+  return launched(ctx, what);
 }
 
-// Launches the persistent tcgen05 GEMM over the plan's work list:
-// X = sum_s A_s B_s^T per matrix with the given epilogue.
-int launchTcGemm(msq_ctx *ctx, const DeviceBatch *b, TcPlan *p, int epilogue, int segments,
-                 const uint8_t *const *a_tiles, const uint8_t *const *b_tiles,
-                 const float *row_scale, const float *eigenvalues, float *x, const char *what,
-                 const uint8_t *scale_tiles = nullptr) {
-  MSQ_TRY(tcAttributes(ctx));
+// The persistent tcgen05 GEMM over the plan's work list: A B^T per matrix
+// with the given epilogue.
+TcArgs tcArgs(msq_ctx *ctx, const DeviceBatch *b, const TcPlan *p, int epilogue) {
   TcArgs args{};
-  args.scales_a = scale_tiles;
-  args.scales_b = scale_tiles;
   args.work = isMirrored(epilogue) ? p->upper_work : p->gemm_work;
   args.items = isMirrored(epilogue) ? p->upper_items : p->gemm_items;
-  args.segments = segments;
-  for (int s = 0; s < segments; ++s) {
-    args.tiles_a[s] = a_tiles[s];
-    args.tiles_b[s] = b_tiles[s];
-  }
   args.tile_base = p->tile_base;
   args.n = b->n;
   args.x_offset = b->offset;
   args.eig_offset = b->eig_offset;
-  args.row_scale = row_scale;
-  args.eigenvalues = eigenvalues;
-  args.x = x;
   args.status = ctx->d_status;
   args.wait_test = waitTestMode() == kWaitTestMbarrier;
-  const unsigned grid = std::min(args.items, kSmCount);
-  const size_t smem = tcSmemBytes(p->kind);
-  if (isBlockScaled(p->kind)) {
-    if (scale_tiles == nullptr || segments != 1 || epilogue != kEpiMirror) {
-      return setError(ctx, MSQ_ERR_INVALID_ARGUMENT, "block-scaled GEMM: one segment, W W^T");
-    }
-    if (p->kind == kOpMxf4) {
-      tcGemmKernel<kOpMxf4, kEpiMirror><<<grid, kTcThreads, smem, ctx->stream>>>(args);
-    } else {
-      tcGemmKernel<kOpMxf8, kEpiMirror><<<grid, kTcThreads, smem, ctx->stream>>>(args);
-    }
-    return launched(ctx, what);
-  }
-  switch (epilogue) {
-    case kEpiRowScale:
-      tcGemmKernel<kOpFp8, kEpiRowScale><<<grid, kTcThreads, smem, ctx->stream>>>(args);
-      break;
-    case kEpiMirror:
-      tcGemmKernel<kOpBf16, kEpiMirror><<<grid, kTcThreads, smem, ctx->stream>>>(args);
-      break;
-    case kEpiInverseH:
-      tcGemmKernel<kOpBf16, kEpiInverseH><<<grid, kTcThreads, smem, ctx->stream>>>(args);
-      break;
-    default:
-      tcGemmKernel<kOpBf16, kEpiStore><<<grid, kTcThreads, smem, ctx->stream>>>(args);
-      break;
-  }
-  return launched(ctx, what);
+  return args;
 }
 
+// X = W W^T from the packed factor (scale_tiles: block-scaled kinds;
+// row_scale: FP8).
 int runTcGemm(msq_ctx *ctx, const DeviceBatch *b, TcPlan *p, const uint8_t *tiles,
-              const float *row_scale, float *x) {
-  const uint8_t *t[1] = {tiles};
-  return launchTcGemm(ctx, b, p, p->kind == kOpFp8 ? kEpiRowScale : kEpiMirror, 1, t, t,
-                      row_scale, nullptr, x, "tcgen05 reconstruction");
+              const uint8_t *scale_tiles, const float *row_scale, float *x) {
+  const char *what = "tcgen05 reconstruction";
+  TcArgs args = tcArgs(ctx, b, p, kEpiMirror);
+  args.tiles_a[0] = args.tiles_b[0] = tiles;
+  args.scales_a = args.scales_b = scale_tiles;
+  args.row_scale = row_scale;
+  args.x = x;
+  switch (p->kind) {
+    case kOpMxf4: return launchTcKernel<kOpMxf4, kEpiMirror>(ctx, args, what);
+    case kOpMxf8: return launchTcKernel<kOpMxf8, kEpiMirror>(ctx, args, what);
+    case kOpFp8: return launchTcKernel<kOpFp8, kEpiRowScale>(ctx, args, what);
+    default: return launchTcKernel<kOpBf16, kEpiMirror>(ctx, args, what);
+  }
 }
 
 template <int kSource>
@@ -948,14 +969,6 @@ int launchPackMx(msq_ctx *ctx, const DeviceBatch *b, TcPlan *p, const float *f,
   args.scale_tiles = scale_tiles;
   packMxKernel<kSource><<<std::min(p->pack_items, kSmCount * 16), 128, 0, ctx->stream>>>(args);
   return launched(ctx, "pack block-scaled operand");
-}
-
-// X = (A * SF)(A * SF)^T from block-scaled operand tiles.
-int runMxGemm(msq_ctx *ctx, const DeviceBatch *b, TcPlan *p, const uint8_t *tiles,
-              const uint8_t *scale_tiles, float *x) {
-  const uint8_t *t[1] = {tiles};
-  return launchTcGemm(ctx, b, p, kEpiMirror, 1, t, t, nullptr, nullptr, x,
-                      "tcgen05 reconstruction", scale_tiles);
 }
 
 // Every matrix of the batch starts a 32-element block and has an order
@@ -1008,7 +1021,7 @@ int packSplit(msq_ctx *ctx, const DeviceBatch *b, TcPlan *p, const float *m, boo
 }
 
 // Scratch for split operands: kBuffers tile buffers of the BF16 plan.
-constexpr int kBuffers = 6;
+constexpr int kBuffers = 8;
 uint8_t *splitBuffers(msq_ctx *ctx, TcPlan *p, uint8_t *bufs[kBuffers]) {
   const size_t one = static_cast<size_t>(p->total_tiles) * kTileBytes;
   uint8_t *mem = static_cast<uint8_t *>(scratch(ctx, one * kBuffers, kScratchGemm));
@@ -1017,13 +1030,19 @@ uint8_t *splitBuffers(msq_ctx *ctx, TcPlan *p, uint8_t *bufs[kBuffers]) {
   return mem;
 }
 
-// C = A B^T with A, B each split in two BF16 pieces: a0 b0 + a0 b1 + a1 b0
-// (the dropped a1 b1 term is ~2^-16 relative).
-int gemmSplit2(msq_ctx *ctx, const DeviceBatch *b, TcPlan *p, uint8_t *const *a, uint8_t *const *bb,
-               int epilogue, const float *eigenvalues, float *out, const char *what) {
-  const uint8_t *sa[3] = {a[0], a[0], a[1]};
-  const uint8_t *sb[3] = {bb[0], bb[1], bb[0]};
-  return launchTcGemm(ctx, b, p, epilogue, 3, sa, sb, nullptr, eigenvalues, out, what);
+// A B^T of split operands, to FP32 (x) or packed (out).
+template <int kEpi>
+int gemmSplit(msq_ctx *ctx, const DeviceBatch *b, TcPlan *p, uint8_t *const *a, uint8_t *const *bb,
+              const float *eigenvalues, uint8_t *const *out, float *x, const char *what) {
+  TcArgs args = tcArgs(ctx, b, p, kEpi);
+  for (int q = 0; q < 2; ++q) {
+    args.tiles_a[q] = a[q];
+    args.tiles_b[q] = bb[q];
+    args.out[q] = out != nullptr ? out[q] : nullptr;
+  }
+  args.eigenvalues = eigenvalues;
+  args.x = x;
+  return launchTcKernel<kOpBf16, kEpi>(ctx, args, what);
 }
 
 }  // namespace
@@ -1034,26 +1053,22 @@ int gemmSplit2(msq_ctx *ctx, const DeviceBatch *b, TcPlan *p, uint8_t *const *a,
 // The correction is residual-sized, so the ~1e-5 relative error of the
 // two-piece products is far below what the next sweep can see.
 int sylvesterTc(msq_ctx *ctx, const DeviceBatch *b, const float *v, const float *lam,
-                const float *r, float *ws0, float *ws1, float **correction, bool basis_packed) {
+                const float *r, float *correction, bool basis_packed) {
   TcPlan *p = tcPlan(ctx, b, kOpBf16);
   if (p == nullptr) return MSQ_ERR_CUDA;
   uint8_t *buf[kBuffers];
   if (splitBuffers(ctx, p, buf) == nullptr) return MSQ_ERR_CUDA;
-  uint8_t *vn[2] = {buf[0], buf[1]}, *vt[2] = {buf[2], buf[3]}, *op[2] = {buf[4], buf[5]};
+  uint8_t *vn[2] = {buf[0], buf[1]}, *vt[2] = {buf[2], buf[3]};
+  uint8_t *even[2] = {buf[4], buf[5]}, *odd[2] = {buf[6], buf[7]};
   if (!basis_packed) {
     MSQ_TRY(packSplit(ctx, b, p, v, false, vn));  // rows = columns of V
     MSQ_TRY(packSplit(ctx, b, p, v, true, vt));   // rows = rows of V
   }
-  MSQ_TRY(packSplit(ctx, b, p, r, false, op));  // R (symmetric)
-  MSQ_TRY(gemmSplit2(ctx, b, p, op, vn, kEpiStore, nullptr, ws0, "tc sylvester G=RV"));
-  MSQ_TRY(packSplit(ctx, b, p, ws0, false, op));
-  MSQ_TRY(gemmSplit2(ctx, b, p, vn, op, kEpiInverseH, lam, ws1, "tc sylvester C=V'G/H"));
-  MSQ_TRY(packSplit(ctx, b, p, ws1, false, op));
-  MSQ_TRY(gemmSplit2(ctx, b, p, op, vt, kEpiStore, nullptr, ws0, "tc sylvester Zt=CV'"));
-  MSQ_TRY(packSplit(ctx, b, p, ws0, false, op));
-  MSQ_TRY(gemmSplit2(ctx, b, p, op, vt, kEpiStore, nullptr, ws1, "tc sylvester E=ZV'"));
-  *correction = ws1;
-  return MSQ_OK;
+  MSQ_TRY(packSplit(ctx, b, p, r, false, even));  // R (symmetric)
+  MSQ_TRY(gemmSplit<kEpiPacked>(ctx, b, p, even, vn, nullptr, odd, nullptr, "tc sylvester G=RV"));
+  MSQ_TRY(gemmSplit<kEpiInverseH>(ctx, b, p, vn, odd, lam, even, nullptr, "tc sylvester C=V'G/H"));
+  MSQ_TRY(gemmSplit<kEpiPacked>(ctx, b, p, even, vt, nullptr, odd, nullptr, "tc sylvester Zt=CV'"));
+  return gemmSplit<kEpiStore>(ctx, b, p, odd, vt, nullptr, nullptr, correction, "tc sylvester E=ZV'");
 }
 
 int reconstructLowBit(msq_ctx *ctx, const DeviceBatch *b, int format, const float *f, float *x) {
@@ -1067,7 +1082,7 @@ int reconstructLowBit(msq_ctx *ctx, const DeviceBatch *b, int format, const floa
                 kScratchOperand));
     if (mem == nullptr) return MSQ_ERR_CUDA;
     MSQ_TRY(launchPackMx<kMxF32Fp4>(ctx, b, p, f, nullptr, nullptr, mem, mem + tile_bytes));
-    return runMxGemm(ctx, b, p, mem, mem + tile_bytes, x);
+    return runTcGemm(ctx, b, p, mem, mem + tile_bytes, nullptr, x);
   }
   const int kind = format == MSQ_FMT_FP8_E4M3FN_ROWSCALE ? kOpFp8 : kOpBf16;
   TcPlan *p = tcPlan(ctx, b, kind);
@@ -1090,7 +1105,7 @@ int reconstructLowBit(msq_ctx *ctx, const DeviceBatch *b, int format, const floa
     default:
       return setError(ctx, MSQ_ERR_UNSUPPORTED, "reconstruction format not supported");
   }
-  return runTcGemm(ctx, b, p, mem, row_scale, x);
+  return runTcGemm(ctx, b, p, mem, nullptr, row_scale, x);
 }
 
 int reconstructEncoded(msq_ctx *ctx, const DeviceBatch *b, int format, const void *values,
@@ -1125,7 +1140,7 @@ int reconstructEncoded(msq_ctx *ctx, const DeviceBatch *b, int format, const voi
     } else {
       MSQ_TRY(launchPackMx<kMxCodesFp8>(ctx, b, p, nullptr, codes, sf, mem, mem + tile_bytes));
     }
-    return runMxGemm(ctx, b, p, mem, mem + tile_bytes, x);
+    return runTcGemm(ctx, b, p, mem, mem + tile_bytes, nullptr, x);
   }
   TcPlan *p = tcPlan(ctx, b, kind);
   if (p == nullptr) return MSQ_ERR_CUDA;
@@ -1146,7 +1161,7 @@ int reconstructEncoded(msq_ctx *ctx, const DeviceBatch *b, int format, const voi
                                           reinterpret_cast<const uint8_t *>(scales), nullptr, mem));
       break;
   }
-  return runTcGemm(ctx, b, p, mem,
+  return runTcGemm(ctx, b, p, mem, nullptr,
                    kind == kOpFp8 ? static_cast<const float *>(scales) : nullptr, x);
 }
 
