@@ -122,6 +122,20 @@ __device__ __forceinline__ uint32_t encodeE2M1Pair(float even, float odd, float 
   return code;
 }
 
+// Two finite values to E4M3 or E5M2 with the hardware conversion (round to
+// nearest even, saturating to the largest finite code), the even element in
+// the low byte.  Same codes as encodeE4M3 / encodeE5M2 for finite values.
+__device__ __forceinline__ uint32_t encodeE4M3Pair(float even, float odd) {
+  uint16_t r;
+  asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(r) : "f"(odd), "f"(even));
+  return r;
+}
+__device__ __forceinline__ uint32_t encodeE5M2Pair(float even, float odd) {
+  uint16_t r;
+  asm("cvt.rn.satfinite.e5m2x2.f32 %0, %1, %2;" : "=h"(r) : "f"(odd), "f"(even));
+  return r;
+}
+
 __device__ __forceinline__ float signedNan(uint32_t negative) {
   return __uint_as_float(0x7fc00000u | (negative ? 0x80000000u : 0u));
 }
@@ -172,6 +186,19 @@ __device__ __forceinline__ float decodeE2M1(uint32_t code) {
 __device__ __forceinline__ float2 decodeE2M1Pair(uint32_t byte) {
   uint32_t h2;
   asm("{\n .reg .b8 t;\n cvt.u8.u32 t, %1;\n cvt.rn.f16x2.e2m1x2 %0, t;\n}" : "=r"(h2) : "r"(byte));
+  return __half22float2(*reinterpret_cast<const __half2 *>(&h2));
+}
+
+// Two E4M3 codes that are not NaN, the even element in the low byte, through
+// the exact hardware conversion to FP16.  Same values as decodeE4M3.
+__device__ __forceinline__ float2 decodeE4M3Pair(uint32_t pair) {
+  uint32_t h2;
+  asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(h2) : "h"(static_cast<uint16_t>(pair)));
+  return __half22float2(*reinterpret_cast<const __half2 *>(&h2));
+}
+// Two E5M2 codes that are not NaN, given as the high bytes of two FP16 values
+// (which they are).  Same values as decodeE5M2.
+__device__ __forceinline__ float2 decodeE5M2Pair(uint32_t h2) {
   return __half22float2(*reinterpret_cast<const __half2 *>(&h2));
 }
 
@@ -236,8 +263,7 @@ __device__ __forceinline__ float mxScale(float decoded, uint32_t scale_byte) {
 // :1888-1907.  A finite magnitude strictly between two codes rounds up with
 // probability (|x| - lo) / (hi - lo) against a 24-bit sample of the hash of
 // (element index, seed, stream); zero, NaN and magnitudes at or above the
-// largest finite code take the nearest code.  Adjacent codes differ by a
-// power of two, so the probability is an exact quotient.
+// largest finite code take the nearest code.
 
 __device__ __forceinline__ uint32_t stochasticHash(uint32_t index, uint32_t seed, uint32_t stream) {
   const uint32_t state = index * 747796405u + seed + stream * 2891336453u;
@@ -245,57 +271,56 @@ __device__ __forceinline__ uint32_t stochasticHash(uint32_t index, uint32_t seed
   return (word >> 22u) ^ word;
 }
 
-__device__ __forceinline__ bool stochasticUp(float probability, uint32_t index, uint32_t seed,
-                                             uint32_t stream) {
-  // 24-bit sample times 2^-24 (exact)
-  const float sample = static_cast<float>(stochasticHash(index, seed, stream) >> 8u) *
-                       5.9604644775390625e-08f;
-  return sample < probability;
-}
-
-// The code below or above a finite magnitude that lies between codes, from
-// its nearest code (codes of one sign are ordered like their values).
-template <class Decode>
-__device__ __forceinline__ uint32_t stochasticCode(uint32_t nearest, float magnitude, Decode dec,
-                                                   uint32_t index, uint32_t seed, uint32_t stream) {
-  const float nearest_value = dec(nearest);
-  if (nearest_value == magnitude) return nearest;
-  const uint32_t lower = nearest_value < magnitude ? nearest : nearest - 1u;
-  const float lo = dec(lower), hi = dec(lower + 1u);
-  const float probability = __fdiv_rn(magnitude - lo, hi - lo);
-  return stochasticUp(probability, index, seed, stream) ? lower + 1u : lower;
+// The code of a finite magnitude below the largest finite value: the code
+// below it, or the next one up with the probability of its place between the
+// two.  The place is the dropped part of the mantissa (of the multiple of the
+// smallest step, below the normal range), so it is exact, and it is compared
+// with the hash's 24 bits as an integer (as a float).
+template <int kMant, int kBias>
+__device__ __forceinline__ uint32_t stochasticMagnitude(float magnitude, uint32_t index,
+                                                        uint32_t seed, uint32_t stream) {
+  constexpr int kEmin = 1 - kBias;
+  const uint32_t sample = stochasticHash(index, seed, stream) >> 8u;
+  const uint32_t bits = __float_as_uint(magnitude);
+  const int exponent = static_cast<int>(bits >> 23) - 127;
+  if (exponent < kEmin) {
+    const float steps = magnitude * __uint_as_float(
+                                        static_cast<uint32_t>(127 + kMant - kEmin) << 23);
+    const float lower = floorf(steps);
+    // 24-bit sample times 2^-24 (exact)
+    const bool up = static_cast<float>(sample) * 5.9604644775390625e-08f < steps - lower;
+    return static_cast<uint32_t>(lower) + up;
+  }
+  constexpr int kDrop = 23 - kMant;
+  const uint32_t lower = (static_cast<uint32_t>(exponent + kBias) << kMant) |
+                         ((bits & 0x007fffffu) >> kDrop);
+  const uint32_t rest = (bits & ((1u << kDrop) - 1u)) << (24 - kDrop);
+  return lower + (sample < rest);
 }
 
 __device__ __forceinline__ uint8_t encodeE4M3Stochastic(float value, uint32_t index, uint32_t seed,
                                                         uint32_t stream) {
   const float magnitude = fabsf(value);
-  if (value != value || magnitude == 0.0f || magnitude >= 448.0f) return encodeE4M3(value);
+  if (!(magnitude < 448.0f) || magnitude == 0.0f) return encodeE4M3(value);
   const uint32_t sign = (__float_as_uint(value) >> 24) & 0x80u;
-  return static_cast<uint8_t>(
-      sign | stochasticCode(encodeE4M3(magnitude), magnitude,
-                            [](uint32_t c) { return decodeE4M3(c); }, index, seed, stream));
+  return static_cast<uint8_t>(sign | stochasticMagnitude<3, 7>(magnitude, index, seed, stream));
 }
 
 __device__ __forceinline__ uint8_t encodeE5M2Stochastic(float value, uint32_t index, uint32_t seed,
                                                         uint32_t stream) {
   const float magnitude = fabsf(value);
-  if (value != value || isinf(magnitude) || magnitude == 0.0f || magnitude >= 57344.0f) {
-    return encodeE5M2(value);
-  }
+  if (!(magnitude < 57344.0f) || magnitude == 0.0f) return encodeE5M2(value);
   const uint32_t sign = (__float_as_uint(value) >> 24) & 0x80u;
-  return static_cast<uint8_t>(
-      sign | stochasticCode(encodeE5M2(magnitude), magnitude,
-                            [](uint32_t c) { return decodeE5M2(c); }, index, seed, stream));
+  return static_cast<uint8_t>(sign | stochasticMagnitude<2, 15>(magnitude, index, seed, stream));
 }
 
 // 4-bit code in the low nibble
 __device__ __forceinline__ uint32_t encodeE2M1Stochastic(float value, uint32_t index, uint32_t seed,
                                                          uint32_t stream) {
   const float magnitude = fabsf(value);
-  if (value != value || magnitude == 0.0f || magnitude >= 6.0f) return encodeE2M1(value);
+  if (!(magnitude < 6.0f) || magnitude == 0.0f) return encodeE2M1(value);
   const uint32_t sign = (__float_as_uint(value) >> 28) & 0x8u;
-  return sign | stochasticCode(encodeE2M1(magnitude), magnitude,
-                               [](uint32_t c) { return decodeE2M1(c); }, index, seed, stream);
+  return sign | stochasticMagnitude<1, 1>(magnitude, index, seed, stream);
 }
 
 __device__ __forceinline__ uint16_t encodeBf16Stochastic(float value, uint32_t index, uint32_t seed,

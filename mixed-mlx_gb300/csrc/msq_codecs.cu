@@ -5,7 +5,7 @@
 // (metal_mixed_sqrt.metal:384-1259, 1661-1909) and is bit-exact with its host
 // codec copyToStorage / storageValueAt (src/storage_codecs.cpp:249-374).
 // HBM-bound streaming work: every thread owns 8 consecutive elements
-// (two 16-byte loads), an MX block of 32 elements is owned by 4 adjacent
+// (one 32-byte access), an MX block of 32 elements is owned by 4 adjacent
 // lanes that agree on the block maximum through two xor-shuffles, and grids
 // are a multiple of the SM count with a grid-stride loop.
 #include "msq_codec_device.cuh"
@@ -23,13 +23,28 @@ struct Group {
   float v[kGroup];
 };
 
-__device__ __forceinline__ Group loadGroup(const float *__restrict__ source,
-                                           size_t base, size_t elements,
-                                           bool vector_ok) {
+// How a float buffer may be accessed: 2 32-byte vectors, 1 16-byte ones, 0
+// element by element.
+__host__ __device__ __forceinline__ int vectorMode(const void *p) {
+  const uintptr_t a = reinterpret_cast<uintptr_t>(p);
+  return (a & 31u) == 0 ? 2 : (a & 15u) == 0 ? 1 : 0;
+}
+
+// Eight elements at `base`, zeros beyond `elements`.  A thread's 32 bytes in
+// one access: half the instructions of two 16-byte ones, and each a whole
+// sector.
+__device__ __forceinline__ Group loadGroup(const float *source, size_t base, size_t elements,
+                                           int mode) {
   Group g;
-  if (vector_ok && base + kGroup <= elements) {
-    const float4 a = __ldcs(reinterpret_cast<const float4 *>(source + base));
-    const float4 b = __ldcs(reinterpret_cast<const float4 *>(source + base + 4));
+  if (mode == 2 && base + kGroup <= elements) {
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(g.v[0]), "=f"(g.v[1]), "=f"(g.v[2]), "=f"(g.v[3]), "=f"(g.v[4]),
+                   "=f"(g.v[5]), "=f"(g.v[6]), "=f"(g.v[7])
+                 : "l"(source + base)
+                 : "memory");
+  } else if (mode == 1 && base + kGroup <= elements) {
+    const float4 a = *reinterpret_cast<const float4 *>(source + base);
+    const float4 b = *reinterpret_cast<const float4 *>(source + base + 4);
     g.v[0] = a.x; g.v[1] = a.y; g.v[2] = a.z; g.v[3] = a.w;
     g.v[4] = b.x; g.v[5] = b.y; g.v[6] = b.z; g.v[7] = b.w;
   } else {
@@ -41,14 +56,16 @@ __device__ __forceinline__ Group loadGroup(const float *__restrict__ source,
   return g;
 }
 
-__device__ __forceinline__ void storeGroup(float *__restrict__ output,
-                                           size_t base, size_t elements,
-                                           bool vector_ok, const Group &g) {
-  if (vector_ok && base + kGroup <= elements) {
-    __stcs(reinterpret_cast<float4 *>(output + base),
-           make_float4(g.v[0], g.v[1], g.v[2], g.v[3]));
-    __stcs(reinterpret_cast<float4 *>(output + base + 4),
-           make_float4(g.v[4], g.v[5], g.v[6], g.v[7]));
+__device__ __forceinline__ void storeGroup(float *output, size_t base, size_t elements, int mode,
+                                           const Group &g) {
+  if (mode == 2 && base + kGroup <= elements) {
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(output + base),
+                 "f"(g.v[0]), "f"(g.v[1]), "f"(g.v[2]), "f"(g.v[3]), "f"(g.v[4]), "f"(g.v[5]),
+                 "f"(g.v[6]), "f"(g.v[7])
+                 : "memory");
+  } else if (mode == 1 && base + kGroup <= elements) {
+    *reinterpret_cast<float4 *>(output + base) = make_float4(g.v[0], g.v[1], g.v[2], g.v[3]);
+    *reinterpret_cast<float4 *>(output + base + 4) = make_float4(g.v[4], g.v[5], g.v[6], g.v[7]);
   } else {
 #pragma unroll
     for (int i = 0; i < kGroup; ++i) {
@@ -57,14 +74,117 @@ __device__ __forceinline__ void storeGroup(float *__restrict__ output,
   }
 }
 
+constexpr float kLargestFinite = 3.402823466e38f;
+
 __device__ __forceinline__ float groupMaxFinite(const Group &g) {
   float m = 0.0f;
 #pragma unroll
   for (int i = 0; i < kGroup; ++i) {
     const float a = fabsf(g.v[i]);
-    if (a <= 3.402823466e38f) m = fmaxf(m, a);  // finite only (NaN fails)
+    if (a <= kLargestFinite) m = fmaxf(m, a);  // finite only (NaN fails)
   }
   return m;
+}
+
+// The largest magnitude, NaN if there is one.
+__device__ __forceinline__ float groupMaxNan(const Group &g) {
+  float m = fabsf(g.v[0]);
+#pragma unroll
+  for (int i = 1; i < kGroup; ++i)
+    asm("max.NaN.f32 %0, %0, %1;" : "+f"(m) : "f"(fabsf(g.v[i])));
+  return m;
+}
+
+// The formats by their parts.
+constexpr bool isMx(int f) {
+  return f == MSQ_FMT_MXFP8_E4M3FN || f == MSQ_FMT_MXFP8_E5M2 || f == MSQ_FMT_MXFP4_E2M1;
+}
+constexpr bool isFp4(int f) { return f == MSQ_FMT_FP4_E2M1 || f == MSQ_FMT_MXFP4_E2M1; }
+constexpr bool isE5M2(int f) { return f == MSQ_FMT_FP8_E5M2 || f == MSQ_FMT_MXFP8_E5M2; }
+constexpr int elementEmax(int f) { return isFp4(f) ? 2 : isE5M2(f) ? 15 : 8; }
+
+// The eight codes of a group (of x / 2^e for MX formats), FP4 in the low 32
+// bits.  A group of finite values takes the hardware conversions, a group
+// with an infinity or a NaN, or with a scale outside the normal powers of
+// two, the conversions in integers: the same codes.
+template <int kFormat>
+__device__ __forceinline__ uint64_t encodeGroup(const Group &g, bool finite, int e) {
+  uint64_t packed = 0;
+  if (finite && (!isMx(kFormat) || (e >= -126 && e <= 126))) {
+    const float s = isMx(kFormat) ? exp2Int(-e) : 1.0f;
+#pragma unroll
+    for (int i = 0; i < kGroup; i += 2) {
+      const float x = isMx(kFormat) ? g.v[i] * s : g.v[i], y = isMx(kFormat) ? g.v[i + 1] * s : g.v[i + 1];
+      const uint32_t pair = isFp4(kFormat)    ? encodeE2M1Pair(x, y, 0.0f, 0.0f)
+                            : isE5M2(kFormat) ? encodeE5M2Pair(x, y)
+                                              : encodeE4M3Pair(x, y);
+      packed |= static_cast<uint64_t>(pair) << ((isFp4(kFormat) ? 4 : 8) * i);
+    }
+  } else {
+#pragma unroll 1
+    for (int i = 0; i < kGroup; ++i) {
+      float x = 0.0f;
+#pragma unroll
+      for (int q = 0; q < kGroup; ++q) x = q == i ? g.v[q] : x;
+      if (isMx(kFormat)) x = mxDivide(x, e);
+      const uint32_t code = isFp4(kFormat) ? encodeE2M1(x) : isE5M2(kFormat) ? encodeE5M2(x) : encodeE4M3(x);
+      packed |= static_cast<uint64_t>(code) << ((isFp4(kFormat) ? 4 : 8) * i);
+    }
+  }
+  return packed;
+}
+
+// The same with stochastic rounding; `index` is the first element's.
+template <int kFormat>
+__device__ __forceinline__ uint64_t encodeGroupStochastic(const Group &g, bool finite, int e,
+                                                          uint32_t index, uint32_t seed,
+                                                          uint32_t stream) {
+  uint64_t packed = 0;
+  const bool plain = finite && e >= -126 && e <= 126;
+  const float s = plain ? exp2Int(-e) : 1.0f;
+#pragma unroll
+  for (int i = 0; i < kGroup; ++i) {
+    const float x = !isMx(kFormat) ? g.v[i] : plain ? g.v[i] * s : mxDivide(g.v[i], e);
+    const uint32_t code = isFp4(kFormat)    ? encodeE2M1Stochastic(x, index + i, seed, stream)
+                          : isE5M2(kFormat) ? encodeE5M2Stochastic(x, index + i, seed, stream)
+                                            : encodeE4M3Stochastic(x, index + i, seed, stream);
+    packed |= static_cast<uint64_t>(code) << ((isFp4(kFormat) ? 4 : 8) * i);
+  }
+  return packed;
+}
+
+// The values of eight codes, times 2^(scale - 127) for MX formats.
+template <int kFormat>
+__device__ __forceinline__ Group decodeGroup(uint64_t packed, uint32_t scale) {
+  Group g;
+  const uint32_t w[2] = {static_cast<uint32_t>(packed), static_cast<uint32_t>(packed >> 32)};
+  bool plain = !isMx(kFormat) || (scale >= 1 && scale <= 254);
+  if (!isFp4(kFormat)) {  // no NaN code
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      plain = plain && (isE5M2(kFormat) ? __vcmpgtu4(w[h] & 0x7f7f7f7fu, 0x7c7c7c7cu)
+                                        : __vcmpeq4(w[h] & 0x7f7f7f7fu, 0x7f7f7f7fu)) == 0;
+  }
+  if (plain) {
+    const float s = isMx(kFormat) ? exp2Int(static_cast<int>(scale) - 127) : 1.0f;
+#pragma unroll
+    for (int q = 0; q < kGroup / 2; ++q) {
+      const float2 d = isFp4(kFormat)    ? decodeE2M1Pair((w[0] >> (8 * q)) & 0xffu)
+                       : isE5M2(kFormat) ? decodeE5M2Pair(__byte_perm(w[q / 2], 0, q % 2 ? 0x3424 : 0x1404))
+                                         : decodeE4M3Pair(w[q / 2] >> (16 * (q % 2)));
+      g.v[2 * q] = isMx(kFormat) ? d.x * s : d.x;
+      g.v[2 * q + 1] = isMx(kFormat) ? d.y * s : d.y;
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < kGroup; ++i) {
+      const uint32_t code = static_cast<uint32_t>(packed >> ((isFp4(kFormat) ? 4 : 8) * i)) &
+                            (isFp4(kFormat) ? 0xfu : 0xffu);
+      const float d = isFp4(kFormat) ? decodeE2M1(code) : isE5M2(kFormat) ? decodeE5M2(code) : decodeE4M3(code);
+      g.v[i] = isMx(kFormat) ? mxScale(d, scale) : d;
+    }
+  }
+  return g;
 }
 
 // Writes `count` bytes of `packed` (little-endian) at byte offset `at`.
@@ -84,23 +204,30 @@ __device__ __forceinline__ void storeBytes(uint8_t *__restrict__ out, size_t at,
 
 // ---------------------------------------------------------------- encoders
 
-template <int kFormat>
+// Eight elements per thread, rounded to nearest or stochastically (the
+// element's flat index feeds the hash).  Bound by memory for the nearest
+// codes; the hash and the place between two codes are some 25 instructions
+// per element.  2^26 elements, E4M3: 53 us nearest (86 with the conversion
+// in integers), 96 stochastic (366 with a thread per element and a
+// division).
+template <int kFormat, bool kStochastic>
 __global__ void __launch_bounds__(kThreads)
-encodeScalarKernel(const float *__restrict__ source, size_t elements,
-                   uint8_t *__restrict__ values, uint8_t *__restrict__ scales,
-                   bool vector_ok) {
+encodeScalarKernel(const float *__restrict__ source, size_t elements, uint32_t seed,
+                   uint32_t stream, uint8_t *__restrict__ values, int mode) {
   const size_t groups = (elements + kGroup - 1) / kGroup;
   for (size_t group = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
        group < groups; group += static_cast<size_t>(gridDim.x) * blockDim.x) {
     const size_t base = group * kGroup;
-    const Group g = loadGroup(source, base, elements, vector_ok);
+    const uint32_t index = static_cast<uint32_t>(base);
+    const Group g = loadGroup(source, base, elements, mode);
     const size_t valid = elements - base < kGroup ? elements - base : kGroup;
     if constexpr (kFormat == MSQ_FMT_BF16) {
       uint16_t h[kGroup];
 #pragma unroll
-      for (int i = 0; i < kGroup; ++i) h[i] = encodeBf16(g.v[i]);
+      for (int i = 0; i < kGroup; ++i)
+        h[i] = kStochastic ? encodeBf16Stochastic(g.v[i], index + i, seed, stream) : encodeBf16(g.v[i]);
       uint16_t *out = reinterpret_cast<uint16_t *>(values);
-      if (vector_ok && valid == kGroup) {
+      if (mode != 0 && valid == kGroup) {
         uint4 packed;
         packed.x = h[0] | (static_cast<uint32_t>(h[1]) << 16);
         packed.y = h[2] | (static_cast<uint32_t>(h[3]) << 16);
@@ -110,40 +237,25 @@ encodeScalarKernel(const float *__restrict__ source, size_t elements,
       } else {
         for (size_t i = 0; i < valid; ++i) out[base + i] = h[i];
       }
-    } else if constexpr (kFormat == MSQ_FMT_FP8_E4M3FN ||
-                         kFormat == MSQ_FMT_FP8_E5M2) {
-      uint64_t packed = 0;
-#pragma unroll
-      for (int i = 0; i < kGroup; ++i) {
-        const uint32_t code = kFormat == MSQ_FMT_FP8_E4M3FN ? encodeE4M3(g.v[i])
-                                                           : encodeE5M2(g.v[i]);
-        packed |= static_cast<uint64_t>(code) << (8 * i);
-      }
-      storeBytes(values, base, packed, static_cast<int>(valid), vector_ok);
-    } else if constexpr (kFormat == MSQ_FMT_FP4_E2M1) {
+    } else {
+      const uint64_t packed =
+          kStochastic ? encodeGroupStochastic<kFormat>(g, true, 0, index, seed, stream)
+                      : encodeGroup<kFormat>(g, groupMaxNan(g) <= kLargestFinite, 0);
       // packFp4 (src/storage_codecs.cpp:138-146): low nibble = even index,
       // the pad nibble of an odd tail is the code of +0 (= 0).
-      uint64_t packed = 0;
-#pragma unroll
-      for (int i = 0; i < kGroup; ++i) {
-        packed |= static_cast<uint64_t>(encodeE2M1(g.v[i])) << (4 * i);
-      }
-      storeBytes(values, base / 2, packed, static_cast<int>((valid + 1) / 2),
-                 vector_ok);
+      if (isFp4(kFormat)) storeBytes(values, base / 2, packed, static_cast<int>((valid + 1) / 2), mode != 0);
+      else storeBytes(values, base, packed, static_cast<int>(valid), mode != 0);
     }
-    (void)scales;
   }
 }
 
-// MX formats: 4 lanes x 8 elements per 32-element scale block.
-template <int kFormat>
+// MX formats: 4 lanes x 8 elements per 32-element scale block.  2^26
+// elements, MXFP8 E4M3: 66 us nearest (120 with the conversion in
+// integers), 125 stochastic (444 with a thread per element and a division).
+template <int kFormat, bool kStochastic>
 __global__ void __launch_bounds__(kThreads)
-encodeMxKernel(const float *__restrict__ source, size_t elements,
-               uint8_t *__restrict__ values, uint8_t *__restrict__ scales,
-               bool vector_ok) {
-  constexpr int kEmax = kFormat == MSQ_FMT_MXFP8_E4M3FN ? 8
-                        : kFormat == MSQ_FMT_MXFP8_E5M2 ? 15
-                                                        : 2;
+encodeMxKernel(const float *__restrict__ source, size_t elements, uint32_t seed, uint32_t stream,
+               uint8_t *__restrict__ values, uint8_t *__restrict__ scales, int mode) {
   const size_t blocks = (elements + 31) / 32;
   const size_t groups = blocks * 4;  // whole blocks; lanes 0-3 share one
   const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
@@ -156,48 +268,26 @@ encodeMxKernel(const float *__restrict__ source, size_t elements,
     const size_t base = group * kGroup;
     Group g;
     if (active) {
-      g = loadGroup(source, base, elements, vector_ok);
+      g = loadGroup(source, base, elements, mode);
     } else {
 #pragma unroll
       for (int i = 0; i < kGroup; ++i) g.v[i] = 0.0f;
     }
-    float m = groupMaxFinite(g);
+    float m = groupMaxNan(g);
+    const bool finite = m <= kLargestFinite;
+    if (!finite) m = groupMaxFinite(g);
     m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
     m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
     if (!active || base >= elements) continue;
-    const int e = mxExponent(m, kEmax);
+    const int e = mxExponent(m, elementEmax(kFormat));
     const size_t valid = elements - base < kGroup ? elements - base : kGroup;
     if (group % 4 == 0) scales[group / 4] = static_cast<uint8_t>(e + 127);
-    if constexpr (kFormat == MSQ_FMT_MXFP4_E2M1) {
-      uint64_t packed = 0;
-      if (e >= -126 && e <= 126) {
-        // x / 2^e is the exact product x * 2^-e; a NaN keeps the sign of x
-        const float s = exp2Int(-e);
-#pragma unroll
-        for (int i = 0; i < kGroup; i += 2) {
-          packed |= static_cast<uint64_t>(encodeE2M1Pair(g.v[i] * s, g.v[i + 1] * s, g.v[i], g.v[i + 1]))
-                    << (4 * i);
-        }
-      } else {
-#pragma unroll
-        for (int i = 0; i < kGroup; i += 2) {
-          const float a = mxDivide(g.v[i], e), b = mxDivide(g.v[i + 1], e);
-          packed |= static_cast<uint64_t>(encodeE2M1Pair(a, b, a, b)) << (4 * i);
-        }
-      }
-      storeBytes(values, base / 2, packed, static_cast<int>((valid + 1) / 2),
-                 vector_ok);
-    } else {
-      uint64_t packed = 0;
-#pragma unroll
-      for (int i = 0; i < kGroup; ++i) {
-        const float scaled = mxDivide(g.v[i], e);
-        const uint32_t code = kFormat == MSQ_FMT_MXFP8_E4M3FN ? encodeE4M3(scaled)
-                                                              : encodeE5M2(scaled);
-        packed |= static_cast<uint64_t>(code) << (8 * i);
-      }
-      storeBytes(values, base, packed, static_cast<int>(valid), vector_ok);
-    }
+    const uint64_t packed =
+        kStochastic
+            ? encodeGroupStochastic<kFormat>(g, finite, e, static_cast<uint32_t>(base), seed, stream)
+            : encodeGroup<kFormat>(g, finite, e);
+    if (isFp4(kFormat)) storeBytes(values, base / 2, packed, static_cast<int>((valid + 1) / 2), mode != 0);
+    else storeBytes(values, base, packed, static_cast<int>(valid), mode != 0);
   }
 }
 
@@ -261,11 +351,57 @@ encodeMxfp4Kernel(const float *__restrict__ source, size_t blocks, uint8_t *__re
 }
 
 // FP8 E4M3FN with one FP32 scale per contiguous row: s = max|row| / 448
-// (1 when the row has no nonzero finite value), code = E4M3(x / s).  One warp
-// per row: a max pass, then an encode pass (the row is re-read from L1/L2).
+// (1 when the row has no nonzero finite value), code = E4M3(x / s).  A max
+// pass, then an encode pass (the row is re-read from L1/L2).
+//
+// Rows of a multiple of eight elements, 16-byte aligned: `sub` lanes (a power
+// of two) per row, eight elements per lane and step, so that short rows fill
+// a warp too.  2^26 elements: rows of 256 97 us (160 with an element per
+// lane), rows of 4096 110 (242).
+template <bool kStochastic>
 __global__ void __launch_bounds__(kThreads)
-encodeRowScaleKernel(const float *__restrict__ source, size_t rows,
-                     size_t row_length, uint8_t *__restrict__ values,
+encodeRowScaleGroupsKernel(const float *__restrict__ source, size_t rows, size_t row_length, int sub,
+                           uint32_t seed, uint32_t stream, uint8_t *__restrict__ values,
+                           float *__restrict__ scales, int mode) {
+  const int lane = threadIdx.x % 32;
+  const size_t per = 32 / sub, groups = row_length / kGroup;
+  const size_t warps = static_cast<size_t>(gridDim.x) * (blockDim.x / 32);
+  for (size_t first = (blockIdx.x * static_cast<size_t>(blockDim.x / 32) + threadIdx.x / 32) * per;
+       first < rows; first += warps * per) {
+    const size_t row = first + lane / sub, q0 = lane % sub;
+    const bool active = row < rows;
+    const float *in = source + row * row_length;
+    Group head = {};
+    if (active && q0 < groups) head = loadGroup(in, q0 * kGroup, row_length, mode);
+    float m = groupMaxFinite(head);
+    if (active) {
+#pragma unroll 4
+      for (size_t q = q0 + sub; q < groups; q += sub)
+        m = fmaxf(m, groupMaxFinite(loadGroup(in, q * kGroup, row_length, mode)));
+    }
+    for (int s = 1; s < sub; s <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, s));
+    const float scale = m == 0.0f ? 1.0f : __fdiv_rn(m, 448.0f);
+    if (active && q0 == 0) scales[row] = scale;
+    if (!active) continue;
+    for (size_t q = q0; q < groups; q += sub) {
+      Group g = q == q0 ? head : loadGroup(in, q * kGroup, row_length, mode);
+#pragma unroll
+      for (int i = 0; i < kGroup; ++i) g.v[i] = rowDivide(g.v[i], scale);
+      const size_t at = row * row_length + q * kGroup;
+      const uint64_t packed =
+          kStochastic ? encodeGroupStochastic<MSQ_FMT_FP8_E4M3FN>(g, true, 0, static_cast<uint32_t>(at), seed, stream)
+                      : encodeGroup<MSQ_FMT_FP8_E4M3FN>(g, groupMaxNan(g) <= kLargestFinite, 0);
+      *reinterpret_cast<uint64_t *>(values + at) = packed;
+    }
+  }
+}
+
+// Other rows: one warp per row, an element per lane (a row's accesses are
+// whole lines whatever its alignment).
+template <bool kStochastic>
+__global__ void __launch_bounds__(kThreads)
+encodeRowScaleKernel(const float *__restrict__ source, size_t rows, size_t row_length,
+                     uint32_t seed, uint32_t stream, uint8_t *__restrict__ values,
                      float *__restrict__ scales) {
   const int lane = threadIdx.x % 32;
   const size_t warps = static_cast<size_t>(gridDim.x) * (blockDim.x / 32);
@@ -273,18 +409,38 @@ encodeRowScaleKernel(const float *__restrict__ source, size_t rows,
        row < rows; row += warps) {
     const float *in = source + row * row_length;
     float m = 0.0f;
+#pragma unroll 4
     for (size_t i = lane; i < row_length; i += 32) {
       const float a = fabsf(in[i]);
-      if (a <= 3.402823466e38f) m = fmaxf(m, a);
+      if (a <= kLargestFinite) m = fmaxf(m, a);
     }
 #pragma unroll
     for (int s = 16; s > 0; s >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, s));
     const float scale = m == 0.0f ? 1.0f : __fdiv_rn(m, 448.0f);
     if (lane == 0) scales[row] = scale;
     uint8_t *out = values + row * row_length;
+#pragma unroll 4
     for (size_t i = lane; i < row_length; i += 32) {
-      out[i] = encodeE4M3(rowDivide(in[i], scale));
+      const float x = rowDivide(in[i], scale);
+      out[i] = kStochastic ? encodeE4M3Stochastic(x, static_cast<uint32_t>(row * row_length + i), seed, stream)
+                           : encodeE4M3(x);
     }
+  }
+}
+
+template <bool kStochastic>
+void launchRowScale(const float *source, size_t rows, size_t row_length, uint32_t seed,
+                    uint32_t stream, uint8_t *values, float *scales, cudaStream_t s) {
+  const int mode = vectorMode(source);
+  if (row_length % kGroup == 0 && mode != 0 && (reinterpret_cast<uintptr_t>(values) & 7u) == 0) {
+    int sub = 1;
+    while (sub < 32 && static_cast<size_t>(sub) * kGroup < row_length) sub *= 2;
+    const size_t per = 32 / sub;
+    encodeRowScaleGroupsKernel<kStochastic><<<gridFor((rows + per - 1) / per * 32, kThreads), kThreads, 0, s>>>(
+        source, rows, row_length, sub, seed, stream, values, scales, mode);
+  } else {
+    encodeRowScaleKernel<kStochastic><<<gridFor(rows * 32, kThreads), kThreads, 0, s>>>(
+        source, rows, row_length, seed, stream, values, scales);
   }
 }
 
@@ -345,10 +501,13 @@ decodeMxfp4Kernel(const uint8_t *__restrict__ values, const uint8_t *__restrict_
   }
 }
 
+// Eight elements per thread; bound by memory.  2^26 elements: MXFP8 E4M3 63 us
+// (76 with 16-byte stores and the conversion in integers), BF16 71 (83), FP4
+// 58 (75).
 template <int kFormat>
 __global__ void __launch_bounds__(kThreads)
 decodeKernel(const uint8_t *__restrict__ values, const uint8_t *__restrict__ scales,
-             size_t elements, float *__restrict__ output, bool vector_ok) {
+             size_t elements, float *__restrict__ output, bool vector_ok, int mode) {
   const size_t groups = (elements + kGroup - 1) / kGroup;
   for (size_t group = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
        group < groups; group += static_cast<size_t>(gridDim.x) * blockDim.x) {
@@ -370,135 +529,66 @@ decodeKernel(const uint8_t *__restrict__ values, const uint8_t *__restrict__ sca
         for (int i = 0; i < kGroup; ++i)
           g.v[i] = i < static_cast<int>(valid) ? decodeBf16(in[base + i]) : 0.0f;
       }
-    } else if constexpr (kFormat == MSQ_FMT_FP4_E2M1 ||
-                         kFormat == MSQ_FMT_MXFP4_E2M1) {
-      uint32_t packed = 0;
-      if (full) {
-        packed = *reinterpret_cast<const uint32_t *>(values + base / 2);
-      } else {
-        for (size_t i = 0; i < (valid + 1) / 2; ++i)
-          packed |= static_cast<uint32_t>(values[base / 2 + i]) << (8 * i);
-      }
-      const uint32_t scale = kFormat == MSQ_FMT_MXFP4_E2M1 ? scales[base / 32] : 127u;
-#pragma unroll
-      for (int i = 0; i < kGroup; ++i) {
-        const float d = decodeE2M1((packed >> (4 * i)) & 0xfu);
-        g.v[i] = kFormat == MSQ_FMT_MXFP4_E2M1 ? mxScale(d, scale) : d;
-      }
     } else {
       uint64_t packed = 0;
+      const size_t at = isFp4(kFormat) ? base / 2 : base;
       if (full) {
-        packed = *reinterpret_cast<const uint64_t *>(values + base);
+        packed = isFp4(kFormat) ? *reinterpret_cast<const uint32_t *>(values + at)
+                                : *reinterpret_cast<const uint64_t *>(values + at);
       } else {
-        for (size_t i = 0; i < valid; ++i)
-          packed |= static_cast<uint64_t>(values[base + i]) << (8 * i);
+        const size_t bytes = isFp4(kFormat) ? (valid + 1) / 2 : valid;
+        for (size_t i = 0; i < bytes; ++i) packed |= static_cast<uint64_t>(values[at + i]) << (8 * i);
       }
-      constexpr bool kMx = kFormat == MSQ_FMT_MXFP8_E4M3FN ||
-                           kFormat == MSQ_FMT_MXFP8_E5M2;
-      constexpr bool kE4M3 = kFormat == MSQ_FMT_FP8_E4M3FN ||
-                             kFormat == MSQ_FMT_MXFP8_E4M3FN;
-      const uint32_t scale = kMx ? scales[base / 32] : 127u;
-#pragma unroll
-      for (int i = 0; i < kGroup; ++i) {
-        const uint32_t code = static_cast<uint32_t>(packed >> (8 * i)) & 0xffu;
-        const float d = kE4M3 ? decodeE4M3(code) : decodeE5M2(code);
-        g.v[i] = kMx ? mxScale(d, scale) : d;
-      }
+      g = decodeGroup<kFormat>(packed, isMx(kFormat) ? scales[base / 32] : 127u);
     }
-    storeGroup(output, base, elements, vector_ok, g);
+    storeGroup(output, base, elements, vector_ok ? mode : 0, g);
   }
 }
 
+// Eight elements per thread and one division for their row (an element's
+// row follows from its neighbour's): 2^26 elements in rows of 256 80 us
+// (221 with a 64-bit division per element).  Index: 32 bits where the element
+// count allows it.
+template <class Index>
 __global__ void __launch_bounds__(kThreads)
-decodeRowScaleKernel(const uint8_t *__restrict__ values,
-                     const float *__restrict__ scales, size_t elements,
-                     size_t row_length, float *__restrict__ output) {
-  for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
-       i < elements; i += static_cast<size_t>(gridDim.x) * blockDim.x) {
-    output[i] = rowScaleDecode(decodeE4M3(values[i]), scales[i / row_length]);
+decodeRowScaleKernel(const uint8_t *__restrict__ values, const float *__restrict__ scales,
+                     size_t elements, size_t row_length, float *__restrict__ output, bool vector_ok,
+                     int mode) {
+  const size_t groups = (elements + kGroup - 1) / kGroup;
+  for (size_t group = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
+       group < groups; group += static_cast<size_t>(gridDim.x) * blockDim.x) {
+    const size_t base = group * kGroup;
+    const size_t valid = elements - base < kGroup ? elements - base : kGroup;
+    uint64_t packed = 0;
+    if (vector_ok && valid == kGroup) {
+      packed = *reinterpret_cast<const uint64_t *>(values + base);
+    } else {
+      for (size_t i = 0; i < valid; ++i) packed |= static_cast<uint64_t>(values[base + i]) << (8 * i);
+    }
+    Group g = decodeGroup<MSQ_FMT_FP8_E4M3FN>(packed, 127u);
+    size_t row = static_cast<Index>(base) / static_cast<Index>(row_length);
+    size_t left = row_length - (base - row * row_length);  // elements of the row from here
+    float scale = scales[row];
+    if (left >= kGroup) {
+#pragma unroll
+      for (int i = 0; i < kGroup; ++i) g.v[i] = rowScaleDecode(g.v[i], scale);
+    } else {
+#pragma unroll
+      for (int i = 0; i < kGroup; ++i) {
+        if (left == 0 && i < static_cast<int>(valid)) {
+          scale = scales[++row];
+          left = row_length;
+        }
+        --left;
+        g.v[i] = rowScaleDecode(g.v[i], scale);
+      }
+    }
+    storeGroup(output, base, elements, vector_ok ? mode : 0, g);
   }
 }
 
 bool aligned16(const void *p) {
   return (reinterpret_cast<uintptr_t>(p) & 15u) == 0;
-}
-
-// ------------------------------------------------- stochastic rounding
-
-// Stochastic encoders (msq_encode_stochastic): one thread per element, the
-// element's flat index feeding the hash; FP4 lanes pair up by shuffle (the
-// even lane writes the byte); MX formats take one warp per 32-element block
-// (the block's finite maximum by a warp reduction, then x / 2^e per lane as
-// the nearest encoders compute it).  The loop is warp-uniform.
-template <int kFormat>
-__global__ void __launch_bounds__(kThreads)
-encodeStochasticKernel(const float *__restrict__ source, size_t elements, uint32_t seed,
-                       uint32_t stream, uint8_t *__restrict__ values,
-                       uint8_t *__restrict__ scales) {
-  constexpr bool kMx = kFormat == MSQ_FMT_MXFP8_E4M3FN || kFormat == MSQ_FMT_MXFP8_E5M2 ||
-                       kFormat == MSQ_FMT_MXFP4_E2M1;
-  constexpr bool kFp4 = kFormat == MSQ_FMT_FP4_E2M1 || kFormat == MSQ_FMT_MXFP4_E2M1;
-  const int lane = threadIdx.x & 31;
-  const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
-  for (size_t base = blockIdx.x * static_cast<size_t>(blockDim.x) + (threadIdx.x & ~31u);
-       base < elements; base += stride) {
-    const size_t i = base + lane;
-    const bool valid = i < elements;
-    float x = valid ? source[i] : 0.0f;
-    if constexpr (kMx) {
-      constexpr int kEmax = kFormat == MSQ_FMT_MXFP8_E4M3FN ? 8 : (kFormat == MSQ_FMT_MXFP8_E5M2 ? 15 : 2);
-      const float a = fabsf(x);
-      // finite magnitudes order like their bits
-      uint32_t m = valid && a <= 3.402823466e38f ? __float_as_uint(a) : 0u;
-      m = __reduce_max_sync(0xffffffffu, m);
-      const int e = mxExponent(__uint_as_float(m), kEmax);
-      if (lane == 0) scales[base / 32] = static_cast<uint8_t>(e + 127);
-      x = mxDivide(x, e);
-    }
-    const uint32_t index = static_cast<uint32_t>(i);
-    if constexpr (kFormat == MSQ_FMT_BF16) {
-      if (valid) reinterpret_cast<uint16_t *>(values)[i] = encodeBf16Stochastic(x, index, seed, stream);
-    } else if constexpr (kFormat == MSQ_FMT_FP8_E4M3FN || kFormat == MSQ_FMT_MXFP8_E4M3FN) {
-      if (valid) values[i] = encodeE4M3Stochastic(x, index, seed, stream);
-    } else if constexpr (kFormat == MSQ_FMT_FP8_E5M2 || kFormat == MSQ_FMT_MXFP8_E5M2) {
-      if (valid) values[i] = encodeE5M2Stochastic(x, index, seed, stream);
-    } else {
-      static_assert(kFp4, "format");
-      const uint32_t code = valid ? encodeE2M1Stochastic(x, index, seed, stream) : 0u;
-      const uint32_t next = __shfl_down_sync(0xffffffffu, code, 1);
-      if (valid && (i & 1) == 0) {
-        values[i / 2] = static_cast<uint8_t>(code | (i + 1 < elements ? next << 4 : 0u));
-      }
-    }
-  }
-}
-
-// Row-scaled FP8 with stochastic rounding: one warp per row as the nearest
-// row-scale encoder, each element rounded with its flat index.
-__global__ void __launch_bounds__(kThreads)
-encodeRowScaleStochasticKernel(const float *__restrict__ source, size_t rows, size_t row_length,
-                               uint32_t seed, uint32_t stream, uint8_t *__restrict__ values,
-                               float *__restrict__ scales) {
-  const int lane = threadIdx.x % 32;
-  const size_t warps = static_cast<size_t>(gridDim.x) * (blockDim.x / 32);
-  for (size_t row = blockIdx.x * static_cast<size_t>(blockDim.x / 32) + threadIdx.x / 32;
-       row < rows; row += warps) {
-    const float *in = source + row * row_length;
-    float m = 0.0f;
-    for (size_t i = lane; i < row_length; i += 32) {
-      const float a = fabsf(in[i]);
-      if (a <= 3.402823466e38f) m = fmaxf(m, a);
-    }
-#pragma unroll
-    for (int s = 16; s > 0; s >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, s));
-    const float scale = m == 0.0f ? 1.0f : __fdiv_rn(m, 448.0f);
-    if (lane == 0) scales[row] = scale;
-    uint8_t *out = values + row * row_length;
-    for (size_t i = lane; i < row_length; i += 32) {
-      out[i] = encodeE4M3Stochastic(rowDivide(in[i], scale),
-                                    static_cast<uint32_t>(row * row_length + i), seed, stream);
-    }
-  }
 }
 
 // ------------------------------------------------- log-spectrum storage
@@ -594,86 +684,61 @@ spectrumDecodeKernel(const uint8_t *__restrict__ values, const float2 *__restric
 // with MX blocks of 32 consecutive elements and scale rows of n elements
 // taken within each matrix (n^2 elements from its offset), so the result is
 // the encode -> decode round trip of each matrix on its own.
+//
+// Eight elements per thread (four lanes per MX block), eight elements per
+// lane and step of a scale row.  Eight matrices of order 384 in MXFP8: 16 us
+// (29 with a thread per block).
 template <int kFormat>
 __global__ void __launch_bounds__(kThreads)
 quantizeBatchKernel(float *__restrict__ x, const int64_t *__restrict__ offset,
                     const int32_t *__restrict__ n, int count) {
-  constexpr bool kMx = kFormat == MSQ_FMT_MXFP8_E4M3FN || kFormat == MSQ_FMT_MXFP8_E5M2 ||
-                       kFormat == MSQ_FMT_MXFP4_E2M1;
-  constexpr int kEmax = kFormat == MSQ_FMT_MXFP8_E4M3FN ? 8 : kFormat == MSQ_FMT_MXFP8_E5M2 ? 15 : 2;
+  const int lane = threadIdx.x % 32;
   for (int mi = blockIdx.y; mi < count; mi += gridDim.y) {
     const int nn = n[mi];
-    const int64_t elements = static_cast<int64_t>(nn) * nn;
+    const size_t elements = static_cast<size_t>(nn) * nn;
     float *p = x + offset[mi];
     if constexpr (kFormat == MSQ_FMT_FP8_E4M3FN_ROWSCALE) {
       // one warp per row of n consecutive elements (encodeRowScaleKernel)
-      const int lane = threadIdx.x % 32;
       const int warps = gridDim.x * (blockDim.x / 32);
       for (int row = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32; row < nn; row += warps) {
         float *in = p + static_cast<int64_t>(row) * nn;
         float m = 0.0f;
+#pragma unroll 4
         for (int i = lane; i < nn; i += 32) {
           const float a = fabsf(in[i]);
-          if (a <= 3.402823466e38f) m = fmaxf(m, a);
+          if (a <= kLargestFinite) m = fmaxf(m, a);
         }
 #pragma unroll
         for (int sh = 16; sh > 0; sh >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, sh));
         const float scale = m == 0.0f ? 1.0f : __fdiv_rn(m, 448.0f);
+#pragma unroll 4
         for (int i = lane; i < nn; i += 32)
           in[i] = rowScaleDecode(decodeE4M3(encodeE4M3(rowDivide(in[i], scale))), scale);
       }
-    } else if constexpr (kMx) {
-      // one thread per 32-element block (encodeMxKernel / decodeKernel)
-      const int64_t blocks = (elements + 31) / 32;
-      for (int64_t blk = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; blk < blocks;
-           blk += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        const int64_t base = blk * 32;
-        float v[32];
-        float m = 0.0f;
-#pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          v[i] = base + i < elements ? p[base + i] : 0.0f;
-          const float a = fabsf(v[i]);
-          if (a <= 3.402823466e38f) m = fmaxf(m, a);  // finite only (NaN fails)
-        }
-        const int e = mxExponent(m, kEmax);
-        const uint32_t scale = static_cast<uint32_t>(e + 127);
-        if constexpr (kFormat == MSQ_FMT_MXFP4_E2M1) {
-          const bool exact = e >= -126 && e <= 126;
-          const float sc = exact ? exp2Int(-e) : 1.0f;
-#pragma unroll
-          for (int i = 0; i < 32; i += 2) {
-            uint32_t pair;
-            if (exact) {
-              pair = encodeE2M1Pair(v[i] * sc, v[i + 1] * sc, v[i], v[i + 1]);
-            } else {
-              const float a = mxDivide(v[i], e), b = mxDivide(v[i + 1], e);
-              pair = encodeE2M1Pair(a, b, a, b);
-            }
-            v[i] = mxScale(decodeE2M1(pair & 0xfu), scale);
-            v[i + 1] = mxScale(decodeE2M1((pair >> 4) & 0xfu), scale);
-          }
-        } else {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const float scaled = mxDivide(v[i], e);
-            const float d = kFormat == MSQ_FMT_MXFP8_E4M3FN ? decodeE4M3(encodeE4M3(scaled))
-                                                            : decodeE5M2(encodeE5M2(scaled));
-            v[i] = mxScale(d, scale);
-          }
-        }
-#pragma unroll
-        for (int i = 0; i < 32; ++i)
-          if (base + i < elements) p[base + i] = v[i];
-      }
     } else {
-      for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < elements;
-           i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        const float y = p[i];
-        if constexpr (kFormat == MSQ_FMT_BF16) p[i] = decodeBf16(encodeBf16(y));
-        else if constexpr (kFormat == MSQ_FMT_FP8_E4M3FN) p[i] = decodeE4M3(encodeE4M3(y));
-        else if constexpr (kFormat == MSQ_FMT_FP8_E5M2) p[i] = decodeE5M2(encodeE5M2(y));
-        else p[i] = decodeE2M1(encodeE2M1(y));  // FP4 E2M1
+      const int mode = vectorMode(p);
+      const size_t groups = isMx(kFormat) ? (elements + 31) / 32 * 4 : (elements + kGroup - 1) / kGroup;
+      // on the warp's first group, as encodeMxKernel
+      for (size_t group = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
+           group - lane < groups; group += static_cast<size_t>(gridDim.x) * blockDim.x) {
+        const size_t base = group * kGroup;
+        Group g = loadGroup(p, base, elements, mode);
+        if constexpr (kFormat == MSQ_FMT_BF16) {
+#pragma unroll
+          for (int i = 0; i < kGroup; ++i) g.v[i] = decodeBf16(encodeBf16(g.v[i]));
+        } else {
+          float m = groupMaxNan(g);
+          const bool finite = m <= kLargestFinite;
+          int e = 0;
+          if constexpr (isMx(kFormat)) {
+            if (!finite) m = groupMaxFinite(g);
+            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
+            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
+            e = mxExponent(m, elementEmax(kFormat));
+          }
+          g = decodeGroup<kFormat>(encodeGroup<kFormat>(g, finite, e), static_cast<uint32_t>(e + 127));
+        }
+        storeGroup(p, base, elements, mode, g);
       }
     }
   }
@@ -684,10 +749,9 @@ quantizeBatchKernel(float *__restrict__ x, const int64_t *__restrict__ offset,
 int quantizeBatch(msq_ctx *ctx, int format, const DeviceBatch *b, float *x) {
   if (format == MSQ_FMT_FP32) return MSQ_OK;
   const int64_t nn = static_cast<int64_t>(b->max_n) * b->max_n;
-  int64_t units = nn;                                               // elements
-  if (format == MSQ_FMT_FP8_E4M3FN_ROWSCALE) units = static_cast<int64_t>(b->max_n) * 32;  // a warp per row
-  else if (format == MSQ_FMT_MXFP8_E4M3FN || format == MSQ_FMT_MXFP8_E5M2 ||
-           format == MSQ_FMT_MXFP4_E2M1) units = (nn + 31) / 32;   // a thread per block
+  // a thread per group of eight elements, a warp per scale row
+  const int64_t units = format == MSQ_FMT_FP8_E4M3FN_ROWSCALE ? static_cast<int64_t>(b->max_n) * 32
+                                                              : (nn + 31) / 32 * 4;
   const dim3 grid(static_cast<unsigned>(std::max<int64_t>(1, std::min<int64_t>((units + kThreads - 1) / kThreads, 64))),
                   static_cast<unsigned>(std::min(b->count, 65535)));
   switch (format) {
@@ -740,6 +804,68 @@ extern "C" size_t msq_scale_bytes(int format, size_t elements, size_t row_length
   }
 }
 
+namespace {
+
+// msq_encode and msq_encode_stochastic after their checks.
+template <bool kStochastic>
+int encode(msq_ctx *ctx, int format, const float *source, size_t elements, size_t row_length,
+           uint32_t seed, uint32_t stream, uint8_t *values, uint8_t *scales, const char *what) {
+  // values are stored in at most 16 bytes
+  const int mode = aligned16(values) ? vectorMode(source) : 0;
+  const unsigned grid = gridFor((elements + kGroup - 1) / kGroup, kThreads);
+  const unsigned mx_grid = gridFor((elements + 31) / 32 * 4, kThreads);
+  cudaStream_t s = ctx->stream;
+  switch (format) {
+    case MSQ_FMT_FP32:
+      return cudaCheck(ctx, cudaMemcpyAsync(values, source, elements * 4, cudaMemcpyDeviceToDevice, s), what);
+#define MSQ_ENCODE_CASE(F)                                                                       \
+    case F:                                                                                      \
+      encodeScalarKernel<F, kStochastic><<<grid, kThreads, 0, s>>>(source, elements, seed, stream, \
+                                                                   values, mode);                \
+      break;
+    MSQ_ENCODE_CASE(MSQ_FMT_BF16)
+    MSQ_ENCODE_CASE(MSQ_FMT_FP8_E4M3FN)
+    MSQ_ENCODE_CASE(MSQ_FMT_FP8_E5M2)
+    MSQ_ENCODE_CASE(MSQ_FMT_FP4_E2M1)
+#undef MSQ_ENCODE_CASE
+    case MSQ_FMT_MXFP8_E4M3FN:
+      encodeMxKernel<MSQ_FMT_MXFP8_E4M3FN, kStochastic><<<mx_grid, kThreads, 0, s>>>(
+          source, elements, seed, stream, values, scales, mode);
+      break;
+    case MSQ_FMT_MXFP8_E5M2:
+      encodeMxKernel<MSQ_FMT_MXFP8_E5M2, kStochastic><<<mx_grid, kThreads, 0, s>>>(
+          source, elements, seed, stream, values, scales, mode);
+      break;
+    case MSQ_FMT_MXFP4_E2M1:
+      if (!kStochastic && mode != 0 && elements >= 32) {
+        const size_t whole = elements / 32, rest = elements - whole * 32;
+        encodeMxfp4Kernel<<<gridFor(whole, kThreads), kThreads, 0, s>>>(source, whole, values, scales);
+        if (rest != 0) {
+          MSQ_TRY(launched(ctx, what));
+          encodeMxKernel<MSQ_FMT_MXFP4_E2M1, false><<<1, kThreads, 0, s>>>(
+              source + whole * 32, rest, 0, 0, values + whole * 16, scales + whole, mode);
+        }
+      } else {
+        encodeMxKernel<MSQ_FMT_MXFP4_E2M1, kStochastic><<<mx_grid, kThreads, 0, s>>>(
+            source, elements, seed, stream, values, scales, mode);
+      }
+      break;
+    case MSQ_FMT_FP8_E4M3FN_ROWSCALE:
+      if (row_length == 0 || elements % row_length != 0) {
+        return setError(ctx, MSQ_ERR_INVALID_ARGUMENT,
+                        std::string(what) + ": elements must be a multiple of row_length");
+      }
+      launchRowScale<kStochastic>(source, elements / row_length, row_length, seed, stream, values,
+                                  reinterpret_cast<float *>(scales), s);
+      break;
+    default:
+      return setError(ctx, MSQ_ERR_INVALID_ARGUMENT, std::string(what) + ": unknown format");
+  }
+  return launched(ctx, what);
+}
+
+}  // namespace
+
 extern "C" int msq_encode(msq_ctx *ctx, int format, const float *source,
                           size_t elements, size_t row_length, uint8_t *values,
                           uint8_t *scales) {
@@ -754,61 +880,7 @@ extern "C" int msq_encode(msq_ctx *ctx, int format, const float *source,
     return setError(ctx, MSQ_ERR_INVALID_ARGUMENT,
                     "msq_encode: this format requires a scale plane");
   }
-  const bool vec = aligned16(source) && aligned16(values);
-  const size_t groups = (elements + kGroup - 1) / kGroup;
-  const unsigned grid = gridFor(groups, kThreads);
-  cudaStream_t s = ctx->stream;
-  switch (format) {
-    case MSQ_FMT_FP32:
-      return cudaCheck(ctx, cudaMemcpyAsync(values, source, elements * 4,
-                                            cudaMemcpyDeviceToDevice, s),
-                       "msq_encode fp32 copy");
-    case MSQ_FMT_BF16:
-      encodeScalarKernel<MSQ_FMT_BF16><<<grid, kThreads, 0, s>>>(source, elements, values, scales, vec);
-      break;
-    case MSQ_FMT_FP8_E4M3FN:
-      encodeScalarKernel<MSQ_FMT_FP8_E4M3FN><<<grid, kThreads, 0, s>>>(source, elements, values, scales, vec);
-      break;
-    case MSQ_FMT_FP8_E5M2:
-      encodeScalarKernel<MSQ_FMT_FP8_E5M2><<<grid, kThreads, 0, s>>>(source, elements, values, scales, vec);
-      break;
-    case MSQ_FMT_FP4_E2M1:
-      encodeScalarKernel<MSQ_FMT_FP4_E2M1><<<grid, kThreads, 0, s>>>(source, elements, values, scales, vec);
-      break;
-    case MSQ_FMT_MXFP8_E4M3FN:
-      encodeMxKernel<MSQ_FMT_MXFP8_E4M3FN><<<gridFor((elements + 31) / 32 * 4, kThreads), kThreads, 0, s>>>(source, elements, values, scales, vec);
-      break;
-    case MSQ_FMT_MXFP8_E5M2:
-      encodeMxKernel<MSQ_FMT_MXFP8_E5M2><<<gridFor((elements + 31) / 32 * 4, kThreads), kThreads, 0, s>>>(source, elements, values, scales, vec);
-      break;
-    case MSQ_FMT_MXFP4_E2M1:
-      if (vec && elements >= 32) {
-        const size_t whole = elements / 32;
-        encodeMxfp4Kernel<<<gridFor(whole, kThreads), kThreads, 0, s>>>(source, whole, values, scales);
-        if (whole * 32 < elements) {
-          MSQ_TRY(launched(ctx, "msq_encode"));
-          const size_t rest = elements - whole * 32;
-          encodeMxKernel<MSQ_FMT_MXFP4_E2M1><<<1, kThreads, 0, s>>>(
-              source + whole * 32, rest, values + whole * 16, scales + whole, vec);
-        }
-      } else {
-        encodeMxKernel<MSQ_FMT_MXFP4_E2M1><<<gridFor((elements + 31) / 32 * 4, kThreads), kThreads, 0, s>>>(source, elements, values, scales, vec);
-      }
-      break;
-    case MSQ_FMT_FP8_E4M3FN_ROWSCALE: {
-      if (row_length == 0 || elements % row_length != 0) {
-        return setError(ctx, MSQ_ERR_INVALID_ARGUMENT,
-                        "msq_encode: elements must be a multiple of row_length");
-      }
-      const size_t rows = elements / row_length;
-      encodeRowScaleKernel<<<gridFor(rows * 32, kThreads), kThreads, 0, s>>>(
-          source, rows, row_length, values, reinterpret_cast<float *>(scales));
-      break;
-    }
-    default:
-      return setError(ctx, MSQ_ERR_INVALID_ARGUMENT, "msq_encode: unknown format");
-  }
-  return launched(ctx, "msq_encode");
+  return encode<false>(ctx, format, source, elements, row_length, 0, 0, values, scales, "msq_encode");
 }
 
 extern "C" int msq_decode(msq_ctx *ctx, int format, const uint8_t *values,
@@ -826,6 +898,7 @@ extern "C" int msq_decode(msq_ctx *ctx, int format, const uint8_t *values,
                     "msq_decode: this format requires a scale plane");
   }
   const bool vec = aligned16(values) && aligned16(output);
+  const int mode = vectorMode(output);
   const size_t groups = (elements + kGroup - 1) / kGroup;
   const unsigned grid = gridFor(groups, kThreads);
   cudaStream_t s = ctx->stream;
@@ -841,14 +914,14 @@ extern "C" int msq_decode(msq_ctx *ctx, int format, const uint8_t *values,
         if (whole * 32 < elements) {
           MSQ_TRY(launched(ctx, "msq_decode"));
           decodeKernel<MSQ_FMT_MXFP4_E2M1><<<1, kThreads, 0, s>>>(
-              values + whole * 16, scales + whole, elements - whole * 32, output + whole * 32, vec);
+              values + whole * 16, scales + whole, elements - whole * 32, output + whole * 32, vec, mode);
         }
       } else {
-        decodeKernel<MSQ_FMT_MXFP4_E2M1><<<grid, kThreads, 0, s>>>(values, scales, elements, output, vec);
+        decodeKernel<MSQ_FMT_MXFP4_E2M1><<<grid, kThreads, 0, s>>>(values, scales, elements, output, vec, mode);
       }
       break;
 #define MSQ_DECODE_CASE(F) \
-    case F: decodeKernel<F><<<grid, kThreads, 0, s>>>(values, scales, elements, output, vec); break;
+    case F: decodeKernel<F><<<grid, kThreads, 0, s>>>(values, scales, elements, output, vec, mode); break;
     MSQ_DECODE_CASE(MSQ_FMT_BF16)
     MSQ_DECODE_CASE(MSQ_FMT_FP8_E4M3FN)
     MSQ_DECODE_CASE(MSQ_FMT_FP8_E5M2)
@@ -861,8 +934,13 @@ extern "C" int msq_decode(msq_ctx *ctx, int format, const uint8_t *values,
         return setError(ctx, MSQ_ERR_INVALID_ARGUMENT,
                         "msq_decode: elements must be a multiple of row_length");
       }
-      decodeRowScaleKernel<<<gridFor(elements, kThreads), kThreads, 0, s>>>(
-          values, reinterpret_cast<const float *>(scales), elements, row_length, output);
+      if (elements <= 0xffffffffu) {
+        decodeRowScaleKernel<uint32_t><<<grid, kThreads, 0, s>>>(
+            values, reinterpret_cast<const float *>(scales), elements, row_length, output, vec, mode);
+      } else {
+        decodeRowScaleKernel<size_t><<<grid, kThreads, 0, s>>>(
+            values, reinterpret_cast<const float *>(scales), elements, row_length, output, vec, mode);
+      }
       break;
     default:
       return setError(ctx, MSQ_ERR_INVALID_ARGUMENT, "msq_decode: unknown format");
@@ -884,48 +962,8 @@ extern "C" int msq_encode_stochastic(msq_ctx *ctx, int format, const float *sour
     return setError(ctx, MSQ_ERR_INVALID_ARGUMENT,
                     "msq_encode_stochastic: this format requires a scale plane");
   }
-  cudaStream_t s = ctx->stream;
-  const unsigned grid = gridFor((elements + 31) / 32 * 32, kThreads);
-  switch (format) {
-    case MSQ_FMT_FP32:
-      return cudaCheck(ctx, cudaMemcpyAsync(values, source, elements * 4,
-                                            cudaMemcpyDeviceToDevice, s),
-                       "msq_encode_stochastic fp32 copy");
-    case MSQ_FMT_BF16:
-      encodeStochasticKernel<MSQ_FMT_BF16><<<grid, kThreads, 0, s>>>(source, elements, seed, stream, values, scales);
-      break;
-    case MSQ_FMT_FP8_E4M3FN:
-      encodeStochasticKernel<MSQ_FMT_FP8_E4M3FN><<<grid, kThreads, 0, s>>>(source, elements, seed, stream, values, scales);
-      break;
-    case MSQ_FMT_FP8_E5M2:
-      encodeStochasticKernel<MSQ_FMT_FP8_E5M2><<<grid, kThreads, 0, s>>>(source, elements, seed, stream, values, scales);
-      break;
-    case MSQ_FMT_FP4_E2M1:
-      encodeStochasticKernel<MSQ_FMT_FP4_E2M1><<<grid, kThreads, 0, s>>>(source, elements, seed, stream, values, scales);
-      break;
-    case MSQ_FMT_MXFP8_E4M3FN:
-      encodeStochasticKernel<MSQ_FMT_MXFP8_E4M3FN><<<grid, kThreads, 0, s>>>(source, elements, seed, stream, values, scales);
-      break;
-    case MSQ_FMT_MXFP8_E5M2:
-      encodeStochasticKernel<MSQ_FMT_MXFP8_E5M2><<<grid, kThreads, 0, s>>>(source, elements, seed, stream, values, scales);
-      break;
-    case MSQ_FMT_MXFP4_E2M1:
-      encodeStochasticKernel<MSQ_FMT_MXFP4_E2M1><<<grid, kThreads, 0, s>>>(source, elements, seed, stream, values, scales);
-      break;
-    case MSQ_FMT_FP8_E4M3FN_ROWSCALE: {
-      if (row_length == 0 || elements % row_length != 0) {
-        return setError(ctx, MSQ_ERR_INVALID_ARGUMENT,
-                        "msq_encode_stochastic: elements must be a multiple of row_length");
-      }
-      const size_t rows = elements / row_length;
-      encodeRowScaleStochasticKernel<<<gridFor(rows * 32, kThreads), kThreads, 0, s>>>(
-          source, rows, row_length, seed, stream, values, reinterpret_cast<float *>(scales));
-      break;
-    }
-    default:
-      return setError(ctx, MSQ_ERR_INVALID_ARGUMENT, "msq_encode_stochastic: unknown format");
-  }
-  return launched(ctx, "msq_encode_stochastic");
+  return encode<true>(ctx, format, source, elements, row_length, seed, stream, values, scales,
+                      "msq_encode_stochastic");
 }
 
 extern "C" size_t msq_spectrum_metadata_bytes(size_t elements) {
