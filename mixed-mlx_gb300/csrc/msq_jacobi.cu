@@ -1345,13 +1345,16 @@ int jacobiEnqueue(msq_ctx *ctx, const DeviceBatch *b, float *matrices, float *ve
   }
   // Large matrices: the grid kernels on the context's stream, overlapping the
   // batched sweeps still running on the internal streams.
+  int busy = serial ? 0 : plan->tl.count;  // one CTA per matrix
+  if (!serial)
+    for (const auto &bucket : plan->buckets) busy += bucket.count;
   for (const int gi : plan->grid_ids) {
     int sweeps = 0;
     double ratio = 0.0, norm2 = 0.0;
     MSQ_TRY(gridJacobiSolve(ctx, matrices + b->host_offset[gi], vectors + b->host_offset[gi],
                             eigenvalues + b->host_eig_offset[gi], b->host_n[gi],
                             tols_host ? tols_host[gi] : tolerance, max_sweeps,
-                            &sweeps, &ratio, &norm2, keep_vectors));
+                            &sweeps, &ratio, &norm2, keep_vectors, busy));
     gridStateKernel<<<1, 1, 0, ctx->stream>>>(args.state + gi, sweeps, ratio, norm2);
     MSQ_TRY(launched(ctx, "jacobi grid state"));
   }

@@ -615,17 +615,28 @@ int gridAttributes(msq_ctx *ctx) {
 
 int gridJacobiSolve(msq_ctx *ctx, float *matrix, float *vectors, float *eigenvalues, int n,
                     double tolerance, int max_sweeps, int *sweeps_out, double *off_ratio_out,
-                    double *norm2_out, bool keep_vectors) {
+                    double *norm2_out, bool keep_vectors, int busy) {
   const int m = padded8(n), nb = m / 4, P = nb / 2, rounds = nb - 1;
   int sms = 0;
   MSQ_TRY(cudaCheck(ctx, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device),
                     "grid SM count"));
-  const int ctas = std::min(sms, kSmCount);  // all resident, one per SM
-  if (P > 2 * kMaxPasses * ctas) return setError(ctx, MSQ_ERR_UNSUPPORTED, "grid jacobi: order too large");
+  // All resident, one per SM, beside the `busy` CTAs of other streams where
+  // they leave half of the SMs and V's rows stay in shared memory: a sweep
+  // waits for all its SMs at once (2048 matrices with 47 fallbacks, three of
+  // them here: 148 ms on every SM, 138 so).
+  sms = std::min(sms, kSmCount);
+  if (P > 2 * kMaxPasses * sms) return setError(ctx, MSQ_ERR_UNSUPPORTED, "grid jacobi: order too large");
+  auto storeFor = [&](int ctas) {
+    int store = kVShared;
+    while (store < kNoneShared && gridSweepSmem(store, P, m, (n + ctas - 1) / ctas) > kGridSmemLimit) ++store;
+    return store;
+  };
+  const int beside = sms - busy;
+  const bool share = busy > 0 && 2 * beside >= sms && P <= 2 * kMaxPasses * beside && storeFor(beside) == kVShared;
+  const int ctas = share ? beside : sms;
   GridArgs g{};
   g.rows = (n + ctas - 1) / ctas;
-  int store = kVShared;
-  while (store < kNoneShared && gridSweepSmem(store, P, m, g.rows) > kGridSmemLimit) ++store;
+  const int store = storeFor(ctas);
   const size_t smem = gridSweepSmem(store, P, m, g.rows);
   const int launch_rounds = store == kVShared ? rounds : std::min(rounds, kLogRounds);
   const int64_t tile_floats = static_cast<int64_t>(nb) * (nb + 1) / 2 * kTileF;
