@@ -17,6 +17,7 @@
 #include "msq_dense.cuh"
 #include "msq_internal.cuh"
 #include "msq_f32x2.cuh"
+#include "msq_gemm_sliced.cuh"
 #include "msq_residual.cuh"
 
 #include <algorithm>
@@ -28,10 +29,6 @@ namespace {
 constexpr int kTile = 64;    // output tile
 constexpr int kBK = 16;      // K step
 constexpr int kThreads = 256;  // 16 x 16 threads, 4 x 4 outputs each
-
-__device__ __forceinline__ float rootOf(float lambda) {
-  return sqrtf(fmaxf(lambda, 0.0f));
-}
 
 // ---- FP32 GEMM ---------------------------------------------------------------
 // C = op(A) op(B) on the CUDA cores, each element the FMA chain over k in
@@ -549,17 +546,19 @@ int gemmClass(const DeviceBatch *b, int n) {
 }
 
 // The tiles (matrix, i, j) of every matrix of one tile class, cached on the
-// batch; `upper`: only those on or above the diagonal.
-int gemmTiles(msq_ctx *ctx, const DeviceBatch *b, int tile, bool upper, const int4 **work,
-              int *items) {
-  return tileWork(ctx, b, tile, upper, kGemmWorkBase + (upper ? 1 : 0) + 2 * tile, work, items,
-                  [&](int n) { return gemmClass(b, n) == tile; });
+// batch; `upper`: only those on or above the diagonal; `unsliced`: of the
+// matrices that slicedMatrix refuses.
+int gemmTiles(msq_ctx *ctx, const DeviceBatch *b, int tile, bool upper, bool unsliced,
+              const int4 **work, int *items) {
+  return tileWork(ctx, b, tile, upper, kGemmWorkBase + (upper ? 1 : 0) + 2 * tile + (unsliced ? 1024 : 0),
+                  work, items, [&](int n) { return gemmClass(b, n) == tile && !(unsliced && slicedMatrix(n)); });
 }
 
 template <int kT, bool kMajorA, bool kMajorB>
-int launchGemm(msq_ctx *ctx, const DeviceBatch *b, GemmArgs args, int epilogue, bool mirror) {
+int launchGemm(msq_ctx *ctx, const DeviceBatch *b, GemmArgs args, int epilogue, bool mirror,
+               bool unsliced) {
   using S = GemmShape<kT>;
-  MSQ_TRY(gemmTiles(ctx, b, kT, mirror, &args.work, &args.items));
+  MSQ_TRY(gemmTiles(ctx, b, kT, mirror, unsliced, &args.work, &args.items));
   if (args.items == 0) return MSQ_OK;
   const unsigned grid = std::min<unsigned>(args.items, kSmCount * S::kCtas * 4);
   if (mirror) {
@@ -574,16 +573,16 @@ int launchGemm(msq_ctx *ctx, const DeviceBatch *b, GemmArgs args, int epilogue, 
 
 template <bool kMajorA, bool kMajorB>
 int launchGemmClasses(msq_ctx *ctx, const DeviceBatch *b, const GemmArgs &args, int epilogue,
-                      bool mirror) {
-  MSQ_TRY((launchGemm<128, kMajorA, kMajorB>(ctx, b, args, epilogue, mirror)));
-  MSQ_TRY((launchGemm<64, kMajorA, kMajorB>(ctx, b, args, epilogue, mirror)));
-  return launchGemm<32, kMajorA, kMajorB>(ctx, b, args, epilogue, mirror);
+                      bool mirror, bool unsliced) {
+  MSQ_TRY((launchGemm<128, kMajorA, kMajorB>(ctx, b, args, epilogue, mirror, unsliced)));
+  MSQ_TRY((launchGemm<64, kMajorA, kMajorB>(ctx, b, args, epilogue, mirror, unsliced)));
+  return launchGemm<32, kMajorA, kMajorB>(ctx, b, args, epilogue, mirror, unsliced);
 }
 
 }  // namespace
 
 int gemmTN(msq_ctx *ctx, const DeviceBatch *b, const float *a, const float *bm, float *c,
-           int epilogue, const float *eigenvalues, bool a_mmajor, bool b_nmajor) {
+           int epilogue, const float *eigenvalues, bool a_mmajor, bool b_nmajor, bool unsliced) {
   GemmArgs args{};
   args.a = a;
   args.b = bm;
@@ -597,10 +596,10 @@ int gemmTN(msq_ctx *ctx, const DeviceBatch *b, const float *a, const float *bm, 
   // one operand against itself in the same layout (F^T F or F F^T): symmetric
   const bool mirror = a == bm && a_mmajor == b_nmajor && epilogue == kEpilogueStore;
   if (a_mmajor)
-    return b_nmajor ? launchGemmClasses<true, true>(ctx, b, args, epilogue, mirror)
-                    : launchGemmClasses<true, false>(ctx, b, args, epilogue, mirror);
-  return b_nmajor ? launchGemmClasses<false, true>(ctx, b, args, epilogue, mirror)
-                  : launchGemmClasses<false, false>(ctx, b, args, epilogue, mirror);
+    return b_nmajor ? launchGemmClasses<true, true>(ctx, b, args, epilogue, mirror, unsliced)
+                    : launchGemmClasses<true, false>(ctx, b, args, epilogue, mirror, unsliced);
+  return b_nmajor ? launchGemmClasses<false, true>(ctx, b, args, epilogue, mirror, unsliced)
+                  : launchGemmClasses<false, false>(ctx, b, args, epilogue, mirror, unsliced);
 }
 
 int residualFF(msq_ctx *ctx, const DeviceBatch *b, const float *a, const float *x_hi,

@@ -35,10 +35,11 @@ struct ResidualArgs {
 int gemmWork(msq_ctx *ctx, const DeviceBatch *b, int tile, const int4 **work, int *items);
 // C = A B per matrix, each element the FP32 FMA chain over k in order; by
 // default A(i,k) = a[k + i*n] and B(k,j) = bm[k + j*n] (C = a^T bm);
-// a_mmajor: A(i,k) = a[i + k*n]; b_nmajor: B(k,j) = bm[j + k*n].
+// a_mmajor: A(i,k) = a[i + k*n]; b_nmajor: B(k,j) = bm[j + k*n]; unsliced:
+// only the matrices that slicedMatrix refuses.
 int gemmTN(msq_ctx *ctx, const DeviceBatch *b, const float *a, const float *bm, float *c,
            int epilogue, const float *eigenvalues, bool a_mmajor = false,
-           bool b_nmajor = false);
+           bool b_nmajor = false, bool unsliced = false);
 // R = (a + a_lo) - (x_hi + x_lo)^2 in float-float; a_lo and x_lo may be null.
 int residualFF(msq_ctx *ctx, const DeviceBatch *b, const float *a, const float *x_hi,
                const float *x_lo, float *r, double *norms, const float *a_lo = nullptr);
@@ -53,5 +54,8 @@ int workingAdd(msq_ctx *ctx, const DeviceBatch *b, float *x_hi, float *x_lo, con
 // C_ij = W_ij / (s_i + s_j) for every matrix of the batch (s at eig_offset).
 int diagonalSylvesterBatch(msq_ctx *ctx, const DeviceBatch *b, const float *w, const float *s,
                            float *c);
+
+// s = sqrt(lambda); an FP32 eigenvalue <= 0 has root 0.
+__device__ __forceinline__ float rootOf(float lambda) { return sqrtf(fmaxf(lambda, 0.0f)); }
 
 }  // namespace msq

@@ -1,0 +1,567 @@
+// FP32 products of large matrices on the tensor cores.
+//
+// The CUDA cores' FP32 rate bounds a plain FP32 product (59% of it at order
+// 1000).  Here both operands are cut into kSlices = 4 digits (msq_slices.cuh),
+// each carrying its weight 2^-7p, and the products of digits p + q < 4 are
+// summed without rounding: one accumulator per weight, at most 4 pairs over
+// 1024 of K.  The pairs of weight 2^-28 join the last accumulator (rounded at
+// 2^-24 of it, far below the result): where a vector meets itself, as on the
+// diagonal of F^T F, they do not average out (a nearly diagonal matrix of order
+// 1000 loses 1.4e-6 without them, 7e-8 with them).  The four are put together in
+// float-float and rounded once.  What is cut off is below 2^-27 of the operands'
+// largest entries.  Relative Frobenius errors against 64 bits, FMA chain and
+// here, order 1000: F^T F of a Wishart matrix 4.3e-7 and 2.2e-8, of condition
+// 1e6 5.9e-7 and 2.9e-8, nearly diagonal and graded over 1e6 2.6e-7 and 7.4e-8;
+// corrections 8.5e-7 and 6.4e-8, 8.2e-7 and 6.7e-8, 8.0e-7 and 1.5e-7; smaller
+// too at orders 256, 512 and 2048.
+//
+// slicedGemmKernel is persistent and warp-specialized as the residual kernel:
+// a producer warp, an MMA warp, sixteen epilogue warps.  Tiles of 128 x 128 (at
+// N = 128 an MMA costs the 68 cycles that its read of A takes, as at N = 64),
+// 32 of K per stage (32 KB of A, 32 KB of B, three stages), four accumulators
+// of 128 columns: all of TMEM.  A stage is 26 MMAs, 1770 cycles, for 64 KB:
+// tensor pipe and operand loads are near balance.
+//
+// The largest magnitude of every column of a result, which the next product's
+// slices are scaled by, is taken in the epilogue.
+#include "msq_dense.cuh"
+#include "msq_gemm_sliced.cuh"
+#include "msq_internal.cuh"
+#include "msq_slices.cuh"
+
+#include <algorithm>
+#include <atomic>
+#include <cstring>
+#include <vector>
+
+namespace msq {
+namespace {
+
+constexpr int kSlices = 4;
+constexpr int kTile = 128, kTileK = 32;
+constexpr int kSliceBytes = kTile * 2 * kTileK;        // one digit of a tile, SWIZZLE_64B
+constexpr int kTileBytes = kSlices * kSliceBytes;
+constexpr int kStageBytes = 2 * kTileBytes;
+constexpr int kStages = 3;
+constexpr int kChunkTiles = 1024 / kTileK;             // K tiles per exact accumulation
+constexpr int kEpilogueWarps = 16;
+constexpr int kCols = kTile / (kEpilogueWarps / 4);    // columns per epilogue thread
+constexpr int kHalf = 16;                              // columns per TMEM load
+constexpr int kSlicedThreads = 32 * (kEpilogueWarps + 2);
+constexpr size_t kSlicedSmem = kStages * kStageBytes + 1024 + 256;
+static_assert(kSlices * kTile == 512, "one accumulator per weight fills TMEM");
+
+// Pairs (p, q) as 16 p + q, (0, g) first of accumulator g = min(p + q, 3).
+constexpr int kPairs = 13;
+__device__ constexpr uint8_t kPairOrder[kPairs] = {0x03, 0x02, 0x01, 0x00, 0x12, 0x11, 0x10,
+                                                   0x21, 0x20, 0x30, 0x13, 0x22, 0x31};
+__host__ __device__ constexpr int pairGroup(int p, int q) { return p + q < kSlices ? p + q : kSlices - 1; }
+
+__device__ __forceinline__ uint32_t finiteBits(float x) {
+  const float a = fabsf(x);
+  return a <= 3.402823466e38f ? __float_as_uint(a) : 0u;  // a NaN or infinity stays one in its digits
+}
+
+struct SliceArgs {
+  const int4 *rows;       // (matrix, tile, -, -)
+  const int4 *work;       // (matrix, tile, k tile, k tiles)
+  int row_items, items;
+  const float *x;
+  const int64_t *offset;
+  const int64_t *eig_offset;
+  const int64_t *tile_base;
+  const int32_t *n;
+  uint32_t *largest;      // bits of the largest finite magnitude per operand row
+  uint8_t *slices;
+};
+
+// Largest magnitudes of the operand's rows: the columns of X (a warp per
+// column, 128 columns per item over the 16 CTAs of grid.y), or with
+// kTranspose its rows (a thread per row, 1 / 16 of K per CTA of grid.y;
+// `largest` is zero before).
+template <bool kTranspose>
+__global__ void __launch_bounds__(256) largestKernel(SliceArgs args) {
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  for (int item = blockIdx.x; item < args.row_items; item += gridDim.x) {
+    const int4 w = args.rows[item];
+    const int n = args.n[w.x];
+    const float *x = args.x + args.offset[w.x];
+    uint32_t *largest = args.largest + args.eig_offset[w.x];
+    uint32_t m = 0;
+    if constexpr (kTranspose) {
+      const int i = w.y * kTile + threadIdx.x % kTile;
+      if (i < n) {
+#pragma unroll 4
+        for (int k = 2 * blockIdx.y + threadIdx.x / kTile; k < n; k += 32)
+          m = max(m, finiteBits(x[i + static_cast<int64_t>(k) * n]));
+        atomicMax(largest + i, m);
+      }
+    } else {
+      const int c = w.y * kTile + 8 * blockIdx.y + warp;
+      if (c < n) {
+#pragma unroll 4
+        for (int k = lane; k < n; k += 32) m = max(m, finiteBits(x[k + static_cast<int64_t>(c) * n]));
+        m = __reduce_max_sync(0xffffffffu, m);
+        if (lane == 0) largest[c] = m;
+      }
+    }
+  }
+}
+
+// The digits of a 128 x 32 piece as an operand tile (K-major): operand row =
+// column of X, or with kTranspose row of X.  A thread cuts 8 elements of a row
+// that are consecutive in K.
+template <bool kTranspose>
+__global__ void __launch_bounds__(256) digitKernel(SliceArgs args) {
+  for (int item = blockIdx.x; item < args.items; item += gridDim.x) {
+    const int4 w = args.work[item];
+    const int n = args.n[w.x];
+    const float *x = args.x + args.offset[w.x];
+    const uint32_t *largest = args.largest + args.eig_offset[w.x];
+    uint8_t *tile = args.slices +
+                    (args.tile_base[w.x] + static_cast<int64_t>(w.y) * w.w + w.z) * kTileBytes;
+    const bool vector = n % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const int unit = threadIdx.x + 256 * half;
+      const int r = kTranspose ? unit % kTile : unit / 4, c = kTranspose ? unit / kTile : unit % 4;
+      const int row = w.y * kTile + r, k0 = w.z * kTileK + 8 * c;
+      float v[8];
+      if (!kTranspose && vector && row < n && k0 + 8 <= n) {
+        const float4 *p = reinterpret_cast<const float4 *>(x + k0 + static_cast<int64_t>(row) * n);
+        const float4 a = p[0], b = p[1];
+        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+        v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+      } else {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          const int64_t at = kTranspose ? row + static_cast<int64_t>(k0 + q) * n
+                                        : k0 + q + static_cast<int64_t>(row) * n;
+          v[q] = row < n && k0 + q < n ? x[at] : 0.0f;
+        }
+      }
+      // to |y| < 64: the first digit is the nearest integer
+      const int e = (row < n ? exponentOf(largest[row]) : 0) - (kDigit - 1);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) v[q] = scaleBy(v[q], -e);
+      uint8_t *out = tile + swizzle64(r, c);
+#pragma unroll
+      for (int p = 0; p < kSlices; ++p) {
+        uint32_t word[4];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          const float d = rintf(v[q]);
+          v[q] = (v[q] - d) * static_cast<float>(1 << kDigit);  // exact
+          // an integer times its weight 2^-7p: BF16 holds it exactly
+          const uint32_t h = __float_as_uint(d * (1.0f / (1 << (kDigit * p)))) >> 16;
+          if (q % 2 == 0) word[q / 2] = h;
+          else word[q / 2] |= h << 16;
+        }
+        *reinterpret_cast<uint4 *>(out + p * kSliceBytes) = make_uint4(word[0], word[1], word[2], word[3]);
+      }
+    }
+  }
+}
+
+struct SlicedArgs {
+  const int4 *work;        // (matrix, tile_i, tile_j, k tiles)
+  int items;
+  const uint8_t *a, *b;    // digits of the operands
+  const uint32_t *largest_a, *largest_b;
+  const int64_t *tile_base;
+  const int32_t *n;
+  const int64_t *offset;
+  const int64_t *eig_offset;
+  const float *eigenvalues;  // kSlicedInverseH
+  float *c;                  // C_ij at i + j n
+  uint32_t *largest_c;       // may be null: largest magnitudes of C's columns (zero before)
+  int *status;
+  int wait_test;             // 1: the producer first waits on a barrier nothing arrives at
+};
+
+enum SlicedEpilogue : int {
+  kSlicedStore = 0,
+  kSlicedInverseH = 1,  // C_ij / (s_i + s_j), s = sqrt(lambda)
+  kSlicedMirror = 2,    // C = A A^T: tiles on or above the diagonal, stored twice
+};
+
+template <int kEpi>
+__global__ void __launch_bounds__(kSlicedThreads, 1) slicedGemmKernel(SlicedArgs args) {
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  unsigned char *base = reinterpret_cast<unsigned char *>(
+      (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  uint64_t *full = reinterpret_cast<uint64_t *>(base + kStages * kStageBytes), *empty = full + kStages;
+  uint64_t *acc_full = empty + kStages, *acc_empty = acc_full + 1;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_empty + 1);
+  volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+  constexpr uint32_t kDesc = instrDescBf16(kTile, kTile);
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kStages; ++s) {
+      mbarInit(smemAddr(&full[s]), 1);
+      mbarInit(smemAddr(&empty[s]), 1);
+    }
+    mbarInit(smemAddr(acc_full), 1);
+    mbarInit(smemAddr(acc_empty), 32 * kEpilogueWarps);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == kEpilogueWarps + 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     smemAddr(tmem_slot)),
+                 "r"(512));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;");
+  const uint32_t tmem = *tmem_slot;
+
+  if (warp == kEpilogueWarps) {
+    if (lane == 0) {
+      int stage = 0;
+      uint32_t phase = 0;
+      if (args.wait_test) {
+        // failure injection: completes only after an MMA commit, which needs
+        // a copy this thread has not issued
+        barWait(smemAddr(&empty[0]), 0, args.status, abort_flag, 4096);
+      }
+      for (int item = blockIdx.x; item < args.items && !*abort_flag; item += gridDim.x) {
+        const int4 w = args.work[item];
+        const uint8_t *ta = args.a + (args.tile_base[w.x] + static_cast<int64_t>(w.y) * w.w) * kTileBytes;
+        const uint8_t *tb = args.b + (args.tile_base[w.x] + static_cast<int64_t>(w.z) * w.w) * kTileBytes;
+        for (int kt = 0; kt < w.w; ++kt) {
+          if (!barWait(smemAddr(&empty[stage]), phase ^ 1, args.status, abort_flag)) break;
+          const uint32_t bar = smemAddr(&full[stage]);
+          const uint32_t dst = smemAddr(base + stage * kStageBytes);
+          mbarArriveExpectTx(bar, kStageBytes);
+          bulkLoad(dst, ta + static_cast<size_t>(kt) * kTileBytes, kTileBytes, bar);
+          bulkLoad(dst + kTileBytes, tb + static_cast<size_t>(kt) * kTileBytes, kTileBytes, bar);
+          if (++stage == kStages) {
+            stage = 0;
+            phase ^= 1;
+          }
+        }
+      }
+    }
+  } else if (warp == kEpilogueWarps + 1) {
+    if (lane == 0) {
+      int stage = 0;
+      uint32_t phase = 0, acc_phase = 0;
+      for (int item = blockIdx.x; item < args.items && !*abort_flag; item += gridDim.x) {
+        const int k_tiles = args.work[item].w;
+        for (int kt = 0; kt < k_tiles; ++kt) {
+          const bool first = kt % kChunkTiles == 0;
+          if (first) {
+            if (!barWait(smemAddr(acc_empty), acc_phase ^ 1, args.status, abort_flag)) break;
+            acc_phase ^= 1;
+          }
+          if (!barWait(smemAddr(&full[stage]), phase, args.status, abort_flag)) break;
+          asm volatile("tcgen05.fence::after_thread_sync;");
+          const uint32_t mem = smemAddr(base + stage * kStageBytes);
+          const uint64_t ad = smemDesc64(mem), bd = smemDesc64(mem + kTileBytes);
+#pragma unroll
+          for (int kk = 0; kk < kTileK / 16; ++kk) {
+#pragma unroll
+            for (int x = 0; x < kPairs; ++x) {
+              const int p = kPairOrder[x] >> 4, q = kPairOrder[x] & 15;
+              mmaBf16(tmem + kTile * pairGroup(p, q), ad + p * (kSliceBytes >> 4) + 2 * kk,
+                      bd + q * (kSliceBytes >> 4) + 2 * kk, kDesc, !(first && p == 0 && kk == 0));
+            }
+          }
+          mmaCommit(smemAddr(&empty[stage]));
+          if (++stage == kStages) {
+            stage = 0;
+            phase ^= 1;
+          }
+          if (kt % kChunkTiles == kChunkTiles - 1 || kt == k_tiles - 1) mmaCommit(smemAddr(acc_full));
+        }
+      }
+    }
+  } else {
+    // Epilogue: warps w, w + 4, .. own accumulator rows 32 (w mod 4) ..; each
+    // thread one row and kCols of the columns.
+    const int quarter = warp % 4, part = warp / 4;
+    uint32_t acc_phase = 0;
+    for (int item = blockIdx.x; item < args.items; item += gridDim.x) {
+      const int4 w = args.work[item];
+      const int mi = w.x, n = args.n[mi];
+      const int i = w.y * kTile + 32 * quarter + lane, j0 = w.z * kTile + kCols * part;
+      const int64_t eig = args.eig_offset[mi];
+      // 2^(e_i + e_j) times the digits' scale; lane q has column j0 + q
+      const int jl = j0 + lane;
+      const int ei = (i < n ? exponentOf(args.largest_a[eig + i]) : 0) - 2 * (kDigit - 1);
+      const int ej = jl < n ? exponentOf(args.largest_b[eig + jl]) : 0;
+      float si = 0.0f, sj = 0.0f;
+      if (kEpi == kSlicedInverseH) {
+        si = i < n ? rootOf(args.eigenvalues[eig + i]) : 0.0f;
+        sj = jl < n ? rootOf(args.eigenvalues[eig + jl]) : 0.0f;
+      }
+      float h[kCols];
+      bool ok = true;
+      const int chunks = (w.w + kChunkTiles - 1) / kChunkTiles;
+      for (int chunk = 0; chunk < chunks; ++chunk) {
+        ok = barWait(smemAddr(acc_full), acc_phase, args.status, abort_flag);
+        if (!ok) break;
+        acc_phase ^= 1;
+        asm volatile("tcgen05.fence::after_thread_sync;");
+        const uint32_t taddr = tmem + ((32u * quarter) << 16) + kCols * part;
+#pragma unroll
+        for (int s = 0; s < kCols; s += kHalf) {
+          // from the smallest weight, in float-float, rounded once per chunk
+          float ch[kHalf], cl[kHalf];
+          tmemLoad16(taddr + kTile * (kSlices - 1) + s, ch);
+#pragma unroll
+          for (int c = 0; c < kHalf; ++c) cl[c] = 0.0f;
+#pragma unroll
+          for (int g = kSlices - 2; g >= 0; --g) {
+            float v[kHalf];
+            tmemLoad16(taddr + kTile * g + s, v);
+#pragma unroll
+            for (int c = 0; c < kHalf; ++c) {
+              const float t = v[c] + ch[c], z = t - v[c];
+              cl[c] += (v[c] - (t - z)) + (ch[c] - z);
+              ch[c] = t;
+            }
+          }
+#pragma unroll
+          for (int c = 0; c < kHalf; ++c) {
+            const float x = ch[c] + cl[c];
+            h[s + c] = chunk == 0 ? x : h[s + c] + x;
+          }
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;");
+        mbarArrive(smemAddr(acc_empty));
+      }
+      if (!ok) break;
+      float *C = args.c + args.offset[mi];
+      uint32_t largest = 0;  // of column j0 + lane
+#pragma unroll
+      for (int q = 0; q < kCols; ++q) {
+        const int j = j0 + q;
+        float x = scaleBy(h[q], ei + __shfl_sync(0xffffffffu, ej, q));
+        if (kEpi == kSlicedInverseH) {
+          const float d = si + __shfl_sync(0xffffffffu, sj, q);
+          x = d > 0.0f ? x / d : 0.0f;  // both roots 0: no correction
+        }
+        if (i < n && j < n) C[i + static_cast<int64_t>(j) * n] = x;
+        if (kEpi != kSlicedMirror) {
+          const uint32_t m = __reduce_max_sync(0xffffffffu, i < n ? finiteBits(x) : 0u);
+          if (lane == q) largest = m;
+        }
+        h[q] = x;
+      }
+      if (kEpi != kSlicedMirror) {
+        if (args.largest_c != nullptr && jl < n) atomicMax(args.largest_c + eig + jl, largest);
+      } else if (w.y != w.z) {
+        transpose32(h, lane);
+        const int i0 = i - lane;
+        if (jl < n) {
+#pragma unroll
+          for (int q = 0; q < 32; ++q)
+            if (i0 + q < n) C[jl + static_cast<int64_t>(i0 + q) * n] = h[q];
+        }
+      }
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;");
+  if (warp == kEpilogueWarps + 1) {
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
+  }
+}
+
+// The work lists of the batch's sliced matrices, kept on it: row blocks of 128; operand tiles; tiles
+// of the product, all and on or above the diagonal, largest matrices first;
+// each matrix's first operand tile (64-bit, two per int4).
+struct SlicedPlan {
+  const int4 *rows, *pack, *gemm, *upper, *bases;
+  int row_items, pack_items, gemm_items, upper_items, base_items;
+};
+
+int slicedPlan(msq_ctx *ctx, const DeviceBatch *b, SlicedPlan *p) {
+  constexpr int kKey = 1 << 21;
+  if (findWork(b, kKey, &p->rows, &p->row_items) && findWork(b, kKey + 1, &p->pack, &p->pack_items) &&
+      findWork(b, kKey + 2, &p->gemm, &p->gemm_items) &&
+      findWork(b, kKey + 3, &p->upper, &p->upper_items) &&
+      findWork(b, kKey + 4, &p->bases, &p->base_items))
+    return MSQ_OK;
+  std::vector<int4> rows, pack, gemm, upper, bases((b->count + 1) / 2);
+  std::vector<int64_t> first(2 * bases.size(), 0);
+  std::vector<int> ids;
+  int64_t tiles = 0;
+  for (int mi = 0; mi < b->count; ++mi) {
+    const int n = b->host_n[mi], mt = (n + kTile - 1) / kTile, kt = (n + kTileK - 1) / kTileK;
+    if (!slicedMatrix(n)) continue;
+    ids.push_back(mi);
+    first[mi] = tiles;
+    tiles += static_cast<int64_t>(mt) * kt;
+    for (int t = 0; t < mt; ++t) {
+      rows.push_back(make_int4(mi, t, 0, 0));
+      for (int k = 0; k < kt; ++k) pack.push_back(make_int4(mi, t, k, kt));
+    }
+  }
+  std::stable_sort(ids.begin(), ids.end(),
+                   [&](int x, int y) { return b->host_n[x] > b->host_n[y]; });
+  for (int mi : ids) {
+    const int n = b->host_n[mi], mt = (n + kTile - 1) / kTile, kt = (n + kTileK - 1) / kTileK;
+    for (int t = 0; t < mt; ++t)
+      for (int u = 0; u < mt; ++u) {
+        gemm.push_back(make_int4(mi, t, u, kt));
+        if (u >= t) upper.push_back(gemm.back());
+      }
+  }
+  std::memcpy(bases.data(), first.data(), bases.size() * sizeof(int4));
+  MSQ_TRY(keepWork(ctx, b, kKey, rows, &p->rows, &p->row_items));
+  MSQ_TRY(keepWork(ctx, b, kKey + 1, pack, &p->pack, &p->pack_items));
+  MSQ_TRY(keepWork(ctx, b, kKey + 2, gemm, &p->gemm, &p->gemm_items));
+  MSQ_TRY(keepWork(ctx, b, kKey + 3, upper, &p->upper, &p->upper_items));
+  return keepWork(ctx, b, kKey + 4, bases, &p->bases, &p->base_items);
+}
+
+// One sliced operand in the scratch.
+struct Operand {
+  uint32_t *largest;
+  uint8_t *slices;
+};
+
+// `count` operands of the batch in the scratch, their largest magnitudes in one block.
+int slicedOperands(msq_ctx *ctx, const DeviceBatch *b, const SlicedPlan &p, int count, Operand *out) {
+  const size_t largest = (count * b->total_order * sizeof(uint32_t) + 1023) & ~size_t(1023);
+  const size_t slices = static_cast<size_t>(p.pack_items) * kTileBytes;
+  uint8_t *mem = static_cast<uint8_t *>(scratch(ctx, largest + 1024 + count * slices, kScratchGemm));
+  if (mem == nullptr) return MSQ_ERR_CUDA;
+  uint8_t *tiles = reinterpret_cast<uint8_t *>(
+      (reinterpret_cast<uintptr_t>(mem) + largest + 1023) & ~static_cast<uintptr_t>(1023));
+  for (int q = 0; q < count; ++q)
+    out[q] = {reinterpret_cast<uint32_t *>(mem) + q * b->total_order, tiles + q * slices};
+  return MSQ_OK;
+}
+
+// The digits of X (kTranspose: of X^T) as an operand; `find`: its largest
+// magnitudes too (else a product has left them).
+template <bool kTranspose>
+int sliceOperand(msq_ctx *ctx, const DeviceBatch *b, const SlicedPlan &p, const float *x,
+                 const Operand &out, bool find) {
+  SliceArgs s{};
+  s.rows = p.rows;
+  s.row_items = p.row_items;
+  s.work = p.pack;
+  s.items = p.pack_items;
+  s.x = x;
+  s.offset = b->offset;
+  s.eig_offset = b->eig_offset;
+  s.tile_base = reinterpret_cast<const int64_t *>(p.bases);
+  s.n = b->n;
+  s.largest = out.largest;
+  s.slices = out.slices;
+  if (find) {
+    const dim3 grid(std::min(p.row_items, kSmCount * 8), kTile / 8);
+    largestKernel<kTranspose><<<grid, 256, 0, ctx->stream>>>(s);
+    MSQ_TRY(launched(ctx, "sliced largest"));
+  }
+  digitKernel<kTranspose><<<std::min(p.pack_items, kSmCount * 8), 256, 0, ctx->stream>>>(s);
+  return launched(ctx, "sliced digits");
+}
+
+template <int kEpi>
+int slicedGemm(msq_ctx *ctx, const DeviceBatch *b, const SlicedPlan &p, const Operand &a,
+               const Operand &bm, const float *eigenvalues, float *c, uint32_t *largest_c) {
+  static std::atomic<uint64_t> done_mask{0};
+  const uint64_t bit = ctx->device >= 0 && ctx->device < 64 ? uint64_t{1} << ctx->device : 0;
+  if (bit == 0 || !(done_mask.load() & bit)) {
+    MSQ_TRY(cudaCheck(ctx, cudaFuncSetAttribute(slicedGemmKernel<kEpi>,
+                                                cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                static_cast<int>(kSlicedSmem)), "sliced attr"));
+    done_mask.fetch_or(bit);
+  }
+  SlicedArgs args{};
+  args.work = kEpi == kSlicedMirror ? p.upper : p.gemm;
+  args.items = kEpi == kSlicedMirror ? p.upper_items : p.gemm_items;
+  args.a = a.slices;
+  args.b = bm.slices;
+  args.largest_a = a.largest;
+  args.largest_b = bm.largest;
+  args.tile_base = reinterpret_cast<const int64_t *>(p.bases);
+  args.n = b->n;
+  args.offset = b->offset;
+  args.eig_offset = b->eig_offset;
+  args.eigenvalues = eigenvalues;
+  args.c = c;
+  args.largest_c = largest_c;
+  args.status = ctx->d_status;
+  args.wait_test = waitTestMode() == kWaitTestMbarrier;
+  slicedGemmKernel<kEpi><<<std::min(args.items, kSmCount), kSlicedThreads, kSlicedSmem, ctx->stream>>>(args);
+  return launched(ctx, "sliced gemm");
+}
+
+// Orders from which a matrix's products may be sliced, and the sum of n^3 of
+// such matrices from which they are.  A tile of 128 is mostly padding below
+// order 256 (a correction of 1000 matrices of order 128: 708 us against 550
+// with FMA chains; 100 of order 200: 333 against 328), and slicing adds ten
+// launches, which little work does not pay for (eight of order 384: 179
+// against 148; 32 of order 256: 180 against 168; but two of order 700, 0.69e9:
+// 225 against 235; 16 of order 384: 204 against 227; 64 of order 256: 273
+// against 286; four of order 1000: 471 against 821; 2048: 752 against 1584).
+constexpr int kSlicedOrder = 256;
+constexpr double kSlicedWork = 0.65e9;
+// The digits of four operands stay below this.
+constexpr int64_t kSlicedBytes = int64_t{16} << 30;
+
+}  // namespace
+
+bool slicedProducts(const DeviceBatch *b) {
+  double work = 0.0;
+  int64_t tiles = 0;
+  for (const int32_t n : b->host_n) {
+    if (n < kSlicedOrder) continue;
+    work += static_cast<double>(n) * n * n;
+    tiles += static_cast<int64_t>((n + kTile - 1) / kTile) * ((n + kTileK - 1) / kTileK);
+  }
+  return work >= kSlicedWork && 4 * tiles * kTileBytes <= kSlicedBytes;
+}
+
+bool slicedMatrix(int n) { return n >= kSlicedOrder; }
+
+int slicedReconstruct(msq_ctx *ctx, const DeviceBatch *b, const float *f, float *x) {
+  SlicedPlan p{};
+  Operand op[1];
+  MSQ_TRY(slicedPlan(ctx, b, &p));
+  MSQ_TRY(slicedOperands(ctx, b, p, 1, op));
+  MSQ_TRY(sliceOperand<false>(ctx, b, p, f, op[0], true));
+  return slicedGemm<kSlicedMirror>(ctx, b, p, op[0], op[0], nullptr, x, nullptr);
+}
+
+int slicedSylvester(msq_ctx *ctx, const DeviceBatch *b, const float *v, const float *lam,
+                    const float *r, float *ws, float *e, bool basis_packed) {
+  SlicedPlan p{};
+  Operand op[4];
+  MSQ_TRY(slicedPlan(ctx, b, &p));
+  MSQ_TRY(slicedOperands(ctx, b, p, 4, op));
+  const Operand vt = op[0], vn = op[1], even = op[2], odd = op[3];
+  const size_t order_bytes = b->total_order * sizeof(uint32_t);
+  auto clear = [&](uint32_t *largest, size_t arrays) {
+    return cudaCheck(ctx, cudaMemsetAsync(largest, 0, arrays * order_bytes, ctx->stream), "sliced reset");
+  };
+  if (!basis_packed) {
+    MSQ_TRY(clear(vt.largest, 4));
+    MSQ_TRY(sliceOperand<false>(ctx, b, p, v, vn, true));  // rows = columns of V
+    MSQ_TRY(sliceOperand<true>(ctx, b, p, v, vt, true));   // rows = rows of V
+  } else {
+    MSQ_TRY(clear(even.largest, 2));
+  }
+  MSQ_TRY(sliceOperand<false>(ctx, b, p, r, even, true));
+  // G = R^T V into ws, C = (V^T G) o H into e, (V C)^T into ws, E into e
+  MSQ_TRY(slicedGemm<kSlicedStore>(ctx, b, p, even, vn, nullptr, ws, odd.largest));
+  MSQ_TRY(sliceOperand<false>(ctx, b, p, ws, odd, false));
+  MSQ_TRY(clear(even.largest, 1));
+  MSQ_TRY(slicedGemm<kSlicedInverseH>(ctx, b, p, vn, odd, lam, e, even.largest));
+  MSQ_TRY(sliceOperand<false>(ctx, b, p, e, even, false));
+  MSQ_TRY(clear(odd.largest, 1));
+  MSQ_TRY(slicedGemm<kSlicedStore>(ctx, b, p, even, vt, nullptr, ws, odd.largest));
+  MSQ_TRY(sliceOperand<false>(ctx, b, p, ws, odd, false));
+  return slicedGemm<kSlicedStore>(ctx, b, p, odd, vt, nullptr, e, nullptr);
+}
+
+}  // namespace msq

@@ -38,7 +38,7 @@
 #include "msq_dense.cuh"
 #include "msq_internal.cuh"
 #include "msq_residual.cuh"
-#include "msq_tcgen05.cuh"
+#include "msq_slices.cuh"
 
 #include <algorithm>
 #include <atomic>
@@ -49,7 +49,6 @@ namespace msq {
 namespace {
 
 constexpr int kSlices = 8;
-constexpr int kDigit = 7;                 // bits per digit after the first
 constexpr int kTileM = 128, kTileN = 64, kTileK = 32;
 // One slice of an operand tile: 64-byte rows (SWIZZLE_64B), A 128 rows, B 64;
 // the kSlices slices of a tile of 128 columns of X are contiguous.
@@ -62,22 +61,8 @@ constexpr int kEpilogueWarps = 16;
 constexpr int kCols = kTileN / (kEpilogueWarps / 4);  // columns per epilogue thread
 constexpr int kResidualThreads = 32 * (kEpilogueWarps + 2);
 constexpr size_t kResidualSmem = kStages * kStageBytes + 1024 + 256;
-constexpr long long kResidualWaitLimit = 1ll << 26;
 constexpr uint32_t kDescResidual = instrDescBf16(kTileM, kTileN);
 static_assert(kSlices * kTileN == 512, "one accumulator per weight fills TMEM");
-
-// Byte offset of 16-byte chunk `chunk` of row `row` in a SWIZZLE_64B K-major
-// operand: 64-byte rows, 8-row atoms, chunk index XOR bits 1..2 of the row.
-__host__ __device__ __forceinline__ uint32_t swizzle64(int row, int chunk) {
-  return (row >> 3) * 512 + (row & 7) * 64 + ((chunk ^ ((row >> 1) & 3)) << 4);
-}
-__device__ __forceinline__ uint64_t smemDesc64(uint32_t addr) {
-  return static_cast<uint64_t>((addr >> 4) & 0x3FFFu) |
-         (static_cast<uint64_t>(1) << 16) |           // LBO (unused)
-         (static_cast<uint64_t>(512 >> 4) << 32) |    // SBO: 8-row atom stride
-         (static_cast<uint64_t>(1) << 46) |           // descriptor version
-         (static_cast<uint64_t>(4) << 61);            // SWIZZLE_64B
-}
 
 // The pairs (p, q), p + q < kSlices, as 16 p + q, (0, g) first of its weight.
 constexpr int kPairs = kSlices * (kSlices + 1) / 2;
@@ -85,17 +70,6 @@ __device__ constexpr uint8_t kPairOrder[kPairs] = {
     0x07, 0x06, 0x05, 0x04, 0x16, 0x15, 0x14, 0x03, 0x25, 0x24, 0x13, 0x23,
     0x34, 0x33, 0x12, 0x22, 0x43, 0x32, 0x02, 0x42, 0x52, 0x21, 0x41, 0x51,
     0x11, 0x31, 0x61, 0x01, 0x00, 0x60, 0x50, 0x70, 0x10, 0x40, 0x30, 0x20};
-
-// 2^k, k clamped to normal exponents
-__device__ __forceinline__ float powerOfTwo(int k) {
-  k = k < -126 ? -126 : (k > 127 ? 127 : k);
-  return __uint_as_float(static_cast<uint32_t>(k + 127) << 23);
-}
-// x 2^k in two exact steps (down to the underflow threshold)
-__device__ __forceinline__ float scaleBy(float x, int k) {
-  const int a = k / 2;
-  return (x * powerOfTwo(a)) * powerOfTwo(k - a);
-}
 
 struct SliceArgs {
   const int4 *rows;       // (matrix, tile_m, -, -)
@@ -133,11 +107,7 @@ __global__ void __launch_bounds__(256) columnExponentKernel(SliceArgs args) {
 #pragma unroll
       for (int s = 16; s > 0; s >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, s));
       if (lane == 0) {
-        const uint32_t bits = __float_as_uint(m);
-        const int field = static_cast<int>(bits >> 23);
-        // m < 2^e; a subnormal by its leading bit
-        const int e = bits == 0 ? 0 : (field != 0 ? field - 126 : (32 - __clz(static_cast<int>(bits))) - 149);
-        args.exponent[args.eig_offset[w.x] + c] = e;
+        args.exponent[args.eig_offset[w.x] + c] = exponentOf(__float_as_uint(m));
       }
     }
   }
@@ -228,33 +198,6 @@ struct ResidualMmaArgs {
   int *status;
   int wait_test;           // 1: the producer first waits on a barrier nothing arrives at
 };
-
-// Bounded wait: false (and the status word set) if the phase never completes.
-__device__ __forceinline__ bool barWait(uint32_t bar, uint32_t parity, int *status,
-                                        volatile int *abort_flag, long long limit = kResidualWaitLimit) {
-  for (long long i = 0; i < limit; ++i) {
-    if (mbarTryWait(bar, parity)) return true;
-    if (*abort_flag) return false;
-  }
-  atomicExch(status, kStatusMbarrierTimeout);
-  *abort_flag = 1;
-  return false;
-}
-
-// 16 consecutive TMEM columns of this warp's 32 lanes (lane = row).
-__device__ __forceinline__ void tmemLoad16(uint32_t taddr, float (&v)[16]) {
-  uint32_t r[16];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, "
-      "%12, %13, %14, %15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-        "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
-}
 
 // Accumulates the sum of squares of normalised float-float values (t, e).
 __device__ __forceinline__ void addSquare(float &s, float &c, float t, float e) {

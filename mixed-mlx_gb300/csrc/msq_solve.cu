@@ -11,6 +11,7 @@
 // Corrections always use the FP32 stable basis, as the reference does
 // (:304-310).
 #include "msq_dense.cuh"
+#include "msq_gemm_sliced.cuh"
 #include "msq_internal.cuh"
 #include "msq_stages.cuh"
 
@@ -25,15 +26,26 @@ namespace {
 
 size_t alignUp(size_t bytes) { return (bytes + 255) & ~static_cast<size_t>(255); }
 
-// One Sylvester sweep on a batch, FP32 GEMMs on the CUDA cores:
+// One Sylvester sweep on a batch in FP32 (sliced products of the larger
+// matrices where they pay, FMA chains on the CUDA cores of the others):
 //   G = R V, C = (V^T G) o H, Z = V C, E = Z V^T, X <- X + (E + E^T)/2.
 int sylvesterFp32(msq_ctx *ctx, const DeviceBatch *b, const float *v, const float *lam,
-                  const float *r, float *x_hi, float *x_lo, float *ws0, float *ws1) {
-  MSQ_TRY(gemmTN(ctx, b, r, v, ws0, kEpilogueStore, nullptr));           // G = R V
-  MSQ_TRY(gemmTN(ctx, b, v, ws0, ws1, kEpilogueInverseH, lam));          // C = V^T G o H
-  MSQ_TRY(gemmTN(ctx, b, v, ws1, ws0, kEpilogueStore, nullptr, true));   // Z = V C
-  MSQ_TRY(gemmTN(ctx, b, ws0, v, ws1, kEpilogueStore, nullptr, true, true));  // E = Z V^T
+                  const float *r, float *x_hi, float *x_lo, float *ws0, float *ws1,
+                  bool basis_packed) {
+  const bool sliced = slicedProducts(b);
+  if (sliced) MSQ_TRY(slicedSylvester(ctx, b, v, lam, r, ws0, ws1, basis_packed));
+  MSQ_TRY(gemmTN(ctx, b, r, v, ws0, kEpilogueStore, nullptr, false, false, sliced));    // G = R V
+  MSQ_TRY(gemmTN(ctx, b, v, ws0, ws1, kEpilogueInverseH, lam, false, false, sliced));  // C = V^T G o H
+  MSQ_TRY(gemmTN(ctx, b, v, ws1, ws0, kEpilogueStore, nullptr, true, false, sliced));   // Z = V C
+  MSQ_TRY(gemmTN(ctx, b, ws0, v, ws1, kEpilogueStore, nullptr, true, true, sliced));    // E = Z V^T
   return symmetricAdd(ctx, b, x_hi, x_lo, ws1);
+}
+
+// X = F^T F in FP32.
+int reconstructFp32(msq_ctx *ctx, const DeviceBatch *b, const float *f, float *x) {
+  const bool sliced = slicedProducts(b);
+  if (sliced) MSQ_TRY(slicedReconstruct(ctx, b, f, x));
+  return gemmTN(ctx, b, f, f, x, kEpilogueStore, nullptr, false, false, sliced);
 }
 
 }  // namespace
@@ -45,7 +57,7 @@ int sylvesterSweep(msq_ctx *ctx, const DeviceBatch *b, int gemm_format, const fl
     MSQ_TRY(sylvesterTc(ctx, b, v, lam, r, ws1, basis_packed));
     return symmetricAdd(ctx, b, x_hi, x_lo, ws1);
   }
-  return sylvesterFp32(ctx, b, v, lam, r, x_hi, x_lo, ws0, ws1);
+  return sylvesterFp32(ctx, b, v, lam, r, x_hi, x_lo, ws0, ws1, basis_packed);
 }
 
 // X0 = F^T F from the FP32 factor F (K-major W^T) in the plan's format.
@@ -53,7 +65,7 @@ int reconstructFromFactor(msq_ctx *ctx, const DeviceBatch *b, int plan_format, c
                           float *x) {
   switch (plan_format) {
     case MSQ_PLAN_FP32:
-      return gemmTN(ctx, b, f, f, x, kEpilogueStore, nullptr);
+      return reconstructFp32(ctx, b, f, x);
     case MSQ_PLAN_BF16:
       return reconstructLowBit(ctx, b, MSQ_FMT_BF16, f, x);
     case MSQ_PLAN_FP8:
@@ -90,7 +102,7 @@ extern "C" int msq_reconstruct(msq_ctx *ctx, int format, const void *values, con
   if (b == nullptr) return MSQ_ERR_INVALID_ARGUMENT;
   if (format == MSQ_FMT_FP32) {
     const float *f = static_cast<const float *>(values);
-    return gemmTN(ctx, b, f, f, root, kEpilogueStore, nullptr);
+    return reconstructFp32(ctx, b, f, root);
   }
   return reconstructEncoded(ctx, b, format, values, scales, root);
 }

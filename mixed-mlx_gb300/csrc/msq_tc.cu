@@ -104,21 +104,6 @@ constexpr bool isMirrored(int epilogue) {
   return epilogue == kEpiRowScale || epilogue == kEpiMirror;
 }
 
-// v[q] of lane l <-> v[l] of lane q.
-__device__ __forceinline__ void transpose32(float *v, int lane) {
-#pragma unroll
-  for (int s = 16; s; s >>= 1) {
-    const bool high = lane & s;
-#pragma unroll
-    for (int q = 0; q < 32; ++q) {
-      if (q & s) continue;
-      const float got = __shfl_xor_sync(0xffffffffu, high ? v[q] : v[q + s], s);
-      if (high) v[q] = got;
-      else v[q + s] = got;
-    }
-  }
-}
-
 // Bounded wait: false (and the status word set) if the phase never completes.
 __device__ __forceinline__ bool mbarWait(uint32_t bar, uint32_t parity, int *status,
                                          volatile int *abort_flag, long long limit = kWaitLimit) {

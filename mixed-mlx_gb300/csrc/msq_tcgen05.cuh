@@ -175,5 +175,20 @@ __device__ __forceinline__ void tmemStore32(uint32_t taddr, const float *v) {
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
+// v[q] of lane l <-> v[l] of lane q.
+__device__ __forceinline__ void transpose32(float *v, int lane) {
+#pragma unroll
+  for (int s = 16; s; s >>= 1) {
+    const bool high = lane & s;
+#pragma unroll
+    for (int q = 0; q < 32; ++q) {
+      if (q & s) continue;
+      const float got = __shfl_xor_sync(0xffffffffu, high ? v[q] : v[q + s], s);
+      if (high) v[q] = got;
+      else v[q + s] = got;
+    }
+  }
+}
+
 }  // namespace
 }  // namespace msq

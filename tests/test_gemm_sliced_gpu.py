@@ -1,0 +1,78 @@
+"""FP32 reconstruction and correction as sliced products on the tensor cores:
+orders around tiles of 128, K steps of 32 and the 1024 of one exact sum, beside
+small matrices that keep the FMA chains, against FP64.
+
+Tolerances.  An element is exact sums, cut off below 2^-27 of the two vectors'
+largest entries and rounded once: relative Frobenius 2 2^-24 for a product of
+matrices of random entries, four of them (and what each rounding does to the
+next) 8 2^-24; the chains' 8 sqrt(n) 2^-24 for the small ones.  For graded
+matrices element (i, j) is off by at most 2 sqrt(n) 2^-27 + 2^-24 of the two
+vectors' norms, doubled for the bound on the largest entry."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+SLICED = 256  # smallest order that may be sliced
+
+
+def _dev(x):
+    import torch
+    return torch.from_numpy(np.ascontiguousarray(x, np.float32)).cuda()
+
+
+@pytest.mark.parametrize("orders", [[870], [256] * 40, [384, 33, 385, 700, 1, 701, 255, 257], [1025], [2049]])
+def test_products_against_fp64(ctx, msq, orders):
+    import torch
+    b = msq.Batch.from_orders(orders)
+    rng = np.random.default_rng(orders[0])
+    mats = [(rng.standard_normal((n, n)) / np.sqrt(n)).astype(np.float32) for n in orders]
+    res = [(rng.standard_normal((n, n)) * 1e-3).astype(np.float32) for n in orders]
+    lam = rng.uniform(0.1, 1.0, int(b.n.sum())).astype(np.float32)
+    f = _dev(b.pack(mats))
+    x = ctx.reconstruct_factor(msq.PLAN_FP32, f, b)
+    hi, lo = torch.zeros_like(f), torch.zeros_like(f)
+    ctx.sylvester_sweep(msq.FP32, f, _dev(lam), _dev(b.pack(res)), b, hi, lo)
+    torch.cuda.synchronize()
+    at = 0
+    for n, v, r, xg, eg in zip(orders, mats, res, b.unpack(x.cpu().numpy()), b.unpack(hi.cpu().numpy())):
+        v, r, s = v.astype(np.float64), r.astype(np.float64), np.sqrt(lam[at:at + n].astype(np.float64))
+        at += n
+        scale = 4 * np.sqrt(n) if n < SLICED else 1.0
+        ref = v.T @ v
+        assert np.linalg.norm(xg - ref) <= 2 * scale * 2.0**-24 * np.linalg.norm(ref), n
+        assert np.array_equal(xg, xg.T)
+        c = (v.T @ r.T @ v) / (s[:, None] + s[None, :])
+        e = v @ c @ v.T
+        e = 0.5 * (e + e.T)
+        assert np.linalg.norm(eg - e) <= 8 * scale * 2.0**-24 * np.linalg.norm(e), n
+
+
+def test_graded_and_extreme_columns(ctx, msq):
+    import torch
+    n = 900
+    b = msq.Batch.from_orders([n])
+    rng = np.random.default_rng(1)
+    f = np.diag(10.0 ** (-3 * np.arange(n) / n)) + 1e-3 * rng.standard_normal((n, n))
+    f = f * 2.0 ** rng.integers(-40, 41, n)[None, :]  # columns of very different sizes
+    f[:, 7] = 0.0
+    f = f.astype(np.float32)
+    x = ctx.reconstruct_factor(msq.PLAN_FP32, _dev(b.pack([f])), b)
+    torch.cuda.synchronize()
+    got = b.unpack(x.cpu().numpy())[0]
+    f64 = f.astype(np.float64)
+    norm = np.linalg.norm(f64, axis=0)
+    bound = 2 * (2 * np.sqrt(n) * 2.0**-27 + 2.0**-24) * np.outer(norm, norm)
+    assert (np.abs(got - f64.T @ f64) <= bound).all()
+
+
+def test_a_nan_stays_in_its_row_and_column(ctx, msq):
+    import torch
+    n, i = 900, 321
+    b = msq.Batch.from_orders([n])
+    f = (np.random.default_rng(2).standard_normal((n, n)) / 30).astype(np.float32)
+    clean = b.unpack(ctx.reconstruct_factor(msq.PLAN_FP32, _dev(b.pack([f])), b).cpu().numpy())[0]
+    f[5, i] = np.nan
+    got = b.unpack(ctx.reconstruct_factor(msq.PLAN_FP32, _dev(b.pack([f])), b).cpu().numpy())[0]
+    assert np.isnan(got[i]).all() and np.isnan(got[:, i]).all()
+    rest = np.delete(np.arange(n), i)
+    assert np.array_equal(got[np.ix_(rest, rest)], clean[np.ix_(rest, rest)])
