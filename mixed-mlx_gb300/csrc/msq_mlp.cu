@@ -44,6 +44,13 @@ struct FloatSum {
     const float q = __fmul_rn(v, v);
     add(q, fmaf(v, v, -q));
   }
+  __device__ __forceinline__ void add(const FloatSum &o) { add(o.s, o.c); }
+  // s the rounded value, c what it leaves
+  __device__ __forceinline__ void normalise() {
+    const float t = s + c;
+    c -= t - s;
+    s = t;
+  }
   // the warp's total in every lane
   __device__ __forceinline__ void warp() {
 #pragma unroll
@@ -57,10 +64,15 @@ struct FloatSum {
 // |a_ji| and a_ji^2 over j != i.  A warp per column, lanes down the column:
 // coalesced, bound by the latency of a few loads per column and, at large
 // orders, by memory.  A thread per column read with a stride of n and summed
-// in FP64; features of 256 matrices of orders 64 .. 512: 417 us, 74 so; of
-// one matrix of order 1024: 1067 and 49; of 4096 of order 64: 275 and 223.
+// in FP64; features of 256 matrices of orders 64 .. 512: 417 us, 53 so; of
+// one matrix of order 1024: 1067 and 35; of 4096 of order 64: 275 and 129.
+//
+// The sums stay float-float (FP64 conversions and comparisons of every column
+// took 30 of 55 us); one whose squares leave FP32's range, or that is not
+// finite, is in `wide` and marked by squares.s < 0.
 struct ColumnStat {
-  double abs_sum, squares;
+  FloatSum abs_sum, squares;
+  double wide_abs_sum, wide_squares;
 };
 constexpr int kStatColumns = 32;  // columns per work item
 
@@ -100,11 +112,10 @@ __global__ void __launch_bounds__(256) columnStatsKernel(const float *__restrict
       }
       sum.warp();
       squares.warp();
-      double rs = sum.value(), r2 = squares.value();
       // Squares that FP32 overflows or loses (a square below 2^-126 beside a
       // sum of 1e-20 is 1e-18 of it), and infinities and NaN: in FP64.
-      if (!(r2 >= 1e-20 && r2 <= 1e37) && rs != 0.0) {
-        rs = r2 = 0.0;
+      double rs = 0.0, r2 = 0.0;
+      if (!(squares.s >= 1e-20f && squares.s <= 1e37f) && sum.s != 0.0f) {
         for (int j = lane; j < n; j += 32) {
           const double y = j == i ? 0.0 : static_cast<double>(col[j]);
           rs += fabs(y);
@@ -115,8 +126,10 @@ __global__ void __launch_bounds__(256) columnStatsKernel(const float *__restrict
           rs += __shfl_xor_sync(0xffffffffu, rs, s);
           r2 += __shfl_xor_sync(0xffffffffu, r2, s);
         }
+        squares.s = -1.0f;
       }
-      if (lane == 0) stats[eoff[mi] + i] = {rs, r2};
+      sum.normalise();
+      if (lane == 0) stats[eoff[mi] + i] = {sum, squares, rs, r2};
     }
   }
 }
@@ -130,27 +143,86 @@ __global__ void __launch_bounds__(256) columnStatsKernel(const float *__restrict
 // 12 std diag / mean diag                     13 fraction of rows diagonally dominant
 // 14 log10 tolerance (filled by the caller; 0 here)   15 bias term 1
 // Lane k forms feature k, so the FP64 logarithms (and square roots) of a
-// matrix are one instruction stream.
-__global__ void __launch_bounds__(128) featuresKernel(const float *__restrict__ a,
-                                                      const int32_t *__restrict__ nn,
-                                                      const int64_t *__restrict__ off,
-                                                      const int64_t *__restrict__ eoff,
-                                                      const ColumnStat *__restrict__ stats, int count,
-                                                      float *__restrict__ out) {
-  const int lane = threadIdx.x % 32, mi = blockIdx.x * 4 + threadIdx.x / 32;
-  if (mi >= count) return;
-  const int n = nn[mi];
-  const float *A = a + off[mi];
-  const ColumnStat *col = stats + eoff[mi];
-  double tr = 0, fro = 0, offm = 0, offabs = 0, dmin = 1e300, dmax = -1e300, d2 = 0;
+// matrix are one instruction stream; the sums before it are float-float, FP64
+// where a diagonal or a column leaves FP32's range.
+struct DiagonalSums {
+  double tr, d2, offm, offabs, dmin, dmax, glo, ghi, rowmax;
+  int dominant;
+};
+
+// a < b for normalised float-float values (false with a NaN)
+__device__ __forceinline__ bool lessThan(const FloatSum &a, const FloatSum &b) {
+  return a.s < b.s || (a.s == b.s && a.c < b.c);
+}
+__device__ __forceinline__ FloatSum shuffled(const FloatSum &v, int s) {
+  return {__shfl_xor_sync(0xffffffffu, v.s, s), __shfl_xor_sync(0xffffffffu, v.c, s)};
+}
+
+// False, with nothing written, if the FP64 sums are needed.
+__device__ bool diagonalSumsFloat(const float *A, const ColumnStat *col, int n, int lane,
+                                  DiagonalSums &out) {
+  FloatSum tr, d2, offm, offabs, glo, ghi, rowmax;
+  glo.s = 3.402823466e38f;
+  ghi.s = -3.402823466e38f;
+  float dmin = 3.402823466e38f, dmax = -3.402823466e38f;
+  int dominant = 0;
+  bool plain = true;
+  for (int i = lane; i < n; i += 32) {
+    const float d = A[i + static_cast<int64_t>(i) * n];
+    const FloatSum rs = col[i].abs_sum, sq = col[i].squares;
+    // squares whose sum over any order stays within FP32's range
+    plain = plain && sq.s >= 0.0f && sq.s <= 1e33f &&
+            ((fabsf(d) >= 1e-10f && fabsf(d) <= 3e16f) || d == 0.0f);
+    tr.add(d);
+    d2.square(d);
+    offm.add(sq);
+    offabs.add(rs);
+    dmin = fminf(dmin, d);
+    dmax = fmaxf(dmax, d);
+    FloatSum lo, hi;
+    lo.add(d);
+    lo.add(-rs.s, -rs.c);
+    lo.normalise();
+    hi.add(d);
+    hi.add(rs);
+    hi.normalise();
+    if (lessThan(lo, glo)) glo = lo;
+    if (lessThan(ghi, hi)) ghi = hi;
+    if (lessThan(rowmax, rs)) rowmax = rs;
+    dominant += lo.s > 0.0f;
+  }
+  if (!__all_sync(0xffffffffu, plain)) return false;
+  tr.warp();
+  d2.warp();
+  offm.warp();
+  offabs.warp();
+#pragma unroll
+  for (int s = 16; s; s >>= 1) {
+    dmin = fminf(dmin, __shfl_xor_sync(0xffffffffu, dmin, s));
+    dmax = fmaxf(dmax, __shfl_xor_sync(0xffffffffu, dmax, s));
+    const FloatSum a = shuffled(glo, s), b = shuffled(ghi, s), c = shuffled(rowmax, s);
+    if (lessThan(a, glo)) glo = a;
+    if (lessThan(ghi, b)) ghi = b;
+    if (lessThan(rowmax, c)) rowmax = c;
+    dominant += __shfl_xor_sync(0xffffffffu, dominant, s);
+  }
+  out = {tr.value(), d2.value(), offm.value(), offabs.value(), dmin, dmax,
+         glo.value(), ghi.value(), rowmax.value(), dominant};
+  return true;
+}
+
+__device__ void diagonalSumsDouble(const float *A, const ColumnStat *col, int n, int lane,
+                                   DiagonalSums &out) {
+  double tr = 0, d2 = 0, offm = 0, offabs = 0, dmin = 1e300, dmax = -1e300;
   double glo = 1e300, ghi = -1e300, rowmax = 0;
   int dominant = 0;
   for (int i = lane; i < n; i += 32) {
     const double d = A[i + static_cast<int64_t>(i) * n];
-    const double rs = col[i].abs_sum, ro2 = col[i].squares;
+    const bool wide = col[i].squares.s < 0.0f;
+    const double rs = wide ? col[i].wide_abs_sum : col[i].abs_sum.value();
+    const double ro2 = wide ? col[i].wide_squares : col[i].squares.value();
     tr += d;
     d2 += d * d;
-    fro += d * d + ro2;
     offm += ro2;
     offabs += rs;
     dmin = fmin(dmin, d);
@@ -165,7 +237,6 @@ __global__ void __launch_bounds__(128) featuresKernel(const float *__restrict__ 
     auto other = [&](double v) { return __shfl_xor_sync(0xffffffffu, v, s); };
     tr += other(tr);
     d2 += other(d2);
-    fro += other(fro);
     offm += other(offm);
     offabs += other(offabs);
     dmin = fmin(dmin, other(dmin));
@@ -175,6 +246,24 @@ __global__ void __launch_bounds__(128) featuresKernel(const float *__restrict__ 
     rowmax = fmax(rowmax, other(rowmax));
     dominant += __shfl_xor_sync(0xffffffffu, dominant, s);
   }
+  out = {tr, d2, offm, offabs, dmin, dmax, glo, ghi, rowmax, dominant};
+}
+
+// One warp per CTA: the FP64 logarithms of few matrices spread over the SMs.
+__global__ void __launch_bounds__(32) featuresKernel(const float *__restrict__ a,
+                                                      const int32_t *__restrict__ nn,
+                                                      const int64_t *__restrict__ off,
+                                                      const int64_t *__restrict__ eoff,
+                                                      const ColumnStat *__restrict__ stats,
+                                                      float *__restrict__ out) {
+  const int lane = threadIdx.x, mi = blockIdx.x;
+  const int n = nn[mi];
+  const float *A = a + off[mi];
+  const ColumnStat *col = stats + eoff[mi];
+  DiagonalSums sums;
+  if (!diagonalSumsFloat(A, col, n, lane, sums)) diagonalSumsDouble(A, col, n, lane, sums);
+  const auto [tr, d2, offm, offabs, dmin, dmax, glo, ghi, rowmax, dominant] = sums;
+  const double fro = d2 + offm;
   if (lane >= kIn) return;
   const double tiny = 1e-30, mean = tr / n, mean_t = fmax(mean, tiny), dmin_t = fmax(dmin, tiny);
   // square roots: ||A||_F, the off-diagonal mass (8), the deviation (12)
@@ -392,8 +481,7 @@ extern "C" int msq_features(msq_ctx *ctx, const float *a, const int32_t *n, cons
   columnStatsKernel<<<std::min(items, kSmCount * 8), 256, 0, ctx->stream>>>(
       a, b->n, b->offset, b->eig_offset, work, items, stats);
   MSQ_TRY(launched(ctx, "mlp column sums"));
-  featuresKernel<<<(count + 3) / 4, 128, 0, ctx->stream>>>(a, b->n, b->offset, b->eig_offset, stats,
-                                                         count, features);
+  featuresKernel<<<count, 32, 0, ctx->stream>>>(a, b->n, b->offset, b->eig_offset, stats, features);
   return launched(ctx, "mlp features");
 }
 

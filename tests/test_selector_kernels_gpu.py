@@ -35,7 +35,7 @@ def _features(a):
 
 
 @pytest.mark.parametrize("orders", [[1], [2, 3, 31], [32, 33, 64, 65, 128], [257, 500, 16]])
-@pytest.mark.parametrize("scale", [1.0, 1e-22, 1e22])
+@pytest.mark.parametrize("scale", [1.0, 1e-22, 1e22, 1e16, 1e17])
 def test_features_against_fp64(ctx, msq, orders, scale):
     import torch
     b = msq.Batch.from_orders(orders)
