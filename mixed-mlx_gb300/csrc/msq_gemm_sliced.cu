@@ -32,6 +32,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cstring>
+#include <initializer_list>
 #include <vector>
 
 namespace msq {
@@ -66,13 +67,15 @@ struct SliceArgs {
   const int4 *rows;       // (matrix, tile, -, -)
   const int4 *work;       // (matrix, tile, k tile, k tiles)
   int row_items, items;
-  const float *x;
   const int64_t *offset;
   const int64_t *eig_offset;
   const int64_t *tile_base;
   const int32_t *n;
-  uint32_t *largest;      // bits of the largest finite magnitude per operand row
-  uint8_t *slices;
+  // operand blockIdx.z: the columns of x, or with `transpose` its rows
+  const float *x[3];
+  uint32_t *largest[3];   // bits of the largest finite magnitude per operand row
+  uint8_t *slices[3];
+  bool transpose[3];
 };
 
 // Largest magnitudes of the operand's rows: the columns of X (a warp per
@@ -80,13 +83,13 @@ struct SliceArgs {
 // kTranspose its rows (a thread per row, 1 / 16 of K per CTA of grid.y;
 // `largest` is zero before).
 template <bool kTranspose>
-__global__ void __launch_bounds__(256) largestKernel(SliceArgs args) {
+__device__ __forceinline__ void largestOf(const SliceArgs &args, int op) {
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   for (int item = blockIdx.x; item < args.row_items; item += gridDim.x) {
     const int4 w = args.rows[item];
     const int n = args.n[w.x];
-    const float *x = args.x + args.offset[w.x];
-    uint32_t *largest = args.largest + args.eig_offset[w.x];
+    const float *x = args.x[op] + args.offset[w.x];
+    uint32_t *largest = args.largest[op] + args.eig_offset[w.x];
     uint32_t m = 0;
     if constexpr (kTranspose) {
       const int i = w.y * kTile + threadIdx.x % kTile;
@@ -108,17 +111,22 @@ __global__ void __launch_bounds__(256) largestKernel(SliceArgs args) {
   }
 }
 
+__global__ void __launch_bounds__(256) largestKernel(const __grid_constant__ SliceArgs args) {
+  if (args.transpose[blockIdx.z]) largestOf<true>(args, blockIdx.z);
+  else largestOf<false>(args, blockIdx.z);
+}
+
 // The digits of a 128 x 32 piece as an operand tile (K-major): operand row =
 // column of X, or with kTranspose row of X.  A thread cuts 8 elements of a row
 // that are consecutive in K.
 template <bool kTranspose>
-__global__ void __launch_bounds__(256) digitKernel(SliceArgs args) {
+__device__ __forceinline__ void digitsOf(const SliceArgs &args, int op) {
   for (int item = blockIdx.x; item < args.items; item += gridDim.x) {
     const int4 w = args.work[item];
     const int n = args.n[w.x];
-    const float *x = args.x + args.offset[w.x];
-    const uint32_t *largest = args.largest + args.eig_offset[w.x];
-    uint8_t *tile = args.slices +
+    const float *x = args.x[op] + args.offset[w.x];
+    const uint32_t *largest = args.largest[op] + args.eig_offset[w.x];
+    uint8_t *tile = args.slices[op] +
                     (args.tile_base[w.x] + static_cast<int64_t>(w.y) * w.w + w.z) * kTileBytes;
     const bool vector = n % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
 #pragma unroll
@@ -161,6 +169,11 @@ __global__ void __launch_bounds__(256) digitKernel(SliceArgs args) {
       }
     }
   }
+}
+
+__global__ void __launch_bounds__(256) digitKernel(const __grid_constant__ SliceArgs args) {
+  if (args.transpose[blockIdx.z]) digitsOf<true>(args, blockIdx.z);
+  else digitsOf<false>(args, blockIdx.z);
 }
 
 struct SlicedArgs {
@@ -439,29 +452,41 @@ int slicedOperands(msq_ctx *ctx, const DeviceBatch *b, const SlicedPlan &p, int 
   return MSQ_OK;
 }
 
-// The digits of X (kTranspose: of X^T) as an operand; `find`: its largest
-// magnitudes too (else a product has left them).
-template <bool kTranspose>
-int sliceOperand(msq_ctx *ctx, const DeviceBatch *b, const SlicedPlan &p, const float *x,
-                 const Operand &out, bool find) {
+// A matrix to cut (transpose: its rows) and the operand it becomes.
+struct Source {
+  const float *x;
+  Operand out;
+  bool transpose;
+};
+
+// The digits of up to three matrices, in one launch (two with `find`: their
+// largest magnitudes first; else a product has left them).  V, V^T and R of a
+// correction of four matrices of order 1000: about 30 us, 62 in six launches.
+int sliceOperands(msq_ctx *ctx, const DeviceBatch *b, const SlicedPlan &p,
+                  std::initializer_list<Source> sources, bool find) {
   SliceArgs s{};
   s.rows = p.rows;
   s.row_items = p.row_items;
   s.work = p.pack;
   s.items = p.pack_items;
-  s.x = x;
   s.offset = b->offset;
   s.eig_offset = b->eig_offset;
   s.tile_base = reinterpret_cast<const int64_t *>(p.bases);
   s.n = b->n;
-  s.largest = out.largest;
-  s.slices = out.slices;
+  unsigned count = 0;
+  for (const Source &q : sources) {
+    s.x[count] = q.x;
+    s.largest[count] = q.out.largest;
+    s.slices[count] = q.out.slices;
+    s.transpose[count++] = q.transpose;
+  }
   if (find) {
-    const dim3 grid(std::min(p.row_items, kSmCount * 8), kTile / 8);
-    largestKernel<kTranspose><<<grid, 256, 0, ctx->stream>>>(s);
+    const dim3 grid(std::min(p.row_items, kSmCount * 8), kTile / 8, count);
+    largestKernel<<<grid, 256, 0, ctx->stream>>>(s);
     MSQ_TRY(launched(ctx, "sliced largest"));
   }
-  digitKernel<kTranspose><<<std::min(p.pack_items, kSmCount * 8), 256, 0, ctx->stream>>>(s);
+  const dim3 grid(std::min(p.pack_items, kSmCount * 8), 1, count);
+  digitKernel<<<grid, 256, 0, ctx->stream>>>(s);
   return launched(ctx, "sliced digits");
 }
 
@@ -499,11 +524,12 @@ int slicedGemm(msq_ctx *ctx, const DeviceBatch *b, const SlicedPlan &p, const Op
 // Orders from which a matrix's products may be sliced, and the sum of n^3 of
 // such matrices from which they are.  A tile of 128 is mostly padding below
 // order 256 (a correction of 1000 matrices of order 128: 708 us against 550
-// with FMA chains; 100 of order 200: 333 against 328), and slicing adds ten
-// launches, which little work does not pay for (eight of order 384: 179
-// against 148; 32 of order 256: 180 against 168; but two of order 700, 0.69e9:
-// 225 against 235; 16 of order 384: 204 against 227; 64 of order 256: 273
-// against 286; four of order 1000: 471 against 821; 2048: 752 against 1584).
+// with FMA chains; 100 of order 200: 333 against 328), and slicing adds six
+// launches, which little work does not pay for (eight of order 384: 158 us
+// against 145; 20 of order 300: 236 against 200; 38 of order 256, 0.64e9: 172
+// against 166; but two of order 700, 0.69e9: 207 against 235; 16 of order 384:
+// 185 against 227; 64 of order 256: 251 against 286; four of order 1000: 445
+// against 821; 2048: 719 against 1584).
 constexpr int kSlicedOrder = 256;
 constexpr double kSlicedWork = 0.65e9;
 // The digits of four operands stay below this.
@@ -529,7 +555,7 @@ int slicedReconstruct(msq_ctx *ctx, const DeviceBatch *b, const float *f, float 
   Operand op[1];
   MSQ_TRY(slicedPlan(ctx, b, &p));
   MSQ_TRY(slicedOperands(ctx, b, p, 1, op));
-  MSQ_TRY(sliceOperand<false>(ctx, b, p, f, op[0], true));
+  MSQ_TRY(sliceOperands(ctx, b, p, {{f, op[0], false}}, true));
   return slicedGemm<kSlicedMirror>(ctx, b, p, op[0], op[0], nullptr, x, nullptr);
 }
 
@@ -546,21 +572,20 @@ int slicedSylvester(msq_ctx *ctx, const DeviceBatch *b, const float *v, const fl
   };
   if (!basis_packed) {
     MSQ_TRY(clear(vt.largest, 4));
-    MSQ_TRY(sliceOperand<false>(ctx, b, p, v, vn, true));  // rows = columns of V
-    MSQ_TRY(sliceOperand<true>(ctx, b, p, v, vt, true));   // rows = rows of V
+    MSQ_TRY(sliceOperands(ctx, b, p, {{v, vn, false}, {v, vt, true}, {r, even, false}}, true));
   } else {
     MSQ_TRY(clear(even.largest, 2));
+    MSQ_TRY(sliceOperands(ctx, b, p, {{r, even, false}}, true));
   }
-  MSQ_TRY(sliceOperand<false>(ctx, b, p, r, even, true));
   // G = R^T V into ws, C = (V^T G) o H into e, (V C)^T into ws, E into e
   MSQ_TRY(slicedGemm<kSlicedStore>(ctx, b, p, even, vn, nullptr, ws, odd.largest));
-  MSQ_TRY(sliceOperand<false>(ctx, b, p, ws, odd, false));
+  MSQ_TRY(sliceOperands(ctx, b, p, {{ws, odd, false}}, false));
   MSQ_TRY(clear(even.largest, 1));
   MSQ_TRY(slicedGemm<kSlicedInverseH>(ctx, b, p, vn, odd, lam, e, even.largest));
-  MSQ_TRY(sliceOperand<false>(ctx, b, p, e, even, false));
+  MSQ_TRY(sliceOperands(ctx, b, p, {{e, even, false}}, false));
   MSQ_TRY(clear(odd.largest, 1));
   MSQ_TRY(slicedGemm<kSlicedStore>(ctx, b, p, even, vt, nullptr, ws, odd.largest));
-  MSQ_TRY(sliceOperand<false>(ctx, b, p, ws, odd, false));
+  MSQ_TRY(sliceOperands(ctx, b, p, {{ws, odd, false}}, false));
   return slicedGemm<kSlicedStore>(ctx, b, p, odd, vt, nullptr, e, nullptr);
 }
 
