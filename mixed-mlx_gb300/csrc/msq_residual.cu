@@ -32,9 +32,9 @@
 // the tensor pipe's read of A: an MMA of M = 128 takes 68 cycles for N = 32,
 // 64 and 128 alike (152 matrices of order 512: 80 per MMA with the drain).
 //
-// Residual of four matrices of order 1000: 216 us with the slicing against
-// 908 on the CUDA cores; 152 of order 512: 1085 against 4247; 1000 of order
-// 128: 346 against 716; one of order 128: 38 against 53.
+// Residual of four matrices of order 1000: 219 us with the slicing against
+// 913 on the CUDA cores; 152 of order 512: 1095 against 4254; 1000 of order
+// 128: 363 against 718; one of order 128: 41 against 54.
 #include "msq_dense.cuh"
 #include "msq_internal.cuh"
 #include "msq_residual.cuh"
@@ -201,10 +201,20 @@ struct ResidualMmaArgs {
 
 // Accumulates the sum of squares of normalised float-float values (t, e).
 __device__ __forceinline__ void addSquare(float &s, float &c, float t, float e) {
-  const float q = t * t, qe = fmaf(t, t, -q) + 2.0f * t * e;
+  const float q = __fmul_rn(t, t), qe = fmaf(t, t, -q) + 2.0f * t * e;
   const float u = s + q, z = u - s;
   c += ((s - (u - z)) + (q - z)) + qe;
   s = u;
+}
+// A thread's sum of at most kCols squares to which every square that FP32
+// loses, and every error term of one (below 2^-126, to within 2^-149), adds
+// less than 2^-48 of it; false for a NaN.
+__device__ __forceinline__ bool inSquareRange(float s) {
+  return s >= 2.5243549e-29f && s <= 1.2676506e30f;  // 2^-95 .. 2^100
+}
+// 4^k as a double, |k| < 500
+__device__ __forceinline__ double squaredPowerOfTwo(int k) {
+  return __hiloint2double((1023 + 2 * k) << 20, 0);
 }
 
 __global__ void __launch_bounds__(kResidualThreads, 1) residualMmaKernel(ResidualMmaArgs args) {
@@ -367,67 +377,95 @@ __global__ void __launch_bounds__(kResidualThreads, 1) residualMmaKernel(Residua
         h[c] = scaleBy(h[c], k);
         l[c] = scaleBy(l[c], k);
       }
-      float rs = 0.0f, rc = 0.0f, as = 0.0f, ac = 0.0f;  // sums of squares, float-float
-      // (a + a_lo) - (s + comp) with a two-sum so the FP32 output rounds once
-      auto element = [&](float a, float a_lo, float s, float comp) {
+      // The squares are summed in float-float (an FP64 operation costs as much
+      // as 64 FP32 ones) at scales that the columns' exponents give: A near 1,
+      // R 2^40 above that.  A sum that leaves inSquareRange, where FP32
+      // loses or overflows squares, is taken again in FP64.
+      int kmax = ei + 12 + __shfl_sync(0xffffffffu, ej, 0);
+#pragma unroll
+      for (int c = 1; c < kCols; ++c) kmax = max(kmax, ei + 12 + __shfl_sync(0xffffffffu, ej, c));
+      kmax = min(max(kmax, -87), 126);  // both scales are normal numbers
+      const float scale_a = powerOfTwo(-kmax), scale_r = powerOfTwo(40 - kmax);
+      double rn = 0.0, an = 0.0;
+      // (a + a_lo) - (s + comp) with a two-sum so the FP32 output rounds once;
+      // after the cancellation t and e are of one size: normalised into t, e
+      auto element = [](float a, float a_lo, float s, float comp, float &t, float &e) {
         const float hi = -s, lo = a_lo - comp;
-        const float t = a + hi, z = t - a;
-        const float e = (a - (t - z)) + (hi - z) + lo;
-        // after the cancellation t and e are of one size: normalised first
-        const float v = t + e, y = v - t;
-        addSquare(rs, rc, v, (t - (v - y)) + (e - y));
-        addSquare(as, ac, a, a_lo);
-        return v;
+        const float u = a + hi, z = u - a;
+        const float f = (a - (u - z)) + (hi - z) + lo;
+        t = u + f;
+        const float y = t - u;
+        e = (u - (t - y)) + (f - y);
       };
-      // All loads of a side before its stores (each thread reads and writes its
-      // own elements only, so R may be A).
-      if (i < n) {
-        float v[kCols];
-        const int64_t at0 = j0 + static_cast<int64_t>(i) * n;
+      // One side of the tile: element c has A's high word v[c] (loaded before
+      // anything is stored: each thread reads and writes its own elements only,
+      // so R may be A), its low word low(c), and R's value goes to store(c, x).
+      auto side = [&](const float (&v)[kCols], auto in, auto low, auto store) {
+        float rs = 0.0f, rc = 0.0f, as = 0.0f, ac = 0.0f;
+        bool any = false;
 #pragma unroll
         for (int c = 0; c < kCols; ++c) {
-          const int j = j0 + c;
-          v[c] = j < n && j >= i ? A[i + static_cast<int64_t>(j) * n] : 0.0f;
+          if (!in(c)) continue;
+          const float a_lo = low(c);
+          float t, e;
+          element(v[c], a_lo, h[c], l[c], t, e);
+          store(c, t);
+          addSquare(rs, rc, t * scale_r, e * scale_r);
+          addSquare(as, ac, v[c] * scale_a, a_lo * scale_a);
+          any = true;
         }
+        if (!any) return;
+        double r2, a2;
+        if (inSquareRange(rs) && inSquareRange(as)) {
+          r2 = (static_cast<double>(rs) + static_cast<double>(rc)) * squaredPowerOfTwo(kmax - 40);
+          a2 = (static_cast<double>(as) + static_cast<double>(ac)) * squaredPowerOfTwo(kmax);
+        } else {
+          r2 = a2 = 0.0;
 #pragma unroll
-        for (int c = 0; c < kCols; ++c) {
-          const int j = j0 + c;
-          if (j < n && j >= i) {
-            const int64_t at = i + static_cast<int64_t>(j) * n;
-            const float x = element(v[c], AL ? AL[at] : 0.0f, h[c], l[c]);
-            if (R) R[at] = x;
+          for (int c = 0; c < kCols; ++c) {
+            if (!in(c)) continue;
+            const float a_lo = low(c);
+            float t, e;
+            element(v[c], a_lo, h[c], l[c], t, e);
+            const double x = static_cast<double>(t) + static_cast<double>(e);
+            const double a = static_cast<double>(v[c]) + static_cast<double>(a_lo);
+            r2 += x * x;
+            a2 += a * a;
           }
         }
+        rn += r2;
+        an += a2;
+      };
+      if (i < n) {
+        float v[kCols];
+        const int64_t at0 = j0 + static_cast<int64_t>(i) * n, column0 = i + static_cast<int64_t>(j0) * n;
+        auto upper = [&](int c) { return j0 + c < n && j0 + c >= i; };
+#pragma unroll
+        for (int c = 0; c < kCols; ++c) v[c] = upper(c) ? A[column0 + static_cast<int64_t>(c) * n] : 0.0f;
+        side(v, upper, [&](int c) { return AL ? AL[column0 + static_cast<int64_t>(c) * n] : 0.0f; },
+             [&](int c, float x) { if (R) R[column0 + static_cast<int64_t>(c) * n] = x; });
         // the mirror image: kCols consecutive elements of column i
         const bool vector = j0 > i && j0 + kCols <= n && n % 4 == 0 &&
                             (reinterpret_cast<uintptr_t>(A) & 15) == 0 && (reinterpret_cast<uintptr_t>(R) & 15) == 0;
+        auto low = [&](int c) { return AL ? AL[at0 + c] : 0.0f; };
         if (vector) {
+          float x[4];
 #pragma unroll
           for (int c = 0; c < kCols; c += 4) {
             const float4 q = *reinterpret_cast<const float4 *>(A + at0 + c);
             v[c] = q.x; v[c + 1] = q.y; v[c + 2] = q.z; v[c + 3] = q.w;
           }
-#pragma unroll
-          for (int c = 0; c < kCols; ++c) v[c] = element(v[c], AL ? AL[at0 + c] : 0.0f, h[c], l[c]);
-          if (R) {
-#pragma unroll
-            for (int c = 0; c < kCols; c += 4)
-              *reinterpret_cast<float4 *>(R + at0 + c) = make_float4(v[c], v[c + 1], v[c + 2], v[c + 3]);
-          }
+          side(v, [](int) { return true; }, low, [&](int c, float y) {
+            x[c % 4] = y;
+            if (R && c % 4 == 3) *reinterpret_cast<float4 *>(R + at0 + c - 3) = make_float4(x[0], x[1], x[2], x[3]);
+          });
         } else {
+          auto mirrored = [&](int c) { return j0 + c < n && j0 + c > i; };
 #pragma unroll
-          for (int c = 0; c < kCols; ++c) v[c] = j0 + c < n && j0 + c > i ? A[at0 + c] : 0.0f;
-#pragma unroll
-          for (int c = 0; c < kCols; ++c) {
-            if (j0 + c < n && j0 + c > i) {
-              const float x = element(v[c], AL ? AL[at0 + c] : 0.0f, h[c], l[c]);
-              if (R) R[at0 + c] = x;
-            }
-          }
+          for (int c = 0; c < kCols; ++c) v[c] = mirrored(c) ? A[at0 + c] : 0.0f;
+          side(v, mirrored, low, [&](int c, float x) { if (R) R[at0 + c] = x; });
         }
       }
-      double rn = static_cast<double>(rs) + static_cast<double>(rc);
-      double an = static_cast<double>(as) + static_cast<double>(ac);
 #pragma unroll
       for (int s = 16; s > 0; s >>= 1) {
         rn += __shfl_xor_sync(0xffffffffu, rn, s);
