@@ -67,6 +67,7 @@ struct GridArgs {
   float *diag;      // diagonal tiles after the pivots of two rounds: 2 x nb x 16
   double *acc;      // off2, diag2 accumulators
   unsigned *barrier;  // arrivals so far
+  int *failed;      // 1 once a launch of this solve gave up
   int *status;      // device status word
   int n, m, nb, P;
   int first, last;  // rounds [first, last) of the sweep
@@ -277,8 +278,9 @@ __global__ void __launch_bounds__(kSweepThreads, 1) gridSweepKernel(GridArgs g) 
 
   if (threadIdx.x == 0) {
     counters[0] = counters[1] = arrived = pair.groups = pair.taken = 0;
-    // an earlier launch gave up: its arrivals are missing from the count
-    give_up = *static_cast<volatile int *>(g.status) != kStatusOk;
+    // an earlier launch of this solve gave up: its arrivals are missing from
+    // the count (the status word may hold another call's report)
+    give_up = *static_cast<volatile int *>(g.failed);
   }
   __syncthreads();
   if (give_up || (quiet && warp != 0 && warp % 4 == 0)) return;
@@ -307,6 +309,7 @@ __global__ void __launch_bounds__(kSweepThreads, 1) gridSweepKernel(GridArgs g) 
         while (static_cast<int>(loadAcquire(g.barrier) - target) < 0) {
           if (++polls > limit) {
             atomicExch(g.status, kStatusFlagTimeout);
+            atomicExch(g.failed, 1);
             give_up = 1;
             break;
           }
@@ -654,6 +657,7 @@ int gridJacobiSolve(msq_ctx *ctx, float *matrix, float *vectors, float *eigenval
   MSQ_TRY(gridAttributes(ctx));
   g.acc = reinterpret_cast<double *>(work);
   g.barrier = reinterpret_cast<unsigned *>(work + 128);
+  g.failed = reinterpret_cast<int *>(work + 192);
   g.tiles[0] = reinterpret_cast<float *>(work + 256);
   g.tiles[1] = g.tiles[0] + tile_floats;
   g.v = g.tiles[1] + tile_floats;

@@ -77,3 +77,24 @@ def test_expired_barrier_is_reported_and_the_context_recovers(ctx, msq):
     ctx.synchronize()
     ref = np.linalg.eigvalsh(a.astype(np.float64))
     np.testing.assert_allclose(np.sort(w.cpu().numpy()), ref, rtol=0, atol=3 * n * 2.0**-24)
+
+
+def test_report_of_an_earlier_call_does_not_stop_the_sweeps(ctx, msq):
+    """A status word left by another call (a log-spectrum that is not positive)
+    is reported by the next check, and the matrix is solved all the same, bit
+    for bit."""
+    import torch
+    n = 1040
+    assert msq.jacobi_route([n])[0] == 1
+    rng = np.random.default_rng(n)
+    a = rng.standard_normal((n, n))
+    a = ((a + a.T) / 2).astype(np.float32)
+    b = msq.Batch.from_orders([n])
+    dev = torch.from_numpy(b.pack([a])).cuda()
+    want = [t.cpu() for t in ctx.jacobi(dev.clone(), b, 1e-6, 15)]
+    ctx.synchronize()
+    ctx.copy_spectrum_to_storage(msq.FP8_E4M3FN, torch.full((8,), -1.0, device="cuda"))
+    got = [t.cpu() for t in ctx.jacobi(dev, b, 1e-6, 15)]
+    with pytest.raises(msq.MsqError, match="log-spectrum"):
+        ctx.synchronize()
+    assert want[2][0] > 1 and all(torch.equal(x, y) for x, y in zip(got, want))
