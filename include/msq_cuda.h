@@ -61,7 +61,11 @@ typedef struct msq_ctx msq_ctx;
 int msq_create(msq_ctx **out, int device);
 void msq_destroy(msq_ctx *ctx);
 const char *msq_last_error(const msq_ctx *ctx);
-/* `stream` is a cudaStream_t (NULL = legacy default stream). */
+/* `stream` is a cudaStream_t (NULL = legacy default stream).  Calls on several
+ * streams in turn share the context's workspaces: a call that needs one waits
+ * on the device for the last that used one (the codecs and the network's
+ * forward and backward passes need none).  Work captured in the caller's own
+ * graphs is not covered: replay those on one stream. */
 int msq_set_stream(msq_ctx *ctx, void *stream);
 /* Concurrency inside a call (default on): the Jacobi forks its size buckets
  * and its V replay onto internal streams that join back into the context's

@@ -232,7 +232,39 @@ int keepWork(msq_ctx *ctx, const DeviceBatch *b, int key, const std::vector<int4
   return MSQ_OK;
 }
 
+namespace {
+// Whether the context's stream is being captured (by this library or by the
+// caller): events of either kind must not cross the capture.
+bool captured(msq_ctx *ctx) {
+  if (ctx->capturing) return true;
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(ctx->stream, &status) == cudaSuccess)
+    return status != cudaStreamCaptureStatusNone;
+  cudaGetLastError();
+  return true;
+}
+}  // namespace
+
+int scratchOrder(msq_ctx *ctx) {
+  ctx->scratch_used = true;
+  if (!ctx->scratch_wait || !ctx->scratch_recorded || captured(ctx)) return MSQ_OK;
+  ctx->scratch_wait = false;
+  return cudaCheck(ctx, cudaStreamWaitEvent(ctx->stream, ctx->scratch_event, 0), "scratch wait");
+}
+
+void scratchRecord(msq_ctx *ctx) {
+  ctx->scratch_used = false;
+  if (captured(ctx)) return;
+  if (ctx->scratch_event == nullptr &&
+      cudaEventCreateWithFlags(&ctx->scratch_event, cudaEventDisableTiming) != cudaSuccess) {
+    ctx->scratch_event = nullptr;
+    return;
+  }
+  ctx->scratch_recorded = cudaEventRecord(ctx->scratch_event, ctx->stream) == cudaSuccess;
+}
+
 void *scratch(msq_ctx *ctx, size_t bytes, int slot) {
+  if (scratchOrder(ctx) != MSQ_OK) return nullptr;
   if (bytes <= ctx->scratch_bytes[slot]) return ctx->scratch[slot];
   if (ctx->scratch[slot] != nullptr) {
     cudaStreamSynchronize(ctx->stream);
@@ -308,6 +340,7 @@ extern "C" void msq_destroy(msq_ctx *ctx) {
   destroyTcPlans(ctx->tc_plans);
   if (ctx->grid_host != nullptr) cudaFreeHost(ctx->grid_host);
   if (ctx->d_status != nullptr) cudaFree(ctx->d_status);
+  if (ctx->scratch_event != nullptr) cudaEventDestroy(ctx->scratch_event);
   recycleTiming(ctx);
   for (cudaEvent_t e : ctx->event_pool) cudaEventDestroy(e);
   for (cudaEvent_t e : ctx->sync_pool) cudaEventDestroy(e);
@@ -323,6 +356,7 @@ extern "C" const char *msq_last_error(const msq_ctx *ctx) {
 extern "C" int msq_set_stream(msq_ctx *ctx, void *stream) {
   if (ctx == nullptr) return MSQ_ERR_INVALID_ARGUMENT;
   ctx->stream = static_cast<cudaStream_t>(stream);
+  ctx->scratch_wait = true;
   return MSQ_OK;
 }
 

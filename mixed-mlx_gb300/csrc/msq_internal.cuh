@@ -102,6 +102,13 @@ struct msq_ctx {
   // one per user so nested stages never share memory.
   void *scratch[7] = {};
   size_t scratch_bytes[7] = {};
+  // Calls on different streams share the arenas: a call that used one leaves
+  // scratch_event behind its work, and after msq_set_stream the next call that
+  // needs one waits for it.
+  cudaEvent_t scratch_event = nullptr;
+  bool scratch_recorded = false;
+  bool scratch_wait = false;  // the stream was set since the last use
+  bool scratch_used = false;  // by the call in progress
   // Batch layouts cached by content hash (at most 32, oldest evicted).
   std::vector<msq::DeviceBatch *> batches;
   // Launch timing (msq_timing_begin/end).  Launches on the context stream
@@ -192,6 +199,11 @@ enum ScratchSlot : int {
   kScratchFallback = 5, kScratchResidual = 6, kScratchSlots = 7
 };
 void *scratch(msq_ctx *ctx, size_t bytes, int slot);
+// Orders the context's stream behind the last call that used an arena, on
+// whatever stream (scratch does this; so must a call that replays a graph).
+int scratchOrder(msq_ctx *ctx);
+// Leaves the event behind the work of a call that used an arena.
+void scratchRecord(msq_ctx *ctx);
 // Work lists (or other per-layout arrays) kept on the batch under a key: the
 // list if it is there (true), or `list` uploaded.
 bool findWork(const DeviceBatch *b, int key, const int4 **work, int *items);
@@ -201,10 +213,12 @@ int keepWork(msq_ctx *ctx, const DeviceBatch *b, int key, const std::vector<int4
 void *pinnedScratch(msq_ctx *ctx, size_t bytes);
 
 // Makes the context's device current for one entry point and restores the
-// caller's device on return (a process may drive several GPUs).
+// caller's device on return (a process may drive several GPUs); marks the end
+// of the call's use of the arenas.
 struct DeviceGuard {
+  msq_ctx *ctx;
   int previous = -1;
-  explicit DeviceGuard(const msq_ctx *ctx) {
+  explicit DeviceGuard(msq_ctx *c) : ctx(c) {
     int current = 0;
     if (cudaGetDevice(&current) == cudaSuccess && current != ctx->device &&
         cudaSetDevice(ctx->device) == cudaSuccess) {
@@ -212,6 +226,7 @@ struct DeviceGuard {
     }
   }
   ~DeviceGuard() {
+    if (ctx->scratch_used) scratchRecord(ctx);
     if (previous >= 0) cudaSetDevice(previous);
   }
   DeviceGuard(const DeviceGuard &) = delete;

@@ -671,6 +671,7 @@ extern "C" int msq_solve_batched(msq_ctx *ctx, const float *a, const int32_t *n,
       ctx->solve_graphs.erase(ctx->solve_graphs.begin() + k);
       break;
     }
+    MSQ_TRY(scratchOrder(ctx));
     MSQ_TRY(cudaCheck(ctx, cudaGraphLaunch(e.exec, ctx->stream), "solve graph launch"));
     ++ctx->graph_launches;
     ctx->launches += e.launches;
@@ -726,7 +727,8 @@ extern "C" int msq_solve_batched(msq_ctx *ctx, const float *a, const int32_t *n,
       cudaGraphExec_t exec = nullptr;
       if (status == MSQ_OK && end == cudaSuccess && generation == ctx->alloc_generation &&
           cudaGraphInstantiate(&exec, graph, 0) == cudaSuccess) {
-        status = cudaCheck(ctx, cudaGraphLaunch(exec, caller), "solve graph launch");
+        status = scratchOrder(ctx);
+        if (status == MSQ_OK) status = cudaCheck(ctx, cudaGraphLaunch(exec, caller), "solve graph launch");
         ++ctx->graph_launches;
         if (ctx->solve_graphs.size() >= 4) {
           cudaGraphExecDestroy(ctx->solve_graphs.front().exec);
