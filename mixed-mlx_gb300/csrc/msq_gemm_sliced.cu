@@ -357,7 +357,10 @@ __global__ void __launch_bounds__(kSlicedThreads, 1) slicedGemmKernel(SlicedArgs
           const float d = si + __shfl_sync(0xffffffffu, sj, q);
           x = d > 0.0f ? x / d : 0.0f;  // both roots 0: no correction
         }
-        if (i < n && j < n) C[i + static_cast<int64_t>(j) * n] = x;
+        // a diagonal tile's (i, j) and (j, i) need not have the same bits (the
+        // last accumulator is rounded, and its pairs come in another order)
+        const bool own = kEpi != kSlicedMirror || w.y != w.z || j >= i;
+        if (own && i < n && j < n) C[i + static_cast<int64_t>(j) * n] = x;
         if (kEpi != kSlicedMirror) {
           const uint32_t m = __reduce_max_sync(0xffffffffu, i < n ? finiteBits(x) : 0u);
           if (lane == q) largest = m;
@@ -366,13 +369,13 @@ __global__ void __launch_bounds__(kSlicedThreads, 1) slicedGemmKernel(SlicedArgs
       }
       if (kEpi != kSlicedMirror) {
         if (args.largest_c != nullptr && jl < n) atomicMax(args.largest_c + eig + jl, largest);
-      } else if (w.y != w.z) {
+      } else {
         transpose32(h, lane);
         const int i0 = i - lane;
         if (jl < n) {
 #pragma unroll
           for (int q = 0; q < 32; ++q)
-            if (i0 + q < n) C[jl + static_cast<int64_t>(i0 + q) * n] = h[q];
+            if (i0 + q < n && (w.y != w.z || jl > i0 + q)) C[jl + static_cast<int64_t>(i0 + q) * n] = h[q];
         }
       }
     }

@@ -76,3 +76,25 @@ def test_a_nan_stays_in_its_row_and_column(ctx, msq):
     assert np.isnan(got[i]).all() and np.isnan(got[:, i]).all()
     rest = np.delete(np.arange(n), i)
     assert np.array_equal(got[np.ix_(rest, rest)], clean[np.ix_(rest, rest)])
+
+
+def test_result_is_symmetric_where_the_last_accumulator_rounds(ctx, msq):
+    """Columns of two kinds, even ones odd and odd ones even under an exchange of
+    the neighbours in K: the three largest weights cancel, and the pairs of the
+    smallest outgrow an exact sum.  (i, j) and (j, i) add them in another order;
+    one of the two is stored twice."""
+    import torch
+    n = 1024
+    rng = np.random.default_rng(n)
+    sign = np.where(np.arange(n) % 2 == 0, 1.0, -1.0)
+    odd = np.arange(n)[None, :] % 2 == 0  # by column: the first three digits change sign
+    first = [np.repeat(d, 2, axis=0) for d in (np.full((n // 2, n), 60.0), rng.integers(-60, 61, (n // 2, n)),
+                                               rng.integers(-60, 61, (n // 2, n)))]
+    y = sum(d * 128.0**-p for p, d in enumerate(first))
+    f = np.where(odd, sign[:, None] * y + 56 * 128.0**-3, y + sign[:, None] * 56 * 128.0**-3) / 64
+    assert np.array_equal(f, f.astype(np.float32))
+    b = msq.Batch.from_orders([n])
+    x = ctx.reconstruct_factor(msq.PLAN_FP32, _dev(b.pack([f])), b)
+    torch.cuda.synchronize()
+    xg = b.unpack(x.cpu().numpy(), np.float32)[0]
+    assert np.array_equal(xg, xg.T)
