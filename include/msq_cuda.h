@@ -299,7 +299,7 @@ int msq_jacobi_noalloc(float *matrix, float *vectors, float *eigenvalues, int n,
  * reconstructLowFactorTiled (src/metal_runtime.cpp:429-534).
  * msq_make_factor builds W^T in K-major order (row i of W contiguous) from V
  * and lambda, FP32.  msq_reconstruct consumes W^T in `format`:
- *   MSQ_FMT_FP32        SIMT FP32 GEMM (the plain FP32 path)
+ *   MSQ_FMT_FP32        FP32 products (below)
  *   MSQ_FMT_BF16        tcgen05 kind::f16 MMA, FP32 accumulate in TMEM
  *   MSQ_FMT_FP8_E4M3FN_ROWSCALE  tcgen05 kind::f8f6f4 (E4M3 x E4M3),
  *                       row scales applied in the epilogue
@@ -313,7 +313,14 @@ int msq_jacobi_noalloc(float *matrix, float *vectors, float *eigenvalues, int n,
  * row-scaled, the codec's scale bytes for MX).  The solver's MXFP4 plan
  * (msq_solve_batched) quantizes W^T per row block and always takes the
  * kind::mxf4 path.
- * Output X (FP32) uses the same batched layout as the input.              */
+ * Output X (FP32) uses the same batched layout as the input.
+ * FP32 products (here, in msq_reconstruct_factor and msq_sylvester_sweep):
+ * each element is within n 2^-24 sum |a_k b_k| of its value, infinities and
+ * NaN as in FP32.  Small matrices and batches run as FMA chains on the CUDA
+ * cores, and orders of 256 and more, where the batch has enough of them, on
+ * the tensor cores (three BF16 pieces per entry, FP32 accumulation, smaller
+ * errors); so the last bits of a large matrix may depend on the batch it is
+ * in.  X is equal to its transpose either way.                            */
 int msq_make_factor(msq_ctx *ctx, const float *vectors,
                     const float *eigenvalues, const int32_t *n,
                     const int64_t *offset, int count, float *factor_t);
@@ -341,7 +348,7 @@ int msq_reconstruct_factor(msq_ctx *ctx, int plan_format, const float *factor_t,
  * refineUpdateAndMeasure (src/metal_runtime.cpp:847-966):
  *   C = (V^T R V) o H, H_ij = 1/(s_i + s_j) recomputed from s = sqrt(lambda),
  *   E = V C V^T,  X <- X + (E + E^T)/2 (float-float add into x_hi/x_lo).
- * `gemm_format` selects the correction GEMMs: MSQ_FMT_FP32 (SIMT FP32) or
+ * `gemm_format` selects the correction GEMMs: MSQ_FMT_FP32 (FP32 products) or
  * MSQ_FMT_BF16 (tcgen05 split-BF16, three products, FP32 accumulate).
  * `workspace` must hold 2 * sum(n^2) floats.                               */
 int msq_residual(msq_ctx *ctx, const float *a, const float *a_lo,

@@ -1,29 +1,41 @@
 // FP32 products of large matrices on the tensor cores.
 //
 // The CUDA cores' FP32 rate bounds a plain FP32 product (59% of it at order
-// 1000).  Here both operands are cut into kSlices = 4 digits (msq_slices.cuh),
-// each carrying its weight 2^-7p, and the products of digits p + q < 4 are
-// summed without rounding: one accumulator per weight, at most 4 pairs over
-// 1024 of K.  The pairs of weight 2^-28 join the last accumulator (rounded at
-// 2^-24 of it, far below the result): where a vector meets itself, as on the
-// diagonal of F^T F, they do not average out (a nearly diagonal matrix of order
-// 1000 loses 1.4e-6 without them, 7e-8 with them).  The four are put together in
-// float-float and rounded once.  What is cut off is below 2^-27 of the operands'
-// largest entries.  Relative Frobenius errors against 64 bits, FMA chain and
-// here, order 1000: F^T F of a Wishart matrix 4.3e-7 and 2.2e-8, of condition
-// 1e6 5.9e-7 and 2.9e-8, nearly diagonal and graded over 1e6 2.6e-7 and 7.4e-8;
-// corrections 8.5e-7 and 6.4e-8, 8.2e-7 and 6.7e-8, 8.0e-7 and 1.5e-7; smaller
-// too at orders 256, 512 and 2048.
+// 1000).  Here every FP32 entry is cut into kSlices = 3 BF16 pieces, each the
+// rounding of what the ones before left over, which hold its 24 bits whatever
+// its size; a product of two pieces is exact, and the pairs (p, q) with
+// p + q < 3 leave out less than 2^-25 of |a_k b_k|.  (The vectors are scaled by
+// powers of two, so that the pieces of entries down to 2^-109 of the largest
+// are normal numbers.)
+//
+// What an FP32 accumulator in TMEM adds is rounded toward zero: about 0.75 2^-24
+// of the sum for each MMA, always the same way.  So the sums are kept short:
+// the pairs (0, 0) of 32 of K (two MMAs) in an accumulator by turns, added up
+// by the epilogue in two levels (in registers, and every kLevel of these in
+// shared memory); the other pairs, 2^-8 of these and less, over all of K.  An
+// element is so within a few 2^-24 of sum |a_k b_k|, for entries of any size.
+//
+// Against 64 bits, FMA chains and here.  Relative Frobenius error of F^T F, F of
+// normal entries, its rows graded over 1e1.5 from the largest: order 256 2.5e-7
+// and 7.3e-8, 3.9e-7 and 8.6e-8; 1000 5.0e-7 and 7.8e-8, 7.8e-7 and 9.2e-8; 4096
+// 1.0e-6 and 9.7e-8, 1.7e-6 and 1.3e-7.  The largest error of an element in
+// units of n 2^-24 sum |a_k b_k|, the identity and 1e-6 of noise: order 256 0.076
+// and 0.030, 1000 0.053 and 0.009.  Corrections at order 1000 7.6e-7 and 1.6e-7,
+// nearly diagonal V 7.3e-7 and 2.4e-7.  (Fixed-point digits of 27 bits have
+// 2.7e-8 of F^T F, but the small entries of that noise are off by 1e-3.)
 //
 // slicedGemmKernel is persistent and warp-specialized as the residual kernel:
 // a producer warp, an MMA warp, sixteen epilogue warps.  Tiles of 128 x 128 (at
 // N = 128 an MMA costs the 68 cycles that its read of A takes, as at N = 64),
-// 32 of K per stage (32 KB of A, 32 KB of B, three stages), four accumulators
-// of 128 columns: all of TMEM.  A stage is 26 MMAs, 1770 cycles, for 64 KB:
-// tensor pipe and operand loads are near balance.
+// 32 of K per stage (24 KB of A, 24 KB of B, three stages), four accumulators of
+// 128 columns, which are all of TMEM: two by turns for the pairs (0, 0), one
+// for p + q = 1, one for p + q = 2 (MMAs into one accumulator follow each other
+// at 164 cycles).  A stage is 12 MMAs, 816 cycles, for 48 KB: bound by the
+// operand loads.
 //
 // The largest magnitude of every column of a result, which the next product's
-// slices are scaled by, is taken in the epilogue.
+// pieces are scaled by, is taken in the epilogue.
+#include "msq_codec_device.cuh"
 #include "msq_dense.cuh"
 #include "msq_gemm_sliced.cuh"
 #include "msq_internal.cuh"
@@ -38,29 +50,29 @@
 namespace msq {
 namespace {
 
-constexpr int kSlices = 4;
+constexpr int kSlices = 3;
 constexpr int kTile = 128, kTileK = 32;
-constexpr int kSliceBytes = kTile * 2 * kTileK;        // one digit of a tile, SWIZZLE_64B
+constexpr int kSliceBytes = kTile * 2 * kTileK;        // one piece of a tile, SWIZZLE_64B
 constexpr int kTileBytes = kSlices * kSliceBytes;
 constexpr int kStageBytes = 2 * kTileBytes;
 constexpr int kStages = 3;
-constexpr int kChunkTiles = 1024 / kTileK;             // K tiles per exact accumulation
+constexpr int kLevel = 8;                              // K tiles per sum in registers
 constexpr int kEpilogueWarps = 16;
 constexpr int kCols = kTile / (kEpilogueWarps / 4);    // columns per epilogue thread
 constexpr int kHalf = 16;                              // columns per TMEM load
 constexpr int kSlicedThreads = 32 * (kEpilogueWarps + 2);
-constexpr size_t kSlicedSmem = kStages * kStageBytes + 1024 + 256;
-static_assert(kSlices * kTile == 512, "one accumulator per weight fills TMEM");
+constexpr int kTotalBytes = kTile * kTile * 4;
+constexpr size_t kSlicedSmem = kStages * kStageBytes + kTotalBytes + 1024 + 256;
 
-// Pairs (p, q) as 16 p + q, (0, g) first of accumulator g = min(p + q, 3).
-constexpr int kPairs = 13;
-__device__ constexpr uint8_t kPairOrder[kPairs] = {0x03, 0x02, 0x01, 0x00, 0x12, 0x11, 0x10,
-                                                   0x21, 0x20, 0x30, 0x13, 0x22, 0x31};
-__host__ __device__ constexpr int pairGroup(int p, int q) { return p + q < kSlices ? p + q : kSlices - 1; }
+// Pairs (p, q) as 16 p + q.  Accumulators: kTile columns each at kTile times 0 or
+// 1 (pair (0, 0) by turns), 2 (p + q = 1), 3 (p + q = 2); the order keeps those
+// of one accumulator apart.
+constexpr int kPairs = 6;
+__device__ constexpr uint8_t kPairOrder[kPairs] = {0x02, 0x01, 0x00, 0x11, 0x10, 0x20};
 
 __device__ __forceinline__ uint32_t finiteBits(float x) {
   const float a = fabsf(x);
-  return a <= 3.402823466e38f ? __float_as_uint(a) : 0u;  // a NaN or infinity stays one in its digits
+  return a <= 3.402823466e38f ? __float_as_uint(a) : 0u;  // a NaN or infinity stays one in its pieces
 }
 
 struct SliceArgs {
@@ -116,11 +128,11 @@ __global__ void __launch_bounds__(256) largestKernel(const __grid_constant__ Sli
   else largestOf<false>(args, blockIdx.z);
 }
 
-// The digits of a 128 x 32 piece as an operand tile (K-major): operand row =
+// The pieces of 128 x 32 entries as an operand tile (K-major): operand row =
 // column of X, or with kTranspose row of X.  A thread cuts 8 elements of a row
 // that are consecutive in K.
 template <bool kTranspose>
-__device__ __forceinline__ void digitsOf(const SliceArgs &args, int op) {
+__device__ __forceinline__ void piecesOf(const SliceArgs &args, int op) {
   for (int item = blockIdx.x; item < args.items; item += gridDim.x) {
     const int4 w = args.work[item];
     const int n = args.n[w.x];
@@ -148,8 +160,8 @@ __device__ __forceinline__ void digitsOf(const SliceArgs &args, int op) {
           v[q] = row < n && k0 + q < n ? x[at] : 0.0f;
         }
       }
-      // to |y| < 64: the first digit is the nearest integer
-      const int e = (row < n ? exponentOf(largest[row]) : 0) - (kDigit - 1);
+      // to |y| < 1
+      const int e = row < n ? exponentOf(largest[row]) : 0;
 #pragma unroll
       for (int q = 0; q < 8; ++q) v[q] = scaleBy(v[q], -e);
       uint8_t *out = tile + swizzle64(r, c);
@@ -158,10 +170,11 @@ __device__ __forceinline__ void digitsOf(const SliceArgs &args, int op) {
         uint32_t word[4];
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
-          const float d = rintf(v[q]);
-          v[q] = (v[q] - d) * static_cast<float>(1 << kDigit);  // exact
-          // an integer times its weight 2^-7p: BF16 holds it exactly
-          const uint32_t h = __float_as_uint(d * (1.0f / (1 << (kDigit * p)))) >> 16;
+          // an infinity or a NaN is its first piece
+          const bool finite = fabsf(v[q]) <= 1.0f;
+          const uint32_t h = finite ? encodeBf16(v[q])
+                                    : (__float_as_uint(v[q]) >> 16) | (v[q] != v[q] ? 0x40u : 0u);
+          v[q] = finite ? v[q] - decodeBf16(static_cast<uint16_t>(h)) : 0.0f;  // exact
           if (q % 2 == 0) word[q / 2] = h;
           else word[q / 2] |= h << 16;
         }
@@ -171,15 +184,15 @@ __device__ __forceinline__ void digitsOf(const SliceArgs &args, int op) {
   }
 }
 
-__global__ void __launch_bounds__(256) digitKernel(const __grid_constant__ SliceArgs args) {
-  if (args.transpose[blockIdx.z]) digitsOf<true>(args, blockIdx.z);
-  else digitsOf<false>(args, blockIdx.z);
+__global__ void __launch_bounds__(256) piecesKernel(const __grid_constant__ SliceArgs args) {
+  if (args.transpose[blockIdx.z]) piecesOf<true>(args, blockIdx.z);
+  else piecesOf<false>(args, blockIdx.z);
 }
 
 struct SlicedArgs {
   const int4 *work;        // (matrix, tile_i, tile_j, k tiles)
   int items;
-  const uint8_t *a, *b;    // digits of the operands
+  const uint8_t *a, *b;    // pieces of the operands
   const uint32_t *largest_a, *largest_b;
   const int64_t *tile_base;
   const int32_t *n;
@@ -203,9 +216,11 @@ __global__ void __launch_bounds__(kSlicedThreads, 1) slicedGemmKernel(SlicedArgs
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char *base = reinterpret_cast<unsigned char *>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  uint64_t *full = reinterpret_cast<uint64_t *>(base + kStages * kStageBytes), *empty = full + kStages;
-  uint64_t *acc_full = empty + kStages, *acc_empty = acc_full + 1;
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_empty + 1);
+  float *totals = reinterpret_cast<float *>(base + kStages * kStageBytes);  // [kCols][epilogue threads]
+  uint64_t *full = reinterpret_cast<uint64_t *>(base + kStages * kStageBytes + kTotalBytes), *empty = full + kStages;
+  // the accumulators of pair (0, 0) by turns, and the other two
+  uint64_t *acc_full = empty + kStages, *acc_empty = acc_full + 2, *rest_empty = acc_empty + 2;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(rest_empty + 1);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
   constexpr uint32_t kDesc = instrDescBf16(kTile, kTile);
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
@@ -214,8 +229,11 @@ __global__ void __launch_bounds__(kSlicedThreads, 1) slicedGemmKernel(SlicedArgs
       mbarInit(smemAddr(&full[s]), 1);
       mbarInit(smemAddr(&empty[s]), 1);
     }
-    mbarInit(smemAddr(acc_full), 1);
-    mbarInit(smemAddr(acc_empty), 32 * kEpilogueWarps);
+    for (int a = 0; a < 2; ++a) {
+      mbarInit(smemAddr(&acc_full[a]), 1);
+      mbarInit(smemAddr(&acc_empty[a]), 32 * kEpilogueWarps);
+    }
+    mbarInit(smemAddr(rest_empty), 32 * kEpilogueWarps);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -259,16 +277,14 @@ __global__ void __launch_bounds__(kSlicedThreads, 1) slicedGemmKernel(SlicedArgs
     }
   } else if (warp == kEpilogueWarps + 1) {
     if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0, acc_phase = 0;
+      int stage = 0, acc = 0;
+      uint32_t phase = 0, acc_phase = 0, rest_phase = 0;
       for (int item = blockIdx.x; item < args.items && !*abort_flag; item += gridDim.x) {
         const int k_tiles = args.work[item].w;
+        if (!barWait(smemAddr(rest_empty), rest_phase ^ 1, args.status, abort_flag)) break;
+        rest_phase ^= 1;
         for (int kt = 0; kt < k_tiles; ++kt) {
-          const bool first = kt % kChunkTiles == 0;
-          if (first) {
-            if (!barWait(smemAddr(acc_empty), acc_phase ^ 1, args.status, abort_flag)) break;
-            acc_phase ^= 1;
-          }
+          if (!barWait(smemAddr(&acc_empty[acc]), acc_phase ^ 1, args.status, abort_flag)) break;
           if (!barWait(smemAddr(&full[stage]), phase, args.status, abort_flag)) break;
           asm volatile("tcgen05.fence::after_thread_sync;");
           const uint32_t mem = smemAddr(base + stage * kStageBytes);
@@ -277,17 +293,23 @@ __global__ void __launch_bounds__(kSlicedThreads, 1) slicedGemmKernel(SlicedArgs
           for (int kk = 0; kk < kTileK / 16; ++kk) {
 #pragma unroll
             for (int x = 0; x < kPairs; ++x) {
-              const int p = kPairOrder[x] >> 4, q = kPairOrder[x] & 15;
-              mmaBf16(tmem + kTile * pairGroup(p, q), ad + p * (kSliceBytes >> 4) + 2 * kk,
-                      bd + q * (kSliceBytes >> 4) + 2 * kk, kDesc, !(first && p == 0 && kk == 0));
+              const int p = kPairOrder[x] >> 4, q = kPairOrder[x] & 15, g = p + q;
+              // the first MMA into an accumulator: (0, 0) of a K tile, (0, 1) and (0, 2) of the item
+              const bool more = g == 0 ? kk > 0 : kk > 0 || p > 0 || kt > 0;
+              mmaBf16(tmem + kTile * (g == 0 ? acc : g + 1), ad + p * (kSliceBytes >> 4) + 2 * kk,
+                      bd + q * (kSliceBytes >> 4) + 2 * kk, kDesc, more);
             }
           }
           mmaCommit(smemAddr(&empty[stage]));
+          mmaCommit(smemAddr(&acc_full[acc]));  // of the last K tile: the item's
           if (++stage == kStages) {
             stage = 0;
             phase ^= 1;
           }
-          if (kt % kChunkTiles == kChunkTiles - 1 || kt == k_tiles - 1) mmaCommit(smemAddr(acc_full));
+          if (++acc == 2) {
+            acc = 0;
+            acc_phase ^= 1;
+          }
         }
       }
     }
@@ -295,15 +317,18 @@ __global__ void __launch_bounds__(kSlicedThreads, 1) slicedGemmKernel(SlicedArgs
     // Epilogue: warps w, w + 4, .. own accumulator rows 32 (w mod 4) ..; each
     // thread one row and kCols of the columns.
     const int quarter = warp % 4, part = warp / 4;
+    const uint32_t taddr = tmem + ((32u * quarter) << 16) + kCols * part;
+    float *total = totals + threadIdx.x;
+    int acc = 0;
     uint32_t acc_phase = 0;
     for (int item = blockIdx.x; item < args.items; item += gridDim.x) {
       const int4 w = args.work[item];
       const int mi = w.x, n = args.n[mi];
       const int i = w.y * kTile + 32 * quarter + lane, j0 = w.z * kTile + kCols * part;
       const int64_t eig = args.eig_offset[mi];
-      // 2^(e_i + e_j) times the digits' scale; lane q has column j0 + q
+      // 2^(e_i + e_j); lane q has column j0 + q
       const int jl = j0 + lane;
-      const int ei = (i < n ? exponentOf(args.largest_a[eig + i]) : 0) - 2 * (kDigit - 1);
+      const int ei = i < n ? exponentOf(args.largest_a[eig + i]) : 0;
       const int ej = jl < n ? exponentOf(args.largest_b[eig + jl]) : 0;
       float si = 0.0f, sj = 0.0f;
       if (kEpi == kSlicedInverseH) {
@@ -312,41 +337,47 @@ __global__ void __launch_bounds__(kSlicedThreads, 1) slicedGemmKernel(SlicedArgs
       }
       float h[kCols];
       bool ok = true;
-      const int chunks = (w.w + kChunkTiles - 1) / kChunkTiles;
-      for (int chunk = 0; chunk < chunks; ++chunk) {
-        ok = barWait(smemAddr(acc_full), acc_phase, args.status, abort_flag);
+      for (int kt = 0; kt < w.w; ++kt) {
+        ok = barWait(smemAddr(&acc_full[acc]), acc_phase, args.status, abort_flag);
         if (!ok) break;
-        acc_phase ^= 1;
         asm volatile("tcgen05.fence::after_thread_sync;");
-        const uint32_t taddr = tmem + ((32u * quarter) << 16) + kCols * part;
 #pragma unroll
         for (int s = 0; s < kCols; s += kHalf) {
-          // from the smallest weight, in float-float, rounded once per chunk
-          float ch[kHalf], cl[kHalf];
-          tmemLoad16(taddr + kTile * (kSlices - 1) + s, ch);
+          float v[kHalf];
+          tmemLoad16(taddr + kTile * acc + s, v);
 #pragma unroll
-          for (int c = 0; c < kHalf; ++c) cl[c] = 0.0f;
-#pragma unroll
-          for (int g = kSlices - 2; g >= 0; --g) {
-            float v[kHalf];
-            tmemLoad16(taddr + kTile * g + s, v);
-#pragma unroll
-            for (int c = 0; c < kHalf; ++c) {
-              const float t = v[c] + ch[c], z = t - v[c];
-              cl[c] += (v[c] - (t - z)) + (ch[c] - z);
-              ch[c] = t;
-            }
-          }
-#pragma unroll
-          for (int c = 0; c < kHalf; ++c) {
-            const float x = ch[c] + cl[c];
-            h[s + c] = chunk == 0 ? x : h[s + c] + x;
-          }
+          for (int c = 0; c < kHalf; ++c) h[s + c] = kt % kLevel == 0 ? v[c] : h[s + c] + v[c];
         }
         asm volatile("tcgen05.fence::before_thread_sync;");
-        mbarArrive(smemAddr(acc_empty));
+        mbarArrive(smemAddr(&acc_empty[acc]));
+        if (++acc == 2) {
+          acc = 0;
+          acc_phase ^= 1;
+        }
+        if (kt % kLevel == kLevel - 1 || kt == w.w - 1) {
+#pragma unroll
+          for (int c = 0; c < kCols; ++c) {
+            float *t = total + c * 32 * kEpilogueWarps;
+            *t = kt < kLevel ? h[c] : *t + h[c];
+          }
+        }
       }
       if (!ok) break;
+      // the other pairs, the smaller first; a sum that is not finite is the
+      // first pieces' alone (zero times infinity in the others)
+#pragma unroll
+      for (int s = 0; s < kCols; s += kHalf) {
+        float v[kHalf], u[kHalf];
+        tmemLoad16(taddr + kTile * 3 + s, u);
+        tmemLoad16(taddr + kTile * 2 + s, v);
+#pragma unroll
+        for (int c = 0; c < kHalf; ++c) {
+          const float t = total[(s + c) * 32 * kEpilogueWarps];
+          h[s + c] = fabsf(t) <= 3.402823466e38f ? t + (v[c] + u[c]) : t;
+        }
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;");
+      mbarArrive(smemAddr(rest_empty));
       float *C = args.c + args.offset[mi];
       uint32_t largest = 0;  // of column j0 + lane
 #pragma unroll
@@ -462,7 +493,7 @@ struct Source {
   bool transpose;
 };
 
-// The digits of up to three matrices, in one launch (two with `find`: their
+// The pieces of up to three matrices, in one launch (two with `find`: their
 // largest magnitudes first; else a product has left them).  V, V^T and R of a
 // correction of four matrices of order 1000: about 30 us, 62 in six launches.
 int sliceOperands(msq_ctx *ctx, const DeviceBatch *b, const SlicedPlan &p,
@@ -489,8 +520,8 @@ int sliceOperands(msq_ctx *ctx, const DeviceBatch *b, const SlicedPlan &p,
     MSQ_TRY(launched(ctx, "sliced largest"));
   }
   const dim3 grid(std::min(p.pack_items, kSmCount * 8), 1, count);
-  digitKernel<<<grid, 256, 0, ctx->stream>>>(s);
-  return launched(ctx, "sliced digits");
+  piecesKernel<<<grid, 256, 0, ctx->stream>>>(s);
+  return launched(ctx, "sliced pieces");
 }
 
 template <int kEpi>
@@ -526,16 +557,16 @@ int slicedGemm(msq_ctx *ctx, const DeviceBatch *b, const SlicedPlan &p, const Op
 
 // Orders from which a matrix's products may be sliced, and the sum of n^3 of
 // such matrices from which they are.  A tile of 128 is mostly padding below
-// order 256 (a correction of 1000 matrices of order 128: 708 us against 550
-// with FMA chains; 100 of order 200: 333 against 328), and slicing adds six
-// launches, which little work does not pay for (eight of order 384: 158 us
-// against 145; 20 of order 300: 236 against 200; 38 of order 256, 0.64e9: 172
-// against 166; but two of order 700, 0.69e9: 207 against 235; 16 of order 384:
-// 185 against 227; 64 of order 256: 251 against 286; four of order 1000: 445
-// against 821; 2048: 719 against 1584).
+// order 256, and slicing adds six launches, which little work does not pay for.
+// Corrections and reconstructions, us, sliced against FMA chains: one of order
+// 512, 0.13e9, 127 and 82, 33 and 15; one of 640, 0.26e9, 141 and 120, 35 and 23;
+// one of 768, 0.45e9, 152 and 158, 39 and 27; 32 of 256, 0.54e9, 145 and 148, 31
+// and 32; one of 900, 0.73e9, 187 and 262, 46 and 40; 16 of 384, 0.9e9, 160 and
+// 208, 34 and 46; one of 1300 242 and 578, 58 and 146; 152 of 512 1934 and 3640,
+// 317 and 507.
 constexpr int kSlicedOrder = 256;
 constexpr double kSlicedWork = 0.65e9;
-// The digits of four operands stay below this.
+// The pieces of four operands stay below this.
 constexpr int64_t kSlicedBytes = int64_t{16} << 30;
 
 }  // namespace

@@ -407,9 +407,8 @@ int enqueuePass(msq_ctx *ctx, const float *a_user, const int32_t *n_user,
     MSQ_TRY(reconstructFromFactor(ctx, sb, g.plan.format, pb->F, pb->Xh));
     // Corrections use the FP32 stable basis V, as the reference's fp32_frozen
     // stage does (src/metal_solver.cpp:304-325).  The plain FP32 plan runs its
-    // GEMMs on the CUDA cores in FP32; low-bit plans run the correction GEMMs
-    // on the tensor cores (split BF16, FP32 accumulation).  Every residual is
-    // float-float.
+    // GEMMs in FP32; low-bit plans run the correction GEMMs on the tensor
+    // cores (split BF16, FP32 accumulation).  Every residual is float-float.
     const int gemm_format = g.plan.format != MSQ_PLAN_FP32 ? MSQ_FMT_BF16 : MSQ_FMT_FP32;
     auto residual = [&]() {
       return residualFF(ctx, sb, pb->A, pb->Xh, pb->Xl, pb->R, norms);
