@@ -64,8 +64,8 @@ struct FloatSum {
 // |a_ji| and a_ji^2 over j != i.  A warp per column, lanes down the column:
 // coalesced, bound by the latency of a few loads per column and, at large
 // orders, by memory.  A thread per column read with a stride of n and summed
-// in FP64; features of 256 matrices of orders 64 .. 512: 417 us, 53 so; of
-// one matrix of order 1024: 1067 and 35; of 4096 of order 64: 275 and 129.
+// in FP64; features of 256 matrices of orders 64 .. 512: 498 us, 85 so; of
+// one matrix of order 1024: 1068 and 39; of 4096 of order 64: 274 and 129.
 //
 // The sums stay float-float (FP64 conversions and comparisons of every column
 // took 30 of 55 us); one whose squares leave FP32's range, or that is not
@@ -143,8 +143,11 @@ __global__ void __launch_bounds__(256) columnStatsKernel(const float *__restrict
 // 12 std diag / mean diag                     13 fraction of rows diagonally dominant
 // 14 log10 tolerance (filled by the caller; 0 here)   15 bias term 1
 // Lane k forms feature k, so the FP64 logarithms (and square roots) of a
-// matrix are one instruction stream; the sums before it are float-float, FP64
-// where a diagonal or a column leaves FP32's range.
+// matrix are one instruction stream.  The sums before it: FP64 of the diagonal,
+// whose deviation is a difference of nearly equal sums (feature 12, and 11 of a
+// nearly constant diagonal); float-float of the columns, each again in FP64
+// where it nearly cancels the diagonal entry (6, 13); all in FP64 where a
+// diagonal or a column leaves FP32's range.
 struct DiagonalSums {
   double tr, d2, offm, offabs, dmin, dmax, glo, ghi, rowmax;
   int dominant;
@@ -158,10 +161,23 @@ __device__ __forceinline__ FloatSum shuffled(const FloatSum &v, int s) {
   return {__shfl_xor_sync(0xffffffffu, v.s, s), __shfl_xor_sync(0xffffffffu, v.c, s)};
 }
 
+// d_i less the sum of |a_ji|, j != i, in FP64 (one thread).
+__device__ FloatSum gershgorinLow(const float *A, int n, int i) {
+  const float *col = A + static_cast<int64_t>(i) * n;
+  double sum = 0.0;
+  for (int j = 0; j < n; ++j) sum += j == i ? 0.0 : fabs(static_cast<double>(col[j]));
+  const double low = static_cast<double>(col[i]) - sum;
+  FloatSum r;
+  r.s = static_cast<float>(low);
+  r.c = static_cast<float>(low - static_cast<double>(r.s));
+  return r;
+}
+
 // False, with nothing written, if the FP64 sums are needed.
 __device__ bool diagonalSumsFloat(const float *A, const ColumnStat *col, int n, int lane,
                                   DiagonalSums &out) {
-  FloatSum tr, d2, offm, offabs, glo, ghi, rowmax;
+  FloatSum offm, offabs, glo, ghi, rowmax;
+  double tr = 0.0, d2 = 0.0;
   glo.s = 3.402823466e38f;
   ghi.s = -3.402823466e38f;
   float dmin = 3.402823466e38f, dmax = -3.402823466e38f;
@@ -173,8 +189,9 @@ __device__ bool diagonalSumsFloat(const float *A, const ColumnStat *col, int n, 
     // squares whose sum over any order stays within FP32's range
     plain = plain && sq.s >= 0.0f && sq.s <= 1e33f &&
             ((fabsf(d) >= 1e-10f && fabsf(d) <= 3e16f) || d == 0.0f);
-    tr.add(d);
-    d2.square(d);
+    const double dd = d;
+    tr += dd;
+    d2 = fma(dd, dd, d2);
     offm.add(sq);
     offabs.add(rs);
     dmin = fminf(dmin, d);
@@ -183,6 +200,8 @@ __device__ bool diagonalSumsFloat(const float *A, const ColumnStat *col, int n, 
     lo.add(d);
     lo.add(-rs.s, -rs.c);
     lo.normalise();
+    // a column's sum is good to 2^-41 of it (order 16384)
+    if (fabsf(lo.s) < 6.1035156e-5f * fabsf(d) && !(lo.s == 0.0f && rs.c == 0.0f)) lo = gershgorinLow(A, n, i);
     hi.add(d);
     hi.add(rs);
     hi.normalise();
@@ -192,12 +211,12 @@ __device__ bool diagonalSumsFloat(const float *A, const ColumnStat *col, int n, 
     dominant += lo.s > 0.0f;
   }
   if (!__all_sync(0xffffffffu, plain)) return false;
-  tr.warp();
-  d2.warp();
   offm.warp();
   offabs.warp();
 #pragma unroll
   for (int s = 16; s; s >>= 1) {
+    tr += __shfl_xor_sync(0xffffffffu, tr, s);
+    d2 += __shfl_xor_sync(0xffffffffu, d2, s);
     dmin = fminf(dmin, __shfl_xor_sync(0xffffffffu, dmin, s));
     dmax = fmaxf(dmax, __shfl_xor_sync(0xffffffffu, dmax, s));
     const FloatSum a = shuffled(glo, s), b = shuffled(ghi, s), c = shuffled(rowmax, s);
@@ -206,7 +225,7 @@ __device__ bool diagonalSumsFloat(const float *A, const ColumnStat *col, int n, 
     if (lessThan(rowmax, c)) rowmax = c;
     dominant += __shfl_xor_sync(0xffffffffu, dominant, s);
   }
-  out = {tr.value(), d2.value(), offm.value(), offabs.value(), dmin, dmax,
+  out = {tr, d2, offm.value(), offabs.value(), dmin, dmax,
          glo.value(), ghi.value(), rowmax.value(), dominant};
   return true;
 }
@@ -370,7 +389,8 @@ __global__ void __launch_bounds__(kMlpThreads) mlpForwardKernel(const float *__r
 // the BF16 rounding as a straight-through identity).  A CTA keeps its rows'
 // sums of the gradient in registers, every thread a fixed set of parameters,
 // and adds them once at the end; at most kGradCtas, so that the additions
-// into the one gradient do not dominate.  loss gets the mean loss.
+// into the one gradient do not dominate.  loss gets the mean loss: summed in
+// float-float by the threads, in FP64 over a CTA, one addition each.
 constexpr int kGradCtas = 64;
 __global__ void __launch_bounds__(kMlpThreads) mlpBackwardKernel(const float *__restrict__ p,
                                                                  const float *__restrict__ x,
@@ -383,7 +403,8 @@ __global__ void __launch_bounds__(kMlpThreads) mlpBackwardKernel(const float *__
   // this thread's parameters: column t of kHid / kRows rows of W2, and of
   // kOut / kRows rows of W3, 4 elements of W1
   constexpr int k2 = kHid / kRows, k3 = kOut / kRows, k1 = kHid * kIn / kMlpThreads;
-  float g1[k1] = {}, g2[k2] = {}, g3[k3] = {}, gb1 = 0.0f, gb2 = 0.0f, gb3 = 0.0f, lsum = 0.0f;
+  float g1[k1] = {}, g2[k2] = {}, g3[k3] = {}, gb1 = 0.0f, gb2 = 0.0f, gb3 = 0.0f;
+  FloatSum lsum;
   const float inv = 1.0f / (static_cast<float>(rows) * kOut);
   mlpLoad(p, m);
   for (int first = blockIdx.x * kRows; first < rows; first += gridDim.x * kRows) {
@@ -394,7 +415,7 @@ __global__ void __launch_bounds__(kMlpThreads) mlpBackwardKernel(const float *__
         const float zz = m.z[r][t], yy = y[static_cast<int64_t>(first + r) * kOut + t];
         const float sig = 1.0f / (1.0f + expf(-zz));
         d = (sig - yy) * inv;
-        lsum += (fmaxf(zz, 0.0f) + log1pf(expf(-fabsf(zz))) - yy * zz) * inv;
+        lsum.add(fmaxf(zz, 0.0f) + log1pf(expf(-fabsf(zz))) - yy * zz);
       }
       dz[r][t] = d;  // rows beyond the last contribute nothing
     }
@@ -438,7 +459,14 @@ __global__ void __launch_bounds__(kMlpThreads) mlpBackwardKernel(const float *__
     atomicAdd(&grad[kB2 + t], gb2);
     if (t < kOut) atomicAdd(&grad[kB3 + t], gb3);
   }
-  if (t < kOut) atomicAdd(loss, lsum);
+  __shared__ double sums[kRows * kOut];
+  if (t < kOut) sums[r * kOut + t] = lsum.value();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double sum = 0.0;
+    for (int i = 0; i < kRows * kOut; ++i) sum += sums[i];
+    atomicAdd(loss, static_cast<float>(sum / (static_cast<double>(rows) * kOut)));
+  }
 }
 
 // Adam (beta1 0.9, beta2 0.999, eps 1e-8) on the FP32 masters.
