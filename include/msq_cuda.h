@@ -96,6 +96,11 @@ int msq_synchronize(msq_ctx *ctx);
  * keep their setting: turn graphs off (msq_set_graphs) around such a test.
  * No counterpart in the reference (its Metal waits are host-side).        */
 int msq_debug_expire_waits(int mode);
+/* The same for workspaces (process-wide, default 0: off): those that a call
+ * can do without are refused above `bytes`, as when the device has no memory
+ * left for them.  The call then takes its path without one (a residual's
+ * digits: the CUDA-core kernel).                                           */
+int msq_debug_scratch_limit(size_t bytes);
 /* Number of this library's kernel launches enqueued so far on `ctx` (a
  * replayed graph counts the launches it holds). */
 uint64_t msq_launch_count(const msq_ctx *ctx);

@@ -74,6 +74,7 @@ _SIGS = {
     "msq_set_stream": (ctypes.c_int, [_P, _P]),
     "msq_synchronize": (ctypes.c_int, [_P]),
     "msq_debug_expire_waits": (ctypes.c_int, [ctypes.c_int]),
+    "msq_debug_scratch_limit": (ctypes.c_int, [ctypes.c_size_t]),
     "msq_launch_count": (ctypes.c_uint64, [_P]),
     "msq_graph_launch_count": (ctypes.c_uint64, [_P]),
     "msq_fma_rate": (ctypes.c_int, [_P, _P]),

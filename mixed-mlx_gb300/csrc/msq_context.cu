@@ -111,6 +111,7 @@ int streamWait(msq_ctx *ctx, cudaStream_t waiter, cudaStream_t source) {
 
 namespace {
 std::atomic<int> g_wait_test{0};
+std::atomic<size_t> g_scratch_limit{0};
 }  // namespace
 
 int waitTestMode() { return g_wait_test.load(std::memory_order_relaxed); }
@@ -146,23 +147,19 @@ static uint64_t hashLayout(const int32_t *n, const int64_t *offset, int count) {
   return h;
 }
 
-const DeviceBatch *prepareBatch(msq_ctx *ctx, const int32_t *n,
-                                const int64_t *offset, int count) {
-  if (count <= 0 || n == nullptr || offset == nullptr) {
-    setError(ctx, MSQ_ERR_INVALID_ARGUMENT, "batch: empty or null layout");
-    return nullptr;
-  }
-  const uint64_t key = hashLayout(n, offset, count);
-  for (DeviceBatch *b : ctx->batches) {
-    if (b->key == key && b->count == count &&
-        std::memcmp(b->host_n.data(), n, count * sizeof(int32_t)) == 0 &&
-        std::memcmp(b->host_offset.data(), offset, count * sizeof(int64_t)) == 0) {
-      return b;
-    }
-  }
+static void freeBatch(DeviceBatch *b) {
+  for (auto &r : b->runs)
+    for (DeviceBatch *run : r.second) freeBatch(run);
+  for (auto &w : b->work_cache) cudaFree(w.work);
+  cudaFree(b->offset);
+  delete b;
+}
+
+// A layout with its device copies; null on error (ctx->error set).
+static DeviceBatch *uploadBatch(msq_ctx *ctx, const int32_t *n, const int64_t *offset, int count) {
   auto *b = new DeviceBatch;
   b->count = count;
-  b->key = key;
+  b->key = hashLayout(n, offset, count);
   b->host_n.assign(n, n + count);
   b->host_offset.assign(offset, offset + count);
   b->host_eig_offset.resize(count);
@@ -196,16 +193,75 @@ const DeviceBatch *prepareBatch(msq_ctx *ctx, const int32_t *n,
     delete b;
     return nullptr;
   }
+  return b;
+}
+
+const DeviceBatch *prepareBatch(msq_ctx *ctx, const int32_t *n,
+                                const int64_t *offset, int count) {
+  if (count <= 0 || n == nullptr || offset == nullptr) {
+    setError(ctx, MSQ_ERR_INVALID_ARGUMENT, "batch: empty or null layout");
+    return nullptr;
+  }
+  const uint64_t key = hashLayout(n, offset, count);
+  for (DeviceBatch *b : ctx->batches) {
+    if (b->key == key && b->count == count &&
+        std::memcmp(b->host_n.data(), n, count * sizeof(int32_t)) == 0 &&
+        std::memcmp(b->host_offset.data(), offset, count * sizeof(int64_t)) == 0) {
+      return b;
+    }
+  }
+  DeviceBatch *b = uploadBatch(ctx, n, offset, count);
+  if (b == nullptr) return nullptr;
   if (ctx->batches.size() >= 32) {
-    DeviceBatch *old = ctx->batches.front();
-    for (auto &w : old->work_cache) cudaFree(w.work);
-    cudaFree(old->offset);
-    delete old;
+    freeBatch(ctx->batches.front());
     ctx->batches.erase(ctx->batches.begin());
     ++ctx->alloc_generation;
   }
   ctx->batches.push_back(b);
   return b;
+}
+
+int batchRuns(msq_ctx *ctx, const DeviceBatch *b, int key, int64_t limit, int64_t (*bytes)(int order),
+              std::vector<BatchRun> *out) {
+  out->clear();
+  const std::vector<DeviceBatch *> *kept = nullptr;
+  for (const auto &r : b->runs)
+    if (r.first == key) kept = &r.second;
+  if (kept == nullptr) {
+    std::vector<int> starts;
+    int64_t sum = 0;
+    for (int i = 0; i < b->count; ++i) {
+      const int64_t mine = bytes(b->host_n[i]);
+      if (i == 0 || (mine > 0 && sum > 0 && sum + mine > limit)) {
+        starts.push_back(i);
+        sum = 0;
+      }
+      sum += mine;
+    }
+    std::vector<DeviceBatch *> runs;
+    if (starts.size() > 1) {
+      for (size_t k = 0; k < starts.size(); ++k) {
+        const int end = k + 1 < starts.size() ? starts[k + 1] : b->count;
+        DeviceBatch *run = uploadBatch(ctx, b->host_n.data() + starts[k], b->host_offset.data() + starts[k],
+                                       end - starts[k]);
+        if (run == nullptr) {
+          for (DeviceBatch *r : runs) freeBatch(r);
+          return MSQ_ERR_CUDA;
+        }
+        runs.push_back(run);
+      }
+    }
+    auto &cache = const_cast<DeviceBatch *>(b)->runs;
+    cache.push_back({key, std::move(runs)});
+    kept = &cache.back().second;
+  }
+  if (kept->empty()) out->push_back({b, 0});
+  int first = 0;
+  for (const DeviceBatch *run : *kept) {
+    out->push_back({run, first});
+    first += run->count;
+  }
+  return MSQ_OK;
 }
 
 bool findWork(const DeviceBatch *b, int key, const int4 **work, int *items) {
@@ -263,9 +319,9 @@ void scratchRecord(msq_ctx *ctx) {
   ctx->scratch_recorded = cudaEventRecord(ctx->scratch_event, ctx->stream) == cudaSuccess;
 }
 
-void *scratch(msq_ctx *ctx, size_t bytes, int slot) {
-  if (scratchOrder(ctx) != MSQ_OK) return nullptr;
-  if (bytes <= ctx->scratch_bytes[slot]) return ctx->scratch[slot];
+// The arena of `slot` with room for `bytes`, or the error of its allocation.
+static cudaError_t growScratch(msq_ctx *ctx, size_t bytes, int slot) {
+  if (bytes <= ctx->scratch_bytes[slot]) return cudaSuccess;
   if (ctx->scratch[slot] != nullptr) {
     cudaStreamSynchronize(ctx->stream);
     cudaFree(ctx->scratch[slot]);
@@ -274,11 +330,29 @@ void *scratch(msq_ctx *ctx, size_t bytes, int slot) {
     ++ctx->alloc_generation;
   }
   const size_t rounded = (bytes + (1u << 20) - 1) & ~static_cast<size_t>((1u << 20) - 1);
-  if (cudaCheck(ctx, cudaMalloc(&ctx->scratch[slot], rounded), "scratch alloc") != MSQ_OK) {
+  const cudaError_t status = cudaMalloc(&ctx->scratch[slot], rounded);
+  if (status != cudaSuccess) {
     ctx->scratch[slot] = nullptr;
-    return nullptr;
+    return status;
   }
   ctx->scratch_bytes[slot] = rounded;
+  return cudaSuccess;
+}
+
+void *scratch(msq_ctx *ctx, size_t bytes, int slot) {
+  if (scratchOrder(ctx) != MSQ_OK) return nullptr;
+  if (cudaCheck(ctx, growScratch(ctx, bytes, slot), "scratch alloc") != MSQ_OK) return nullptr;
+  return ctx->scratch[slot];
+}
+
+void *tryScratch(msq_ctx *ctx, size_t bytes, int slot) {
+  const size_t limit = g_scratch_limit.load(std::memory_order_relaxed);
+  if (limit != 0 && bytes > limit) return nullptr;
+  if (scratchOrder(ctx) != MSQ_OK) return nullptr;
+  if (bytes > ctx->scratch_bytes[slot] && captured(ctx)) return nullptr;
+  const cudaError_t status = growScratch(ctx, bytes, slot);
+  if (status == cudaErrorMemoryAllocation) cudaGetLastError();  // not an error of the call
+  else if (cudaCheck(ctx, status, "scratch alloc") != MSQ_OK) return nullptr;
   return ctx->scratch[slot];
 }
 
@@ -326,11 +400,7 @@ extern "C" void msq_destroy(msq_ctx *ctx) {
   cudaSetDevice(ctx->device);
   if (ctx->stream != nullptr) cudaStreamSynchronize(ctx->stream);
   else cudaDeviceSynchronize();
-  for (DeviceBatch *b : ctx->batches) {
-    for (auto &w : b->work_cache) cudaFree(w.work);
-    cudaFree(b->offset);
-    delete b;
-  }
+  for (DeviceBatch *b : ctx->batches) freeBatch(b);
   for (int slot = 0; slot < msq::kScratchSlots; ++slot)
     if (ctx->scratch[slot] != nullptr) cudaFree(ctx->scratch[slot]);
   for (auto &g : ctx->jacobi_graphs) cudaGraphExecDestroy(g.exec);
@@ -375,6 +445,11 @@ extern "C" int msq_set_graphs(msq_ctx *ctx, int enable) {
 extern "C" int msq_debug_expire_waits(int mode) {
   if (mode < msq::kWaitTestOff || mode > msq::kWaitTestMbarrier) return MSQ_ERR_INVALID_ARGUMENT;
   msq::g_wait_test.store(mode, std::memory_order_relaxed);
+  return MSQ_OK;
+}
+
+extern "C" int msq_debug_scratch_limit(size_t bytes) {
+  msq::g_scratch_limit.store(bytes, std::memory_order_relaxed);
   return MSQ_OK;
 }
 

@@ -636,25 +636,38 @@ int gemmTN(msq_ctx *ctx, const DeviceBatch *b, const float *a, const float *bm, 
 
 int residualFF(msq_ctx *ctx, const DeviceBatch *b, const float *a, const float *x_hi,
                const float *x_lo, float *r, double *norms, const float *a_lo) {
-  ResidualArgs args{};
-  // upper tiles of the small matrices; the others on the tensor cores
-  MSQ_TRY(tileWork(ctx, b, kTile, true, kResidualWork, &args.work, &args.items,
-                   [](int n) { return !residualOnTensorCores(n); }));
-  args.a = a;
-  args.a_lo = a_lo;
-  args.x_hi = x_hi;
-  args.x_lo = x_lo;
-  args.r = r;
-  args.norms = norms;
-  args.offset = b->offset;
-  args.n = b->n;
   MSQ_TRY(cudaCheck(ctx, cudaMemsetAsync(norms, 0, 2 * b->count * sizeof(double), ctx->stream),
                     "norm reset"));
-  MSQ_TRY(residualMma(ctx, b, a, x_hi, x_lo, r, norms, a_lo));
-  if (args.items == 0) return MSQ_OK;
-  const unsigned grid = std::min<unsigned>(args.items, kSmCount * 8);
-  residualFFKernel<false><<<grid, kThreads, 0, ctx->stream>>>(args);
-  return launched(ctx, "residual float-float");
+  // the upper tiles of the matrices of `part` that `in` accepts
+  auto cudaCores = [&](const DeviceBatch *part, int key, double *part_norms, auto in) {
+    ResidualArgs args{};
+    MSQ_TRY(tileWork(ctx, part, kTile, true, key, &args.work, &args.items, in));
+    if (args.items == 0) return static_cast<int>(MSQ_OK);
+    args.a = a;
+    args.a_lo = a_lo;
+    args.x_hi = x_hi;
+    args.x_lo = x_lo;
+    args.r = r;
+    args.norms = part_norms;
+    args.offset = part->offset;
+    args.n = part->n;
+    const unsigned grid = std::min<unsigned>(args.items, kSmCount * 8);
+    residualFFKernel<false><<<grid, kThreads, 0, ctx->stream>>>(args);
+    return launched(ctx, "residual float-float");
+  };
+  // the larger matrices on the tensor cores, as many at a time as kResidualDigits
+  // holds; on the CUDA cores where there is no memory for their digits
+  std::vector<BatchRun> runs;
+  MSQ_TRY(batchRuns(ctx, b, kResidualWork, kResidualDigits, residualDigitBytes, &runs));
+  for (const BatchRun &run : runs) {
+    const int status = residualMma(ctx, run.b, a, x_hi, x_lo, r, norms + 2 * run.first, a_lo);
+    if (status == kNoScratch) {
+      MSQ_TRY(cudaCores(run.b, kResidualWork + 1, norms + 2 * run.first, residualOnTensorCores));
+    } else {
+      MSQ_TRY(status);
+    }
+  }
+  return cudaCores(b, kResidualWork, norms, [](int n) { return !residualOnTensorCores(n); });
 }
 
 int makeFactor(msq_ctx *ctx, const DeviceBatch *b, const float *v, const float *lam, float *f) {

@@ -6,6 +6,7 @@
 #include <cstddef>
 #include <cstdint>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/msq_cuda.h"
@@ -58,6 +59,8 @@ struct DeviceBatch {
   std::vector<int64_t> host_offset;
   std::vector<int64_t> host_eig_offset;
   std::vector<WorkList> work_cache;  // tile work lists (msq_dense.cu)
+  // runs of the batch's matrices as batches of their own, by key (batchRuns)
+  std::vector<std::pair<int, std::vector<DeviceBatch *>>> runs;
 };
 
 // The context's cached Jacobi launch plans (msq_jacobi.cu) and tcgen05 tile
@@ -199,6 +202,9 @@ enum ScratchSlot : int {
   kScratchFallback = 5, kScratchResidual = 6, kScratchSlots = 7
 };
 void *scratch(msq_ctx *ctx, size_t bytes, int slot);
+// The same for a user that can do without: nullptr, with no error, where the
+// device has no memory for it (or while a stream is captured).
+void *tryScratch(msq_ctx *ctx, size_t bytes, int slot);
 // Orders the context's stream behind the last call that used an arena, on
 // whatever stream (scratch does this; so must a call that replays a graph).
 int scratchOrder(msq_ctx *ctx);
@@ -209,6 +215,16 @@ void scratchRecord(msq_ctx *ctx);
 bool findWork(const DeviceBatch *b, int key, const int4 **work, int *items);
 int keepWork(msq_ctx *ctx, const DeviceBatch *b, int key, const std::vector<int4> &list,
              const int4 **work, int *items);
+// Consecutive runs of the batch's matrices whose bytes(order) add up to at most
+// `limit`, a matrix above it in a run of its own, so that an arena serves one
+// run after another.  Each has the batch's offsets; first: its first matrix.
+// One run is the batch itself.  Kept on the batch under `key`.
+struct BatchRun {
+  const DeviceBatch *b;
+  int first;
+};
+int batchRuns(msq_ctx *ctx, const DeviceBatch *b, int key, int64_t limit, int64_t (*bytes)(int order),
+              std::vector<BatchRun> *out);
 // Grow-only pinned host staging (for reports copied back inside a graph).
 void *pinnedScratch(msq_ctx *ctx, size_t bytes);
 

@@ -532,6 +532,11 @@ int residualWork(msq_ctx *ctx, const DeviceBatch *b, const int4 **rows, int *row
 
 bool residualOnTensorCores(int n) { return n >= kResidualMmaOrder; }
 
+int64_t residualDigitBytes(int n) {
+  if (!residualOnTensorCores(n)) return 0;
+  return int64_t{(n + kTileM - 1) / kTileM} * ((n + kTileK - 1) / kTileK) * kTileBytes;
+}
+
 int residualMma(msq_ctx *ctx, const DeviceBatch *b, const float *a, const float *x_hi,
                 const float *x_lo, float *r, double *norms, const float *a_lo) {
   const int4 *rows = nullptr, *pack = nullptr, *gemm = nullptr, *bases = nullptr;
@@ -541,9 +546,9 @@ int residualMma(msq_ctx *ctx, const DeviceBatch *b, const float *a, const float 
   if (row_items == 0) return MSQ_OK;
   const int64_t *tile_base = reinterpret_cast<const int64_t *>(bases);
   const size_t exp_bytes = (b->total_order * sizeof(int32_t) + 255) & ~size_t(255);
-  uint8_t *mem = static_cast<uint8_t *>(scratch(ctx, exp_bytes + 1024 + static_cast<size_t>(pack_items) * kTileBytes,
-                                                  kScratchResidual));
-  if (mem == nullptr) return MSQ_ERR_CUDA;
+  uint8_t *mem = static_cast<uint8_t *>(
+      tryScratch(ctx, exp_bytes + 1024 + static_cast<size_t>(pack_items) * kTileBytes, kScratchResidual));
+  if (mem == nullptr) return kNoScratch;
   static std::atomic<uint64_t> done_mask{0};
   const uint64_t bit = ctx->device >= 0 && ctx->device < 64 ? uint64_t{1} << ctx->device : 0;
   if (bit == 0 || !(done_mask.load() & bit)) {

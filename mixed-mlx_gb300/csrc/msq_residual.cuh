@@ -11,9 +11,16 @@ namespace msq {
 // one tile each, and a 128 x 64 tile would be half padding).
 constexpr int kResidualMmaOrder = 65;
 bool residualOnTensorCores(int n);
+// Bytes of a matrix's digits, and how many of them are kept at a time: a batch
+// with more runs in several passes over one arena (152 of
+// order 512 have 0.64 GB; three more launches per pass).
+int64_t residualDigitBytes(int n);
+constexpr int64_t kResidualDigits = int64_t{2} << 30;
 // R = (a + a_lo) - X^T X, X = x_hi + x_lo (x_lo, a_lo and r may be null), and
 // ||R||^2, ||A||^2 added to `norms` (2 per matrix), for the matrices of the
-// batch whose order residualOnTensorCores accepts.
+// batch whose order residualOnTensorCores accepts.  kNoScratch: nothing done,
+// there is no memory for the digits.
+constexpr int kNoScratch = -1;
 int residualMma(msq_ctx *ctx, const DeviceBatch *b, const float *a, const float *x_hi,
                 const float *x_lo, float *r, double *norms, const float *a_lo);
 
