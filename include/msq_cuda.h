@@ -99,7 +99,8 @@ int msq_debug_expire_waits(int mode);
 /* The same for workspaces (process-wide, default 0: off): those that a call
  * can do without are refused above `bytes`, as when the device has no memory
  * left for them.  The call then takes its path without one (a residual's
- * digits: the CUDA-core kernel).                                           */
+ * digits and the pieces of FP32 products: the CUDA-core kernels; the split
+ * operands of a BF16 correction: fewer buffers).                           */
 int msq_debug_scratch_limit(size_t bytes);
 /* Number of this library's kernel launches enqueued so far on `ctx` (a
  * replayed graph counts the launches it holds). */

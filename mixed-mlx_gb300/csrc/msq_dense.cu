@@ -578,19 +578,21 @@ int gemmClass(const DeviceBatch *b, int n) {
 }
 
 // The tiles (matrix, i, j) of every matrix of one tile class, cached on the
-// batch; `upper`: only those on or above the diagonal; `unsliced`: of the
-// matrices that slicedMatrix refuses.
-int gemmTiles(msq_ctx *ctx, const DeviceBatch *b, int tile, bool upper, bool unsliced,
+// batch; `upper`: only those on or above the diagonal.
+int gemmTiles(msq_ctx *ctx, const DeviceBatch *b, int tile, bool upper, GemmPart part,
               const int4 **work, int *items) {
-  return tileWork(ctx, b, tile, upper, kGemmWorkBase + (upper ? 1 : 0) + 2 * tile + (unsliced ? 1024 : 0),
-                  work, items, [&](int n) { return gemmClass(b, n) == tile && !(unsliced && slicedMatrix(n)); });
+  return tileWork(ctx, b, tile, upper, kGemmWorkBase + (upper ? 1 : 0) + 2 * tile + 1024 * static_cast<int>(part),
+                  work, items, [&](int n) {
+                    return gemmClass(b, n) == tile &&
+                           (part == GemmPart::kAll || slicedMatrix(n) == (part == GemmPart::kSliced));
+                  });
 }
 
 template <int kT, bool kMajorA, bool kMajorB>
 int launchGemm(msq_ctx *ctx, const DeviceBatch *b, GemmArgs args, int epilogue, bool mirror,
-               bool unsliced) {
+               GemmPart part) {
   using S = GemmShape<kT>;
-  MSQ_TRY(gemmTiles(ctx, b, kT, mirror, unsliced, &args.work, &args.items));
+  MSQ_TRY(gemmTiles(ctx, b, kT, mirror, part, &args.work, &args.items));
   if (args.items == 0) return MSQ_OK;
   const unsigned grid = std::min<unsigned>(args.items, kSmCount * S::kCtas * 4);
   if (mirror) {
@@ -605,16 +607,16 @@ int launchGemm(msq_ctx *ctx, const DeviceBatch *b, GemmArgs args, int epilogue, 
 
 template <bool kMajorA, bool kMajorB>
 int launchGemmClasses(msq_ctx *ctx, const DeviceBatch *b, const GemmArgs &args, int epilogue,
-                      bool mirror, bool unsliced) {
-  MSQ_TRY((launchGemm<128, kMajorA, kMajorB>(ctx, b, args, epilogue, mirror, unsliced)));
-  MSQ_TRY((launchGemm<64, kMajorA, kMajorB>(ctx, b, args, epilogue, mirror, unsliced)));
-  return launchGemm<32, kMajorA, kMajorB>(ctx, b, args, epilogue, mirror, unsliced);
+                      bool mirror, GemmPart part) {
+  MSQ_TRY((launchGemm<128, kMajorA, kMajorB>(ctx, b, args, epilogue, mirror, part)));
+  MSQ_TRY((launchGemm<64, kMajorA, kMajorB>(ctx, b, args, epilogue, mirror, part)));
+  return launchGemm<32, kMajorA, kMajorB>(ctx, b, args, epilogue, mirror, part);
 }
 
 }  // namespace
 
 int gemmTN(msq_ctx *ctx, const DeviceBatch *b, const float *a, const float *bm, float *c,
-           int epilogue, const float *eigenvalues, bool a_mmajor, bool b_nmajor, bool unsliced) {
+           int epilogue, const float *eigenvalues, bool a_mmajor, bool b_nmajor, GemmPart part) {
   GemmArgs args{};
   args.a = a;
   args.b = bm;
@@ -628,10 +630,10 @@ int gemmTN(msq_ctx *ctx, const DeviceBatch *b, const float *a, const float *bm, 
   // one operand against itself in the same layout (F^T F or F F^T): symmetric
   const bool mirror = a == bm && a_mmajor == b_nmajor && epilogue == kEpilogueStore;
   if (a_mmajor)
-    return b_nmajor ? launchGemmClasses<true, true>(ctx, b, args, epilogue, mirror, unsliced)
-                    : launchGemmClasses<true, false>(ctx, b, args, epilogue, mirror, unsliced);
-  return b_nmajor ? launchGemmClasses<false, true>(ctx, b, args, epilogue, mirror, unsliced)
-                  : launchGemmClasses<false, false>(ctx, b, args, epilogue, mirror, unsliced);
+    return b_nmajor ? launchGemmClasses<true, true>(ctx, b, args, epilogue, mirror, part)
+                    : launchGemmClasses<true, false>(ctx, b, args, epilogue, mirror, part);
+  return b_nmajor ? launchGemmClasses<false, true>(ctx, b, args, epilogue, mirror, part)
+                  : launchGemmClasses<false, false>(ctx, b, args, epilogue, mirror, part);
 }
 
 int residualFF(msq_ctx *ctx, const DeviceBatch *b, const float *a, const float *x_hi,

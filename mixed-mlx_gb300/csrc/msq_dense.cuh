@@ -10,6 +10,10 @@ enum GemmEpilogue : int {
   kEpilogueInverseH = 1,  // C_ij / (sqrt(lambda_i) + sqrt(lambda_j))
 };
 
+// The matrices of a batch that a product is for: all, those that slicedMatrix
+// refuses, those that it accepts.
+enum class GemmPart : int { kAll = 0, kUnsliced = 1, kSliced = 2 };
+
 struct GemmArgs {
   const int4 *work;
   int items;
@@ -35,11 +39,10 @@ struct ResidualArgs {
 int gemmWork(msq_ctx *ctx, const DeviceBatch *b, int tile, const int4 **work, int *items);
 // C = A B per matrix, each element the FP32 FMA chain over k in order; by
 // default A(i,k) = a[k + i*n] and B(k,j) = bm[k + j*n] (C = a^T bm);
-// a_mmajor: A(i,k) = a[i + k*n]; b_nmajor: B(k,j) = bm[j + k*n]; unsliced:
-// only the matrices that slicedMatrix refuses.
+// a_mmajor: A(i,k) = a[i + k*n]; b_nmajor: B(k,j) = bm[j + k*n].
 int gemmTN(msq_ctx *ctx, const DeviceBatch *b, const float *a, const float *bm, float *c,
            int epilogue, const float *eigenvalues, bool a_mmajor = false,
-           bool b_nmajor = false, bool unsliced = false);
+           bool b_nmajor = false, GemmPart part = GemmPart::kAll);
 // R = (a + a_lo) - (x_hi + x_lo)^2 in float-float; a_lo and x_lo may be null.
 int residualFF(msq_ctx *ctx, const DeviceBatch *b, const float *a, const float *x_hi,
                const float *x_lo, float *r, double *norms, const float *a_lo = nullptr);

@@ -477,8 +477,8 @@ struct Operand {
 int slicedOperands(msq_ctx *ctx, const DeviceBatch *b, const SlicedPlan &p, int count, Operand *out) {
   const size_t largest = (count * b->total_order * sizeof(uint32_t) + 1023) & ~size_t(1023);
   const size_t slices = static_cast<size_t>(p.pack_items) * kTileBytes;
-  uint8_t *mem = static_cast<uint8_t *>(scratch(ctx, largest + 1024 + count * slices, kScratchGemm));
-  if (mem == nullptr) return MSQ_ERR_CUDA;
+  uint8_t *mem = static_cast<uint8_t *>(tryScratch(ctx, largest + 1024 + count * slices, kScratchGemm));
+  if (mem == nullptr) return kNoScratch;
   uint8_t *tiles = reinterpret_cast<uint8_t *>(
       (reinterpret_cast<uintptr_t>(mem) + largest + 1023) & ~static_cast<uintptr_t>(1023));
   for (int q = 0; q < count; ++q)
@@ -566,23 +566,22 @@ int slicedGemm(msq_ctx *ctx, const DeviceBatch *b, const SlicedPlan &p, const Op
 // 317 and 507.
 constexpr int kSlicedOrder = 256;
 constexpr double kSlicedWork = 0.65e9;
-// The pieces of four operands stay below this.
-constexpr int64_t kSlicedBytes = int64_t{16} << 30;
 
 }  // namespace
 
+bool slicedMatrix(int n) { return n >= kSlicedOrder; }
+
 bool slicedProducts(const DeviceBatch *b) {
   double work = 0.0;
-  int64_t tiles = 0;
-  for (const int32_t n : b->host_n) {
-    if (n < kSlicedOrder) continue;
-    work += static_cast<double>(n) * n * n;
-    tiles += static_cast<int64_t>((n + kTile - 1) / kTile) * ((n + kTileK - 1) / kTileK);
-  }
-  return work >= kSlicedWork && 4 * tiles * kTileBytes <= kSlicedBytes;
+  for (const int32_t n : b->host_n)
+    if (slicedMatrix(n)) work += static_cast<double>(n) * n * n;
+  return work >= kSlicedWork;
 }
 
-bool slicedMatrix(int n) { return n >= kSlicedOrder; }
+int64_t slicedBytes(int n) {
+  if (!slicedMatrix(n)) return 0;
+  return int64_t{4} * ((n + kTile - 1) / kTile) * ((n + kTileK - 1) / kTileK) * kTileBytes;
+}
 
 int slicedReconstruct(msq_ctx *ctx, const DeviceBatch *b, const float *f, float *x) {
   SlicedPlan p{};

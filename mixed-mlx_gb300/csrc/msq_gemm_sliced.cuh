@@ -10,7 +10,13 @@ namespace msq {
 // matrices, those that slicedMatrix accepts, run as sliced products.
 bool slicedProducts(const DeviceBatch *b);
 bool slicedMatrix(int n);
-// The functions below do those matrices only.  X = F^T F.
+// Bytes of the pieces of a matrix's four operands, and how many of them are kept
+// at a time: a batch with more runs in several passes over one arena (152 of
+// order 512 have 0.95 GB).
+int64_t slicedBytes(int n);
+constexpr int64_t kSlicedBytes = int64_t{2} << 30;
+// The functions below do those matrices only, and may return kNoScratch.
+// X = F^T F.
 int slicedReconstruct(msq_ctx *ctx, const DeviceBatch *b, const float *f, float *x);
 // E of one Sylvester sweep, G = R^T V, C = (V^T G) o H, E = V C V^T.
 // basis_packed: the pieces of V are still those of the previous call on the

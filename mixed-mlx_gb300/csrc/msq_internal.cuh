@@ -205,6 +205,9 @@ void *scratch(msq_ctx *ctx, size_t bytes, int slot);
 // The same for a user that can do without: nullptr, with no error, where the
 // device has no memory for it (or while a stream is captured).
 void *tryScratch(msq_ctx *ctx, size_t bytes, int slot);
+// Internal status of a stage that can be replaced: nothing done, no memory for
+// its workspace.
+constexpr int kNoScratch = -1;
 // Orders the context's stream behind the last call that used an arena, on
 // whatever stream (scratch does this; so must a call that replays a graph).
 int scratchOrder(msq_ctx *ctx);

@@ -18,9 +18,7 @@ int64_t residualDigitBytes(int n);
 constexpr int64_t kResidualDigits = int64_t{2} << 30;
 // R = (a + a_lo) - X^T X, X = x_hi + x_lo (x_lo, a_lo and r may be null), and
 // ||R||^2, ||A||^2 added to `norms` (2 per matrix), for the matrices of the
-// batch whose order residualOnTensorCores accepts.  kNoScratch: nothing done,
-// there is no memory for the digits.
-constexpr int kNoScratch = -1;
+// batch whose order residualOnTensorCores accepts.  May return kNoScratch.
 int residualMma(msq_ctx *ctx, const DeviceBatch *b, const float *a, const float *x_hi,
                 const float *x_lo, float *r, double *norms, const float *a_lo);
 

@@ -26,26 +26,56 @@ namespace {
 
 size_t alignUp(size_t bytes) { return (bytes + 255) & ~static_cast<size_t>(255); }
 
-// One Sylvester sweep on a batch in FP32 (sliced products of the larger
-// matrices where they pay, FMA chains on the CUDA cores of the others):
-//   G = R V, C = (V^T G) o H, Z = V C, E = Z V^T, X <- X + (E + E^T)/2.
+// E of one Sylvester sweep by FMA chains on the CUDA cores, of the matrices of
+// `part`: G = R V into ws, C = (V^T G) o H into e, Z = V C into ws, E = Z V^T.
+int sylvesterChains(msq_ctx *ctx, const DeviceBatch *b, const float *v, const float *lam,
+                    const float *r, float *ws, float *e, GemmPart part) {
+  MSQ_TRY(gemmTN(ctx, b, r, v, ws, kEpilogueStore, nullptr, false, false, part));
+  MSQ_TRY(gemmTN(ctx, b, v, ws, e, kEpilogueInverseH, lam, false, false, part));
+  MSQ_TRY(gemmTN(ctx, b, v, e, ws, kEpilogueStore, nullptr, true, false, part));
+  return gemmTN(ctx, b, ws, v, e, kEpilogueStore, nullptr, true, true, part);
+}
+
+// The larger matrices of a batch whose products are sliced, as many at a time
+// as kSlicedBytes holds: stage(run), or chains(run) where there is no memory
+// for it; then the others as chains.
+template <class Stage, class Chains>
+int slicedOrChains(msq_ctx *ctx, const DeviceBatch *b, Stage stage, Chains chains) {
+  constexpr int kRuns = 1 << 21;
+  if (!slicedProducts(b)) return chains(BatchRun{b, 0}, GemmPart::kAll);
+  std::vector<BatchRun> runs;
+  MSQ_TRY(batchRuns(ctx, b, kRuns, kSlicedBytes, slicedBytes, &runs));
+  for (const BatchRun &run : runs) {
+    const int status = stage(run, runs.size() == 1);
+    MSQ_TRY(status == kNoScratch ? chains(run, GemmPart::kSliced) : status);
+  }
+  return chains(BatchRun{b, 0}, GemmPart::kUnsliced);
+}
+
+// One Sylvester sweep on a batch in FP32, X <- X + (E + E^T)/2.
 int sylvesterFp32(msq_ctx *ctx, const DeviceBatch *b, const float *v, const float *lam,
                   const float *r, float *x_hi, float *x_lo, float *ws0, float *ws1,
                   bool basis_packed) {
-  const bool sliced = slicedProducts(b);
-  if (sliced) MSQ_TRY(slicedSylvester(ctx, b, v, lam, r, ws0, ws1, basis_packed));
-  MSQ_TRY(gemmTN(ctx, b, r, v, ws0, kEpilogueStore, nullptr, false, false, sliced));    // G = R V
-  MSQ_TRY(gemmTN(ctx, b, v, ws0, ws1, kEpilogueInverseH, lam, false, false, sliced));  // C = V^T G o H
-  MSQ_TRY(gemmTN(ctx, b, v, ws1, ws0, kEpilogueStore, nullptr, true, false, sliced));   // Z = V C
-  MSQ_TRY(gemmTN(ctx, b, ws0, v, ws1, kEpilogueStore, nullptr, true, true, sliced));    // E = Z V^T
+  auto roots = [&](const BatchRun &run) { return lam + b->host_eig_offset[run.first]; };
+  MSQ_TRY(slicedOrChains(
+      ctx, b,
+      [&](const BatchRun &run, bool alone) {
+        // another run's pieces take the place of V's
+        return slicedSylvester(ctx, run.b, v, roots(run), r, ws0, ws1, basis_packed && alone);
+      },
+      [&](const BatchRun &run, GemmPart part) {
+        return sylvesterChains(ctx, run.b, v, roots(run), r, ws0, ws1, part);
+      }));
   return symmetricAdd(ctx, b, x_hi, x_lo, ws1);
 }
 
 // X = F^T F in FP32.
 int reconstructFp32(msq_ctx *ctx, const DeviceBatch *b, const float *f, float *x) {
-  const bool sliced = slicedProducts(b);
-  if (sliced) MSQ_TRY(slicedReconstruct(ctx, b, f, x));
-  return gemmTN(ctx, b, f, f, x, kEpilogueStore, nullptr, false, false, sliced);
+  return slicedOrChains(
+      ctx, b, [&](const BatchRun &run, bool) { return slicedReconstruct(ctx, run.b, f, x); },
+      [&](const BatchRun &run, GemmPart part) {
+        return gemmTN(ctx, run.b, f, f, x, kEpilogueStore, nullptr, false, false, part);
+      });
 }
 
 }  // namespace

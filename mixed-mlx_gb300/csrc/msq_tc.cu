@@ -1005,14 +1005,26 @@ int packSplit(msq_ctx *ctx, const DeviceBatch *b, TcPlan *p, const float *m, boo
   return launched(ctx, "pack split-BF16");
 }
 
-// Scratch for split operands: kBuffers tile buffers of the BF16 plan.
-constexpr int kBuffers = 8;
-uint8_t *splitBuffers(msq_ctx *ctx, TcPlan *p, uint8_t *bufs[kBuffers]) {
+// Tile buffers of the BF16 plan for split operands, two per operand: V, V^T and
+// two by turns.  Where there is no memory for eight, six, and V^T takes V's.
+struct SplitBuffers {
+  uint8_t *vn[2], *vt[2], *even[2], *odd[2];
+  bool shared;  // V and V^T in the same
+};
+
+int splitBuffers(msq_ctx *ctx, TcPlan *p, SplitBuffers *out) {
   const size_t one = static_cast<size_t>(p->total_tiles) * kTileBytes;
-  uint8_t *mem = static_cast<uint8_t *>(scratch(ctx, one * kBuffers, kScratchGemm));
-  if (mem == nullptr) return nullptr;
-  for (int q = 0; q < kBuffers; ++q) bufs[q] = mem + q * one;
-  return mem;
+  uint8_t *mem = static_cast<uint8_t *>(tryScratch(ctx, 8 * one, kScratchGemm));
+  out->shared = mem == nullptr;
+  if (out->shared) mem = static_cast<uint8_t *>(scratch(ctx, 6 * one, kScratchGemm));
+  if (mem == nullptr) return MSQ_ERR_CUDA;
+  for (int q = 0; q < 2; ++q) {
+    out->vn[q] = mem + q * one;
+    out->even[q] = mem + (2 + q) * one;
+    out->odd[q] = mem + (4 + q) * one;
+    out->vt[q] = out->shared ? out->vn[q] : mem + (6 + q) * one;
+  }
+  return MSQ_OK;
 }
 
 // A B^T of split operands, to FP32 (x) or packed (out).
@@ -1041,17 +1053,15 @@ int sylvesterTc(msq_ctx *ctx, const DeviceBatch *b, const float *v, const float 
                 const float *r, float *correction, bool basis_packed) {
   TcPlan *p = tcPlan(ctx, b, kOpBf16);
   if (p == nullptr) return MSQ_ERR_CUDA;
-  uint8_t *buf[kBuffers];
-  if (splitBuffers(ctx, p, buf) == nullptr) return MSQ_ERR_CUDA;
-  uint8_t *vn[2] = {buf[0], buf[1]}, *vt[2] = {buf[2], buf[3]};
-  uint8_t *even[2] = {buf[4], buf[5]}, *odd[2] = {buf[6], buf[7]};
-  if (!basis_packed) {
-    MSQ_TRY(packSplit(ctx, b, p, v, false, vn));  // rows = columns of V
-    MSQ_TRY(packSplit(ctx, b, p, v, true, vt));   // rows = rows of V
-  }
+  SplitBuffers buf;
+  MSQ_TRY(splitBuffers(ctx, p, &buf));
+  uint8_t **vn = buf.vn, **vt = buf.vt, **even = buf.even, **odd = buf.odd;
+  if (!basis_packed || buf.shared) MSQ_TRY(packSplit(ctx, b, p, v, false, vn));  // rows = columns of V
+  if (!basis_packed && !buf.shared) MSQ_TRY(packSplit(ctx, b, p, v, true, vt));  // rows = rows of V
   MSQ_TRY(packSplit(ctx, b, p, r, false, even));  // R (symmetric)
   MSQ_TRY(gemmSplit<kEpiPacked>(ctx, b, p, even, vn, nullptr, odd, nullptr, "tc sylvester G=RV"));
   MSQ_TRY(gemmSplit<kEpiInverseH>(ctx, b, p, vn, odd, lam, even, nullptr, "tc sylvester C=V'G/H"));
+  if (buf.shared) MSQ_TRY(packSplit(ctx, b, p, v, true, vt));
   MSQ_TRY(gemmSplit<kEpiPacked>(ctx, b, p, even, vt, nullptr, odd, nullptr, "tc sylvester Zt=CV'"));
   return gemmSplit<kEpiStore>(ctx, b, p, odd, vt, nullptr, nullptr, correction, "tc sylvester E=ZV'");
 }

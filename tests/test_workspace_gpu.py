@@ -97,3 +97,64 @@ def test_solve_without_memory_for_workspaces(ctx, msq, refuse):
     finally:
         refuse(0)
         fresh.close()
+
+
+def _correct(ctx, msq, fmt, b, v, w, r):
+    import torch
+    hi, lo = torch.zeros_like(v), torch.zeros_like(v)
+    ctx.sylvester_sweep(fmt, v, w, r, b, hi, lo)
+    return hi, lo
+
+
+def test_products_of_more_pieces_than_are_kept_at_a_time(ctx, msq):
+    """30 matrices of order 2048 have 3 GB of pieces: two runs, each matrix as
+    alone."""
+    import torch
+    orders = [2048] * 12 + [70, 300] + [2048] * 18
+    b, v = _batch(msq, orders)
+    w = torch.linspace(0.5, 1.5, int(b.n.sum()), device="cuda")
+    x = ctx.reconstruct_factor(msq.PLAN_FP32, v, b)
+    hi, _ = _correct(ctx, msq, msq.FP32, b, v, w, v)
+    eig = b.eig_offset
+    for i, (one, vi) in enumerate(_members(msq, b, v)):
+        n, o, k = int(b.n[i]), int(b.offset[i]), int(eig[i])
+        if n < 2048 or i % 5:
+            continue
+        vi = vi.contiguous()
+        assert torch.equal(x[o:o + n * n], ctx.reconstruct_factor(msq.PLAN_FP32, vi, one))
+        assert torch.equal(hi[o:o + n * n], _correct(ctx, msq, msq.FP32, one, vi, w[k:k + n].contiguous(), vi)[0])
+
+
+@pytest.mark.parametrize("orders", [[900], [512, 130, 700, 33, 300]])
+def test_products_without_memory_for_pieces(ctx, msq, refuse, orders):
+    """FMA chains: each of the four within sqrt(n) 2^-24 and a little of its terms'
+    norms, as in test_gemm_tiles_gpu.py."""
+    import torch
+    b, v = _batch(msq, orders)
+    w = torch.linspace(0.5, 1.5, int(b.n.sum()), device="cuda")
+    assert refuse(1) == 0
+    x = b.unpack(ctx.reconstruct_factor(msq.PLAN_FP32, v, b).cpu().numpy())
+    hi = b.unpack(_correct(ctx, msq, msq.FP32, b, v, w, v)[0].cpu().numpy())
+    refuse(0)
+    for i, (_, vi) in enumerate(_members(msq, b, v)):
+        n = int(b.n[i])
+        m = vi.reshape(n, n).double().cpu().numpy()
+        s = np.sqrt(w[int(b.eig_offset[i]):int(b.eig_offset[i]) + n].double().cpu().numpy())
+        ref = m @ m
+        assert np.linalg.norm(x[i] - ref) <= 8 * np.sqrt(n) * 2.0**-24 * np.linalg.norm(ref)
+        h = 1.0 / (s[:, None] + s[None, :])
+        e = m @ ((m @ m @ m) * h) @ m
+        size = np.linalg.norm(np.abs(m) @ ((np.abs(m) @ np.abs(m) @ np.abs(m)) * h) @ np.abs(m))
+        assert np.linalg.norm(hi[i] - (e + e.T) / 2) <= 8 * np.sqrt(n) * 2.0**-24 * size
+
+
+def test_split_products_with_six_buffers(ctx, msq, refuse):
+    """V and its transpose take the same buffers in turn: the same bits."""
+    import torch
+    b, v = _batch(msq, [300, 64, 129])
+    w = torch.linspace(0.5, 1.5, int(b.n.sum()), device="cuda")
+    want = _correct(ctx, msq, msq.BF16, b, v, w, v)
+    assert refuse(1) == 0
+    got = _correct(ctx, msq, msq.BF16, b, v, w, v)
+    refuse(0)
+    assert all(torch.equal(x, y) for x, y in zip(got, want))
