@@ -42,7 +42,7 @@ constexpr int kThreads = 256;  // 16 x 16 threads, 4 x 4 outputs each
 // of the rest being the last wave): the four products of a correction of
 // four matrices of order 1000 take 802 us (40 TFLOP/s) against 1437 us with
 // 64 x 64 tiles of 4 x 4 outputs per thread and a load-barrier-compute loop;
-// order 256 alone 46 us against 97.  Tile sizes: gemmClass.
+// order 256 alone 46 us against 97.  Tile sizes: GemmClasses.
 template <int kT>
 struct GemmShape {
   static constexpr int kM = kT == 32 ? 4 : 8;              // outputs per thread and dimension
@@ -566,26 +566,31 @@ namespace {
 // the batch's 128-tiles nearly give every SM one (order 2048: 1565 us
 // against 1724; 1500: 648 against 719; 1000 alone, 64 tiles: 443 against
 // 295).  64 otherwise (20 of order 777: 2058 us against 2087 with 128).
-int gemmClass(const DeviceBatch *b, int n) {
-  int64_t tiles64 = 0, tiles128 = 0;
-  for (const int32_t m : b->host_n) {
-    const int64_t t = (m + 63) / 64, u = (m + 127) / 128;
-    tiles64 += t * t;
-    if (m >= kGemmLargeOrder) tiles128 += u * u;
+struct GemmClasses {
+  int64_t tiles64 = 0, tiles128 = 0;  // of the whole batch
+  explicit GemmClasses(const DeviceBatch *b) {
+    for (const int32_t m : b->host_n) {
+      const int64_t t = (m + 63) / 64, u = (m + 127) / 128;
+      tiles64 += t * t;
+      if (m >= kGemmLargeOrder) tiles128 += u * u;
+    }
   }
-  if (n <= 32 || tiles64 < 3 * kSmCount / 2) return 32;
-  return n >= kGemmLargeOrder && tiles128 >= 4 * kSmCount / 5 ? 128 : 64;
-}
+  int operator()(int n) const {
+    if (n <= 32 || tiles64 < 3 * kSmCount / 2) return 32;
+    return n >= kGemmLargeOrder && tiles128 >= 4 * kSmCount / 5 ? 128 : 64;
+  }
+};
 
 // The tiles (matrix, i, j) of every matrix of one tile class, cached on the
 // batch; `upper`: only those on or above the diagonal.
 int gemmTiles(msq_ctx *ctx, const DeviceBatch *b, int tile, bool upper, GemmPart part,
               const int4 **work, int *items) {
-  return tileWork(ctx, b, tile, upper, kGemmWorkBase + (upper ? 1 : 0) + 2 * tile + 1024 * static_cast<int>(part),
-                  work, items, [&](int n) {
-                    return gemmClass(b, n) == tile &&
-                           (part == GemmPart::kAll || slicedMatrix(n) == (part == GemmPart::kSliced));
-                  });
+  const int key = kGemmWorkBase + (upper ? 1 : 0) + 2 * tile + 1024 * static_cast<int>(part);
+  if (findWork(b, key, work, items)) return MSQ_OK;
+  const GemmClasses classOf(b);
+  return tileWork(ctx, b, tile, upper, key, work, items, [&](int n) {
+    return classOf(n) == tile && (part == GemmPart::kAll || slicedMatrix(n) == (part == GemmPart::kSliced));
+  });
 }
 
 template <int kT, bool kMajorA, bool kMajorB>
