@@ -150,7 +150,8 @@ static uint64_t hashLayout(const int32_t *n, const int64_t *offset, int count) {
 static void freeBatch(DeviceBatch *b) {
   for (auto &r : b->runs)
     for (DeviceBatch *run : r.second) freeBatch(run);
-  for (auto &w : b->work_cache) cudaFree(w.work);
+  for (auto &w : b->work_cache)
+    if (w.owner) cudaFree(w.work);
   cudaFree(b->offset);
   delete b;
 }
@@ -274,17 +275,33 @@ bool findWork(const DeviceBatch *b, int key, const int4 **work, int *items) {
   return false;
 }
 
+int keepWorks(msq_ctx *ctx, const DeviceBatch *b, int key,
+              std::initializer_list<const std::vector<int4> *> lists) {
+  std::vector<int4> all;
+  for (const std::vector<int4> *list : lists) all.insert(all.end(), list->begin(), list->end());
+  int4 *dev = nullptr;
+  if (!all.empty()) {
+    MSQ_TRY(cudaCheck(ctx, cudaMalloc(&dev, all.size() * sizeof(int4)), "work list alloc"));
+    const int status = cudaCheck(ctx, cudaMemcpy(dev, all.data(), all.size() * sizeof(int4),
+                                                 cudaMemcpyHostToDevice), "work list upload");
+    if (status != MSQ_OK) {
+      cudaFree(dev);
+      return status;
+    }
+  }
+  bool owner = true;
+  for (const std::vector<int4> *list : lists) {
+    const_cast<DeviceBatch *>(b)->work_cache.push_back({key++, dev, static_cast<int>(list->size()), owner});
+    if (dev != nullptr) dev += list->size();
+    owner = false;
+  }
+  return MSQ_OK;
+}
+
 int keepWork(msq_ctx *ctx, const DeviceBatch *b, int key, const std::vector<int4> &list,
              const int4 **work, int *items) {
-  int4 *dev = nullptr;
-  if (!list.empty()) {
-    MSQ_TRY(cudaCheck(ctx, cudaMalloc(&dev, list.size() * sizeof(int4)), "work list alloc"));
-    MSQ_TRY(cudaCheck(ctx, cudaMemcpy(dev, list.data(), list.size() * sizeof(int4),
-                                      cudaMemcpyHostToDevice), "work list upload"));
-  }
-  const_cast<DeviceBatch *>(b)->work_cache.push_back({key, dev, static_cast<int>(list.size())});
-  *work = dev;
-  *items = static_cast<int>(list.size());
+  MSQ_TRY(keepWorks(ctx, b, key, {&list}));
+  findWork(b, key, work, items);
   return MSQ_OK;
 }
 

@@ -526,12 +526,9 @@ constexpr int kGemmLargeOrder = 1000;
 constexpr int kGemmWorkBase = 1 << 16;
 constexpr int kResidualWork = 1 << 18;
 
-// One work list per (batch layout, key), cached on the batch: the tiles of
-// every matrix whose order `in` accepts.
+// The tiles of every matrix whose order `in` accepts.
 template <class In>
-int tileWork(msq_ctx *ctx, const DeviceBatch *b, int size, bool upper, int key, const int4 **work,
-             int *items, In in) {
-  if (findWork(b, key, work, items)) return MSQ_OK;
+std::vector<int4> tileList(const DeviceBatch *b, int size, bool upper, In in) {
   std::vector<int4> list;
   // largest matrices first: their long K loops start early
   std::vector<int> ids;
@@ -544,7 +541,15 @@ int tileWork(msq_ctx *ctx, const DeviceBatch *b, int size, bool upper, int key, 
     for (int ti = 0; ti < t; ++ti)
       for (int tj = upper ? ti : 0; tj < t; ++tj) list.push_back(make_int4(mi, ti, tj, 0));
   }
-  return keepWork(ctx, b, key, list, work, items);
+  return list;
+}
+
+// One such list per (batch layout, key), cached on the batch.
+template <class In>
+int tileWork(msq_ctx *ctx, const DeviceBatch *b, int size, bool upper, int key, const int4 **work,
+             int *items, In in) {
+  if (findWork(b, key, work, items)) return MSQ_OK;
+  return keepWork(ctx, b, key, tileList(b, size, upper, in), work, items);
 }
 
 }  // namespace
@@ -585,12 +590,19 @@ struct GemmClasses {
 // batch; `upper`: only those on or above the diagonal.
 int gemmTiles(msq_ctx *ctx, const DeviceBatch *b, int tile, bool upper, GemmPart part,
               const int4 **work, int *items) {
-  const int key = kGemmWorkBase + (upper ? 1 : 0) + 2 * tile + 1024 * static_cast<int>(part);
+  const int keys = kGemmWorkBase + 4 * (2 * static_cast<int>(part) + (upper ? 1 : 0));
+  const int key = keys + (tile == 32 ? 0 : tile == 64 ? 1 : 2);
   if (findWork(b, key, work, items)) return MSQ_OK;
   const GemmClasses classOf(b);
-  return tileWork(ctx, b, tile, upper, key, work, items, [&](int n) {
-    return classOf(n) == tile && (part == GemmPart::kAll || slicedMatrix(n) == (part == GemmPart::kSliced));
-  });
+  std::vector<int4> list[3];
+  int sizes[3] = {32, 64, 128};
+  for (int q = 0; q < 3; ++q)
+    list[q] = tileList(b, sizes[q], upper, [&](int n) {
+      return classOf(n) == sizes[q] && (part == GemmPart::kAll || slicedMatrix(n) == (part == GemmPart::kSliced));
+    });
+  MSQ_TRY(keepWorks(ctx, b, keys, {&list[0], &list[1], &list[2]}));
+  findWork(b, key, work, items);
+  return MSQ_OK;
 }
 
 template <int kT, bool kMajorA, bool kMajorB>

@@ -43,7 +43,6 @@
 
 #include <algorithm>
 #include <atomic>
-#include <cstring>
 #include <initializer_list>
 #include <vector>
 
@@ -51,7 +50,8 @@ namespace msq {
 namespace {
 
 constexpr int kSlices = 3;
-constexpr int kTile = 128, kTileK = 32;
+constexpr int kTile = kSliceRows, kTileK = kSliceK;
+constexpr int kSlicedWorkKey = 1 << 21;
 constexpr int kSliceBytes = kTile * 2 * kTileK;        // one piece of a tile, SWIZZLE_64B
 constexpr int kTileBytes = kSlices * kSliceBytes;
 constexpr int kStageBytes = 2 * kTileBytes;
@@ -419,54 +419,6 @@ __global__ void __launch_bounds__(kSlicedThreads, 1) slicedGemmKernel(SlicedArgs
   }
 }
 
-// The work lists of the batch's sliced matrices, kept on it: row blocks of 128; operand tiles; tiles
-// of the product, all and on or above the diagonal, largest matrices first;
-// each matrix's first operand tile (64-bit, two per int4).
-struct SlicedPlan {
-  const int4 *rows, *pack, *gemm, *upper, *bases;
-  int row_items, pack_items, gemm_items, upper_items, base_items;
-};
-
-int slicedPlan(msq_ctx *ctx, const DeviceBatch *b, SlicedPlan *p) {
-  constexpr int kKey = 1 << 21;
-  if (findWork(b, kKey, &p->rows, &p->row_items) && findWork(b, kKey + 1, &p->pack, &p->pack_items) &&
-      findWork(b, kKey + 2, &p->gemm, &p->gemm_items) &&
-      findWork(b, kKey + 3, &p->upper, &p->upper_items) &&
-      findWork(b, kKey + 4, &p->bases, &p->base_items))
-    return MSQ_OK;
-  std::vector<int4> rows, pack, gemm, upper, bases((b->count + 1) / 2);
-  std::vector<int64_t> first(2 * bases.size(), 0);
-  std::vector<int> ids;
-  int64_t tiles = 0;
-  for (int mi = 0; mi < b->count; ++mi) {
-    const int n = b->host_n[mi], mt = (n + kTile - 1) / kTile, kt = (n + kTileK - 1) / kTileK;
-    if (!slicedMatrix(n)) continue;
-    ids.push_back(mi);
-    first[mi] = tiles;
-    tiles += static_cast<int64_t>(mt) * kt;
-    for (int t = 0; t < mt; ++t) {
-      rows.push_back(make_int4(mi, t, 0, 0));
-      for (int k = 0; k < kt; ++k) pack.push_back(make_int4(mi, t, k, kt));
-    }
-  }
-  std::stable_sort(ids.begin(), ids.end(),
-                   [&](int x, int y) { return b->host_n[x] > b->host_n[y]; });
-  for (int mi : ids) {
-    const int n = b->host_n[mi], mt = (n + kTile - 1) / kTile, kt = (n + kTileK - 1) / kTileK;
-    for (int t = 0; t < mt; ++t)
-      for (int u = 0; u < mt; ++u) {
-        gemm.push_back(make_int4(mi, t, u, kt));
-        if (u >= t) upper.push_back(gemm.back());
-      }
-  }
-  std::memcpy(bases.data(), first.data(), bases.size() * sizeof(int4));
-  MSQ_TRY(keepWork(ctx, b, kKey, rows, &p->rows, &p->row_items));
-  MSQ_TRY(keepWork(ctx, b, kKey + 1, pack, &p->pack, &p->pack_items));
-  MSQ_TRY(keepWork(ctx, b, kKey + 2, gemm, &p->gemm, &p->gemm_items));
-  MSQ_TRY(keepWork(ctx, b, kKey + 3, upper, &p->upper, &p->upper_items));
-  return keepWork(ctx, b, kKey + 4, bases, &p->bases, &p->base_items);
-}
-
 // One sliced operand in the scratch.
 struct Operand {
   uint32_t *largest;
@@ -474,7 +426,7 @@ struct Operand {
 };
 
 // `count` operands of the batch in the scratch, their largest magnitudes in one block.
-int slicedOperands(msq_ctx *ctx, const DeviceBatch *b, const SlicedPlan &p, int count, Operand *out) {
+int slicedOperands(msq_ctx *ctx, const DeviceBatch *b, const SlicePlan &p, int count, Operand *out) {
   const size_t largest = (count * b->total_order * sizeof(uint32_t) + 1023) & ~size_t(1023);
   const size_t slices = static_cast<size_t>(p.pack_items) * kTileBytes;
   uint8_t *mem = static_cast<uint8_t *>(tryScratch(ctx, largest + 1024 + count * slices, kScratchGemm));
@@ -496,7 +448,7 @@ struct Source {
 // The pieces of up to three matrices, in one launch (two with `find`: their
 // largest magnitudes first; else a product has left them).  V, V^T and R of a
 // correction of four matrices of order 1000: about 30 us, 62 in six launches.
-int sliceOperands(msq_ctx *ctx, const DeviceBatch *b, const SlicedPlan &p,
+int sliceOperands(msq_ctx *ctx, const DeviceBatch *b, const SlicePlan &p,
                   std::initializer_list<Source> sources, bool find) {
   SliceArgs s{};
   s.rows = p.rows;
@@ -505,7 +457,7 @@ int sliceOperands(msq_ctx *ctx, const DeviceBatch *b, const SlicedPlan &p,
   s.items = p.pack_items;
   s.offset = b->offset;
   s.eig_offset = b->eig_offset;
-  s.tile_base = reinterpret_cast<const int64_t *>(p.bases);
+  s.tile_base = p.tileBase();
   s.n = b->n;
   unsigned count = 0;
   for (const Source &q : sources) {
@@ -525,7 +477,7 @@ int sliceOperands(msq_ctx *ctx, const DeviceBatch *b, const SlicedPlan &p,
 }
 
 template <int kEpi>
-int slicedGemm(msq_ctx *ctx, const DeviceBatch *b, const SlicedPlan &p, const Operand &a,
+int slicedGemm(msq_ctx *ctx, const DeviceBatch *b, const SlicePlan &p, const Operand &a,
                const Operand &bm, const float *eigenvalues, float *c, uint32_t *largest_c) {
   static std::atomic<uint64_t> done_mask{0};
   const uint64_t bit = ctx->device >= 0 && ctx->device < 64 ? uint64_t{1} << ctx->device : 0;
@@ -542,7 +494,7 @@ int slicedGemm(msq_ctx *ctx, const DeviceBatch *b, const SlicedPlan &p, const Op
   args.b = bm.slices;
   args.largest_a = a.largest;
   args.largest_b = bm.largest;
-  args.tile_base = reinterpret_cast<const int64_t *>(p.bases);
+  args.tile_base = p.tileBase();
   args.n = b->n;
   args.offset = b->offset;
   args.eig_offset = b->eig_offset;
@@ -584,9 +536,9 @@ int64_t slicedBytes(int n) {
 }
 
 int slicedReconstruct(msq_ctx *ctx, const DeviceBatch *b, const float *f, float *x) {
-  SlicedPlan p{};
+  SlicePlan p{};
   Operand op[1];
-  MSQ_TRY(slicedPlan(ctx, b, &p));
+  MSQ_TRY(slicePlan(ctx, b, kSlicedWorkKey, kTile, true, slicedMatrix, &p));
   MSQ_TRY(slicedOperands(ctx, b, p, 1, op));
   MSQ_TRY(sliceOperands(ctx, b, p, {{f, op[0], false}}, true));
   return slicedGemm<kSlicedMirror>(ctx, b, p, op[0], op[0], nullptr, x, nullptr);
@@ -594,9 +546,9 @@ int slicedReconstruct(msq_ctx *ctx, const DeviceBatch *b, const float *f, float 
 
 int slicedSylvester(msq_ctx *ctx, const DeviceBatch *b, const float *v, const float *lam,
                     const float *r, float *ws, float *e, bool basis_packed) {
-  SlicedPlan p{};
+  SlicePlan p{};
   Operand op[4];
-  MSQ_TRY(slicedPlan(ctx, b, &p));
+  MSQ_TRY(slicePlan(ctx, b, kSlicedWorkKey, kTile, true, slicedMatrix, &p));
   MSQ_TRY(slicedOperands(ctx, b, p, 4, op));
   const Operand vt = op[0], vn = op[1], even = op[2], odd = op[3];
   const size_t order_bytes = b->total_order * sizeof(uint32_t);

@@ -5,6 +5,7 @@
 
 #include <cstddef>
 #include <cstdint>
+#include <initializer_list>
 #include <string>
 #include <utility>
 #include <vector>
@@ -43,6 +44,7 @@ struct WorkList {
   int tile;
   int4 *work;
   int items;
+  bool owner;  // of the allocation, which lists kept together share
 };
 
 // Batched layout uploaded to the device once per distinct (n, offset) set.
@@ -218,6 +220,9 @@ void scratchRecord(msq_ctx *ctx);
 bool findWork(const DeviceBatch *b, int key, const int4 **work, int *items);
 int keepWork(msq_ctx *ctx, const DeviceBatch *b, int key, const std::vector<int4> &list,
              const int4 **work, int *items);
+// Several lists under key, key + 1, .. in one upload; read them with findWork.
+int keepWorks(msq_ctx *ctx, const DeviceBatch *b, int key,
+              std::initializer_list<const std::vector<int4> *> lists);
 // Consecutive runs of the batch's matrices whose bytes(order) add up to at most
 // `limit`, a matrix above it in a run of its own, so that an arena serves one
 // run after another.  Each has the batch's offsets; first: its first matrix.

@@ -42,14 +42,13 @@
 
 #include <algorithm>
 #include <atomic>
-#include <cstring>
-#include <vector>
 
 namespace msq {
 namespace {
 
 constexpr int kSlices = 8;
-constexpr int kTileM = 128, kTileN = 64, kTileK = 32;
+constexpr int kTileM = kSliceRows, kTileN = 64, kTileK = kSliceK;
+constexpr int kResidualWorkKey = 1 << 20;
 // One slice of an operand tile: 64-byte rows (SWIZZLE_64B), A 128 rows, B 64;
 // the kSlices slices of a tile of 128 columns of X are contiguous.
 constexpr int kSliceA = 8192, kSliceB = 4096;
@@ -485,49 +484,6 @@ __global__ void __launch_bounds__(kResidualThreads, 1) residualMmaKernel(Residua
   }
 }
 
-// The work lists of the matrices this path takes, kept on the batch: row
-// blocks of 128 columns of X; operand tiles; 128 x 64 tiles of the product
-// that reach the diagonal or lie above it, largest matrices first; and each
-// matrix's first operand tile (64-bit, two per int4).
-int residualWork(msq_ctx *ctx, const DeviceBatch *b, const int4 **rows, int *row_items,
-                 const int4 **pack, int *pack_items, const int4 **gemm, int *gemm_items,
-                 const int4 **bases, int *base_items) {
-  constexpr int kRows = 1 << 20, kPack = kRows + 1, kGemm = kRows + 2, kBases = kRows + 3;
-  if (findWork(b, kRows, rows, row_items) && findWork(b, kPack, pack, pack_items) &&
-      findWork(b, kGemm, gemm, gemm_items) && findWork(b, kBases, bases, base_items))
-    return MSQ_OK;
-  std::vector<int4> r, p, g, base((b->count + 1) / 2);
-  std::vector<int64_t> first(2 * base.size(), 0);
-  std::vector<int> ids;
-  int64_t tiles = 0;
-  for (int mi = 0; mi < b->count; ++mi) {
-    const int n = b->host_n[mi];
-    if (!residualOnTensorCores(n)) continue;
-    ids.push_back(mi);
-    const int mt = (n + kTileM - 1) / kTileM, kt = (n + kTileK - 1) / kTileK;
-    first[mi] = tiles;
-    tiles += static_cast<int64_t>(mt) * kt;
-    for (int t = 0; t < mt; ++t) {
-      r.push_back(make_int4(mi, t, 0, 0));
-      for (int k = 0; k < kt; ++k) p.push_back(make_int4(mi, t, k, kt));
-    }
-  }
-  std::stable_sort(ids.begin(), ids.end(),
-                   [&](int x, int y) { return b->host_n[x] > b->host_n[y]; });
-  static_assert(kTileM == 2 * kTileN, "tile u >= 2 t reaches the diagonal of tile row t");
-  for (int mi : ids) {
-    const int n = b->host_n[mi];
-    const int mt = (n + kTileM - 1) / kTileM, nt = (n + kTileN - 1) / kTileN, kt = (n + kTileK - 1) / kTileK;
-    for (int t = 0; t < mt; ++t)
-      for (int u = 2 * t; u < nt; ++u) g.push_back(make_int4(mi, t, u, kt));
-  }
-  std::memcpy(base.data(), first.data(), base.size() * sizeof(int4));
-  MSQ_TRY(keepWork(ctx, b, kRows, r, rows, row_items));
-  MSQ_TRY(keepWork(ctx, b, kPack, p, pack, pack_items));
-  MSQ_TRY(keepWork(ctx, b, kGemm, g, gemm, gemm_items));
-  return keepWork(ctx, b, kBases, base, bases, base_items);
-}
-
 }  // namespace
 
 bool residualOnTensorCores(int n) { return n >= kResidualMmaOrder; }
@@ -539,15 +495,12 @@ int64_t residualDigitBytes(int n) {
 
 int residualMma(msq_ctx *ctx, const DeviceBatch *b, const float *a, const float *x_hi,
                 const float *x_lo, float *r, double *norms, const float *a_lo) {
-  const int4 *rows = nullptr, *pack = nullptr, *gemm = nullptr, *bases = nullptr;
-  int row_items = 0, pack_items = 0, gemm_items = 0, base_items = 0;
-  MSQ_TRY(residualWork(ctx, b, &rows, &row_items, &pack, &pack_items, &gemm, &gemm_items, &bases,
-                       &base_items));
-  if (row_items == 0) return MSQ_OK;
-  const int64_t *tile_base = reinterpret_cast<const int64_t *>(bases);
+  SlicePlan p{};
+  MSQ_TRY(slicePlan(ctx, b, kResidualWorkKey, kTileN, false, residualOnTensorCores, &p));
+  if (p.row_items == 0) return MSQ_OK;
   const size_t exp_bytes = (b->total_order * sizeof(int32_t) + 255) & ~size_t(255);
   uint8_t *mem = static_cast<uint8_t *>(
-      tryScratch(ctx, exp_bytes + 1024 + static_cast<size_t>(pack_items) * kTileBytes, kScratchResidual));
+      tryScratch(ctx, exp_bytes + 1024 + static_cast<size_t>(p.pack_items) * kTileBytes, kScratchResidual));
   if (mem == nullptr) return kNoScratch;
   static std::atomic<uint64_t> done_mask{0};
   const uint64_t bit = ctx->device >= 0 && ctx->device < 64 ? uint64_t{1} << ctx->device : 0;
@@ -557,20 +510,20 @@ int residualMma(msq_ctx *ctx, const DeviceBatch *b, const float *a, const float 
     done_mask.fetch_or(bit);
   }
   SliceArgs s{};
-  s.rows = rows;
-  s.row_items = row_items;
-  s.work = pack;
-  s.items = pack_items;
+  s.rows = p.rows;
+  s.row_items = p.row_items;
+  s.work = p.pack;
+  s.items = p.pack_items;
   s.hi = x_hi;
   s.lo = x_lo;
   s.offset = b->offset;
   s.eig_offset = b->eig_offset;
-  s.tile_base = tile_base;
+  s.tile_base = p.tileBase();
   s.n = b->n;
   s.exponent = reinterpret_cast<int32_t *>(mem);
   s.slices = mem + ((exp_bytes + 1023) & ~size_t(1023));
-  const dim3 row_grid(std::min(row_items, kSmCount * 8), kTileM / 8);
-  const unsigned pack_grid = std::min(pack_items, kSmCount * 8);
+  const dim3 row_grid(std::min(p.row_items, kSmCount * 8), kTileM / 8);
+  const unsigned pack_grid = std::min(p.pack_items, kSmCount * 8);
   if (x_lo != nullptr) {
     columnExponentKernel<true><<<row_grid, 256, 0, ctx->stream>>>(s);
     MSQ_TRY(launched(ctx, "residual exponents"));
@@ -582,10 +535,10 @@ int residualMma(msq_ctx *ctx, const DeviceBatch *b, const float *a, const float 
   }
   MSQ_TRY(launched(ctx, "residual slices"));
   ResidualMmaArgs args{};
-  args.work = gemm;
-  args.items = gemm_items;
+  args.work = p.upper;
+  args.items = p.upper_items;
   args.slices = s.slices;
-  args.tile_base = tile_base;
+  args.tile_base = p.tileBase();
   args.n = b->n;
   args.offset = b->offset;
   args.eig_offset = b->eig_offset;
@@ -596,7 +549,7 @@ int residualMma(msq_ctx *ctx, const DeviceBatch *b, const float *a, const float 
   args.norms = norms;
   args.status = ctx->d_status;
   args.wait_test = waitTestMode() == kWaitTestMbarrier;
-  residualMmaKernel<<<std::min(gemm_items, kSmCount), kResidualThreads, kResidualSmem, ctx->stream>>>(args);
+  residualMmaKernel<<<std::min(p.upper_items, kSmCount), kResidualThreads, kResidualSmem, ctx->stream>>>(args);
   return launched(ctx, "residual float-float");
 }
 

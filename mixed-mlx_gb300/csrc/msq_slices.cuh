@@ -8,11 +8,69 @@
 // Internal.
 #pragma once
 
+#include <algorithm>
+#include <cstring>
+#include <vector>
+
 #include "msq_internal.cuh"
 #include "msq_tcgen05.cuh"
 
 namespace msq {
 namespace {
+
+// The work lists of a batch's matrices that `in` accepts, kept on it from `key`
+// on: row blocks of 128 of an operand (matrix, block, -, -); its tiles of 128 x 32
+// (matrix, block, K tile, K tiles); tiles of 128 x `columns` of the product
+// (matrix, tile_i, tile_j, K tiles) that reach the diagonal or lie above it, and
+// with `all` every one, largest matrices first; and each matrix's first operand
+// tile.
+constexpr int kSliceRows = 128, kSliceK = 32;
+struct SlicePlan {
+  const int4 *rows, *pack, *upper, *gemm, *bases;
+  int row_items, pack_items, upper_items, gemm_items, base_items;
+  const int64_t *tileBase() const { return reinterpret_cast<const int64_t *>(bases); }
+};
+
+inline int slicePlan(msq_ctx *ctx, const DeviceBatch *b, int key, int columns, bool all, bool (*in)(int),
+                     SlicePlan *p) {
+  auto find = [&] {
+    return findWork(b, key, &p->rows, &p->row_items) && findWork(b, key + 1, &p->pack, &p->pack_items) &&
+           findWork(b, key + 2, &p->upper, &p->upper_items) &&
+           findWork(b, key + 3, &p->gemm, &p->gemm_items) &&
+           findWork(b, key + 4, &p->bases, &p->base_items);
+  };
+  if (find()) return MSQ_OK;
+  std::vector<int4> rows, pack, upper, gemm, bases((b->count + 1) / 2);  // 64-bit bases, two per int4
+  std::vector<int64_t> first(2 * bases.size(), 0);
+  std::vector<int> ids;
+  int64_t tiles = 0;
+  for (int mi = 0; mi < b->count; ++mi) {
+    const int n = b->host_n[mi], mt = (n + kSliceRows - 1) / kSliceRows, kt = (n + kSliceK - 1) / kSliceK;
+    if (!in(n)) continue;
+    ids.push_back(mi);
+    first[mi] = tiles;
+    tiles += static_cast<int64_t>(mt) * kt;
+    for (int t = 0; t < mt; ++t) {
+      rows.push_back(make_int4(mi, t, 0, 0));
+      for (int k = 0; k < kt; ++k) pack.push_back(make_int4(mi, t, k, kt));
+    }
+  }
+  std::stable_sort(ids.begin(), ids.end(),
+                   [&](int x, int y) { return b->host_n[x] > b->host_n[y]; });
+  for (int mi : ids) {
+    const int n = b->host_n[mi], kt = (n + kSliceK - 1) / kSliceK;
+    for (int t = 0; t < (n + kSliceRows - 1) / kSliceRows; ++t)
+      for (int u = 0; u < (n + columns - 1) / columns; ++u) {
+        const int4 w = make_int4(mi, t, u, kt);
+        if (all) gemm.push_back(w);
+        if ((u + 1) * columns > t * kSliceRows) upper.push_back(w);
+      }
+  }
+  std::memcpy(bases.data(), first.data(), bases.size() * sizeof(int4));
+  MSQ_TRY(keepWorks(ctx, b, key, {&rows, &pack, &upper, &gemm, &bases}));
+  find();
+  return MSQ_OK;
+}
 
 constexpr int kDigit = 7;                     // bits per digit after the first
 constexpr long long kSliceWaitLimit = 1ll << 26;
