@@ -69,7 +69,12 @@ constexpr int kGridFewLarge = 8;
 // the sweep count): one matrix on one CTA takes about 3.8e-7 n^3 ms, and
 // batched matrices above 256 saturate at about 40 in flight (their tiles
 // stream from L2 / HBM), those up to 256 at about 300; the grid kernels take
-// about 5 + 3.8e-5 n^2 ms per matrix, one matrix at a time.
+// about 5 + 3.8e-5 n^2 ms per matrix, one matrix at a time.  The figures are of
+// kernels with two launches per round: a grid solve now takes 6.1 ms at order
+// 512, 12.6 at 1024 and 40 at 2048 (the model: 15, 45, 164), a one-CTA solve of
+// order 256 5.2 (6.4).  So where it chooses the grid it gains more than it
+// takes, and there are batches left on one CTA each that the grid would solve
+// sooner.
 constexpr double kCtaSolveMs = 3.8e-7;    // x n^3
 constexpr double kGridSolveMs0 = 5.0;     // + kGridSolveMs2 x n^2
 constexpr double kGridSolveMs2 = 3.8e-5;
@@ -1343,8 +1348,11 @@ int jacobiEnqueue(msq_ctx *ctx, const DeviceBatch *b, float *matrices, float *ve
       MSQ_TRY(cudaCheck(ctx, cudaEventRecord(replay_done[parity], rs), "event record"));
     }
   }
-  // Large matrices: the grid kernels on the context's stream, overlapping the
-  // batched sweeps still running on the internal streams.
+  // Large matrices: the grid kernels on the context's stream, beside the
+  // batched sweeps on the internal streams where these leave enough SMs, else
+  // in turn with them (a cooperative launch waits for its SMs).  Solves of 1000
+  // matrices of orders 64 .. 512 with one and eight of 1100: 150 and 248 ms,
+  // 199 and 528 with launches per round that overlapped them.
   int busy = serial ? 0 : plan->tl.count;  // one CTA per matrix
   if (!serial)
     for (const auto &bucket : plan->buckets) busy += bucket.count;

@@ -149,8 +149,6 @@ __device__ __forceinline__ int64_t tileElement(int t, int i, int j) {
   return static_cast<int64_t>(t) * kTileF + (((i ^ tileSwizzle(t)) << 2) | j);
 }
 
-// Loads block (R, C) of A (4x4, row-major in t) from packed tile ti, which
-// holds (min, max) of the two block indices (transposed when R > C).
 // 16-byte asynchronous global -> shared copies (cp.async, L2 only).
 __device__ __forceinline__ void copyAsync16(void *smem, const void *gmem) {
   const unsigned dst = static_cast<unsigned>(__cvta_generic_to_shared(smem));
@@ -159,40 +157,7 @@ __device__ __forceinline__ void copyAsync16(void *smem, const void *gmem) {
 __device__ __forceinline__ void copyAsyncCommit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void copyAsyncWaitAll() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
 
-__device__ __forceinline__ void loadTile(const float *tiles, int ti, bool transposed, float (&t)[4][4]) {
-  const float4 *src = reinterpret_cast<const float4 *>(tiles + static_cast<int64_t>(ti) * kTileF);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float4 v = src[i ^ tileSwizzle(ti)];
-    if (!transposed) {
-      t[i][0] = v.x; t[i][1] = v.y; t[i][2] = v.z; t[i][3] = v.w;
-    } else {
-      t[0][i] = v.x; t[1][i] = v.y; t[2][i] = v.z; t[3][i] = v.w;
-    }
-  }
-}
-
-__device__ __forceinline__ void storeTile(float *tiles, int ti, bool transposed, const float (&t)[4][4]) {
-  float4 *dst = reinterpret_cast<float4 *>(tiles + static_cast<int64_t>(ti) * kTileF);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    dst[i ^ tileSwizzle(ti)] = transposed ? make_float4(t[0][i], t[1][i], t[2][i], t[3][i])
-                                   : make_float4(t[i][0], t[i][1], t[i][2], t[i][3]);
-  }
-}
-
-// Block (R, C) through a table tri[J] = J (J + 1) / 2 (shared memory) ...
-__device__ __forceinline__ void loadBlock(const float *tiles, const int *tri, int R, int C, float (&t)[4][4]) {
-  if (R <= C) loadTile(tiles, tileIndex(tri, R, C), false, t);
-  else loadTile(tiles, tileIndex(tri, C, R), true, t);
-}
-
-__device__ __forceinline__ void storeBlock(float *tiles, const int *tri, int R, int C, const float (&t)[4][4]) {
-  if (R <= C) storeTile(tiles, tileIndex(tri, R, C), false, t);
-  else storeTile(tiles, tileIndex(tri, C, R), true, t);
-}
-
-// ... or with the index computed (grid kernels).
+// Index of tile (I, J), I <= J.
 __device__ __forceinline__ int triTile(int I, int J) { return J * (J + 1) / 2 + I; }
 
 // ---------------------------------------------------------------------------
@@ -387,16 +352,14 @@ __host__ __device__ __forceinline__ int sweepPairOf(int block, int round, int m)
 // grid kernels: a round's critical path is one pivot): the same rotations
 // and the same bits.
 //
-// In tournament positions as well.  Lane (t, j) holds the 2x2 block of pairs lo = min(t, j), hi = max(t, j): rows
-// (lo, 7 - lo), columns (hi, 7 - hi), row rotation first, then the column
-// rotation, which is the sequential order of the upper triangle (the lower
-// one is its transpose bit for bit: each of its elements sees the same two
-// operations).  Lanes (t, j) and (j, t) do the same work and write the two
-// triangles.  The diagonal lanes compute the four angles of a group at once;
-// the blocks move through shared memory, double-buffered (no bank conflict
-// in either direction for the two pivots of a warp).  Positions order a pair
-// by tournament slot, the angle by index: where they differ the angle is
-// taken of the swapped pair and s negated (x - y and x + (-y) round alike).
+// In tournament positions as above.  Lane (t, j) holds the 2x2 block of pairs
+// lo = min(t, j), hi = max(t, j): rows (lo, 7 - lo), columns (hi, 7 - hi), row
+// rotation first, then the column rotation, which is the sequential order of
+// the upper triangle (the lower one is its transpose bit for bit: each of its
+// elements sees the same two operations).  Lanes (t, j) and (j, t) do the same
+// work and write the two triangles.  The diagonal lanes compute the four angles
+// of a group at once; the blocks move through shared memory, double-buffered
+// (no bank conflict in either direction for the two pivots of a warp).
 // Q is formed by another warp that follows the pivot warp (PivotQ): the
 // diagonal lanes leave each group's (c, s) in shared memory and a flag says
 // how far they are; 32 more rotations per group would otherwise sit on the
@@ -564,6 +527,8 @@ __device__ __forceinline__ float &tileAt(const Mem &mem, int64_t e) {
   return mem.base(static_cast<int>(e >> 4))[e & 15];
 }
 
+// Block (R, C) of A (4x4, row-major in t) from the packed tile ti at p, which
+// holds (min, max) of the two block indices (transposed when R > C).
 __device__ __forceinline__ void loadTileAt(const float *p, int ti, bool transposed, float (&t)[4][4]) {
   const float4 *src = reinterpret_cast<const float4 *>(p);
 #pragma unroll
