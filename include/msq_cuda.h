@@ -349,7 +349,13 @@ int msq_reconstruct_factor(msq_ctx *ctx, int plan_format, const float *factor_t,
  * A as a (high, low) pair: metal_mixed_sqrt.metal:1268-1317,
  * src/metal_solver.cpp:186-196); writes R as FP32 (may be NULL) and
  * per-matrix ||R||_F^2, ||A||_F^2 (FP64, device, 2 per matrix).  a_lo and
- * x_lo may be NULL (treated as zero).
+ * x_lo may be NULL (treated as zero).  X must be symmetric.  Orders up to 64
+ * run on the CUDA cores, larger ones on the tensor cores with X in digits of
+ * its columns: R_ij is then off by its rounding to FP32 and by at most
+ * n 2^-51 of the product of the largest entries of columns i and j (2e-15 to
+ * 6e-15 of ||A|| measured for n = 64 .. 512, the CUDA cores 2e-14 to 3e-13);
+ * an entry of X below 2^-8 of its column's largest has fewer than 48 bits
+ * there.
  * msq_sylvester_sweep: one frozen-basis correction of
  * refineUpdateAndMeasure (src/metal_runtime.cpp:847-966):
  *   C = (V^T R V) o H, H_ij = 1/(s_i + s_j) recomputed from s = sqrt(lambda),

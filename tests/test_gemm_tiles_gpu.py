@@ -41,3 +41,40 @@ def test_reconstruction_and_correction_at_tile_edges(ctx, msq, orders):
         e = v @ c @ v.T
         e = 0.5 * (e + e.T)
         assert np.linalg.norm(eg - e) <= tol * np.linalg.norm(e)
+
+
+@pytest.mark.parametrize("orders", [
+    [1, 31, 33], [63, 64, 65] * 30,             # 32- and 64-tiles
+    [1000, 1001, 1023, 1025], [1409, 40]])      # 128-tiles
+@pytest.mark.parametrize("trans", [(0, 0), (1, 0), (0, 1), (1, 1)])
+@pytest.mark.parametrize("mode", ["plain", "same", "roots"])
+def test_general_products_at_tile_edges(ctx, msq, orders, trans, mode):
+    """msq_gemm, which is FMA chains at every order: every layout of the operands,
+    an operand with itself (mirrored where the layouts agree) and the division by
+    the sums of roots.  An element is within n 2^-24 sum |a_k b_k|, and the roots,
+    their sum and the quotient round four times."""
+    import ctypes
+    import torch
+    b = msq.Batch.from_orders(orders)
+    rng = np.random.default_rng(len(orders))
+    am = [rng.standard_normal((n, n)).astype(np.float32) for n in orders]
+    bm = am if mode == "same" else [rng.standard_normal((n, n)).astype(np.float32) for n in orders]
+    lam = rng.uniform(0.1, 1.0, int(b.n.sum())).astype(np.float32)
+    a = torch.from_numpy(b.pack(am)).cuda()
+    bb = a if mode == "same" else torch.from_numpy(b.pack(bm)).cuda()
+    w, c = torch.from_numpy(lam).cuda(), torch.zeros_like(a)
+    ptr = lambda t: ctypes.c_void_p(t.data_ptr())  # noqa: E731
+    ctx.check(msq.lib().msq_gemm(
+        ctypes.c_void_p(ctx.handle.value), trans[0], trans[1], ptr(a), ptr(bb), ctypes.c_void_p(b.n.ctypes.data),
+        ctypes.c_void_p(b.offset.ctypes.data), b.count, ptr(w) if mode == "roots" else None, ptr(c)), "msq_gemm")
+    ctx.synchronize()
+    at = 0
+    for n, x, y, got in zip(orders, am, bm, b.unpack(c.cpu().numpy())):
+        x, y = (m.astype(np.float64).T if t else m.astype(np.float64) for m, t in zip((x, y), trans))
+        s = np.sqrt(lam[at:at + n].astype(np.float64))
+        at += n
+        h = 1.0 / (s[:, None] + s[None, :]) if mode == "roots" else 1.0
+        bound = (n + 4) * 2.0**-24 * (np.abs(x) @ np.abs(y)) * h
+        assert (np.abs(got - (x @ y) * h) <= bound).all()
+        if mode == "same" and trans[0] != trans[1]:
+            assert np.array_equal(got, got.T)
