@@ -12,7 +12,8 @@ low-bit speed-up.
 
 Usage: python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference]
 Under torchrun each rank solves its own batch (weak scaling, no collective
-on the data path); rank 0 prints one JSON line.
+on the data path); rank 0 prints one JSON line (and every measurement behind it
+on the error stream).
 """
 from __future__ import annotations
 
@@ -200,6 +201,22 @@ def cpu_baseline(oracle, mats, budget_s: float) -> dict:
     return {"value": ok / per_solve, "unit": "solves/s", "cores": cores, "kind": "port",
             "sample": f"{done} of {len(mats)} matrices (stratified by n), "
                       f"{per_solve * done:.1f}s, OpenBLAS threads={os.environ.get('OPENBLAS_NUM_THREADS', cores)}"}
+
+
+# Keys of the default workload's line; the others go to the error stream.
+SHORT_KEYS = ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better",
+              "scaling", "vs_baseline", "dtype", "data", "config", "e2e", "clocks", "gpu_launches",
+              "accepted", "fallback", "speedup_vs_plain_fp32", "roofline")
+SHORT_ROOFLINE = ("bound", "achieved", "peak", "unit", "frac", "traffic", "kernel", "share")
+
+
+def emit(line: dict) -> None:
+    """Every measurement on the error stream, then the result as one line that
+    fits where only the end of a run's output is kept."""
+    print("all measurements: " + json.dumps(line), file=sys.stderr, flush=True)
+    short = {k: line[k] for k in SHORT_KEYS}
+    short["roofline"] = {k: line["roofline"][k] for k in SHORT_ROOFLINE}
+    print(json.dumps(short), flush=True)
 
 
 def run_reference(args):
@@ -988,7 +1005,7 @@ def main():
         "kernels_source": "launch timer over one extra step with concurrency off (serial)",
         "autotune": [l for l in ctx.autotune_report().splitlines() if l],
     }
-    print(json.dumps(line), flush=True)
+    emit(line)
     if world > 1:
         torch.distributed.barrier()
 
