@@ -471,79 +471,119 @@ __device__ __forceinline__ uint32_t tileWord(int row, int word) {
   return swizzle128(row, word >> 2) + 4 * (word & 3);
 }
 
-// One CTA of 128 threads per tile, a warp per 32 of its rows: lane l forms
-// word l of a row, so a row is read and written as whole lines, kBatch rows
-// in flight.  Bound by memory.  (A thread per row, each lane on its own
-// line: 522 us for the BF16 factors of 4096 matrices of orders 16 .. 512, 247
-// so.)
+constexpr int kPackThreads = 256;  // packKernel
+constexpr int kMxWarps = 8;        // packMxKernel
+constexpr int kSplitWarps = 4;     // packSplitKernel
+
+// The E4M3 codes of v[e] / scale: by the hardware where the four are finite
+// (the same codes), else by the conversion in integers.
+__device__ __forceinline__ uint32_t fp8Word(const float (&v)[4], float scale) {
+  float x[4];
+  bool finite = true;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    x[e] = rowDivide(v[e], scale);
+    finite = finite && fabsf(x[e]) <= 3.402823466e38f;
+  }
+  if (finite) return encodeE4M3Pair(x[0], x[1]) | (encodeE4M3Pair(x[2], x[3]) << 16);
+  uint32_t word = 0;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) word |= static_cast<uint32_t>(encodeE4M3(x[e])) << (8 * e);
+  return word;
+}
+
+// One CTA per tile.  The words of the rows that the matrix has
+// (a row's rounded up to whole 16-byte chunks) are dealt to the threads in
+// order, kBatch in flight of each: a warp reads and writes whole lines of one
+// row of a large matrix, of several of a small one, and the tile's other chunks
+// are zeroed.  Bound by memory.  (A thread per row, each lane on its own line:
+// 1240 us for the BF16 factors of 4096 matrices of orders 16 .. 512, 613 so.  A
+// warp per row, whatever its length: 35.5 us for the FP8 factors of 1000
+// matrices of order 65, 25.2 so; with 128 threads a latency-bound single order
+// 1000 takes 28.3 us, 18.0 with 256.)
 template <int kSource>
-__global__ void __launch_bounds__(128) packKernel(PackArgs args) {
+__global__ void __launch_bounds__(kPackThreads) packKernel(PackArgs args) {
   constexpr bool kFp8 = kSource == kPackF32Fp8Row || kSource == kPackFp8Codes;
   constexpr bool kF32 = kSource == kPackF32Fp8Row || kSource == kPackF32Bf16;
   constexpr int kElems = kFp8 ? 128 : 64;  // elements per 128-byte row
-  constexpr int kWord = kElems / 32;       // elements per lane
-  constexpr int kBatch = 8;
-  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  constexpr int kWord = kElems / 32;       // elements per 32-bit word
+  constexpr int kBatch = 8, kThreads = kPackThreads;
   for (int item = blockIdx.x; item < args.items; item += gridDim.x) {
     const int4 w = args.work[item];
     const int mi = w.x, n = args.n[mi];
-    const int k = w.z * kElems + kWord * lane;
+    const int i0 = w.y * kTileRows, k0 = w.z * kElems;
     const int64_t off = args.f_offset[mi];
     uint8_t *tile = args.tiles + (args.tile_base[mi] + static_cast<int64_t>(w.y) * w.w + w.z) *
                                      kTileBytes;
+    const int rows = min(n - i0, kTileRows);
+    const int chunks = min((n - k0 + 4 * kWord - 1) / (4 * kWord), 8);
+    if (rows < kTileRows || chunks < 8) {
+#pragma unroll
+      for (int c = threadIdx.x; c < kTileBytes / 16; c += kThreads)
+        if (c / 8 >= rows || c % 8 >= chunks)
+          *reinterpret_cast<uint4 *>(tile + swizzle128(c / 8, c % 8)) = make_uint4(0, 0, 0, 0);
+    }
+    // j / words for j < 4096 and words <= 32: the inverse is less than 1 too
+    // large, the quotient less than 2^12 / 2^20 < 1 / words
+    const int words = 4 * chunks;
+    const uint32_t inverse = ((1u << 20) + words - 1) / words;
     const float *f = args.f + off;
     const bool vec = kF32 && rowsAligned<kWord>(f, n);
 #pragma unroll 1
-    for (int r0 = 32 * warp; r0 < 32 * warp + 32; r0 += kBatch) {
-      const int i0 = w.y * kTileRows + r0;
+    for (int j0 = threadIdx.x; j0 < rows * words; j0 += kThreads * kBatch) {
+      int row[kBatch], col[kBatch];  // row -1: no word
+#pragma unroll
+      for (int q = 0; q < kBatch; ++q) {
+        const int j = j0 + kThreads * q;
+        row[q] = static_cast<int>((j * inverse) >> 20);
+        col[q] = j - row[q] * words;
+        if (row[q] >= rows) row[q] = -1;
+      }
+      uint32_t word[kBatch] = {};
       if constexpr (kF32) {
         float v[kBatch][kWord] = {};
         float scale[kBatch];
 #pragma unroll
         for (int q = 0; q < kBatch; ++q) {
-          if (i0 + q < n) loadRow<kWord>(f + static_cast<int64_t>(i0 + q) * n, k, n, vec, v[q]);
-          scale[q] = kSource == kPackF32Fp8Row && i0 + q < n
-                         ? args.row_scale[args.eig_offset[mi] + i0 + q]
+          if (row[q] >= 0)
+            loadRow<kWord>(f + static_cast<int64_t>(i0 + row[q]) * n, k0 + kWord * col[q], n, vec,
+                           v[q]);
+          scale[q] = kSource == kPackF32Fp8Row && row[q] >= 0
+                         ? args.row_scale[args.eig_offset[mi] + i0 + row[q]]
                          : 1.0f;
         }
 #pragma unroll
         for (int q = 0; q < kBatch; ++q) {
-          uint32_t word = 0;
-#pragma unroll
-          for (int e = 0; e < kWord; ++e) {
-            if (kFp8) word |= static_cast<uint32_t>(encodeE4M3(rowDivide(v[q][e], scale[q]))) << (8 * e);
-            else word |= static_cast<uint32_t>(encodeBf16(v[q][e])) << (16 * e);
-          }
-          *reinterpret_cast<uint32_t *>(tile + tileWord(r0 + q, lane)) = word;
+          if (row[q] < 0) continue;
+          if constexpr (kFp8) word[q] = fp8Word(v[q], scale[q]);
+          else word[q] = encodeBf16(v[q][0]) | (static_cast<uint32_t>(encodeBf16(v[q][1])) << 16);
         }
       } else {
-        uint32_t word[kBatch] = {};
 #pragma unroll
         for (int q = 0; q < kBatch; ++q) {
-          const int64_t at0 = off + k + static_cast<int64_t>(i0 + q) * n;
-          if (i0 + q < n) {
+          const int k = k0 + kWord * col[q];
+          if (row[q] < 0) continue;
 #pragma unroll
-            for (int e = 0; e < kWord; ++e) {
-              if (k + e >= n) continue;
-              const int64_t at = at0 + e;
-              if (kSource == kPackFp8Codes) {
-                word[q] |= static_cast<uint32_t>(args.codes[at]) << (8 * e);
-              } else if (kSource == kPackBf16Codes) {
-                word[q] |= static_cast<uint32_t>(reinterpret_cast<const uint16_t *>(args.codes)[at])
-                           << (16 * e);
-              } else {  // kPackMxfp4Codes: exact, at most 2 significant bits
-                const uint32_t byte = args.codes[at / 2];
-                const float d = decodeE2M1((byte >> ((at & 1) * 4)) & 0xfu);
-                word[q] |= static_cast<uint32_t>(encodeBf16(mxScale(d, args.mx_scales[at / 32])))
-                           << (16 * e);
-              }
+          for (int e = 0; e < kWord; ++e) {
+            if (k + e >= n) continue;
+            const int64_t at = off + k + e + static_cast<int64_t>(i0 + row[q]) * n;
+            if (kSource == kPackFp8Codes) {
+              word[q] |= static_cast<uint32_t>(args.codes[at]) << (8 * e);
+            } else if (kSource == kPackBf16Codes) {
+              word[q] |= static_cast<uint32_t>(reinterpret_cast<const uint16_t *>(args.codes)[at])
+                         << (16 * e);
+            } else {  // kPackMxfp4Codes: exact, at most 2 significant bits
+              const uint32_t byte = args.codes[at / 2];
+              const float d = decodeE2M1((byte >> ((at & 1) * 4)) & 0xfu);
+              word[q] |= static_cast<uint32_t>(encodeBf16(mxScale(d, args.mx_scales[at / 32])))
+                         << (16 * e);
             }
           }
         }
-#pragma unroll
-        for (int q = 0; q < kBatch; ++q)
-          *reinterpret_cast<uint32_t *>(tile + tileWord(r0 + q, lane)) = word[q];
       }
+#pragma unroll
+      for (int q = 0; q < kBatch; ++q)
+        if (row[q] >= 0) *reinterpret_cast<uint32_t *>(tile + tileWord(row[q], col[q])) = word[q];
     }
   }
 }
@@ -556,10 +596,11 @@ __global__ void __launch_bounds__(128) packKernel(PackArgs args) {
 //   kMxCodesFp4  flat MXFP4 codes and scales (order divisible by 32, so
 //                the flat 32-element blocks are row blocks)
 //   kMxCodesFp8  flat MXFP8 E4M3 codes and scales (same condition)
-// One CTA of 128 threads per tile, a warp per 32 of its rows, lane l word l
-// of a row (8 or 4 elements: a block is 4 or 8 lanes).  Blocks beyond the
-// order get zero codes and the unit scale (byte 127).  Bound by memory: the
-// FP32 factor of order 8192 in 64 us (244 with a thread per row).
+// One CTA per tile, a warp every eighth row (four warps: 11.8 us for 64 factors
+// of order 16, 8.9 with eight), lane l word l of a row (8 or 4 elements: a
+// block is 4 or 8 lanes).  Blocks beyond the order get zero codes and the unit
+// scale (byte 127).  Bound by memory: the FP32 factor of order 8192 in 70 us
+// (256 with a thread per row).
 enum MxSource : int { kMxF32Fp4 = 0, kMxCodesFp4 = 1, kMxCodesFp8 = 2 };
 
 struct MxPackArgs {
@@ -576,7 +617,7 @@ struct MxPackArgs {
 };
 
 template <int kSource>
-__global__ void __launch_bounds__(128) packMxKernel(MxPackArgs args) {
+__global__ void __launch_bounds__(32 * kMxWarps) packMxKernel(MxPackArgs args) {
   constexpr bool kFp4 = kSource != kMxCodesFp8;
   constexpr int kElems = kFp4 ? 256 : 128;  // K per 128-byte tile row
   constexpr int kWord = kElems / 32;
@@ -594,17 +635,31 @@ __global__ void __launch_bounds__(128) packMxKernel(MxPackArgs args) {
     const bool block_ok = k / 32 * 32 < n;  // the lane's block has an element
     const float *f = args.f + off;
     const bool vec = kSource == kMxF32Fp4 && rowsAligned<kWord>(f, n);
+    // the steps of kStep rows that have one of the matrix; the others hold zeros
+    // and unit scales
+    constexpr int kStep = kMxWarps * kBatch;
+    const int rows = min((n - w.y * kTileRows + kStep - 1) / kStep * kStep, kTileRows);
+    for (int c = 8 * rows + threadIdx.x; c < kTileBytes / 16; c += 32 * kMxWarps)
+      *reinterpret_cast<uint4 *>(tile + 16 * c) = make_uint4(0, 0, 0, 0);
+    for (int r = rows + threadIdx.x; r < kTileRows; r += 32 * kMxWarps)
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        *reinterpret_cast<uint32_t *>(sft + h * kScaleAtomBytes + 16 * (r % 32) + 4 * (r / 32)) =
+            0x7f7f7f7fu;
 #pragma unroll 1
-    for (int r0 = 32 * warp; r0 < 32 * warp + 32; r0 += kBatch) {
+    for (int r0 = warp; r0 < rows; r0 += kStep) {
       const int i0 = w.y * kTileRows + r0;
       uint32_t word[kBatch] = {}, sf[kBatch];
       if constexpr (kSource == kMxF32Fp4) {
         float v[kBatch][kWord] = {};
 #pragma unroll
         for (int q = 0; q < kBatch; ++q)
-          if (i0 + q < n) loadRow<kWord>(f + static_cast<int64_t>(i0 + q) * n, k, n, vec, v[q]);
+          if (i0 + kMxWarps * q < n)
+            loadRow<kWord>(f + static_cast<int64_t>(i0 + kMxWarps * q) * n, k, n, vec, v[q]);
 #pragma unroll
         for (int q = 0; q < kBatch; ++q) {
+          sf[q] = 127;
+          if (i0 + kMxWarps * q >= n) continue;  // a row beyond the order (the whole warp's)
           float m = 0.0f;
 #pragma unroll
           for (int e = 0; e < kWord; ++e) {
@@ -613,8 +668,9 @@ __global__ void __launch_bounds__(128) packMxKernel(MxPackArgs args) {
           }
 #pragma unroll
           for (int s = 1; s < kGroup; s <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, s));
+          if (!block_ok) continue;
           const int ex = mxExponent(m, 2);
-          sf[q] = i0 + q < n && block_ok ? static_cast<uint32_t>(ex + 127) : 127u;
+          sf[q] = static_cast<uint32_t>(ex + 127);
           if (ex >= -126 && ex <= 126) {
             const float s = exp2Int(-ex);
 #pragma unroll
@@ -633,8 +689,8 @@ __global__ void __launch_bounds__(128) packMxKernel(MxPackArgs args) {
 #pragma unroll
         for (int q = 0; q < kBatch; ++q) {
           sf[q] = 127;
-          if (i0 + q < n && block_ok) {
-            const int64_t at = off + k + static_cast<int64_t>(i0 + q) * n;
+          if (i0 + kMxWarps * q < n && block_ok) {
+            const int64_t at = off + k + static_cast<int64_t>(i0 + kMxWarps * q) * n;
             word[q] = *reinterpret_cast<const uint32_t *>(args.codes + (kFp4 ? at / 2 : at));
             sf[q] = args.mx_scales[at / 32];
           }
@@ -642,13 +698,13 @@ __global__ void __launch_bounds__(128) packMxKernel(MxPackArgs args) {
       }
 #pragma unroll
       for (int q = 0; q < kBatch; ++q) {
-        *reinterpret_cast<uint32_t *>(tile + tileWord(r0 + q, lane)) = word[q];
+        *reinterpret_cast<uint32_t *>(tile + tileWord(r0 + kMxWarps * q, lane)) = word[q];
         // the four scale bytes of an atom's row: 4 bytes at 16 (r mod 32) + 4 (r / 32)
         uint32_t bytes = sf[q] << (8 * (lane / kGroup % 4));
         bytes |= __shfl_xor_sync(0xffffffffu, bytes, kGroup);
         bytes |= __shfl_xor_sync(0xffffffffu, bytes, 2 * kGroup);
         if (lane % (4 * kGroup) == 0) {
-          const int r = r0 + q;
+          const int r = r0 + kMxWarps * q;
           *reinterpret_cast<uint32_t *>(sft + lane / (4 * kGroup) * kScaleAtomBytes +
                                         16 * (r % 32) + 4 * (r / 32)) = bytes;
         }
@@ -680,8 +736,8 @@ __device__ __forceinline__ void splitPair(float x, float y, uint32_t &first, uin
 }
 
 // Bound by memory: both directions read M and write the tiles in whole
-// lines.  kTranspose false: a warp per 32 rows, lane l word l (two elements)
-// of a row, as packKernel.  kTranspose true: a thread per operand row reads
+// lines.  kTranspose false: a warp every fourth row, lane l word l (two
+// elements) of a row, as packKernel.  kTranspose true: a thread per operand row reads
 // along M's columns with its warp, and the tile goes through shared memory
 // in its own (swizzled) layout, from which it is copied out in order.
 template <bool kTranspose>
@@ -731,19 +787,21 @@ __global__ void __launch_bounds__(128) packSplitKernel(SplitArgs args) {
       const int k = k0 + 2 * lane;
       const bool vec = rowsAligned<2>(M, n);
 #pragma unroll 1
-      for (int r0 = 32 * warp; r0 < 32 * warp + 32; r0 += kBatch) {
+      for (int r0 = warp; r0 < kTileRows; r0 += kSplitWarps * kBatch) {
         const int i0 = w.y * kTileRows + r0;
         float v[kBatch][2] = {};
 #pragma unroll
         for (int q = 0; q < kBatch; ++q)
-          if (i0 + q < n) loadRow<2>(M + static_cast<int64_t>(i0 + q) * n, k, n, vec, v[q]);
+          if (i0 + kSplitWarps * q < n)
+            loadRow<2>(M + static_cast<int64_t>(i0 + kSplitWarps * q) * n, k, n, vec, v[q]);
 #pragma unroll
         for (int q = 0; q < kBatch; ++q) {
           uint32_t word[2];
           splitPair(v[q][0], v[q][1], word[0], word[1]);
 #pragma unroll
           for (int p = 0; p < 2; ++p)
-            *reinterpret_cast<uint32_t *>(args.out[p] + tile + tileWord(r0 + q, lane)) = word[p];
+            *reinterpret_cast<uint32_t *>(args.out[p] + tile +
+                                          tileWord(r0 + kSplitWarps * q, lane)) = word[p];
         }
       }
     }
@@ -952,7 +1010,8 @@ int launchPackMx(msq_ctx *ctx, const DeviceBatch *b, TcPlan *p, const float *f,
   args.n = b->n;
   args.tiles = tiles;
   args.scale_tiles = scale_tiles;
-  packMxKernel<kSource><<<std::min(p->pack_items, kSmCount * 16), 128, 0, ctx->stream>>>(args);
+  packMxKernel<kSource>
+      <<<std::min(p->pack_items, kSmCount * 8), 32 * kMxWarps, 0, ctx->stream>>>(args);
   return launched(ctx, "pack block-scaled operand");
 }
 
@@ -980,7 +1039,7 @@ int launchPack(msq_ctx *ctx, const DeviceBatch *b, TcPlan *p, const float *f,
   args.tile_base = p->tile_base;
   args.n = b->n;
   args.tiles = tiles;
-  packKernel<kSource><<<std::min(p->pack_items, kSmCount * 16), 128, 0, ctx->stream>>>(args);
+  packKernel<kSource><<<std::min(p->pack_items, kSmCount * 8), kPackThreads, 0, ctx->stream>>>(args);
   return launched(ctx, "pack operand");
 }
 

@@ -73,3 +73,20 @@ def test_factor_and_split_correction(ctx, msq, orders):
         e = m @ c @ m.T
         e = 0.5 * (e + e.T)
         assert np.linalg.norm(eg - e) <= (12 * 2.0**-18 + 4 * ACC) * np.linalg.norm(e), n
+
+
+@pytest.mark.parametrize("n", [5, 33, 130])
+def test_fp8_factor_with_an_infinity_and_a_nan(ctx, msq, n):
+    """Words of four codes with an entry that the hardware conversion would not
+    code as the codec does."""
+    import torch
+    b = msq.Batch.from_orders([n])
+    f = np.random.default_rng(n).standard_normal((n, n)).astype(np.float32)
+    f[2, 1], f[3, n - 1] = np.inf, np.nan
+    x = b.unpack(ctx.reconstruct_factor(2, _dev(b.pack([f])), b).cpu().numpy())[0]
+    torch.cuda.synchronize()
+    q = _quantized(8, f)
+    ref = q.T @ q
+    assert np.array_equal(np.isnan(x), np.isnan(ref))
+    ok = np.isfinite(ref)
+    assert np.linalg.norm(x[ok] - ref[ok]) <= ACC * np.linalg.norm(ref[ok])
