@@ -96,10 +96,10 @@ constexpr int ringStages(int epilogue) { return isSplit(epilogue) ? 3 : kStages;
 constexpr int epilogueWarps(int epilogue) { return isSplit(epilogue) ? 16 : 4; }
 constexpr int tcThreads(int epilogue) { return 32 * (epilogueWarps(epilogue) + 2); }
 // X = W W^T: its tiles below the diagonal are the transposes, bit for bit, of
-// those above it (the same products in the same order), so the work list
-// holds the upper ones and the epilogue stores both.  Half the MMAs and half
-// the operand traffic, which is what bounds a large order: MXFP4 at order
-// 8192 205 us (369 with every tile computed).
+// those above it (the same products in the same order), so the work list holds
+// the upper ones (in all but the smallest batches: tcArgs) and the epilogue
+// stores both.  Half the MMAs and half the operand traffic, which is what bounds
+// a large order: MXFP4 at order 8192 205 us (369 with every tile computed).
 constexpr bool isMirrored(int epilogue) {
   return epilogue == kEpiRowScale || epilogue == kEpiMirror;
 }
@@ -156,6 +156,7 @@ struct TcArgs {
   const float *eigenvalues;// kEpiInverseH: lambda, s = sqrt(max(lambda, 0))
   float *x;
   int *status;
+  int mirror;              // 1: the work list has a mirrored product's upper tiles only
   int wait_test;           // 1: the producer first waits on a barrier nothing arrives at
 };
 
@@ -388,7 +389,7 @@ __global__ void __launch_bounds__(tcThreads(kEpi), 1) tcGemmKernel(TcArgs args) 
             }
           }
         }
-        if (isMirrored(kEpi) && w.y != w.z) {
+        if (isMirrored(kEpi) && args.mirror && w.y != w.z) {
           transpose32(v, lane);
           const int j = j0 + lane, i0 = i - lane;
           if (j < n) {
@@ -966,8 +967,14 @@ int launchTcKernel(msq_ctx *ctx, const TcArgs &args, const char *what) {
 // with the given epilogue.
 TcArgs tcArgs(msq_ctx *ctx, const DeviceBatch *b, const TcPlan *p, int epilogue) {
   TcArgs args{};
-  args.work = isMirrored(epilogue) ? p->upper_work : p->gemm_work;
-  args.items = isMirrored(epilogue) ? p->upper_items : p->gemm_items;
+  // The upper tiles alone where there is more than one tile per CTA.  With a CTA
+  // for every tile the launch lasts as long as one of them, and a mirrored one
+  // is stored twice: BF16 at order 400 11.9 us with the upper tiles, 9.9 with
+  // all; at order 1000 14.3 and 11.9.  (Sixteen epilogue warps do not change
+  // that.)
+  args.mirror = isMirrored(epilogue) && p->gemm_items > kSmCount;
+  args.work = args.mirror ? p->upper_work : p->gemm_work;
+  args.items = args.mirror ? p->upper_items : p->gemm_items;
   args.tile_base = p->tile_base;
   args.n = b->n;
   args.x_offset = b->offset;

@@ -75,6 +75,23 @@ def test_factor_and_split_correction(ctx, msq, orders):
         assert np.linalg.norm(eg - e) <= (12 * 2.0**-18 + 4 * ACC) * np.linalg.norm(e), n
 
 
+@pytest.mark.parametrize("plan", [1, 2, 3])
+def test_mirrored_tiles_are_the_computed_ones(ctx, msq, plan):
+    """A batch of more tiles than SMs (its lower tiles mirrored) against the
+    same matrices one at a time (every tile computed), bit for bit."""
+    import torch
+    orders = [257, 130, 33, 600] * 5  # 39 tiles a group
+    b = msq.Batch.from_orders(orders)
+    rng = np.random.default_rng(plan)
+    fs = [rng.standard_normal((n, n)).astype(np.float32) for n in orders]
+    x = ctx.reconstruct_factor(plan, _dev(b.pack(fs)), b)
+    torch.cuda.synchronize()
+    for f, xg in zip(fs, b.unpack(x.cpu().numpy())):
+        one = msq.Batch.from_orders([f.shape[0]])
+        alone = ctx.reconstruct_factor(plan, _dev(one.pack([f])), one)
+        assert np.array_equal(xg, one.unpack(alone.cpu().numpy())[0]), f.shape
+
+
 @pytest.mark.parametrize("n", [5, 33, 130])
 def test_fp8_factor_with_an_infinity_and_a_nan(ctx, msq, n):
     """Words of four codes with an entry that the hardware conversion would not
