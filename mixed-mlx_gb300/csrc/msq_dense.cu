@@ -43,16 +43,24 @@ constexpr int kThreads = 256;  // 16 x 16 threads, 4 x 4 outputs each
 // four matrices of order 1000 take 802 us (40 TFLOP/s) against 1437 us with
 // 64 x 64 tiles of 4 x 4 outputs per thread and a load-barrier-compute loop;
 // order 256 alone 46 us against 97.  Tile sizes: GemmClasses.
-template <int kT>
+//
+// kC is a tile size or kOneStep: 32 x 32 tiles of matrices up to order 32, whose
+// K loop is one step.  Its latency is all there is, so one stage instead of
+// three, only the elements that exist, and room for more CTAs: a product of
+// 10000 matrices of order 7 22 us with three stages and 8 CTAs per SM, 18 so;
+// of 4096 of order 16 14 and 12.
+constexpr int kOneStep = 1;
+template <int kC>
 struct GemmShape {
+  static constexpr int kT = kC == kOneStep ? 32 : kC;
   static constexpr int kM = kT == 32 ? 4 : 8;              // outputs per thread and dimension
   static constexpr int kSide = kT / kM;                    // threads per dimension
   static constexpr int kThr = kSide * kSide;               // 256, 64, 64
   static constexpr int kK = kT == 32 ? 32 : 16;            // K step
-  static constexpr int kStages = kT == 128 ? 2 : 3;
+  static constexpr int kStages = kC == kOneStep ? 1 : kT == 128 ? 2 : 3;
   static constexpr int kLd = kT + 4;
   static constexpr int kQ = kT / (kM / 4);                 // stride between a thread's groups of 4
-  static constexpr int kCtas = kT == 128 ? 2 : 8;          // resident CTAs per SM
+  static constexpr int kCtas = kC == kOneStep ? 20 : kT == 128 ? 2 : 8;  // resident CTAs per SM
 };
 
 __device__ __forceinline__ void copyAsync4(float *smem, const float *gmem, bool valid) {
@@ -64,9 +72,10 @@ __device__ __forceinline__ void copyAsync4(float *smem, const float *gmem, bool 
 
 // One operand's K step into its [k][m] stage.  kMajorM: element (m, k) at
 // m + k n (m is the fast thread index), else at k + m n (k fast).
-template <int kT, bool kMajorM>
+template <int kC, bool kMajorM>
 __device__ __forceinline__ void gemmStage(float *dst, const float *src, int n, int m0, int k0) {
-  using S = GemmShape<kT>;
+  using S = GemmShape<kC>;
+  constexpr int kT = S::kT;
   constexpr int kFast = kMajorM ? kT : S::kK;
   constexpr int kStep = S::kThr / kFast;                   // slow index per element
   constexpr int kElems = kT * S::kK / S::kThr;
@@ -83,14 +92,15 @@ __device__ __forceinline__ void gemmStage(float *dst, const float *src, int n, i
 #pragma unroll
   for (int e = 0; e < kElems; ++e) {
     const bool valid = fast_left > 0 && slow_left > e * kStep;
-    copyAsync4(s + e * kSmem, valid ? g + e * gstep : src, valid);
+    // of one step only the rows and columns of the matrix are used
+    if (kC != kOneStep || valid) copyAsync4(s + e * kSmem, valid ? g + e * gstep : src, valid);
   }
 }
 
-template <int kT>
+template <int kC>
 __device__ __forceinline__ void gemmStep(const float *as, const float *bs,
-                                         f32x2 (&acc)[GemmShape<kT>::kM / 2][GemmShape<kT>::kM]) {
-  using S = GemmShape<kT>;
+                                         f32x2 (&acc)[GemmShape<kC>::kM / 2][GemmShape<kC>::kM]) {
+  using S = GemmShape<kC>;
   f32x2 a[S::kM / 2];
   float b[S::kM];
 #pragma unroll
@@ -113,11 +123,11 @@ __device__ __forceinline__ void gemmStep(const float *as, const float *bs,
 // the tiles on or above the diagonal and an off-diagonal tile also writes
 // its mirror image (the same products in the same order, so the same bits
 // as a direct tile).
-template <int kT, bool kMajorA, bool kMajorB, int kEpilogue, bool kMirror>
-__global__ void __launch_bounds__(GemmShape<kT>::kThr, GemmShape<kT>::kCtas)
+template <int kC, bool kMajorA, bool kMajorB, int kEpilogue, bool kMirror>
+__global__ void __launch_bounds__(GemmShape<kC>::kThr, GemmShape<kC>::kCtas)
 gemmKernel(GemmArgs args) {
-  using S = GemmShape<kT>;
-  constexpr int kM = S::kM;
+  using S = GemmShape<kC>;
+  constexpr int kT = S::kT, kM = S::kM;
   __shared__ __align__(16) float As[S::kStages][S::kK][S::kLd];
   __shared__ __align__(16) float Bs[S::kStages][S::kK][S::kLd];
   const int tx = threadIdx.x % S::kSide, ty = threadIdx.x / S::kSide;
@@ -136,24 +146,25 @@ gemmKernel(GemmArgs args) {
     const int steps = (n + S::kK - 1) / S::kK;
     auto stage = [&](int s) {
       if (s < steps) {
-        gemmStage<kT, kMajorA>(&As[s % S::kStages][0][0], A, n, i0, s * S::kK);
-        gemmStage<kT, kMajorB>(&Bs[s % S::kStages][0][0], B, n, j0, s * S::kK);
+        gemmStage<kC, kMajorA>(&As[s % S::kStages][0][0], A, n, i0, s * S::kK);
+        gemmStage<kC, kMajorB>(&Bs[s % S::kStages][0][0], B, n, j0, s * S::kK);
       }
       asm volatile("cp.async.commit_group;\n" ::: "memory");
     };
+    constexpr int kAhead = kC == kOneStep ? 1 : S::kStages - 1;
 #pragma unroll
-    for (int s = 0; s < S::kStages - 1; ++s) stage(s);
-    for (int s = 0; s < steps; ++s) {
-      asm volatile("cp.async.wait_group %0;\n" ::"n"(S::kStages - 2) : "memory");
+    for (int s = 0; s < kAhead; ++s) stage(s);
+    for (int s = 0; s < (kC == kOneStep ? 1 : steps); ++s) {
+      asm volatile("cp.async.wait_group %0;\n" ::"n"(kAhead - 1) : "memory");
       __syncthreads();  // step s landed for every thread; step s - 1's slot is free
-      stage(s + S::kStages - 1);
+      if (kC != kOneStep) stage(s + kAhead);
       const float *as = &As[s % S::kStages][0][4 * tx], *bs = &Bs[s % S::kStages][0][4 * ty];
       const int left = n - s * S::kK;
       if (left >= S::kK) {
 #pragma unroll
-        for (int k = 0; k < S::kK; ++k) gemmStep<kT>(as + k * S::kLd, bs + k * S::kLd, acc);
+        for (int k = 0; k < S::kK; ++k) gemmStep<kC>(as + k * S::kLd, bs + k * S::kLd, acc);
       } else {
-        for (int k = 0; k < left; ++k) gemmStep<kT>(as + k * S::kLd, bs + k * S::kLd, acc);
+        for (int k = 0; k < left; ++k) gemmStep<kC>(as + k * S::kLd, bs + k * S::kLd, acc);
       }
     }
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
@@ -407,6 +418,25 @@ __global__ void __launch_bounds__(256) makeFactorKernel(
   }
 }
 
+// The same for a batch of matrices of at most kSmallOrder, as
+// smallSymmetricAddKernel: lane k has the root of column k (4096 of order 16:
+// 31 us with 64 x 64 tiles, 28 so).
+constexpr int kSmallOrder = 32;
+__global__ void __launch_bounds__(256) makeSmallFactorKernel(
+    const float *__restrict__ v, const float *__restrict__ lam, const int32_t *__restrict__ nn,
+    const int64_t *__restrict__ off, const int64_t *__restrict__ eoff, float *__restrict__ f,
+    int count) {
+  const int k = threadIdx.x % 32, warp = threadIdx.x / 32;
+  for (int mi = blockIdx.x; mi < count; mi += gridDim.x) {
+    const int n = nn[mi];
+    if (k >= n) continue;
+    const float *V = v + off[mi];
+    float *F = f + off[mi];
+    const float root = sqrtf(rootOf(lam[eoff[mi] + k]));
+    for (int i = warp; i < n; i += 8) F[k + i * n] = V[i + k * n] * root;
+  }
+}
+
 __global__ void transposeKernel(const float *__restrict__ src, const int32_t *__restrict__ nn,
                                 const int64_t *__restrict__ off, float *__restrict__ dst,
                                 const int4 *__restrict__ work, int items) {
@@ -428,6 +458,17 @@ __global__ void transposeKernel(const float *__restrict__ src, const int32_t *__
     if (i < n && j < n) D[j + static_cast<int64_t>(i) * n] = tile[threadIdx.x][r];
   }
   }
+}
+
+// (hi, lo) <- (h, l) + corr: two-sum of the high word and the correction, the
+// error and the low word renormalised.
+__device__ __forceinline__ void addFF(float h, float l, float corr, float *hi, float *lo) {
+  const float s = h + corr;
+  const float vr = s - h;
+  const float err = (h - (s - vr)) + (corr - vr) + l;
+  const float t = s + err;
+  *hi = t;
+  *lo = err - (t - s);
 }
 
 // X <- X + (E + E^T)/2 in float-float (working_add_symmetric_correction,
@@ -479,13 +520,28 @@ __global__ void __launch_bounds__(256) symmetricAddKernel(
         if (s >= sides || i >= n || j >= n) continue;
         const int64_t at = i + static_cast<int64_t>(j) * n;
         const float corr = 0.5f * (own[s][q] + tile[sides - 1 - s][lane][warp + 8 * q]);
-        const float t = h[s][q] + corr;
-        const float vr = t - h[s][q];
-        const float err = (h[s][q] - (t - vr)) + (corr - vr) + l[s][q];
-        const float hi = t + err;
-        H[at] = hi;
-        L[at] = err - (hi - t);
+        addFF(h[s][q], l[s][q], corr, &H[at], &L[at]);
       }
+  }
+}
+
+// The same for a batch of matrices of one tile each: what is read across its
+// columns is in L1 already, and without barriers a CTA has all its loads in
+// flight (10000 of order 7: 37 us through shared memory, 11 so; 4096 of order 16
+// 16 and 10).
+__global__ void __launch_bounds__(256) smallSymmetricAddKernel(
+    float *__restrict__ x_hi, float *__restrict__ x_lo, const float *__restrict__ e,
+    const int32_t *__restrict__ nn, const int64_t *__restrict__ off, int count) {
+  const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
+  for (int mi = blockIdx.x; mi < count; mi += gridDim.x) {
+    const int n = nn[mi];
+    const float *E = e + off[mi];
+    float *H = x_hi + off[mi], *L = x_lo + off[mi];
+    for (int j = warp; j < n; j += 8) {
+      if (lane >= n) continue;
+      const int at = lane + j * n;
+      addFF(H[at], L[at], 0.5f * (E[at] + E[j + lane * n]), &H[at], &L[at]);
+    }
   }
 }
 
@@ -562,12 +618,13 @@ int gemmWork(msq_ctx *ctx, const DeviceBatch *b, int tile, const int4 **work, in
 
 namespace {
 
-// Tile size of a matrix in the FP32 GEMM.  32 up to order 32 (a 64-tile is
-// mostly padding: a correction of 1000 matrices of order 24 takes 33 us
-// against 53) and for batches with fewer 64-tiles than 1.5 per SM, where
-// one CTA's K loop is the whole launch and a 32-tile's is a quarter as long
-// (order 256 alone: 46 us against 90; order 512 alone: 82 against 150; eight
-// of order 384, 288 tiles: 162 against 133).  128 from order 1000 where
+// Tile class of a matrix in the FP32 GEMM.  32 for batches with fewer 64-tiles
+// than 1.5 per SM, where one CTA's K loop is the whole launch and a 32-tile's is
+// a quarter as long (order 256 alone: 46 us against 90; order 512 alone: 82
+// against 150; eight of order 384, 288 tiles: 162 against 133).  In larger ones
+// kOneStep up to order 32 (a 64-tile is mostly padding: a correction of 1000
+// matrices of order 24 takes 53 us with it, 33 with 32-tiles).  128 from order
+// 1000 where
 // the batch's 128-tiles nearly give every SM one (order 2048: 1565 us
 // against 1724; 1500: 648 against 719; 1000 alone, 64 tiles: 443 against
 // 295).  64 otherwise (20 of order 777: 2058 us against 2087 with 128).
@@ -581,7 +638,8 @@ struct GemmClasses {
     }
   }
   int operator()(int n) const {
-    if (n <= 32 || tiles64 < 3 * kSmCount / 2) return 32;
+    if (tiles64 < 3 * kSmCount / 2) return 32;
+    if (n <= 32) return kOneStep;
     return n >= kGemmLargeOrder && tiles128 >= 4 * kSmCount / 5 ? 128 : 64;
   }
 };
@@ -591,33 +649,34 @@ struct GemmClasses {
 int gemmTiles(msq_ctx *ctx, const DeviceBatch *b, int tile, bool upper, GemmPart part,
               const int4 **work, int *items) {
   const int keys = kGemmWorkBase + 4 * (2 * static_cast<int>(part) + (upper ? 1 : 0));
-  const int key = keys + (tile == 32 ? 0 : tile == 64 ? 1 : 2);
+  const int key = keys + (tile == kOneStep ? 3 : tile == 32 ? 0 : tile == 64 ? 1 : 2);
   if (findWork(b, key, work, items)) return MSQ_OK;
   const GemmClasses classOf(b);
-  std::vector<int4> list[3];
-  int sizes[3] = {32, 64, 128};
-  for (int q = 0; q < 3; ++q)
-    list[q] = tileList(b, sizes[q], upper, [&](int n) {
-      return classOf(n) == sizes[q] && (part == GemmPart::kAll || slicedMatrix(n) == (part == GemmPart::kSliced));
+  std::vector<int4> list[4];
+  const int classes[4] = {32, 64, 128, kOneStep};
+  for (int q = 0; q < 4; ++q)
+    list[q] = tileList(b, classes[q] == kOneStep ? 32 : classes[q], upper, [&](int n) {
+      return classOf(n) == classes[q] &&
+             (part == GemmPart::kAll || slicedMatrix(n) == (part == GemmPart::kSliced));
     });
-  MSQ_TRY(keepWorks(ctx, b, keys, {&list[0], &list[1], &list[2]}));
+  MSQ_TRY(keepWorks(ctx, b, keys, {&list[0], &list[1], &list[2], &list[3]}));
   findWork(b, key, work, items);
   return MSQ_OK;
 }
 
-template <int kT, bool kMajorA, bool kMajorB>
+template <int kC, bool kMajorA, bool kMajorB>
 int launchGemm(msq_ctx *ctx, const DeviceBatch *b, GemmArgs args, int epilogue, bool mirror,
                GemmPart part) {
-  using S = GemmShape<kT>;
-  MSQ_TRY(gemmTiles(ctx, b, kT, mirror, part, &args.work, &args.items));
+  using S = GemmShape<kC>;
+  MSQ_TRY(gemmTiles(ctx, b, kC, mirror, part, &args.work, &args.items));
   if (args.items == 0) return MSQ_OK;
   const unsigned grid = std::min<unsigned>(args.items, kSmCount * S::kCtas * 4);
   if (mirror) {
-    gemmKernel<kT, kMajorA, kMajorA, kEpilogueStore, true><<<grid, S::kThr, 0, ctx->stream>>>(args);
+    gemmKernel<kC, kMajorA, kMajorA, kEpilogueStore, true><<<grid, S::kThr, 0, ctx->stream>>>(args);
   } else if (epilogue == kEpilogueInverseH) {
-    gemmKernel<kT, kMajorA, kMajorB, kEpilogueInverseH, false><<<grid, S::kThr, 0, ctx->stream>>>(args);
+    gemmKernel<kC, kMajorA, kMajorB, kEpilogueInverseH, false><<<grid, S::kThr, 0, ctx->stream>>>(args);
   } else {
-    gemmKernel<kT, kMajorA, kMajorB, kEpilogueStore, false><<<grid, S::kThr, 0, ctx->stream>>>(args);
+    gemmKernel<kC, kMajorA, kMajorB, kEpilogueStore, false><<<grid, S::kThr, 0, ctx->stream>>>(args);
   }
   return launched(ctx, "gemm TN fp32");
 }
@@ -627,7 +686,8 @@ int launchGemmClasses(msq_ctx *ctx, const DeviceBatch *b, const GemmArgs &args, 
                       bool mirror, GemmPart part) {
   MSQ_TRY((launchGemm<128, kMajorA, kMajorB>(ctx, b, args, epilogue, mirror, part)));
   MSQ_TRY((launchGemm<64, kMajorA, kMajorB>(ctx, b, args, epilogue, mirror, part)));
-  return launchGemm<32, kMajorA, kMajorB>(ctx, b, args, epilogue, mirror, part);
+  MSQ_TRY((launchGemm<32, kMajorA, kMajorB>(ctx, b, args, epilogue, mirror, part)));
+  return launchGemm<kOneStep, kMajorA, kMajorB>(ctx, b, args, epilogue, mirror, part);
 }
 
 }  // namespace
@@ -692,6 +752,11 @@ int residualFF(msq_ctx *ctx, const DeviceBatch *b, const float *a, const float *
 int makeFactor(msq_ctx *ctx, const DeviceBatch *b, const float *v, const float *lam, float *f) {
   const int4 *work;
   int items;
+  if (b->max_n <= kSmallOrder) {
+    makeSmallFactorKernel<<<std::min(b->count, kSmCount * 16), 256, 0, ctx->stream>>>(
+        v, lam, b->n, b->offset, b->eig_offset, f, b->count);
+    return launched(ctx, "make factor");
+  }
   MSQ_TRY(gemmWork(ctx, b, kFactorTile, &work, &items));
   makeFactorKernel<<<std::min(items, kSmCount * 8), 256, 0, ctx->stream>>>(
       v, lam, b->n, b->offset, b->eig_offset, f, work, items);
@@ -770,6 +835,11 @@ int workingAdd(msq_ctx *ctx, const DeviceBatch *b, float *x_hi, float *x_lo, con
 int symmetricAdd(msq_ctx *ctx, const DeviceBatch *b, float *x_hi, float *x_lo, const float *e) {
   const int4 *work;
   int items;
+  if (b->max_n <= kSmallOrder) {
+    smallSymmetricAddKernel<<<std::min(b->count, kSmCount * 16), 256, 0, ctx->stream>>>(
+        x_hi, x_lo, e, b->n, b->offset, b->count);
+    return launched(ctx, "symmetric add");
+  }
   MSQ_TRY(gemmWork(ctx, b, -32, &work, &items));
   symmetricAddKernel<<<std::min(items, kSmCount * 8), 256, 0, ctx->stream>>>(
       x_hi, x_lo, e, b->n, b->offset, work, items);

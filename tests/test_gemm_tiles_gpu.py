@@ -78,3 +78,38 @@ def test_general_products_at_tile_edges(ctx, msq, orders, trans, mode):
         assert (np.abs(got - (x @ y) * h) <= bound).all()
         if mode == "same" and trans[0] != trans[1]:
             assert np.array_equal(got, got.T)
+
+
+def test_batches_of_small_orders(ctx, msq):
+    """Orders 1 .. 32 in a batch large enough for the one-step products and the
+    kernels without shared memory, bit for bit what the same matrices give
+    beside one of order 33 in a small batch."""
+    import ctypes
+    import torch
+    orders = list(range(1, 33))
+    many, few = msq.Batch.from_orders(orders * 10), msq.Batch.from_orders(orders + [33])
+    rng = np.random.default_rng(32)
+    vm, rm = ([rng.standard_normal((n, n)).astype(np.float32) for n in orders + [33]] for _ in range(2))
+    lam = rng.uniform(0.1, 1.0, int(few.n.sum())).astype(np.float32)
+    own = int(sum(orders))
+
+    def run(b, times):
+        pick = (lambda m: m) if times == 1 else (lambda m: m[:-1] * times)
+        v, r = (torch.from_numpy(b.pack(pick(m))).cuda() for m in (vm, rm))
+        w = torch.from_numpy(lam if times == 1 else np.tile(lam[:own], times)).cuda()
+        out = [ctx.make_factor(v, w, b), ctx.reconstruct_factor(msq.PLAN_FP32, v, b)]
+        ptr = lambda t: ctypes.c_void_p(t.data_ptr())  # noqa: E731
+        for ta, tb in ((0, 0), (1, 0), (0, 1), (1, 1)):
+            c = torch.zeros_like(v)
+            ctx.check(msq.lib().msq_gemm(
+                ctypes.c_void_p(ctx.handle.value), ta, tb, ptr(v), ptr(r), ctypes.c_void_p(b.n.ctypes.data),
+                ctypes.c_void_p(b.offset.ctypes.data), b.count, ptr(w), ptr(c)), "msq_gemm")
+            out.append(c)
+        hi, lo = out[1].clone(), torch.zeros_like(v)
+        ctx.sylvester_sweep(msq.FP32, v, w, r, b, hi, lo)
+        ctx.synchronize()
+        return [b.unpack(t.cpu().numpy()) for t in out + [hi, lo]]
+
+    for got, ref in zip(run(many, 10), run(few, 1)):
+        for i, g in enumerate(got):
+            assert np.array_equal(g, ref[i % len(orders)]), g.shape
