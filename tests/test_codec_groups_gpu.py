@@ -70,3 +70,41 @@ def test_rows_equal_the_oracle(ctx, msq, row, shift):
     w_ref, _ = O.encode_stochastic(8, x, 7, 3, row_length=row)
     w, _ = ctx.copy_to_storage_stochastic(8, dev, 7, 3, row)
     assert np.array_equal(w.cpu().numpy().view(np.uint8).ravel(), w_ref)
+
+
+@pytest.mark.parametrize("shift", [0, 1, 4])
+@pytest.mark.parametrize("n", [7, 256, 264, 511, 4103])
+@pytest.mark.parametrize("fmt,row", [(1, 0), (2, 0), (3, 0), (4, 0), (5, 0), (6, 0), (7, 0), (8, 1), (8, 11)])
+def test_decoding_into_a_shifted_buffer(ctx, msq, fmt, row, n, shift):
+    """Outputs 4, 16 and 32 bytes aligned, of whole warps and with tails; what
+    lies before and behind the output stays as it was."""
+    import ctypes
+    import torch
+    n = n // row * row if row else n
+    if n == 0:
+        return
+    x = _values(n, n + shift)
+    kw = {"row_length": row} if row else {}
+    v_ref, s_ref = O.encode(fmt, x, **kw)
+    want = O.decode(fmt, v_ref, s_ref, n, **kw).astype(np.float32)
+    v, s = ctx.copy_to_storage(fmt, torch.from_numpy(x).cuda(), row)
+    buf = torch.full((ALIGN + shift + n + ALIGN,), 3.0, device="cuda")
+    out = buf[ALIGN + shift:]
+    ctx.check(msq.lib().msq_decode(
+        ctypes.c_void_p(ctx.handle.value), fmt, ctypes.c_void_p(v.data_ptr()),
+        ctypes.c_void_p(s.data_ptr()) if s is not None else None, n, row, ctypes.c_void_p(out.data_ptr())), "decode")
+    ctx.synchronize()
+    got = buf.cpu().numpy()
+    at = ALIGN + shift
+    assert np.array_equal(got[at:at + n].view(np.uint32), want.view(np.uint32))
+    assert (got[:at] == 3.0).all() and (got[at + n:] == 3.0).all()
+
+
+@pytest.mark.parametrize("row", [31, 32, 33, 127, 128, 129])
+def test_row_lengths_around_a_lanes_first_elements(ctx, msq, row):
+    import torch
+    x = _values(row * 19, row)
+    v_ref, s_ref = O.encode(8, x, row_length=row)
+    v, s = ctx.copy_to_storage(8, _placed(torch, x, torch.float32, 1), row)
+    assert np.array_equal(v.cpu().numpy().view(np.uint8).ravel()[:len(v_ref)], v_ref)
+    assert np.array_equal(s.cpu().numpy().view(np.uint8).ravel()[:len(s_ref)], s_ref)
