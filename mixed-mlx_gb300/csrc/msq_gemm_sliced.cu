@@ -525,9 +525,10 @@ constexpr double kSlicedWork = 0.65e9;
 bool slicedMatrix(int n) { return n >= kSlicedOrder; }
 
 bool slicedProducts(const DeviceBatch *b) {
+  if (!slicedMatrix(b->max_n)) return false;
   double work = 0.0;
   for (const int32_t n : b->host_n)
-    if (slicedMatrix(n)) work += static_cast<double>(n) * n * n;
+    if (n >= kSlicedOrder) work += static_cast<double>(n) * n * n;
   return work >= kSlicedWork;
 }
 
