@@ -32,9 +32,9 @@
 // the tensor pipe's read of A: an MMA of M = 128 takes 68 cycles for N = 32,
 // 64 and 128 alike (152 matrices of order 512: 80 per MMA with the drain).
 //
-// Residual of four matrices of order 1000: 219 us with the slicing against
-// 913 on the CUDA cores; 152 of order 512: 1095 against 4254; 1000 of order
-// 128: 363 against 718; one of order 128: 41 against 54.
+// Residual of four matrices of order 1000: 214 us with the slicing against
+// 913 on the CUDA cores; 152 of order 512: 1090 against 4254; 1000 of order
+// 128: 347 against 718; one of order 128: 39 against 54.
 #include "msq_dense.cuh"
 #include "msq_internal.cuh"
 #include "msq_residual.cuh"
@@ -216,6 +216,9 @@ __device__ __forceinline__ double squaredPowerOfTwo(int k) {
   return __hiloint2double((1023 + 2 * k) << 20, 0);
 }
 
+// kLow: A has a low word.  Without one the epilogue has registers enough: 1000
+// matrices of order 65 300 us with the choice at run time, 274 so.
+template <bool kLow>
 __global__ void __launch_bounds__(kResidualThreads, 1) residualMmaKernel(ResidualMmaArgs args) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char *base = reinterpret_cast<unsigned char *>(
@@ -368,7 +371,7 @@ __global__ void __launch_bounds__(kResidualThreads, 1) residualMmaKernel(Residua
         }
       }
       if (!ok) break;
-      const float *A = args.a + off, *AL = args.a_lo ? args.a_lo + off : nullptr;
+      const float *A = args.a + off, *AL = kLow ? args.a_lo + off : nullptr;
       float *R = args.r ? args.r + off : nullptr;
 #pragma unroll
       for (int c = 0; c < kCols; ++c) {
@@ -380,10 +383,8 @@ __global__ void __launch_bounds__(kResidualThreads, 1) residualMmaKernel(Residua
       // as 64 FP32 ones) at scales that the columns' exponents give: A near 1,
       // R 2^40 above that.  A sum that leaves inSquareRange, where FP32
       // loses or overflows squares, is taken again in FP64.
-      int kmax = ei + 12 + __shfl_sync(0xffffffffu, ej, 0);
-#pragma unroll
-      for (int c = 1; c < kCols; ++c) kmax = max(kmax, ei + 12 + __shfl_sync(0xffffffffu, ej, c));
-      kmax = min(max(kmax, -87), 126);  // both scales are normal numbers
+      const int cols_max = __reduce_max_sync(0xffffffffu, lane < kCols && j0 + lane < n ? ej : -300);
+      const int kmax = min(max(ei + 12 + cols_max, -87), 126);  // both scales are normal numbers
       const float scale_a = powerOfTwo(-kmax), scale_r = powerOfTwo(40 - kmax);
       double rn = 0.0, an = 0.0;
       // (a + a_lo) - (s + comp) with a two-sum so the FP32 output rounds once;
@@ -401,7 +402,7 @@ __global__ void __launch_bounds__(kResidualThreads, 1) residualMmaKernel(Residua
       // so R may be A), its low word low(c), and R's value goes to store(c, x).
       auto side = [&](const float (&v)[kCols], auto in, auto low, auto store) {
         float rs = 0.0f, rc = 0.0f, as = 0.0f, ac = 0.0f;
-        bool any = false;
+        uint32_t r_bits = 0, a_bits = 0;
 #pragma unroll
         for (int c = 0; c < kCols; ++c) {
           if (!in(c)) continue;
@@ -409,13 +410,15 @@ __global__ void __launch_bounds__(kResidualThreads, 1) residualMmaKernel(Residua
           float t, e;
           element(v[c], a_lo, h[c], l[c], t, e);
           store(c, t);
+          r_bits |= __float_as_uint(t);
+          a_bits |= __float_as_uint(v[c]) | __float_as_uint(a_lo);
           addSquare(rs, rc, t * scale_r, e * scale_r);
           addSquare(as, ac, v[c] * scale_a, a_lo * scale_a);
-          any = true;
         }
-        if (!any) return;
+        const bool r_plain = inSquareRange(rs) || r_bits << 1 == 0, a_plain = inSquareRange(as) || a_bits << 1 == 0;
         double r2, a2;
-        if (inSquareRange(rs) && inSquareRange(as)) {
+        if (r_plain && a_plain) {  // zeros are exact (1000 diagonal matrices of order 128
+                                   // 347 us, 858 with zeros in FP64)
           r2 = (static_cast<double>(rs) + static_cast<double>(rc)) * squaredPowerOfTwo(kmax - 40);
           a2 = (static_cast<double>(as) + static_cast<double>(ac)) * squaredPowerOfTwo(kmax);
         } else {
@@ -441,12 +444,12 @@ __global__ void __launch_bounds__(kResidualThreads, 1) residualMmaKernel(Residua
         auto upper = [&](int c) { return j0 + c < n && j0 + c >= i; };
 #pragma unroll
         for (int c = 0; c < kCols; ++c) v[c] = upper(c) ? A[column0 + static_cast<int64_t>(c) * n] : 0.0f;
-        side(v, upper, [&](int c) { return AL ? AL[column0 + static_cast<int64_t>(c) * n] : 0.0f; },
+        side(v, upper, [&](int c) { return kLow ? AL[column0 + static_cast<int64_t>(c) * n] : 0.0f; },
              [&](int c, float x) { if (R) R[column0 + static_cast<int64_t>(c) * n] = x; });
         // the mirror image: kCols consecutive elements of column i
         const bool vector = j0 > i && j0 + kCols <= n && n % 4 == 0 &&
                             (reinterpret_cast<uintptr_t>(A) & 15) == 0 && (reinterpret_cast<uintptr_t>(R) & 15) == 0;
-        auto low = [&](int c) { return AL ? AL[at0 + c] : 0.0f; };
+        auto low = [&](int c) { return kLow ? AL[at0 + c] : 0.0f; };
         if (vector) {
           float x[4];
 #pragma unroll
@@ -505,8 +508,9 @@ int residualMma(msq_ctx *ctx, const DeviceBatch *b, const float *a, const float 
   static std::atomic<uint64_t> done_mask{0};
   const uint64_t bit = ctx->device >= 0 && ctx->device < 64 ? uint64_t{1} << ctx->device : 0;
   if (bit == 0 || !(done_mask.load() & bit)) {
-    MSQ_TRY(cudaCheck(ctx, cudaFuncSetAttribute(residualMmaKernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                static_cast<int>(kResidualSmem)), "residual attr"));
+    for (auto kernel : {residualMmaKernel<false>, residualMmaKernel<true>})
+      MSQ_TRY(cudaCheck(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                  static_cast<int>(kResidualSmem)), "residual attr"));
     done_mask.fetch_or(bit);
   }
   SliceArgs s{};
@@ -549,7 +553,8 @@ int residualMma(msq_ctx *ctx, const DeviceBatch *b, const float *a, const float 
   args.norms = norms;
   args.status = ctx->d_status;
   args.wait_test = waitTestMode() == kWaitTestMbarrier;
-  residualMmaKernel<<<std::min(p.upper_items, kSmCount), kResidualThreads, kResidualSmem, ctx->stream>>>(args);
+  auto kernel = a_lo ? residualMmaKernel<true> : residualMmaKernel<false>;
+  kernel<<<std::min(p.upper_items, kSmCount), kResidualThreads, kResidualSmem, ctx->stream>>>(args);
   return launched(ctx, "residual float-float");
 }
 

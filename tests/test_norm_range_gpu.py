@@ -71,6 +71,23 @@ def test_norms_of_blocks_in_different_units(ctx, msq, n):
     assert abs(norms[0] - norms[1]) <= 1e-12 * norms[1] and norms[1] > 0.0
 
 
+@pytest.mark.parametrize("n", [65, 129, 260])
+def test_norms_of_sparse_matrices(ctx, msq, n):
+    """Tiles, rows and residuals of zeros beside single entries whose squares FP32
+    does not hold: X a diagonal of powers of two, A its square and one such entry."""
+    x = np.diag(2.0 ** np.random.default_rng(n).integers(-3, 4, n)).astype(np.float32)
+    z = np.zeros_like(x)
+    b = msq.Batch.from_orders([n])
+    for small in (0.0, 2.0**-100, 1.0):
+        a = x * x
+        a[n - 1, 1] = a[1, n - 1] = np.float32(small)
+        norms = _norms(ctx, msq, b, a, x, z)
+        want = 2.0 * float(np.float32(small))**2
+        assert abs(norms[0] - want) <= 1e-12 * want
+        full = np.sum(a.astype(np.float64)**2)
+        assert abs(norms[1] - full) <= 1e-12 * full
+
+
 @pytest.mark.parametrize("n", [64, 65, 130])
 def test_acceptance_does_not_depend_on_units(ctx, msq, n):
     """An MXFP4 root without a correction misses 1e-5 and falls back at every
