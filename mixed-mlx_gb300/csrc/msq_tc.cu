@@ -36,6 +36,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <type_traits>
 #include <vector>
 
 namespace msq {
@@ -472,9 +473,12 @@ __device__ __forceinline__ uint32_t tileWord(int row, int word) {
   return swizzle128(row, word >> 2) + 4 * (word & 3);
 }
 
-constexpr int kPackThreads = 256;  // packKernel
-constexpr int kMxWarps = 8;        // packMxKernel
-constexpr int kSplitWarps = 4;     // packSplitKernel
+constexpr int kSplitWarps = 4;  // packSplitKernel
+// Warps of a CTA of the other packs.  Eight where the tiles are few, since the
+// launch then is one CTA's latency (MXFP4 of order 1000: 14.0 us, 20.5 with four),
+// else four, which spend less of a tile's time on finding it (MXFP4 of 152 of
+// order 512: 41 us, 47 with eight).
+int packWarps(int items) { return items <= 4 * kSmCount ? 8 : 4; }
 
 // The E4M3 codes of v[e] / scale: by the hardware where the four are finite
 // (the same codes), else by the conversion in integers.
@@ -493,22 +497,28 @@ __device__ __forceinline__ uint32_t fp8Word(const float (&v)[4], float scale) {
   return word;
 }
 
-// One CTA per tile.  The words of the rows that the matrix has
-// (a row's rounded up to whole 16-byte chunks) are dealt to the threads in
-// order, kBatch in flight of each: a warp reads and writes whole lines of one
-// row of a large matrix, of several of a small one, and the tile's other chunks
-// are zeroed.  Bound by memory.  (A thread per row, each lane on its own line:
-// 1240 us for the BF16 factors of 4096 matrices of orders 16 .. 512, 613 so.  A
-// warp per row, whatever its length: 35.5 us for the FP8 factors of 1000
-// matrices of order 65, 25.2 so; with 128 threads a latency-bound single order
-// 1000 takes 28.3 us, 18.0 with 256.)
-template <int kSource>
-__global__ void __launch_bounds__(kPackThreads) packKernel(PackArgs args) {
+// One CTA per tile.  A warp reads and writes a row at a time, as whole lines,
+// kBatch rows in flight; where the matrix has less than whole rows of a tile, the
+// words that it has (a row's rounded up to whole 16-byte chunks) are dealt to the
+// threads in order, several rows to a warp.  The tile's other chunks are zeroed.
+// Bound by memory.  (A thread per row, each lane on its own line: 1240 us for the
+// BF16 factors of 4096 matrices of orders 16 .. 512, 511 so.  A warp per row,
+// whatever its length: 35.5 us for the FP8 factors of 1000 matrices of order 65,
+// 26.2 so.  Every tile dealt word by word: 61 us for the BF16 factors of 152
+// matrices of order 512, 49 so.)
+// Resident CTAs per SM: loads in flight come from warps, not from one's unrolling.
+constexpr int packBlocks(int source, int warps) {
+  const int of_four = source == kPackF32Bf16 ? 10 : source == kPackF32Fp8Row ? 6 : 12;
+  return of_four * 4 / warps;
+}
+template <int kSource, int kWarps>
+__global__ void __launch_bounds__(32 * kWarps, packBlocks(kSource, kWarps))
+packKernel(PackArgs args) {
   constexpr bool kFp8 = kSource == kPackF32Fp8Row || kSource == kPackFp8Codes;
   constexpr bool kF32 = kSource == kPackF32Fp8Row || kSource == kPackF32Bf16;
   constexpr int kElems = kFp8 ? 128 : 64;  // elements per 128-byte row
   constexpr int kWord = kElems / 32;       // elements per 32-bit word
-  constexpr int kBatch = 8, kThreads = kPackThreads;
+  constexpr int kBatch = 8, kThreads = 32 * kWarps;
   for (int item = blockIdx.x; item < args.items; item += gridDim.x) {
     const int4 w = args.work[item];
     const int mi = w.x, n = args.n[mi];
@@ -524,50 +534,40 @@ __global__ void __launch_bounds__(kPackThreads) packKernel(PackArgs args) {
         if (c / 8 >= rows || c % 8 >= chunks)
           *reinterpret_cast<uint4 *>(tile + swizzle128(c / 8, c % 8)) = make_uint4(0, 0, 0, 0);
     }
-    // j / words for j < 4096 and words <= 32: the inverse is less than 1 too
-    // large, the quotient less than 2^12 / 2^20 < 1 / words
-    const int words = 4 * chunks;
-    const uint32_t inverse = ((1u << 20) + words - 1) / words;
     const float *f = args.f + off;
     const bool vec = kF32 && rowsAligned<kWord>(f, n);
-#pragma unroll 1
-    for (int j0 = threadIdx.x; j0 < rows * words; j0 += kThreads * kBatch) {
-      int row[kBatch], col[kBatch];  // row -1: no word
-#pragma unroll
-      for (int q = 0; q < kBatch; ++q) {
-        const int j = j0 + kThreads * q;
-        row[q] = static_cast<int>((j * inverse) >> 20);
-        col[q] = j - row[q] * words;
-        if (row[q] >= rows) row[q] = -1;
-      }
+    // kBatch words of a thread: the q-th is word colOf(q) of row rowOf(q), which
+    // may be none of the matrix's unless `full`
+    auto pack = [&](auto full, auto rowOf, auto colOf) {
+      constexpr bool kFull = decltype(full)::value;
       uint32_t word[kBatch] = {};
       if constexpr (kF32) {
         float v[kBatch][kWord] = {};
         float scale[kBatch];
 #pragma unroll
         for (int q = 0; q < kBatch; ++q) {
-          if (row[q] >= 0)
-            loadRow<kWord>(f + static_cast<int64_t>(i0 + row[q]) * n, k0 + kWord * col[q], n, vec,
-                           v[q]);
-          scale[q] = kSource == kPackF32Fp8Row && row[q] >= 0
-                         ? args.row_scale[args.eig_offset[mi] + i0 + row[q]]
+          const int row = rowOf(q);
+          if (kFull || row < rows)
+            loadRow<kWord>(f + static_cast<int64_t>(i0 + row) * n, k0 + kWord * colOf(q), n, vec, v[q]);
+          scale[q] = kSource == kPackF32Fp8Row && (kFull || row < rows)
+                         ? args.row_scale[args.eig_offset[mi] + i0 + row]
                          : 1.0f;
         }
 #pragma unroll
         for (int q = 0; q < kBatch; ++q) {
-          if (row[q] < 0) continue;
+          if (!kFull && rowOf(q) >= rows) continue;
           if constexpr (kFp8) word[q] = fp8Word(v[q], scale[q]);
           else word[q] = encodeBf16(v[q][0]) | (static_cast<uint32_t>(encodeBf16(v[q][1])) << 16);
         }
       } else {
 #pragma unroll
         for (int q = 0; q < kBatch; ++q) {
-          const int k = k0 + kWord * col[q];
-          if (row[q] < 0) continue;
+          const int k = k0 + kWord * colOf(q);
+          if (!kFull && rowOf(q) >= rows) continue;
 #pragma unroll
           for (int e = 0; e < kWord; ++e) {
             if (k + e >= n) continue;
-            const int64_t at = off + k + e + static_cast<int64_t>(i0 + row[q]) * n;
+            const int64_t at = off + k + e + static_cast<int64_t>(i0 + rowOf(q)) * n;
             if (kSource == kPackFp8Codes) {
               word[q] |= static_cast<uint32_t>(args.codes[at]) << (8 * e);
             } else if (kSource == kPackBf16Codes) {
@@ -584,7 +584,27 @@ __global__ void __launch_bounds__(kPackThreads) packKernel(PackArgs args) {
       }
 #pragma unroll
       for (int q = 0; q < kBatch; ++q)
-        if (row[q] >= 0) *reinterpret_cast<uint32_t *>(tile + tileWord(row[q], col[q])) = word[q];
+        if (kFull || rowOf(q) < rows)
+          *reinterpret_cast<uint32_t *>(tile + tileWord(rowOf(q), colOf(q))) = word[q];
+    };
+    // whole tiles of the packs that memory bounds (the others are as fast without)
+    bool whole = false;
+    if constexpr (kSource == kPackF32Bf16) whole = rows == kTileRows && chunks == 8;
+    if (whole) {
+      const int lane = threadIdx.x % 32;
+#pragma unroll 1
+      for (int r0 = threadIdx.x / 32; r0 < kTileRows; r0 += kThreads / 32 * kBatch)
+        pack(std::true_type{}, [&](int q) { return r0 + kThreads / 32 * q; }, [&](int) { return lane; });
+    } else {
+      // j / words for j < 4096 and words <= 32: the inverse is less than 1 too
+      // large, the quotient less than 2^12 / 2^20 < 1 / words
+      const int words = 4 * chunks;
+      const uint32_t inverse = ((1u << 20) + words - 1) / words;
+#pragma unroll 1
+      for (int j0 = threadIdx.x; j0 < rows * words; j0 += kThreads * kBatch) {
+        auto rowOf = [&](int q) { return static_cast<int>(((j0 + kThreads * q) * inverse) >> 20); };
+        pack(std::false_type{}, rowOf, [&](int q) { return j0 + kThreads * q - rowOf(q) * words; });
+      }
     }
   }
 }
@@ -597,9 +617,8 @@ __global__ void __launch_bounds__(kPackThreads) packKernel(PackArgs args) {
 //   kMxCodesFp4  flat MXFP4 codes and scales (order divisible by 32, so
 //                the flat 32-element blocks are row blocks)
 //   kMxCodesFp8  flat MXFP8 E4M3 codes and scales (same condition)
-// One CTA per tile, a warp every eighth row (four warps: 11.8 us for 64 factors
-// of order 16, 8.9 with eight), lane l word l of a row (8 or 4 elements: a
-// block is 4 or 8 lanes).  Blocks beyond the order get zero codes and the unit
+// One CTA per tile, a warp every kWarps-th row, lane l word l of a row (8 or 4
+// elements: a block is 4 or 8 lanes).  Blocks beyond the order get zero codes and the unit
 // scale (byte 127).  Bound by memory: the FP32 factor of order 8192 in 70 us
 // (256 with a thread per row).
 enum MxSource : int { kMxF32Fp4 = 0, kMxCodesFp4 = 1, kMxCodesFp8 = 2 };
@@ -617,8 +636,8 @@ struct MxPackArgs {
   uint8_t *scale_tiles;
 };
 
-template <int kSource>
-__global__ void __launch_bounds__(32 * kMxWarps) packMxKernel(MxPackArgs args) {
+template <int kSource, int kWarps>
+__global__ void __launch_bounds__(32 * kWarps) packMxKernel(MxPackArgs args) {
   constexpr bool kFp4 = kSource != kMxCodesFp8;
   constexpr int kElems = kFp4 ? 256 : 128;  // K per 128-byte tile row
   constexpr int kWord = kElems / 32;
@@ -638,29 +657,30 @@ __global__ void __launch_bounds__(32 * kMxWarps) packMxKernel(MxPackArgs args) {
     const bool vec = kSource == kMxF32Fp4 && rowsAligned<kWord>(f, n);
     // the steps of kStep rows that have one of the matrix; the others hold zeros
     // and unit scales
-    constexpr int kStep = kMxWarps * kBatch;
+    constexpr int kStep = kWarps * kBatch;
     const int rows = min((n - w.y * kTileRows + kStep - 1) / kStep * kStep, kTileRows);
-    for (int c = 8 * rows + threadIdx.x; c < kTileBytes / 16; c += 32 * kMxWarps)
+    for (int c = 8 * rows + threadIdx.x; c < kTileBytes / 16; c += 32 * kWarps)
       *reinterpret_cast<uint4 *>(tile + 16 * c) = make_uint4(0, 0, 0, 0);
-    for (int r = rows + threadIdx.x; r < kTileRows; r += 32 * kMxWarps)
+    for (int r = rows + threadIdx.x; r < kTileRows; r += 32 * kWarps)
 #pragma unroll
       for (int h = 0; h < 2; ++h)
         *reinterpret_cast<uint32_t *>(sft + h * kScaleAtomBytes + 16 * (r % 32) + 4 * (r / 32)) =
             0x7f7f7f7fu;
-#pragma unroll 1
-    for (int r0 = warp; r0 < rows; r0 += kStep) {
+    // the rows r0, r0 + kWarps, .., which may not be the matrix's unless `full`
+    auto pack = [&](auto full, int r0) {
+      constexpr bool kFull = decltype(full)::value;
       const int i0 = w.y * kTileRows + r0;
       uint32_t word[kBatch] = {}, sf[kBatch];
       if constexpr (kSource == kMxF32Fp4) {
         float v[kBatch][kWord] = {};
 #pragma unroll
         for (int q = 0; q < kBatch; ++q)
-          if (i0 + kMxWarps * q < n)
-            loadRow<kWord>(f + static_cast<int64_t>(i0 + kMxWarps * q) * n, k, n, vec, v[q]);
+          if (kFull || i0 + kWarps * q < n)
+            loadRow<kWord>(f + static_cast<int64_t>(i0 + kWarps * q) * n, k, n, vec, v[q]);
 #pragma unroll
         for (int q = 0; q < kBatch; ++q) {
           sf[q] = 127;
-          if (i0 + kMxWarps * q >= n) continue;  // a row beyond the order (the whole warp's)
+          if (!kFull && i0 + kWarps * q >= n) continue;  // a row beyond the order (the whole warp's)
           float m = 0.0f;
 #pragma unroll
           for (int e = 0; e < kWord; ++e) {
@@ -690,8 +710,8 @@ __global__ void __launch_bounds__(32 * kMxWarps) packMxKernel(MxPackArgs args) {
 #pragma unroll
         for (int q = 0; q < kBatch; ++q) {
           sf[q] = 127;
-          if (i0 + kMxWarps * q < n && block_ok) {
-            const int64_t at = off + k + static_cast<int64_t>(i0 + kMxWarps * q) * n;
+          if ((kFull || i0 + kWarps * q < n) && block_ok) {
+            const int64_t at = off + k + static_cast<int64_t>(i0 + kWarps * q) * n;
             word[q] = *reinterpret_cast<const uint32_t *>(args.codes + (kFp4 ? at / 2 : at));
             sf[q] = args.mx_scales[at / 32];
           }
@@ -699,17 +719,24 @@ __global__ void __launch_bounds__(32 * kMxWarps) packMxKernel(MxPackArgs args) {
       }
 #pragma unroll
       for (int q = 0; q < kBatch; ++q) {
-        *reinterpret_cast<uint32_t *>(tile + tileWord(r0 + kMxWarps * q, lane)) = word[q];
+        *reinterpret_cast<uint32_t *>(tile + tileWord(r0 + kWarps * q, lane)) = word[q];
         // the four scale bytes of an atom's row: 4 bytes at 16 (r mod 32) + 4 (r / 32)
         uint32_t bytes = sf[q] << (8 * (lane / kGroup % 4));
         bytes |= __shfl_xor_sync(0xffffffffu, bytes, kGroup);
         bytes |= __shfl_xor_sync(0xffffffffu, bytes, 2 * kGroup);
         if (lane % (4 * kGroup) == 0) {
-          const int r = r0 + kMxWarps * q;
+          const int r = r0 + kWarps * q;
           *reinterpret_cast<uint32_t *>(sft + lane / (4 * kGroup) * kScaleAtomBytes +
                                         16 * (r % 32) + 4 * (r / 32)) = bytes;
         }
       }
+    };
+    if (n - w.y * kTileRows >= kTileRows) {
+#pragma unroll 1
+      for (int r0 = warp; r0 < kTileRows; r0 += kStep) pack(std::true_type{}, r0);
+    } else {
+#pragma unroll 1
+      for (int r0 = warp; r0 < rows; r0 += kStep) pack(std::false_type{}, r0);
     }
   }
 }
@@ -1017,8 +1044,9 @@ int launchPackMx(msq_ctx *ctx, const DeviceBatch *b, TcPlan *p, const float *f,
   args.n = b->n;
   args.tiles = tiles;
   args.scale_tiles = scale_tiles;
-  packMxKernel<kSource>
-      <<<std::min(p->pack_items, kSmCount * 8), 32 * kMxWarps, 0, ctx->stream>>>(args);
+  const int warps = packWarps(p->pack_items);
+  auto kernel = warps == 8 ? packMxKernel<kSource, 8> : packMxKernel<kSource, 4>;
+  kernel<<<std::min(p->pack_items, kSmCount * 16), 32 * warps, 0, ctx->stream>>>(args);
   return launched(ctx, "pack block-scaled operand");
 }
 
@@ -1046,7 +1074,11 @@ int launchPack(msq_ctx *ctx, const DeviceBatch *b, TcPlan *p, const float *f,
   args.tile_base = p->tile_base;
   args.n = b->n;
   args.tiles = tiles;
-  packKernel<kSource><<<std::min(p->pack_items, kSmCount * 8), kPackThreads, 0, ctx->stream>>>(args);
+  // FP8's conversions bound it, not the tile's start: eight at any size (4096
+  // matrices of orders 16 .. 512 685 us, 765 with four)
+  const int warps = kSource == kPackF32Fp8Row ? 8 : packWarps(p->pack_items);
+  auto kernel = warps == 8 ? packKernel<kSource, 8> : packKernel<kSource, 4>;
+  kernel<<<std::min(p->pack_items, kSmCount * 16), 32 * warps, 0, ctx->stream>>>(args);
   return launched(ctx, "pack operand");
 }
 

@@ -92,6 +92,41 @@ def test_mirrored_tiles_are_the_computed_ones(ctx, msq, plan):
         assert np.array_equal(xg, one.unpack(alone.cpu().numpy())[0]), f.shape
 
 
+@pytest.mark.parametrize("source", ["bf16", "fp8", "mxfp4", "bf16 codes", "fp8 codes", "mxfp4 flat codes",
+                                    "mxfp4 codes", "mxfp8 codes"])
+def test_packs_of_many_tiles(ctx, msq, source):
+    """More operand tiles than four per SM (CTAs of four warps) against the
+    matrices one at a time (of eight), bit for bit."""
+    import torch
+    aligned = source in ("mxfp4 codes", "mxfp8 codes")
+    orders = ([256, 128, 32, 608] if aligned else [257, 130, 33, 600]) * 30
+    b = msq.Batch.from_orders(orders)
+    rng = np.random.default_rng(len(source))
+    flat = _dev((rng.standard_normal(b.total) * 2.0 ** rng.integers(-12, 1, b.total)).astype(np.float32))
+    fmt = {"bf16 codes": 1, "fp8 codes": 8, "mxfp8 codes": 4}.get(source, 7)
+    if fmt == 8:  # row scales: matrix by matrix
+        values, scales = torch.zeros(b.total, dtype=torch.uint8, device="cuda"), []
+        for n, o in zip(b.n.tolist(), b.offset.tolist()):
+            v, sc = ctx.copy_to_storage(fmt, flat[o:o + n * n].clone(), n)
+            values[o:o + n * n] = v.view(torch.uint8).reshape(-1)
+            scales.append(sc.view(torch.float32).reshape(-1))
+        scales = torch.cat(scales)
+    elif "codes" in source:
+        values, scales = ctx.copy_to_storage(fmt, flat)
+
+    def run(batch, first):
+        out = torch.zeros_like(flat)
+        if "codes" not in source:
+            return ctx.reconstruct_factor({"bf16": 1, "fp8": 2, "mxfp4": 3}[source], flat, batch, out)
+        return ctx.reconstruct(fmt, values, scales[first:] if fmt == 8 else scales, batch, out)
+
+    x = b.unpack(run(b, 0).cpu().numpy())
+    for i in [*range(4), *range(len(orders) - 4, len(orders))]:
+        one = msq.Batch(b.n[i:i + 1].copy(), b.offset[i:i + 1].copy(), b.total)
+        alone = one.unpack(run(one, int(b.eig_offset[i])).cpu().numpy())[0]
+        assert np.abs(alone).max() > 0.0 and np.array_equal(x[i], alone), orders[i]
+
+
 @pytest.mark.parametrize("n", [5, 33, 130])
 def test_fp8_factor_with_an_infinity_and_a_nan(ctx, msq, n):
     """Words of four codes with an entry that the hardware conversion would not
