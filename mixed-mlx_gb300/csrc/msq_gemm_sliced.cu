@@ -338,7 +338,8 @@ __global__ void __launch_bounds__(kSlicedThreads, 1) slicedGemmKernel(SlicedArgs
       float h[kCols];
       bool ok = true;
       for (int kt = 0; kt < w.w; ++kt) {
-        ok = barWait(smemAddr(&acc_full[acc]), acc_phase, args.status, abort_flag);
+        // a warp gives up as one: its TMEM loads and shuffles need every lane
+        ok = __all_sync(0xffffffffu, barWait(smemAddr(&acc_full[acc]), acc_phase, args.status, abort_flag));
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;");
 #pragma unroll

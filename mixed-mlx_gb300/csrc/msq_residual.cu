@@ -331,7 +331,8 @@ __global__ void __launch_bounds__(kResidualThreads, 1) residualMmaKernel(Residua
       bool ok = true;
       const int chunks = (w.w + kChunkTiles - 1) / kChunkTiles;
       for (int chunk = 0; chunk < chunks; ++chunk) {
-        ok = barWait(smemAddr(acc_full), acc_phase, args.status, abort_flag);
+        // a warp gives up as one: its TMEM loads and shuffles need every lane
+        ok = __all_sync(0xffffffffu, barWait(smemAddr(acc_full), acc_phase, args.status, abort_flag));
         if (!ok) break;
         acc_phase ^= 1;
         asm volatile("tcgen05.fence::after_thread_sync;");

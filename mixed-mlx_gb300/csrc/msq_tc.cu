@@ -323,7 +323,9 @@ __global__ void __launch_bounds__(tcThreads(kEpi), 1) tcGemmKernel(TcArgs args) 
     uint32_t acc_phase = 0;
     for (int item = blockIdx.x; item < args.items; item += gridDim.x) {
       const int4 w = args.work[item];
-      if (!mbarWait(smemAddr(&acc_full[acc]), acc_phase, args.status, abort_flag)) break;
+      // a warp gives up as one: its TMEM loads and shuffles need every lane
+      if (!__all_sync(0xffffffffu, mbarWait(smemAddr(&acc_full[acc]), acc_phase, args.status, abort_flag)))
+        break;
       asm volatile("tcgen05.fence::after_thread_sync;");
       const int mi = w.x;
       const int n = args.n[mi];
