@@ -499,20 +499,22 @@ __device__ __forceinline__ uint32_t fp8Word(const float (&v)[4], float scale) {
   return word;
 }
 
-// One CTA per tile.  A warp reads and writes a row at a time, as whole lines,
-// kBatch rows in flight; where the matrix has less than whole rows of a tile, the
-// words that it has (a row's rounded up to whole 16-byte chunks) are dealt to the
-// threads in order, several rows to a warp.  The tile's other chunks are zeroed.
+// Resident CTAs of packKernel per SM: loads in flight come from warps, not from
+// one's unrolling (FP8 with 106 registers 835 us, with 78 685; sizes as below).
+constexpr int packBlocks(int source, int warps) {
+  const int of_four = source == kPackF32Bf16 ? 10 : source == kPackF32Fp8Row ? 6 : 12;
+  return of_four * 4 / warps;
+}
+
+// One CTA per tile.  The words that the matrix has of it (a row's rounded up to
+// whole 16-byte chunks) are dealt to the threads in order, so that a warp reads
+// and writes whole lines, of several rows if these are short, kBatch words of each
+// thread in flight; the other chunks are zeroed.  Whole BF16 tiles, a warp a row.
 // Bound by memory.  (A thread per row, each lane on its own line: 1240 us for the
 // BF16 factors of 4096 matrices of orders 16 .. 512, 511 so.  A warp per row,
 // whatever its length: 35.5 us for the FP8 factors of 1000 matrices of order 65,
 // 26.2 so.  Every tile dealt word by word: 61 us for the BF16 factors of 152
 // matrices of order 512, 49 so.)
-// Resident CTAs per SM: loads in flight come from warps, not from one's unrolling.
-constexpr int packBlocks(int source, int warps) {
-  const int of_four = source == kPackF32Bf16 ? 10 : source == kPackF32Fp8Row ? 6 : 12;
-  return of_four * 4 / warps;
-}
 template <int kSource, int kWarps>
 __global__ void __launch_bounds__(32 * kWarps, packBlocks(kSource, kWarps))
 packKernel(PackArgs args) {
