@@ -234,6 +234,23 @@ __device__ __forceinline__ bool applyWait(uint32_t bar, uint32_t parity, int *st
   *abort_flag = 1;
   return false;
 }
+// The same for a whole warp, which gives up as one: what follows needs every lane
+// (and a lane may see the phase complete as another sees the flag).
+__device__ __forceinline__ bool applyWaitWarp(uint32_t bar, uint32_t parity, int *status,
+                                              volatile int *abort_flag) {
+  return __all_sync(0xffffffffu, applyWait(bar, parity, status, abort_flag));
+}
+// Barrier 1 of 128 threads; whether `ok` holds in all of them.
+__device__ __forceinline__ bool barrierAll(bool ok) {
+  uint32_t all;
+  asm volatile(
+      "{\n .reg .pred p, q;\n setp.ne.b32 p, %1, 0;\n bar.red.and.pred q, 1, 128, p;\n"
+      " selp.b32 %0, 1, 0, q;\n}\n"
+      : "=r"(all)
+      : "r"(static_cast<uint32_t>(ok))
+      : "memory");
+  return all != 0;
+}
 
 __global__ void __launch_bounds__(kApplyThreads, 1) tcvApplyKernel(ApplyArgs args) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -377,13 +394,13 @@ __global__ void __launch_bounds__(kApplyThreads, 1) tcvApplyKernel(ApplyArgs arg
         if (!stagePair(s, x, supers, real, Ps, Qs)) continue;
         const int buf = it % kOperandBuffers;
         if (it >= kOperandBuffers &&
-            !applyWait(smemAddr(&a_empty[buf]), ((it / kOperandBuffers) - 1) & 1, args.status,
-                       abort_flag)) {
+            !applyWaitWarp(smemAddr(&a_empty[buf]), ((it / kOperandBuffers) - 1) & 1, args.status,
+                           abort_flag)) {
           ok = false;
           break;
         }
         if (first && s > 0 &&
-            !applyWait(smemAddr(stage_done), (s - 1) & 1, args.status, abort_flag)) {
+            !applyWaitWarp(smemAddr(stage_done), (s - 1) & 1, args.status, abort_flag)) {
           ok = false;
           break;
         }
@@ -414,7 +431,7 @@ __global__ void __launch_bounds__(kApplyThreads, 1) tcvApplyKernel(ApplyArgs arg
         ++it;
       }
     }
-    if (ok && applyWait(smemAddr(stage_done), (stages - 1) & 1, args.status, abort_flag)) {
+    if (ok && applyWaitWarp(smemAddr(stage_done), (stages - 1) & 1, args.status, abort_flag)) {
       asm volatile("tcgen05.fence::after_thread_sync;");
 #pragma unroll 1
       for (int cb = half; cb < real; cb += 2) {
@@ -870,10 +887,11 @@ __global__ void __launch_bounds__(kPassThreads, 1) tlPassKernel(PassArgs args) {
         const int y = x - 1, b = y & 1, u = y >> 1;
         int Ps, Qs;
         rrPair(y, args.stage, supers, Ps, Qs);
-        if (!applyWait(smemAddr(&d_full[b]), u & 1, args.status, abort_flag)) {
-          ok = false;
-          break;
-        }
+        ok = applyWaitWarp(smemAddr(&d_full[b]), u & 1, args.status, abort_flag);
+        // pass 1: the four warps meet below, so they give up as one; the drain
+        // before has been read from `stage`
+        if constexpr (!kSecond) ok = barrierAll(ok);
+        if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;");
         float d[64];
         tmemLoad32(tmem + ((32u * warp) << 16) + 64 * b, d);
@@ -907,7 +925,6 @@ __global__ void __launch_bounds__(kPassThreads, 1) tlPassKernel(PassArgs args) {
               if (g >= 0) Dst[g + static_cast<int64_t>(R) * n] = stage[rr * kStageLd + 32 * h + lane];
             }
           }
-          asm volatile("bar.sync 1, 128;" ::: "memory");
         }
       }
     }
